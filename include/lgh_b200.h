@@ -716,6 +716,11 @@ int lgh_test_spmm_strip (lgh_Mat A, int w, const double *X, double *Y,
                          int fp32, int R, int *R_used);
 int lgh_test_zsolve (lgh_prior_t *prior, int w, const double *X, double *Y,
                      int fp32);
+/* Y = V(X): one block V-cycle of the prior's multigrid preconditioner on
+ * n x w row-major host blocks (fp32 != 0: the float V-cycle); *nlev gets
+ * the level count and smax (cap entries) each level's lambda_max estimate */
+int lgh_test_vcycle (lgh_prior_t *prior, int w, const double *X, double *Y,
+                     int fp32, double *smax, int cap, int *nlev);
 /* one Chebyshev-Jacobi smoothing step of a square CSR Mat (n x w row-major
  * host blocks) with the smoother's kernel: X in place, Rout = Ro - A d_new,
  * Dout = d_new (flags & 4), d_new = a Do + b D^{-1} Ro (flags & 1: a Do

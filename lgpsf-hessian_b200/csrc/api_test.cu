@@ -77,7 +77,43 @@ test_cheb (lgh_Mat A, int w, double a, double b, int flags, double *X, const dou
   return 0;
 }
 
+template <typename T>
+static int
+test_vcycle (lgh_prior_t *p, int w, const double *X, double *Y)
+{
+  const int64_t n = p->n;
+  const int ld = round_ld (w);
+  std::vector<T> h ((size_t) n * ld, T (0));
+  for (int64_t i = 0; i < n; i++)
+    for (int j = 0; j < w; j++) h[i * ld + j] = (T) X[i * w + j];
+  DBuf<T> dx, dy;
+  LGH_TRY (up (dx, h.data (), h.size ()));
+  LGH_TRY (dy.alloc (h.size ()));
+  LGH_TRY (mg_vcycle<T> (p->mg, dx.p, dy.p, ld, w, stream ()));
+  LGH_CUDA (cudaStreamSynchronize (stream ()));
+  LGH_TRY (down (h.data (), dy, h.size ()));
+  for (int64_t i = 0; i < n; i++)
+    for (int j = 0; j < w; j++) Y[i * w + j] = (double) h[i * ld + j];
+  return 0;
+}
+
 extern "C" {
+
+int
+lgh_test_vcycle (lgh_prior_t *prior, int w, const double *X, double *Y,
+                 int fp32, double *smax, int cap, int *nlev)
+{
+  LGH_TRY (ensure_init ());
+  LGH_CHECK (prior && X && Y && smax && nlev && w > 0, LGH_ERR_ARG_NULL,
+             "lgh_test_vcycle: NULL");
+  LGH_CHECK (prior->mg && !prior->rows, LGH_ERR_SUP,
+             "lgh_test_vcycle: the prior has no multigrid hierarchy");
+  *nlev = (int) prior->mg->lev.size ();
+  LGH_CHECK (*nlev <= cap, LGH_ERR_ARG_SIZ, "lgh_test_vcycle: levels");
+  for (int l = 0; l < *nlev; l++) smax[l] = prior->mg->lev[l].smax;
+  return fp32 ? test_vcycle<float> (prior, w, X, Y)
+              : test_vcycle<double> (prior, w, X, Y);
+}
 
 /* out (n x k, row-major) = Omega columns j0 .. j0+k-1 */
 int

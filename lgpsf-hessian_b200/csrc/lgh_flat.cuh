@@ -1,0 +1,125 @@
+/* lgh_flat.cuh -- the flat row mapping of the gather kernels.
+ *
+ * A row of nvec 16-byte packs is covered by L = ceil (nvec / CH) threads of
+ * CH packs each (thread l: packs l, l + L, ...), and a CTA of 256 threads
+ * holds 256 / L rows, whatever L is: rows straddle warps, so no lanes are
+ * lost to rounding L up to a power of two (18 packs: 9 threads x 2, 28 rows
+ * per CTA, against 16 threads x 2 with 14 of 32 packs idle).  Every thread
+ * reads its row's (column, value) entries itself: the threads of a row read
+ * the same address (one broadcast from L1), which costs the load pipe less
+ * than the three shuffles per entry of a lane-distributed row and leaves
+ * the entry loop free of lane masks.  The loop takes one entry at a time:
+ * the kernels are bound by L1 wavefronts and by how many warps are
+ * resident, so registers spent on more entries in flight cost more than
+ * they hide (first smoothing step, 512^2 x 220 columns FP64: 180 us with
+ * one entry in flight at 4 CTAs per SM, 206 with two, 275 with five).
+ * Packs per thread: 4 above 32 packs, 2 down to 3, 1 below (4 columns
+ * FP64); fewer where the grid would not reach two CTAs per SM.  At 64
+ * columns FP64, 2 packs 59 us, 4 packs 62, 1 pack 72; at 4 columns, 1 pack
+ * 8.6 us, 2 packs 10.6. */
+
+#ifndef LGH_FLAT_CUH
+#define LGH_FLAT_CUH
+
+#include <algorithm>
+
+#include "lgh_device.cuh"
+#include "lgh_internal.h"
+
+namespace lgh
+{
+
+constexpr int FLAT_THREADS = 256;
+constexpr int FLAT_MAXPACKS = FLAT_THREADS * 4;   /* packs of one launch */
+
+/* threads per row, packs per thread, rows per CTA */
+struct FlatShape
+{
+  int L, ch, rpc;
+};
+
+inline FlatShape
+flat_shape_ch (int nvec, int ch)
+{
+  FlatShape f;
+  f.ch = ch;
+  f.L = (nvec + ch - 1) / ch;
+  f.rpc = FLAT_THREADS / f.L;
+  return f;
+}
+
+inline FlatShape
+flat_shape (int nvec, int64_t n)
+{
+  int ch = nvec > 32 ? 4 : (nvec > 2 ? 2 : 1);
+  FlatShape f = flat_shape_ch (nvec, ch);
+  while (ch > 1 && (nvec + ch / 2 - 1) / (ch / 2) <= FLAT_THREADS
+         && (n + f.rpc - 1) / f.rpc < 2 * num_sms ()) {
+    ch /= 2;
+    f = flat_shape_ch (nvec, ch);
+  }
+  return f;
+}
+
+/* CTAs that cover n rows once */
+inline int
+flat_grid (const FlatShape &f, int64_t n)
+{
+  const int64_t g = (n + f.rpc - 1) / f.rpc;
+  return (int) std::max<int64_t> (1, std::min<int64_t> (g, 1 << 20));
+}
+
+/* CTAs per SM each shape is built for: 4 packs fit 64 registers, 2 packs
+ * 42, 1 pack 32 (without spills in the single-gather kernels) */
+template <int CH>
+struct FlatOcc
+{
+  static constexpr int v = CH == 4 ? 4 : (CH == 2 ? 6 : 8);
+};
+
+/* one row's product: acc += sum_k v_k X[c_k, :] over its entries k0, k0 +
+ * step, ... below k1 (entry offsets in 32 bits: operators of fewer than
+ * 2^31 entries) */
+template <typename T, int CH>
+__device__ __forceinline__ void
+flat_gather (const int32_t *__restrict__ ci, const T *__restrict__ va, int k0,
+             int k1, int step, const T *__restrict__ X, int ld, int lane,
+             int L, int nvec, T (&acc)[CH][Pack<T>::W])
+{
+  constexpr int W = Pack<T>::W;
+  for (int k = k0; k < k1; k += step) {
+    const int c = __ldg (ci + k);
+    const T v = __ldg (va + k);
+    const T *xr = X + (int64_t) c * ld;
+#pragma unroll
+    for (int h = 0; h < CH; h++) {
+      const int vi = lane + h * L;
+      if (h < CH - 1 || vi < nvec) {
+        const Pack<T> x = ldp (xr + vi * W);
+#pragma unroll
+        for (int e = 0; e < W; e++) acc[h][e] = fma (v, x.v[e], acc[h][e]);
+      }
+    }
+  }
+}
+
+template <typename T, int CH>
+__device__ __forceinline__ void
+flat_zero (T (&acc)[CH][Pack<T>::W])
+{
+#pragma unroll
+  for (int h = 0; h < CH; h++)
+#pragma unroll
+    for (int e = 0; e < Pack<T>::W; e++) acc[h][e] = T (0);
+}
+
+#define LGH_FLAT_DISPATCH(CHV, ...)                                          \
+  switch (CHV) {                                                             \
+  case 1: { constexpr int CH_ = 1; __VA_ARGS__; } break;                     \
+  case 2: { constexpr int CH_ = 2; __VA_ARGS__; } break;                     \
+  default: { constexpr int CH_ = 4; __VA_ARGS__; } break;                    \
+  }
+
+} /* namespace lgh */
+
+#endif /* LGH_FLAT_CUH */

@@ -191,21 +191,23 @@ template <typename T>
 int launch_spmm_mode (const Csr &A, const T *X, int ldx, T *Y, int ldy, int w,
                       int mode, const T *Bm, int ldb, cudaStream_t s);
 
-/* the last two steps of a two-step post-smoothing sequence in one pass:
- * with F1 = b1 Z D^{-1} (values fl(b1 vd_ij)) and R0 the residual,
- * r1 = R0 - F1 R0, d0 = (bp dinv) R0, X += d0, X += (b dinv) r1 + a d0 */
+/* the V-cycle's passes over one smoothed level (k_flat.cu), blocks of ld
+ * columns; F1 = b1 A D^{-1}:
+ *   first   R1 = R0 - F1 R0
+ *   second  R2 = R1 - a2 (R0 - R1) - s2 F1 R1
+ *   finish  Z = D^{-1} (g (R0 + R2) + b2 (R1 + R2 - F1 R2)) + Q Xc
+ * and Y = A X for the restriction (rows split over thread groups) */
 template <typename T>
-int launch_spmm_cheb_post (const Csr &F1, const T *R0, T *X, int ld, int w,
-                           const T *dinv, double a, double b, double bp,
-                           cudaStream_t s);
-
-/* the coarse correction and the whole two-step post-smoothing in one
- * pass: X += P Xc (the prolongation), then the two steps of
- * launch_spmm_cheb_post from the post residual R */
+int launch_vc_first (const Csr &F1, const T *R0, T *R1, int ld, cudaStream_t s);
 template <typename T>
-int launch_post_prolong (const Csr &F1, const Csr &P, const T *R, const T *Xc,
-                         T *X, int ld, int w, const T *dinv, double a,
-                         double b, double bp, cudaStream_t s);
+int launch_vc_second (const Csr &F1, const T *R0, const T *R1, T *R2, int ld,
+                      double a2, double s2, cudaStream_t s);
+template <typename T>
+int launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
+                      const T *R1, const T *R2, const T *Xc, T *Z, int ld,
+                      double g, double b2, cudaStream_t s);
+template <typename T>
+int launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s);
 
 /* Y = (TO) X over count elements of two blocks with the same layout */
 template <typename TI, typename TO>

@@ -26,10 +26,11 @@ struct MgLevel
   Csr F1;
   double *f1v = nullptr;
   float *f1v32 = nullptr;
-  /* A P (n_l x n_{l+1}): the post residual after the coarse correction is
-   * r2 - (A P) xc, from the pre-smoothing residual r2, without the fine
-   * product A (x + P xc) (owned; empty on the coarsest level) */
-  Csr AP;
+  /* Q = (I - S A) P (n_l x n_{l+1}), S the two-step smoother from zero: the
+   * coarse correction followed by post-smoothing, as one operator on the
+   * coarse solution (k_flat.cu; owned, empty on the coarsest level and at
+   * other smoother degrees) */
+  Csr Q;
 };
 
 struct MgWork

@@ -13,12 +13,15 @@
  * interval [0.1, smoother_top] * lambda_max(D^{-1} A_l) from CG-Lanczos
  * (zsolve_impl.h:284-313, 340-341) and nu = 2 Chebyshev-Jacobi terms.
  *
- * Solve (device): the block V-cycle in correction form, every operation on
- * row-major blocks: Chebyshev-Jacobi pre-smoothing (the fused k_cheb kernel
- * keeps the residual current), restriction R_c = P^T R (CSR of P^T),
- * recursion, prolongation X += P X_c and the residual refresh R = B - A X
- * (the accumulate and residual forms of the row-group CSR product),
- * post-smoothing; coarse level X = A_0^{-1} B as a dense product.
+ * Solve (device): the block V-cycle, every operation on row-major blocks.
+ * At the default degree 2 a level takes the four passes of k_flat.cu
+ * (first step, second step, restriction, and the correction with the whole
+ * post-smoothing); other degrees run in correction form: Chebyshev-Jacobi
+ * pre-smoothing (k_cheb keeps the residual current), restriction R_c =
+ * P^T R (CSR of P^T), recursion, prolongation X += P X_c and the residual
+ * refresh R = B - A X (the accumulate and residual forms of the row-group
+ * CSR product), post-smoothing.  Coarse level X = A_0^{-1} B as a dense
+ * product.
  */
 
 #include <math.h>
@@ -673,7 +676,7 @@ Hierarchy::~Hierarchy ()
     csr_free (l.R);
     dfree (l.f1v);
     dfree (l.f1v32);
-    csr_free (l.AP);
+    csr_free (l.Q);
   }
 }
 
@@ -697,7 +700,7 @@ first_step_operator (MgLevel &lv)
   const Csr &A = lv.A;
   if (!A.vd || !A.vd32 || A.nnz == 0) return 0;
   const double theta = 0.5 * (lv.shi + lv.slo);
-  const double b1 = 1.0 / theta;      /* mg_smooth's first coefficient */
+  const double b1 = 1.0 / theta;      /* the first step's coefficient */
   int rc = dalloc ((void **) &lv.f1v, (size_t) A.nnz * sizeof (double) + 16);
   if (!rc) rc = dalloc ((void **) &lv.f1v32, (size_t) A.nnz * sizeof (float) + 16);
   if (rc) {
@@ -725,8 +728,7 @@ mg_destroy (Hierarchy *h)
 }
 
 /* smoothed-aggregation hierarchy of Z (level 0 borrows Z's device arrays) */
-/* the Galerkin step of one level: R = P^T, A P (kept for the post
- * residual) and Ac = P^T (A P), symmetrised against rounding: every entry
+/* the Galerkin step of one level: R = P^T, A P and Ac = P^T (A P), symmetrised against rounding: every entry
  * (i, j) averaged with its mirror (j, i), found in row j's sorted columns
  * (the pattern of P^T A P is symmetric); the averages go to a copy so that
  * each pair reads the unsymmetrised values */
@@ -749,6 +751,93 @@ galerkin (const HCsr &A, const HCsr &P, HCsr &R, HCsr &AP, HCsr &Ac)
     }
   Ac.v.swap (vs);
   Ac.m = Ac.n;
+}
+
+/* the two-step Chebyshev-Jacobi coefficients on [slo, shi]: the first
+ * step d = b1 D^{-1} r, the second d = a2 d + b2 D^{-1} r */
+static void
+cheb2_coeffs (const MgLevel &lv, double *b1, double *a2, double *b2)
+{
+  const double theta = 0.5 * (lv.shi + lv.slo);
+  const double delta = 0.5 * (lv.shi - lv.slo);
+  const double sigma1 = theta / delta;
+  const double rho_old = 1.0 / sigma1;
+  const double rho = 1.0 / (2.0 * sigma1 - rho_old);
+  *b1 = 1.0 / theta;
+  *a2 = rho * rho_old;
+  *b2 = 2.0 * rho / delta;
+}
+
+/* U + c V row by row, columns ascending in both (a merge) */
+static HCsr
+hcsr_add (const HCsr &U, double c, const HCsr &V)
+{
+  HCsr C;
+  C.n = U.n;
+  C.m = U.m;
+  C.rp.assign (C.n + 1, 0);
+#pragma omp parallel for schedule(static)
+  for (int64_t i = 0; i < C.n; i++) {
+    int64_t a = U.rp[i], b = V.rp[i], cnt = 0;
+    const int64_t ae = U.rp[i + 1], be = V.rp[i + 1];
+    while (a < ae || b < be) {
+      const int32_t ca = a < ae ? U.ci[a] : INT32_MAX;
+      const int32_t cb = b < be ? V.ci[b] : INT32_MAX;
+      if (ca <= cb) a++;
+      if (cb <= ca) b++;
+      cnt++;
+    }
+    C.rp[i + 1] = cnt;
+  }
+  for (int64_t i = 0; i < C.n; i++) C.rp[i + 1] += C.rp[i];
+  C.ci.resize (C.rp[C.n]);
+  C.v.resize (C.rp[C.n]);
+#pragma omp parallel for schedule(static)
+  for (int64_t i = 0; i < C.n; i++) {
+    int64_t a = U.rp[i], b = V.rp[i], o = C.rp[i];
+    const int64_t ae = U.rp[i + 1], be = V.rp[i + 1];
+    while (a < ae || b < be) {
+      const int32_t ca = a < ae ? U.ci[a] : INT32_MAX;
+      const int32_t cb = b < be ? V.ci[b] : INT32_MAX;
+      double v = 0.;
+      if (ca <= cb) v += U.v[a++];
+      if (cb <= ca) v += c * V.v[b++];
+      C.ci[o] = ca < cb ? ca : cb;
+      C.v[o++] = v;
+    }
+  }
+  return C;
+}
+
+/* Q = (I - S A) P = P + D^{-1} A (b1 b2 D^{-1} (A P) - (g + b2) P), with
+ * g = b1 (1 + a2): S A x = D^{-1} ((g + b2) A x - b2 b1 A D^{-1} A x).  Its
+ * rows hold 7 entries in 2D (A P: 5, P: 2.5), 17 to 30 in 3D (9 to 14 and
+ * 4 to 5): gathers from the coarse block, which caches, instead of two
+ * more passes over the fine one. */
+static HCsr
+smoothed_correction (const HCsr &A, const HCsr &P, const HCsr &AP,
+                     const MgLevel &lv)
+{
+  double b1, a2, b2;
+  cheb2_coeffs (lv, &b1, &a2, &b2);
+  const double g = b1 * (1. + a2);
+  std::vector<double> di (A.n);
+#pragma omp parallel for schedule(static)
+  for (int64_t i = 0; i < A.n; i++) {
+    const double d = hcsr_diag (A, i);
+    di[i] = d != 0. ? 1. / d : 0.;
+  }
+  auto scale_rows = [&] (HCsr &M, double c) {
+#pragma omp parallel for schedule(static)
+    for (int64_t i = 0; i < M.n; i++)
+      for (int64_t k = M.rp[i]; k < M.rp[i + 1]; k++) M.v[k] *= c * di[i];
+  };
+  HCsr U = AP;
+  scale_rows (U, b1 * b2);
+  U = hcsr_add (U, -(g + b2), P);
+  HCsr W = hcsr_gemm (A, U);
+  scale_rows (W, 1.);
+  return hcsr_add (W, 1., P);
 }
 
 /* The first coarsening of a square host CSR on the host alone (no device
@@ -917,7 +1006,11 @@ mg_build (const Csr &Z, int tile, double smoother_top, int nu, Hierarchy **out)
     lap (3);
     rc = csr_upload (P, lv.P);
     if (!rc) rc = csr_upload (R, lv.R);
-    if (!rc && lv.f1v) rc = csr_upload (AP, lv.AP);
+    if (!rc && lv.f1v && A.rp[A.n] < INT32_MAX) {
+      /* the fused passes index an operator's entries in 32 bits */
+      const HCsr Q = smoothed_correction (A, P, AP, lv);
+      if (Q.rp[Q.n] < INT32_MAX) rc = csr_upload (Q, lv.Q);
+    }
     if (rc) { delete h; return rc; }
     h->lev.push_back (lv);
     A = std::move (Ac);
@@ -934,6 +1027,13 @@ mg_build (const Csr &Z, int tile, double smoother_top, int nu, Hierarchy **out)
 }
 
 /* ---- the block V-cycle ---------------------------------------------------- */
+
+/* the level runs the fused two-step passes (k_flat.cu) */
+static bool
+two_step (const MgLevel &lv)
+{
+  return lv.nu == 2 && lv.f1v != nullptr && lv.Q.n == lv.n;
+}
 
 template <typename T>
 static int
@@ -955,7 +1055,7 @@ mg_work (Hierarchy *h, int ld, MgWork **w0, std::vector<MgWork> *own)
     if (l + 1 < h->lev.size ()) {
       LGH_TRY (w.R0.alloc (bytes));
       LGH_TRY (w.R1.alloc (bytes));
-      if (h->lev[l].nu != 2) {
+      if (!two_step (h->lev[l])) {
         LGH_TRY (w.D0.alloc (bytes));
         LGH_TRY (w.D1.alloc (bytes));
       }
@@ -972,21 +1072,6 @@ zdinv_of (const Csr &A)
 {
   if constexpr (std::is_same<T, double>::value) return A.dinv;
   else return A.dinv32;
-}
-
-/* the two-step Chebyshev-Jacobi coefficients on [slo, shi]: the first
- * step d = b1 D^{-1} r, the second d = a2 d + b2 D^{-1} r */
-static void
-cheb2_coeffs (const MgLevel &lv, double *b1, double *a2, double *b2)
-{
-  const double theta = 0.5 * (lv.shi + lv.slo);
-  const double delta = 0.5 * (lv.shi - lv.slo);
-  const double sigma1 = theta / delta;
-  const double rho_old = 1.0 / sigma1;
-  const double rho = 1.0 / (2.0 * sigma1 - rho_old);
-  *b1 = 1.0 / theta;
-  *a2 = rho * rho_old;
-  *b2 = 2.0 * rho / delta;
 }
 
 /* Chebyshev-Jacobi smoothing in correction form on level l: R holds
@@ -1011,59 +1096,6 @@ mg_smooth (const MgLevel &lv, T *X, const T *B, T *R, T *Ra, T *D0, T *D1,
   const T *Ro = pre ? B : R;
   T *Rn = pre ? R : Ra;
   T *Do = D0, *Dn = D1;
-  if (lv.nu == 2) {
-    /* the two-step polynomial in 6 block passes instead of 9: the first
-     * step stores its residual alone, the second forms the first step's d
-     * and x from that step's input residual (the same roundings, so the
-     * same bits as two ordinary steps) */
-    const double b1 = 1.0 / theta;
-    const double rho = 1.0 / (2.0 * sigma1 - rho_old);
-    const double a2 = rho * rho_old, b2 = 2.0 * rho / delta;
-    const int f1 = CHEB_FIRST | CHEB_R_ONLY | (pre ? CHEB_ZERO_X : 0);
-    if (lv.f1v && !pre) {
-      /* post: both steps in one pass over r0 (gathered) and x; reads x
-       * and r0, writes x (r1 stays in registers) */
-      if (tr) LGH_TRY (tr->begin (K_MG_POST, sbase + 3. * sblk
-                                  + (double) lv.n * sizeof (T), s));
-      LGH_TRY (launch_spmm_cheb_post<T> (lv.F1, Ro, X, ld, ld,
-                                         zdinv_of<T> (lv.A), a2,
-                                         b2, b1, s));
-      if (tr) LGH_TRY (tr->end (s));
-      if (Rout) *Rout = nullptr;
-      return 0;
-    }
-    if (lv.f1v) {
-      /* r1 = r0 - (b1 Z D^{-1}) r0 with the products fl(b1 vd_ij) formed
-       * once at set-up: the same products and order as the Chebyshev
-       * kernel's first step, without its direction and x streams */
-      if (tr) LGH_TRY (tr->begin (K_MG_FIRST, sbase + 2. * sblk, s));
-      LGH_TRY (launch_spmm_mode<T> (lv.F1, Ro, ld, Rn, ld, ld, 2, Ro, ld, s));
-      if (tr) LGH_TRY (tr->end (s));
-    } else {
-      if (tr) LGH_TRY (tr->begin (K_MG_SMOOTH, sbase + 2. * sblk, s));
-      LGH_TRY (launch_cheb_step<T> (lv.A, X, Ro, Rn, nullptr, nullptr, ld, 0.,
-                                    b1, f1, s));
-      if (tr) LGH_TRY (tr->end (s));
-    }
-    T *R2 = (Rn == R) ? Ra : R;
-    if (pre) {
-      /* reads r1 (gathered), r0 = B (gathered); writes x, r2 */
-      if (tr) LGH_TRY (tr->begin (K_MG_SMOOTH, sbase + 4. * sblk
-                                  + (double) lv.n * sizeof (T), s));
-      LGH_TRY (launch_cheb_step<T> (lv.A, X, Rn, R2, Ro, nullptr, ld, a2, b2,
-                                    CHEB_PREV_R | CHEB_ZERO_X, s, b1));
-      if (tr) LGH_TRY (tr->end (s));
-      if (Rout) *Rout = R2;
-    } else {
-      /* reads x, r0, r1; writes x (no Z product) */
-      if (tr) LGH_TRY (tr->begin (K_MG_TAIL, 4. * sblk
-                                  + (double) lv.n * sizeof (T), s));
-      LGH_TRY (launch_cheb_tail<T> (lv.A, X, Rn, Ro, ld, a2, b2, 0, s, b1));
-      if (tr) LGH_TRY (tr->end (s));
-      if (Rout) *Rout = nullptr;
-    }
-    return 0;
-  }
   for (int k = 1; k <= lv.nu; k++) {
     double a, b;
     if (k == 1) { a = 0.; b = 1.0 / theta; }
@@ -1116,6 +1148,31 @@ vcycle_level (Hierarchy *h, MgWork *W, size_t l, const T *B, T *X, int ld,
   MgWork &wk = W[l];
   T *R = (T *) wk.R0.p, *Ra = (T *) wk.R1.p;
   T *D0 = (T *) wk.D0.p, *D1 = (T *) wk.D1.p;
+  if (two_step (lv)) {
+    double b1, a2, b2;
+    cheb2_coeffs (lv, &b1, &a2, &b2);
+    const double mb = (4. + sizeof (T)) * lv.F1.nnz + 8. * (n + 1);
+    const double cb = (double) h->lev[l + 1].n * ld * sizeof (T);
+    T *Bc = (T *) W[l + 1].B.p, *Xc = (T *) W[l + 1].X.p;
+    if (tr) LGH_TRY (tr->begin (K_MG_FIRST, mb + 2. * blk, s));
+    LGH_TRY (launch_vc_first<T> (lv.F1, B, R, ld, s));
+    if (tr) LGH_TRY (tr->end (s));
+    if (tr) LGH_TRY (tr->begin (K_MG_SECOND, mb + 3. * blk, s));
+    LGH_TRY (launch_vc_second<T> (lv.F1, B, R, Ra, ld, a2, b2 / b1, s));
+    if (tr) LGH_TRY (tr->end (s));
+    if (tr) LGH_TRY (tr->begin (K_MG_RESTRICT, blk + cb
+                                + (4. + sizeof (T)) * lv.R.nnz, s));
+    LGH_TRY (launch_flat_mult<T> (lv.R, Ra, Bc, ld, s));
+    if (tr) LGH_TRY (tr->end (s));
+    LGH_TRY (vcycle_level<T> (h, W, l + 1, Bc, Xc, ld, w, s, trace));
+    if (tr) LGH_TRY (tr->begin (K_MG_FINISH, mb + 4. * blk + cb
+                                + (4. + sizeof (T)) * lv.Q.nnz + 8. * (n + 1)
+                                + (double) n * sizeof (T), s));
+    LGH_TRY (launch_vc_finish<T> (lv.F1, lv.Q, zdinv_of<T> (lv.A), B, R, Ra, Xc,
+                                  X, ld, b1 * (1. + a2), b2, s));
+    if (tr) LGH_TRY (tr->end (s));
+    return 0;
+  }
   /* pre-smoothing from X = 0 (the first step writes X without reading
    * it and reads the residual straight from B) */
   T *Rc = nullptr;
@@ -1128,26 +1185,6 @@ vcycle_level (Hierarchy *h, MgWork *W, size_t l, const T *B, T *X, int ld,
   LGH_TRY (launch_spmm<T> (lv.R, Rc, ld, Bc, ld, ld, s));
   if (tr) LGH_TRY (tr->end (s));
   LGH_TRY (vcycle_level<T> (h, W, l + 1, Bc, Xc, ld, w, s, trace));
-  constexpr int PW = Pack<T>::W;
-  if (lv.nu == 2 && lv.f1v && lv.AP.n == n && Rc && ld <= 32 * 10 * PW) {
-    /* r = r2 - (A P) xc: the residual of x + P xc from the pre-smoothing
-     * residual r2 (the same value in exact arithmetic as B - A (x + P xc));
-     * then the prolongation and both post-smoothing steps in one pass */
-    T *Rp = (Rc == R) ? Ra : R;
-    double b1, a2, b2;
-    cheb2_coeffs (lv, &b1, &a2, &b2);
-    if (tr) LGH_TRY (tr->begin (K_MG_RESID, 2. * blk + cblk
-                                + (4. + sizeof (T)) * lv.AP.nnz, s));
-    LGH_TRY (launch_spmm_mode<T> (lv.AP, Xc, ld, Rp, ld, ld, 2, Rc, ld, s));
-    if (tr) LGH_TRY (tr->end (s));
-    if (tr) LGH_TRY (tr->begin (K_MG_POSTP, 3. * blk + cblk + (double) n * sizeof (T)
-                                + (4. + sizeof (T)) * (lv.F1.nnz + lv.P.nnz)
-                                + 16. * (n + 1), s));
-    LGH_TRY (launch_post_prolong<T> (lv.F1, lv.P, Rp, Xc, X, ld, ld,
-                                     zdinv_of<T> (lv.A), a2, b2, b1, s));
-    if (tr) LGH_TRY (tr->end (s));
-    return 0;
-  }
   if (tr) LGH_TRY (tr->begin (K_MG_PROLONG, 2. * blk + cblk + 12. * lv.P.nnz, s));
   LGH_TRY (launch_spmm_mode<T> (lv.P, Xc, ld, X, ld, ld, 1, nullptr, 0, s));
   if (tr) LGH_TRY (tr->end (s));

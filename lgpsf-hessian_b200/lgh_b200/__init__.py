@@ -331,6 +331,8 @@ SIGNATURES = {
     "lgh_test_spmm_strip": (ctypes.c_int, [P, ctypes.c_int, P, P, ctypes.c_int,
                                            ctypes.c_int, P]),
     "lgh_test_zsolve": (ctypes.c_int, [P, ctypes.c_int, P, P, ctypes.c_int]),
+    "lgh_test_vcycle": (ctypes.c_int, [P, ctypes.c_int, P, P, ctypes.c_int,
+                                       P, ctypes.c_int, P]),
     "lgh_test_cheb_step": (ctypes.c_int, [P, ctypes.c_int, ctypes.c_double,
                                           ctypes.c_double, ctypes.c_int,
                                           ctypes.c_int, P, P, P, P, P,
@@ -1057,6 +1059,19 @@ def test_zsolve(prior, X, fp32=False):
                                 Y.ctypes.data, 1 if fp32 else 0),
          "lgh_test_zsolve")
     return Y
+
+
+def test_vcycle(prior, X, fp32=False):
+    """One V-cycle of the prior's preconditioner; (V(X), each level's
+    lambda_max estimate)."""
+    X = np.ascontiguousarray(X, dtype=np.float64)
+    Y = np.empty_like(X)
+    smax, nl = np.zeros(16), ctypes.c_int(0)
+    _chk(load().lgh_test_vcycle(prior.h, X.shape[1], X.ctypes.data,
+                                Y.ctypes.data, 1 if fp32 else 0,
+                                smax.ctypes.data, 16, ctypes.addressof(nl)),
+         "lgh_test_vcycle")
+    return Y, smax[:nl.value]
 
 
 CHEB_FIRST, CHEB_ZERO_X, CHEB_STORE_D = 1, 2, 4
