@@ -232,6 +232,20 @@ k_strip_spmm (int64_t n, int64_t nstrips, const int64_t *__restrict__ sptr,
   }
 }
 
+} /* namespace */
+
+int
+launch_scan_counts (int64_t m, const int64_t *counts, int64_t *ptr,
+                    cudaStream_t s)
+{
+  k_scan_counts<<<1, 1024, 0, s>>> (m, counts, ptr);
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+namespace
+{
+
 template <int R>
 int
 merge_pass (const Csr &A, int64_t nstrips, int64_t *counts,
@@ -329,8 +343,7 @@ strip_build (const Csr &A, int force_R, StripForm &S)
   LGH_TRY (dalloc ((void **) &S.scol, (size_t) S.nent * sizeof (int32_t) + 16));
   LGH_TRY (dalloc ((void **) &S.sval, (size_t) S.nent * R * sizeof (double) + 16));
   LGH_TRY (dalloc ((void **) &S.sval32, (size_t) S.nent * R * sizeof (float) + 16));
-  k_scan_counts<<<1, 1024, 0, s>>> (S.nstrips, counts, S.sptr);
-  LGH_LAUNCH_CHECK ();
+  LGH_TRY (launch_scan_counts (S.nstrips, counts, S.sptr, s));
   LGH_TRY (merge_any (R, A, S.nstrips, nullptr, nullptr, &S, s));
   LGH_CUDA (cudaStreamSynchronize (s));
   return 0;

@@ -191,6 +191,10 @@ template <typename T>
 int launch_spmm_mode (const Csr &A, const T *X, int ldx, T *Y, int ldy, int w,
                       int mode, const T *Bm, int ldb, cudaStream_t s);
 
+/* ptr[0 .. m] = exclusive scan of counts[0 .. m - 1] */
+int launch_scan_counts (int64_t m, const int64_t *counts, int64_t *ptr,
+                        cudaStream_t s);
+
 /* the V-cycle's passes over one smoothed level (k_flat.cu), blocks of ld
  * columns; F1 = b1 A D^{-1}:
  *   first   R1 = R0 - F1 R0

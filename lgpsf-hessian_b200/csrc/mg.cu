@@ -721,6 +721,214 @@ first_step_operator (MgLevel &lv)
   return 0;
 }
 
+/* the two-step Chebyshev-Jacobi coefficients on [slo, shi]: the first
+ * step d = b1 D^{-1} r, the second d = a2 d + b2 D^{-1} r */
+static void
+cheb2_coeffs (const MgLevel &lv, double *b1, double *a2, double *b2)
+{
+  const double theta = 0.5 * (lv.shi + lv.slo);
+  const double delta = 0.5 * (lv.shi - lv.slo);
+  const double sigma1 = theta / delta;
+  const double rho_old = 1.0 / sigma1;
+  const double rho = 1.0 / (2.0 * sigma1 - rho_old);
+  *b1 = 1.0 / theta;
+  *a2 = rho * rho_old;
+  *b2 = 2.0 * rho / delta;
+}
+
+/* ---- sparse products on the device ------------------------------------------
+ * Row i of the result is a sum of scaled rows of other operators (columns
+ * ascending), formed as a merge: the lists of a row are dealt to the G
+ * lanes of a group (C lists per lane), the group takes the smallest current
+ * column, sums the values there in a fixed order and advances the lists
+ * that held it.  A counting pass, a scan, then the fill; the same bits on
+ * every run.  SumAP: A P.  SumQ: Q = P + D^{-1} (b2 F1 (A P) - (g + b2) A P),
+ * the smoothed correction (I - S A) P of the two-step smoother. */
+struct SumAP
+{
+  Csr A, P;
+  __device__ int lists (int64_t i) const
+  {
+    return (int) (A.rowptr[i + 1] - A.rowptr[i]);
+  }
+  __device__ double list (int64_t i, int t, const Csr *&src, int64_t &row) const
+  {
+    const int64_t k = A.rowptr[i] + t;
+    src = &P;
+    row = A.colidx[k];
+    return A.vals[k];
+  }
+};
+
+struct SumQ
+{
+  Csr F1, P, AP;
+  const double *dinv;
+  double b2, gb2;
+  __device__ int lists (int64_t i) const
+  {
+    return (int) (F1.rowptr[i + 1] - F1.rowptr[i]) + 2;
+  }
+  __device__ double list (int64_t i, int t, const Csr *&src, int64_t &row) const
+  {
+    const int64_t k = F1.rowptr[i] + t;
+    if (k < F1.rowptr[i + 1]) {
+      src = &AP;
+      row = F1.colidx[k];
+      return dinv[i] * b2 * F1.vals[k];
+    }
+    row = i;
+    if (k == F1.rowptr[i + 1]) {
+      src = &AP;
+      return -dinv[i] * gb2;
+    }
+    src = &P;
+    return 1.;
+  }
+};
+
+template <typename Sum, int G, int C>
+__global__ void __launch_bounds__ (256)
+k_row_sum (int64_t n, Sum op, int64_t *counts, const int64_t *ptr,
+           int32_t *col, double *val)
+{
+  const int lane = threadIdx.x & (G - 1);
+  const unsigned gmask = G == 32 ? 0xffffffffu
+                         : ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
+  const int64_t stride = (int64_t) gridDim.x * (256 / G);
+  for (int64_t i = (int64_t) blockIdx.x * (256 / G) + threadIdx.x / G; i < n;
+       i += stride) {
+    const int nl = op.lists (i);
+    const int32_t *cc[C];
+    const double *cv[C];
+    int left[C];
+    double coef[C];
+#pragma unroll
+    for (int q = 0; q < C; q++) {
+      const int t = lane + q * G;
+      left[q] = 0;
+      if (t < nl) {
+        const Csr *src;
+        int64_t row;
+        coef[q] = op.list (i, t, src, row);
+        const int64_t k = src->rowptr[row];
+        left[q] = (int) (src->rowptr[row + 1] - k);
+        cc[q] = src->colidx + k;
+        cv[q] = src->vals + k;
+      }
+    }
+    int64_t pos = col ? ptr[i] : 0;
+    for (;;) {
+      int cur = INT32_MAX;
+#pragma unroll
+      for (int q = 0; q < C; q++)
+        if (left[q] > 0 && *cc[q] < cur) cur = *cc[q];
+      const int m = (int) __reduce_min_sync (gmask, (unsigned) cur);
+      if (m == INT32_MAX) break;
+      double v = 0.;
+#pragma unroll
+      for (int q = 0; q < C; q++)
+        if (left[q] > 0 && *cc[q] == m) {
+          if (col) v += coef[q] * *cv[q];
+          cc[q]++;
+          cv[q]++;
+          left[q]--;
+        }
+      if (col) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync (gmask, v, o);
+        if (lane == 0) {
+          col[pos] = m;
+          val[pos] = v;
+        }
+      }
+      pos++;
+    }
+    if (!col && lane == 0) counts[i] = pos;
+  }
+}
+
+/* the result as a device Csr of n rows and m columns (rowptr, colidx and
+ * vals alone; csr_finish adds the rest); maxlists: the most lists of a row;
+ * *fits = 0 (and no result) if they exceed 32 per lane or the entries 2^31 */
+template <typename Sum>
+static int
+row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
+{
+  cudaStream_t s = stream ();
+  DBuf<int64_t> counts;
+  LGH_TRY (counts.alloc (n));
+  out = Csr ();
+  out.n = n;
+  out.ncols = m;
+  *fits = 1;
+  auto pass = [&] (bool fill) -> int {
+    auto run = [&] (auto g, auto c) -> int {
+      constexpr int G = decltype (g)::value, C = decltype (c)::value;
+      const int grid = (int) std::max<int64_t> (1, std::min<int64_t> (
+          (n * G + 255) / 256, (int64_t) num_sms () * 8));
+      k_row_sum<Sum, G, C><<<grid, 256, 0, s>>> (
+          n, op, counts.p, out.rowptr, fill ? out.colidx : nullptr,
+          fill ? out.vals : nullptr);
+      LGH_LAUNCH_CHECK ();
+      return 0;
+    };
+    using std::integral_constant;
+    if (maxlists <= 8)
+      return run (integral_constant<int, 8> (), integral_constant<int, 1> ());
+    if (maxlists <= 16)
+      return run (integral_constant<int, 16> (), integral_constant<int, 1> ());
+    if (maxlists <= 32)
+      return run (integral_constant<int, 32> (), integral_constant<int, 1> ());
+    if (maxlists <= 96)
+      return run (integral_constant<int, 32> (), integral_constant<int, 3> ());
+    if (maxlists <= 256)
+      return run (integral_constant<int, 32> (), integral_constant<int, 8> ());
+    if (maxlists <= 1024)
+      return run (integral_constant<int, 32> (), integral_constant<int, 32> ());
+    *fits = 0;
+    return 0;
+  };
+  int rc = pass (false);
+  if (rc || !*fits) return rc;
+  rc = dalloc ((void **) &out.rowptr, (size_t) (n + 1) * sizeof (int64_t));
+  if (!rc) rc = launch_scan_counts (n, counts.p, out.rowptr, s);
+  if (!rc && (cudaMemcpyAsync (&out.nnz, out.rowptr + n, sizeof (int64_t),
+                               cudaMemcpyDeviceToHost, s) != cudaSuccess
+              || cudaStreamSynchronize (s) != cudaSuccess))
+    rc = set_error (LGH_ERR_GPU, "mg: sparse product sizes");
+  if (!rc && out.nnz >= INT32_MAX) *fits = 0;
+  if (!rc && *fits) {
+    rc = dalloc ((void **) &out.colidx, (size_t) out.nnz * sizeof (int32_t) + 16);
+    if (!rc) rc = dalloc ((void **) &out.vals, (size_t) out.nnz * sizeof (double) + 16);
+    if (!rc) rc = pass (true);
+  }
+  if (rc || !*fits) csr_free (out);
+  return rc;
+}
+
+/* lv.Q from the level's device operators (A, F1, P).  Left empty, and the
+ * level on the correction form, where an operator's entries pass 32 bits
+ * or a row of A holds more than 1022. */
+static int
+smoothed_correction (MgLevel &lv)
+{
+  if (lv.A.nnz >= INT32_MAX || lv.P.nnz >= INT32_MAX || lv.R.nnz >= INT32_MAX)
+    return 0;
+  double b1, a2, b2;
+  cheb2_coeffs (lv, &b1, &a2, &b2);
+  const int64_t m = lv.P.ncols;
+  int fits = 0;
+  Csr AP;
+  LGH_TRY (row_sum (lv.n, m, lv.A.max_row_nnz, SumAP{ lv.A, lv.P }, AP, &fits));
+  if (!fits) return 0;
+  const SumQ q{ lv.F1, lv.P, AP, lv.A.dinv, b2, b1 * (1. + a2) + b2 };
+  int rc = row_sum (lv.n, m, lv.A.max_row_nnz + 2, q, lv.Q, &fits);
+  csr_free (AP);
+  if (!rc && fits) rc = csr_finish (lv.Q);
+  return rc;
+}
+
 void
 mg_destroy (Hierarchy *h)
 {
@@ -751,93 +959,6 @@ galerkin (const HCsr &A, const HCsr &P, HCsr &R, HCsr &AP, HCsr &Ac)
     }
   Ac.v.swap (vs);
   Ac.m = Ac.n;
-}
-
-/* the two-step Chebyshev-Jacobi coefficients on [slo, shi]: the first
- * step d = b1 D^{-1} r, the second d = a2 d + b2 D^{-1} r */
-static void
-cheb2_coeffs (const MgLevel &lv, double *b1, double *a2, double *b2)
-{
-  const double theta = 0.5 * (lv.shi + lv.slo);
-  const double delta = 0.5 * (lv.shi - lv.slo);
-  const double sigma1 = theta / delta;
-  const double rho_old = 1.0 / sigma1;
-  const double rho = 1.0 / (2.0 * sigma1 - rho_old);
-  *b1 = 1.0 / theta;
-  *a2 = rho * rho_old;
-  *b2 = 2.0 * rho / delta;
-}
-
-/* U + c V row by row, columns ascending in both (a merge) */
-static HCsr
-hcsr_add (const HCsr &U, double c, const HCsr &V)
-{
-  HCsr C;
-  C.n = U.n;
-  C.m = U.m;
-  C.rp.assign (C.n + 1, 0);
-#pragma omp parallel for schedule(static)
-  for (int64_t i = 0; i < C.n; i++) {
-    int64_t a = U.rp[i], b = V.rp[i], cnt = 0;
-    const int64_t ae = U.rp[i + 1], be = V.rp[i + 1];
-    while (a < ae || b < be) {
-      const int32_t ca = a < ae ? U.ci[a] : INT32_MAX;
-      const int32_t cb = b < be ? V.ci[b] : INT32_MAX;
-      if (ca <= cb) a++;
-      if (cb <= ca) b++;
-      cnt++;
-    }
-    C.rp[i + 1] = cnt;
-  }
-  for (int64_t i = 0; i < C.n; i++) C.rp[i + 1] += C.rp[i];
-  C.ci.resize (C.rp[C.n]);
-  C.v.resize (C.rp[C.n]);
-#pragma omp parallel for schedule(static)
-  for (int64_t i = 0; i < C.n; i++) {
-    int64_t a = U.rp[i], b = V.rp[i], o = C.rp[i];
-    const int64_t ae = U.rp[i + 1], be = V.rp[i + 1];
-    while (a < ae || b < be) {
-      const int32_t ca = a < ae ? U.ci[a] : INT32_MAX;
-      const int32_t cb = b < be ? V.ci[b] : INT32_MAX;
-      double v = 0.;
-      if (ca <= cb) v += U.v[a++];
-      if (cb <= ca) v += c * V.v[b++];
-      C.ci[o] = ca < cb ? ca : cb;
-      C.v[o++] = v;
-    }
-  }
-  return C;
-}
-
-/* Q = (I - S A) P = P + D^{-1} A (b1 b2 D^{-1} (A P) - (g + b2) P), with
- * g = b1 (1 + a2): S A x = D^{-1} ((g + b2) A x - b2 b1 A D^{-1} A x).  Its
- * rows hold 7 entries in 2D (A P: 5, P: 2.5), 17 to 30 in 3D (9 to 14 and
- * 4 to 5): gathers from the coarse block, which caches, instead of two
- * more passes over the fine one. */
-static HCsr
-smoothed_correction (const HCsr &A, const HCsr &P, const HCsr &AP,
-                     const MgLevel &lv)
-{
-  double b1, a2, b2;
-  cheb2_coeffs (lv, &b1, &a2, &b2);
-  const double g = b1 * (1. + a2);
-  std::vector<double> di (A.n);
-#pragma omp parallel for schedule(static)
-  for (int64_t i = 0; i < A.n; i++) {
-    const double d = hcsr_diag (A, i);
-    di[i] = d != 0. ? 1. / d : 0.;
-  }
-  auto scale_rows = [&] (HCsr &M, double c) {
-#pragma omp parallel for schedule(static)
-    for (int64_t i = 0; i < M.n; i++)
-      for (int64_t k = M.rp[i]; k < M.rp[i + 1]; k++) M.v[k] *= c * di[i];
-  };
-  HCsr U = AP;
-  scale_rows (U, b1 * b2);
-  U = hcsr_add (U, -(g + b2), P);
-  HCsr W = hcsr_gemm (A, U);
-  scale_rows (W, 1.);
-  return hcsr_add (W, 1., P);
 }
 
 /* The first coarsening of a square host CSR on the host alone (no device
@@ -1006,11 +1127,7 @@ mg_build (const Csr &Z, int tile, double smoother_top, int nu, Hierarchy **out)
     lap (3);
     rc = csr_upload (P, lv.P);
     if (!rc) rc = csr_upload (R, lv.R);
-    if (!rc && lv.f1v && A.rp[A.n] < INT32_MAX) {
-      /* the fused passes index an operator's entries in 32 bits */
-      const HCsr Q = smoothed_correction (A, P, AP, lv);
-      if (Q.rp[Q.n] < INT32_MAX) rc = csr_upload (Q, lv.Q);
-    }
+    if (!rc && lv.f1v) rc = smoothed_correction (lv);
     if (rc) { delete h; return rc; }
     h->lev.push_back (lv);
     A = std::move (Ac);

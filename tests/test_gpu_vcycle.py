@@ -96,3 +96,30 @@ def test_vcycle_matches_correction_form(problems, name, fp32, w):
     ref = memo["ref"][:, :w]
     err = np.linalg.norm(Y - ref) / np.linalg.norm(ref)
     assert err < (1e-4 if fp32 else 1e-10), err
+
+
+def _wide_rows(n=1700, half=330, seed=4):
+    """A banded SPD operator of up to 2 half + 1 entries a row: more lists
+    per row than the merge that forms the correction operator keeps in
+    registers."""
+    i = np.arange(n)
+    o = np.arange(-half, half + 1)
+    j = i[:, None] + o[None, :]
+    ok = (j >= 0) & (j < n)
+    w = -np.exp(-np.abs(o) / 60.0)[None, :] * np.ones((n, 1))
+    w[:, half] = 0.0
+    w = np.where(ok, w, 0.0)
+    w[:, half] = -w.sum(1) + 0.05
+    rp = np.concatenate([[0], np.cumsum(ok.sum(1))]).astype(np.int64)
+    return dict(n=n, rowptr=rp, colidx=j[ok].astype(np.int32), vals=w[ok])
+
+
+@pytest.mark.parametrize("half", [20, 120, 330])
+def test_vcycle_wide_rows(cuda_device, half):
+    Z = _wide_rows(half=half)
+    prior = L.Prior(Z=L.Mat(Z), mass=np.ones(Z["n"]))
+    X = np.random.default_rng(6).standard_normal((Z["n"], 13))
+    Y, smax = L.test_vcycle(prior, X)
+    levels, Ac = _hierarchy(Z, len(smax))
+    ref = _vcycle(levels, Ac, smax, X)
+    assert np.linalg.norm(Y - ref) / np.linalg.norm(ref) < 1e-10
