@@ -432,55 +432,89 @@ launch_shift_combine_variant (int variant, int64_t n, int kept, int m,
   return 0;
 }
 
-/* Y = A^{-1} B on the dense coarse level: A^{-1} n0 x n0 column-major,
- * B and Y n0 x ld row-major; columns w .. ld - 1 of Y are set to zero */
-template <typename T>
-__global__ void __launch_bounds__ (128)
+/* Y = A^{-1} B on the dense coarse level: A^{-1} n0 x n0 column-major (and
+ * symmetric), B and Y n0 x ld row-major; columns w .. ld - 1 of Y are set to
+ * zero.  n0 is 33 to 1500 and w as small as one, so the product is bound by
+ * latency, not by the FP64 tensor pipe: a CTA takes a small tile (8 MT rows
+ * x 8 NT columns) and its NW warps split the n0 terms, each reading its
+ * fragments straight from L2 (for a fixed k, 8 consecutive rows of A^{-1}
+ * and 8 consecutive columns of B: whole 32-byte sectors) with the loads of
+ * several k steps in flight; the warps' partial tiles are added in warp
+ * order through shared memory.  A 64 x 64 tile with one serial pass over n0
+ * left 9 to 36 CTAs on the chip: 45 us at n0 = 559 x 220 columns and 46 us
+ * at 704 x 1; now see the launch rule below. */
+template <typename T, int MT, int NT, int NW>
+__global__ void __launch_bounds__ (NW * 32)
 k_dense_apply (int n0, const double *__restrict__ Ainv, const T *__restrict__ B,
                T *__restrict__ Y, int w, int ld)
 {
-  __shared__ double As[GK][SLD], Bs[GK][SLD];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  const int i0 = blockIdx.x * GB, c0 = blockIdx.y * GB;
-  double acc[4][4][2];
+  constexpr int TM = 8 * MT, TN = 8 * NT;
+  extern __shared__ double red[];              /* [NW][TM * TN] */
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * TM, c0 = blockIdx.y * TN;
+  /* this warp's k range, in steps of 4 */
+  const int steps = (n0 + 3) / 4;
+  const int s0 = (int) ((int64_t) steps * warp / NW);
+  const int s1 = (int) ((int64_t) steps * (warp + 1) / NW);
+  const int kl = lane & 3, ml = lane >> 2;
+  double acc[MT][NT][2];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < MT; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b][0] = acc[a][b][1] = 0.;
-  /* staging: thread -> k row (tid / 8), 8 consecutive rows / columns */
-  const int lk = tid >> 3, lc = (tid & 7) * 8;
-  double ra[8], rb[8];
-  auto fetch = [&] (int k0) {
-    const int gk = k0 + lk;
+    for (int b = 0; b < NT; b++) acc[a][b][0] = acc[a][b][1] = 0.;
+#pragma unroll 4
+  for (int s = s0; s < s1; s++) {
+    const int k = 4 * s + kl;
+    double a[MT], b[NT];
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-      const int gi = i0 + lc + e, gc = c0 + lc + e;
-      ra[e] = (gk < n0 && gi < n0) ? Ainv[gi + (size_t) gk * n0] : 0.;
-      rb[e] = (gk < n0 && gc < w) ? (double) B[(size_t) gk * ld + gc] : 0.;
+    for (int t = 0; t < MT; t++) {
+      const int i = i0 + t * 8 + ml;
+      a[t] = (k < n0 && i < n0) ? __ldg (Ainv + i + (size_t) k * n0) : 0.;
     }
-  };
-  fetch (0);
-  for (int k0 = 0; k0 < n0; k0 += GK) {
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-      As[lk][lc + e] = ra[e];
-      Bs[lk][lc + e] = rb[e];
+    for (int t = 0; t < NT; t++) {
+      const int c = c0 + t * 8 + ml;
+      b[t] = (k < n0 && c < w) ? (double) B[(size_t) k * ld + c] : 0.;
     }
-    __syncthreads ();
-    if (k0 + GK < n0) fetch (k0 + GK);
-    dmma_block (As, Bs, wm, wn, lane, acc);
-    __syncthreads ();
+#pragma unroll
+    for (int ti = 0; ti < MT; ti++)
+#pragma unroll
+      for (int tj = 0; tj < NT; tj++)
+        asm volatile ("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
+                      "{%0, %1}, {%2}, {%3}, {%0, %1};"
+                      : "+d"(acc[ti][tj][0]), "+d"(acc[ti][tj][1])
+                      : "d"(a[ti]), "d"(b[tj]));
   }
 #pragma unroll
-  for (int ti = 0; ti < 4; ti++)
+  for (int ti = 0; ti < MT; ti++)
 #pragma unroll
-    for (int tj = 0; tj < 4; tj++)
+    for (int tj = 0; tj < NT; tj++)
 #pragma unroll
-      for (int c = 0; c < 2; c++) {
-        const int gi = i0 + dmma_row (wm, ti, lane), gc = c0 + dmma_col (wn, tj, c, lane);
-        if (gi < n0 && gc < ld) Y[(size_t) gi * ld + gc] = (gc < w) ? (T) acc[ti][tj][c] : T (0);
-      }
+      for (int c = 0; c < 2; c++)
+        red[warp * (TM * TN) + (ti * 8 + ml) * TN + tj * 8 + kl * 2 + c]
+            = acc[ti][tj][c];
+  __syncthreads ();
+  for (int e = threadIdx.x; e < TM * TN; e += NW * 32) {
+    double v = 0.;
+#pragma unroll
+    for (int q = 0; q < NW; q++) v += red[q * (TM * TN) + e];
+    const int gi = i0 + e / TN, gc = c0 + e % TN;
+    if (gi < n0 && gc < ld) Y[(size_t) gi * ld + gc] = gc < w ? (T) v : T (0);
+  }
+}
+
+template <typename T, int MT, int NT, int NW>
+static int
+dense_apply_tile (int n0, const double *Ainv, const T *B, T *Y, int w, int ld,
+                  cudaStream_t s)
+{
+  const int smem = NW * 64 * MT * NT * (int) sizeof (double);
+  static_assert (NW * 64 * MT * NT * 8 <= 48 * 1024, "static shared limit");
+  dim3 grid ((unsigned) ((n0 + 8 * MT - 1) / (8 * MT)),
+             (unsigned) ((ld + 8 * NT - 1) / (8 * NT)));
+  k_dense_apply<T, MT, NT, NW><<<grid, NW * 32, smem, s>>> (n0, Ainv, B, Y, w, ld);
+  LGH_LAUNCH_CHECK ();
+  return 0;
 }
 
 template <typename T>
@@ -488,10 +522,12 @@ int
 launch_dense_apply (int n0, const double *Ainv, const T *B, T *Y, int w, int ld,
                     cudaStream_t s)
 {
-  dim3 grid ((unsigned) ((n0 + GB - 1) / GB), (unsigned) ((ld + GB - 1) / GB));
-  k_dense_apply<T><<<grid, 128, 0, s>>> (n0, Ainv, B, Y, w, ld);
-  LGH_LAUNCH_CHECK ();
-  return 0;
+  /* narrow blocks: 16 rows x 8 columns over 16 warps, so that n0 = 560
+   * still makes 35 CTAs and a warp's share of the terms stays near 10
+   * steps; wide ones: 32 x 32 over 4 warps (126 CTAs at 559 x 220) */
+  if (ld <= 8) return dense_apply_tile<T, 2, 1, 16> (n0, Ainv, B, Y, w, ld, s);
+  if (ld <= 64) return dense_apply_tile<T, 2, 2, 16> (n0, Ainv, B, Y, w, ld, s);
+  return dense_apply_tile<T, 4, 4, 4> (n0, Ainv, B, Y, w, ld, s);
 }
 
 template int launch_dense_apply<double> (int, const double *, const double *,
