@@ -49,7 +49,7 @@ k_flat_resid (int64_t n, const int64_t *__restrict__ rowptr,
       k1n = (int) rowptr[i + stride + 1];
     }
     T acc[CH][W];
-    flat_zero<T, CH> (acc);
+    flat_zero<T, CH, W> (acc);
     flat_gather<T, CH> (colidx, vals, k0, k1, 1, X, ld, lane, L, nvec, acc);
 #pragma unroll
     for (int h = 0; h < CH; h++) {
@@ -90,7 +90,7 @@ k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
       k1n = (int) rowptr[i + stride + 1];
     }
     T acc[CH][W];
-    flat_zero<T, CH> (acc);
+    flat_zero<T, CH, W> (acc);
     flat_gather<T, CH> (colidx, vals, k0, k1, 1, R1, ld, lane, L, nvec, acc);
 #pragma unroll
     for (int h = 0; h < CH; h++) {
@@ -115,7 +115,7 @@ k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
 /* z = dinv (g (r0 + r2) + b2 (r1 + r2 - F1 r2)) + Q xc: reads r0, r1, r2
  * (gathered) and the coarse block (gathered), writes z */
 template <typename T, int CH>
-__global__ void __launch_bounds__ (FLAT_THREADS, CH == 2 ? 5 : FlatOcc<CH>::v)
+__global__ void __launch_bounds__ (FLAT_THREADS, CH == 2 ? 5 : (CH == 3 ? 4 : FlatOcc<CH>::v))
 k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
                const int32_t *__restrict__ fci, const T *__restrict__ fv,
                const int64_t *__restrict__ qrp,
@@ -141,7 +141,7 @@ k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
       q1n = (int) qrp[i + stride + 1];
     }
     T acc[CH][W];
-    flat_zero<T, CH> (acc);
+    flat_zero<T, CH, W> (acc);
     flat_gather<T, CH> (fci, fv, k0, k1, 1, R2, ld, lane, L, nvec, acc);
     const T di = dinv[i];
 #pragma unroll
@@ -196,7 +196,7 @@ k_flat_mult (int64_t n, const int64_t *__restrict__ rowptr,
     const int64_t i = i0 + rl;
     const bool on = rl < rows && i < n;
     T acc[CH][W];
-    flat_zero<T, CH> (acc);
+    flat_zero<T, CH, W> (acc);
     if (on) {
       flat_gather<T, CH> (colidx, vals, (int) rowptr[i] + sp, (int) rowptr[i + 1],
                           SPLIT ? S : 1, X, ld, lane, L, nvec, acc);
@@ -336,7 +336,17 @@ launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
   LGH_TRY (flat_check<T> (Q, Xc, Z, nullptr, ld));
   LGH_CHECK (dinv && Q.n == F1.n, LGH_ERR_ARG_WRONG, "V-cycle finish: operators");
   return flat_slices (F1.n, F1.bandwidth, ld, ld / W, sizeof (T), [&] (int v0, int nv) {
-    const FlatShape f = flat_shape (nv, F1.n);
+    /* three packs per thread where that wastes under 5 % of them and the
+     * rows are long (3D: 25 entries with Q's; 46 packs FP64 305 us against
+     * 375 with four and 340 with two, 110 packs 802, 1036, 824), or divides
+     * a 2D block of up to 64 packs (48: 210, 218, 230); 110 packs in 2D
+     * keep four (470, three 522) */
+    FlatShape f = flat_shape (nv, F1.n);
+    const int L3 = (nv + 2) / 3;
+    const bool lng = F1.nnz + Q.nnz > 16 * F1.n;
+    if (f.ch > 1 && nv > 16 && L3 <= FLAT_THREADS && 20 * (3 * L3 - nv) <= 3 * L3
+        && (lng || (nv % 3 == 0 && nv <= 64)))
+      f = flat_shape_ch (nv, 3);
     LGH_FLAT_DISPATCH (f.ch, {
       auto k = k_flat_finish<T, CH_>;
       k<<<fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,

@@ -1,0 +1,655 @@
+/* k_pcg.cu -- the passes of blocked PCG around an explicit preconditioner
+ * z = V(r) (the reference's per-column CG + PCGAMG, zsolve_impl.h:674-683,
+ * 808-818), every column of the block with its own scalars and mask.
+ *
+ * One iteration is four passes over the block besides the V-cycle, 12 block
+ * transfers: direction with the deferred x update (z, p, x in; p, x out: the
+ * direction is formed in place), product with (p, q) (p gathered in, q
+ * out), residual (r, q in; r out), dots (r, z in).  Column sums: a thread
+ * keeps the sums of its packs over all its rows in registers, the CTA adds
+ * its rows in shared memory, and the per-CTA partials are summed in a fixed
+ * order, one warp per column.  Up to 32 columns the last CTA to finish does
+ * that; wider blocks leave it to a small launch of one warp per column,
+ * since one CTA takes 40 us over the 592 partials of 220 columns and the
+ * launch 4 us (the whole product pass: 347 us with the last-CTA sum).
+ *
+ * The preconditioner's output may be FP32 (a mixed solve's float V-cycle):
+ * the passes that read z widen it as they load it, which gives the values a
+ * separate widening pass would have stored, and the residual pass stores
+ * r's FP32 copy beside r.  Separate passes took 98 and 49 us of an
+ * iteration's 1900 at 64^3 x 90 columns. */
+
+#include <type_traits>
+
+#include "lgh_flat.cuh"
+#include "lgh_pcg.h"
+
+namespace lgh
+{
+
+namespace
+{
+
+/* z packs: 16 bytes of T's width in elements, loaded from TZ */
+template <typename T, typename TZ>
+__device__ __forceinline__ Pack<T>
+ldz (const TZ *p)
+{
+  if constexpr (std::is_same<T, TZ>::value) {
+    return ldp (p);
+  } else {
+    static_assert (sizeof (T) == 8 && sizeof (TZ) == 4, "widening only");
+    const float2 f = *reinterpret_cast<const float2 *> (p);
+    Pack<T> r;
+    r.v[0] = (T) f.x;
+    r.v[1] = (T) f.y;
+    return r;
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void
+st32 (float *p, const Pack<T> &r)
+{
+  if constexpr (sizeof (T) == 8)
+    *reinterpret_cast<float2 *> (p) = make_float2 ((float) r.v[0], (float) r.v[1]);
+  else
+    stp (p, r);
+}
+
+/* a thread's pack sums -> this CTA's column sums -> part[c * grid + block].
+ * red: rpc * ld doubles and, behind them, 256 more. */
+template <typename T, int CH>
+__device__ __forceinline__ void
+flat_colsum (const double (&acc)[CH][Pack<T>::W], int rl, int lane, int L,
+             int rpc, int nvec, int ld, double *red, double *part)
+{
+  constexpr int W = Pack<T>::W;
+  __syncthreads ();
+  if (rl < rpc) {
+#pragma unroll
+    for (int h = 0; h < CH; h++) {
+      const int vi = lane + h * L;
+      if (h < CH - 1 || vi < nvec)
+#pragma unroll
+        for (int e = 0; e < W; e++) red[rl * ld + vi * W + e] = acc[h][e];
+    }
+  }
+  __syncthreads ();
+  /* narrow blocks hold many rows per CTA: nseg threads share a column */
+  int nseg = 1;
+  while (nseg < 16 && 2 * nseg * ld <= FLAT_THREADS) nseg *= 2;
+  if (nseg == 1) {
+    for (int c = threadIdx.x; c < ld; c += FLAT_THREADS) {
+      double s = 0.;
+      for (int r = 0; r < rpc; r++) s += red[r * ld + c];
+      part[(size_t) c * gridDim.x + blockIdx.x] = s;
+    }
+    return;
+  }
+  double *red2 = red + rpc * ld;
+  const int seg = threadIdx.x / ld, c = threadIdx.x - seg * ld;
+  if (seg < nseg) {
+    double s = 0.;
+    for (int r = seg; r < rpc; r += nseg) s += red[r * ld + c];
+    red2[seg * ld + c] = s;
+  }
+  __syncthreads ();
+  if (threadIdx.x < ld) {
+    double s = 0.;
+    for (int q = 0; q < nseg; q++) s += red2[q * ld + threadIdx.x];
+    part[(size_t) threadIdx.x * gridDim.x + blockIdx.x] = s;
+  }
+}
+
+/* the sum of one column's nb partials by one warp, in a fixed order */
+__device__ __forceinline__ double
+part_sum (const double *part, int nb, int lane)
+{
+  double s[4] = { 0., 0., 0., 0. };
+  for (int b = lane; b < nb; b += 128) {
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (b + 32 * q < nb) s[q] += __ldcg (part + b + 32 * q);
+  }
+  return warp_sum ((s[0] + s[1]) + (s[2] + s[3]));
+}
+
+struct PcgCols
+{
+  double *scal;
+  int *ival;
+  int cap, w;
+  double rtol;
+  int first, iter;
+  double *hist;
+  const int *fresh;
+
+  /* alpha from (p, q) */
+  __device__ void prod (int c, double pq) const
+  {
+    double *al = scal + S_ALPHA * cap;
+    int *act = ival + I_ACTIVE * cap;
+    if (act[c]) {
+      if (pq != 0. && isfinite (pq)) al[c] = scal[S_RZ * cap + c] / pq;
+      else { al[c] = 0.; act[c] = 0; }
+    } else {
+      al[c] = 0.;
+    }
+  }
+
+  /* the start of a column, or beta and the convergence test */
+  __device__ void dots (int c, double srz, double szz) const
+  {
+    double *rz = scal + S_RZ * cap, *be = scal + S_BETA * cap;
+    double *al = scal + S_ALPHA * cap, *n0 = scal + S_NORM0 * cap;
+    int *act = ival + I_ACTIVE * cap, *its = ival + I_ITS * cap;
+    if (first || (fresh != nullptr && fresh[c])) {
+      rz[c] = srz;
+      n0[c] = sqrt (szz);
+      act[c] = (c < w && szz > 0.) ? 1 : 0;
+      al[c] = 0.;
+      be[c] = 0.;
+      its[c] = 0;
+      return;
+    }
+    if (!act[c]) { be[c] = 0.; return; }
+    const double b = (rz[c] != 0.) ? srz / rz[c] : 0.;
+    if (hist != nullptr && c == 0 && iter < 10000) {
+      hist[2 * iter] = al[0];
+      hist[2 * iter + 1] = b;
+    }
+    rz[c] = srz;
+    be[c] = b;
+    /* a converged column keeps its alpha: its x update may still be
+     * pending (launch_pcg_dir or launch_pcg_out applies it), and the next
+     * product zeroes alpha for inactive columns */
+    if (sqrt (szz) <= rtol * n0[c] || srz == 0.) {
+      act[c] = 0;
+      be[c] = 0.;
+      its[c] = iter + 1;
+    }
+  }
+
+  /* the active columns, counted by the whole CTA */
+  __device__ void count (int ld) const
+  {
+    int cnt = 0;
+    for (int c = threadIdx.x; c - (int) threadIdx.x < ld; c += blockDim.x)
+      cnt += __syncthreads_count (
+          c < ld && ((volatile int *) ival)[I_ACTIVE * cap + c] != 0);
+    if (threadIdx.x == 0) ival[I_NSLOT * cap] = cnt;
+  }
+};
+
+/* columns up to which the last CTA sums the partials */
+constexpr int PCG_TAIL_COLS = 32;
+
+template <bool DOTS>
+__device__ __forceinline__ void
+pcg_columns (const double *partA, const double *partB, int nb, int c0, int cstep,
+             int ld, const PcgCols &pc)
+{
+  const int lane = threadIdx.x & 31;
+  for (int c = c0; c < ld; c += cstep) {
+    const double a = part_sum (partA + (size_t) c * nb, nb, lane);
+    const double b = DOTS ? part_sum (partB + (size_t) c * nb, nb, lane) : 0.;
+    if (lane == 0) {
+      if (DOTS) pc.dots (c, a, b);
+      else pc.prod (c, a);
+    }
+  }
+}
+
+template <bool DOTS>
+__device__ __forceinline__ void
+pcg_tail (const double *partA, const double *partB, int ld, unsigned *counter,
+          const PcgCols &pc)
+{
+  if (!last_block_ticket (counter)) return;
+  pcg_columns<DOTS> (partA, partB, gridDim.x, threadIdx.x >> 5,
+                     FLAT_THREADS / 32, ld, pc);
+  __syncthreads ();
+  if (DOTS) pc.count (ld);
+  if (threadIdx.x == 0) *counter = 0u;
+}
+
+/* the partials of a wide block: one warp per column over all CTAs; the
+ * last CTA counts the active columns */
+template <bool DOTS>
+__global__ void __launch_bounds__ (FLAT_THREADS)
+k_pcg_columns (const double *partA, const double *partB, int nb, int ld,
+               unsigned *counter, PcgCols pc)
+{
+  pcg_columns<DOTS> (partA, partB, nb,
+                     (int) (blockIdx.x * (FLAT_THREADS / 32) + (threadIdx.x >> 5)),
+                     (int) (gridDim.x * (FLAT_THREADS / 32)), ld, pc);
+  if (!DOTS) return;
+  if (!last_block_ticket (counter)) return;
+  pc.count (ld);
+  if (threadIdx.x == 0) *counter = 0u;
+}
+
+/* ---- the passes ----------------------------------------------------------- */
+
+template <typename T>
+__global__ void __launch_bounds__ (256)
+k_pcg_start (int64_t n, int w, int ld, const T *__restrict__ B, int ldb,
+             const double *__restrict__ rs, T *__restrict__ R,
+             float *__restrict__ R32, int vec)
+{
+  constexpr int W = Pack<T>::W;
+  const int nvec = ld / W;
+  const int64_t total = n * nvec;
+  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (int64_t) gridDim.x * blockDim.x) {
+    const int64_t i = e / nvec;
+    const int c = (int) (e - i * nvec) * W;
+    const double sc = rs ? rs[i] : 1.0;
+    Pack<T> r;
+    if (vec && c + W <= w) {
+      r = ldp (B + i * ldb + c);
+    } else {
+      /* a single vector (ldb = 1), an unaligned view or the pad columns */
+#pragma unroll
+      for (int k = 0; k < W; k++) r.v[k] = c + k < w ? B[i * ldb + c + k] : T (0);
+    }
+#pragma unroll
+    for (int k = 0; k < W; k++) r.v[k] = (T) (sc * (double) r.v[k]);
+    stp (R + i * ld + c, r);
+    if (R32) st32<T> (R32 + i * ld + c, r);
+  }
+}
+
+template <typename T, typename TZ, int CH, bool TAIL>
+__global__ void __launch_bounds__ (FLAT_THREADS, CH == 4 ? 3 : (CH == 2 ? 5 : 6))
+k_pcg_dots (int64_t n, int ld, int nvec, int L, int rpc, const T *__restrict__ R,
+            const TZ *__restrict__ Zb, double *partA, double *partB,
+            unsigned *counter, PcgCols pc)
+{
+  constexpr int W = Pack<T>::W;
+  extern __shared__ double red[];
+  const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
+  double arz[CH][W], azz[CH][W];
+  flat_zero<double, CH, W> (arz);
+  flat_zero<double, CH, W> (azz);
+  if (rl < rpc)
+    for (int64_t i = (int64_t) blockIdx.x * rpc + rl; i < n;
+         i += (int64_t) gridDim.x * rpc) {
+#pragma unroll
+      for (int h = 0; h < CH; h++) {
+        const int vi = lane + h * L;
+        if (h < CH - 1 || vi < nvec) {
+          const Pack<T> r = ldp (R + i * ld + vi * W);
+          const Pack<T> z = ldz<T, TZ> (Zb + i * ld + vi * W);
+#pragma unroll
+          for (int e = 0; e < W; e++) {
+            arz[h][e] += (double) r.v[e] * (double) z.v[e];
+            azz[h][e] += (double) z.v[e] * (double) z.v[e];
+          }
+        }
+      }
+    }
+  flat_colsum<T, CH> (arz, rl, lane, L, rpc, nvec, ld, red, partA);
+  flat_colsum<T, CH> (azz, rl, lane, L, rpc, nvec, ld, red, partB);
+  if (TAIL) pcg_tail<true> (partA, partB, ld, counter, pc);
+}
+
+template <typename T, typename TZ, int FLAGS>
+__global__ void __launch_bounds__ (256)
+k_pcg_dir (int64_t n, int ld, const TZ *__restrict__ Zb, T *__restrict__ P,
+           T *__restrict__ X, const double *__restrict__ beta,
+           const double *__restrict__ alpha)
+{
+  constexpr int W = Pack<T>::W;
+  const int nvec = ld / W;
+  const int64_t total = n * nvec;
+  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (int64_t) gridDim.x * blockDim.x) {
+    const int64_t i = e / nvec;
+    const int vi = (int) (e - i * nvec);
+    const int64_t o = i * ld + vi * W;
+    Pack<T> z = ldz<T, TZ> (Zb + o);
+    if constexpr (!(FLAGS & PCG_P_FIRST)) {
+      const Pack<T> p = ldp (P + o);
+      if constexpr (FLAGS & (PCG_X_FIRST | PCG_X_ADD)) {
+        Pack<T> x = (FLAGS & PCG_X_ADD) ? ldp (X + o) : pzero<T> ();
+#pragma unroll
+        for (int k = 0; k < W; k++)
+          x.v[k] = fma ((T) alpha[vi * W + k], p.v[k], x.v[k]);
+        stp (X + o, x);
+      }
+#pragma unroll
+      for (int k = 0; k < W; k++)
+        z.v[k] = fma ((T) beta[vi * W + k], p.v[k], z.v[k]);
+    }
+    stp (P + o, z);
+  }
+}
+
+/* 4 packs: 16 gather and 16 sum registers in 80 (3 CTAs per SM; 512^2 x 220
+ * columns 250 us, 304 at 4 CTAs with spills, 299 with 2 packs).  I: entry
+ * offsets in 32 bits, or 64 for an operator of 2^31 entries or more. */
+template <typename T, typename I, int CH, bool TAIL>
+__global__ void __launch_bounds__ (FLAT_THREADS, CH == 4 ? 3 : (CH == 2 ? 4 : 6))
+k_pcg_prod (int64_t n, const int64_t *__restrict__ rowptr,
+            const int32_t *__restrict__ colidx, const T *__restrict__ vals,
+            const T *__restrict__ P, T *__restrict__ Q, int ld, int nvec, int L,
+            int rpc, double *partA, unsigned *counter, PcgCols pc)
+{
+  constexpr int W = Pack<T>::W;
+  extern __shared__ double red[];
+  const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
+  const int64_t stride = (int64_t) gridDim.x * rpc;
+  double apq[CH][W];
+  flat_zero<double, CH, W> (apq);
+  int64_t i = (int64_t) blockIdx.x * rpc + rl;
+  if (rl < rpc && i < n) {
+    I k0 = (I) rowptr[i], k1 = (I) rowptr[i + 1];
+    for (; i < n; i += stride) {
+      I k0n = 0, k1n = 0;
+      if (i + stride < n) {
+        k0n = (I) rowptr[i + stride];
+        k1n = (I) rowptr[i + stride + 1];
+      }
+      T acc[CH][W];
+      flat_zero<T, CH, W> (acc);
+      flat_gather<T, CH> (colidx, vals, k0, k1, 1, P, ld, lane, L, nvec, acc);
+#pragma unroll
+      for (int h = 0; h < CH; h++) {
+        const int vi = lane + h * L;
+        if (h < CH - 1 || vi < nvec) {
+          const int64_t o = i * ld + vi * W;
+          const Pack<T> p = ldp (P + o);
+          Pack<T> q;
+#pragma unroll
+          for (int e = 0; e < W; e++) {
+            q.v[e] = acc[h][e];
+            apq[h][e] += (double) p.v[e] * (double) q.v[e];
+          }
+          stp (Q + o, q);
+        }
+      }
+      k0 = k0n;
+      k1 = k1n;
+    }
+  }
+  flat_colsum<T, CH> (apq, rl, lane, L, rpc, nvec, ld, red, partA);
+  if (TAIL) pcg_tail<false> (partA, nullptr, ld, counter, pc);
+}
+
+template <typename T, bool WITHX>
+__global__ void __launch_bounds__ (256)
+k_pcg_resid (int64_t n, int ld, T *__restrict__ R, const T *__restrict__ Qv,
+             float *__restrict__ R32, T *__restrict__ X,
+             const T *__restrict__ P, const double *__restrict__ alpha)
+{
+  constexpr int W = Pack<T>::W;
+  const int nvec = ld / W;
+  const int64_t total = n * nvec;
+  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (int64_t) gridDim.x * blockDim.x) {
+    const int64_t i = e / nvec;
+    const int vi = (int) (e - i * nvec);
+    const int64_t o = i * ld + vi * W;
+    Pack<T> r = ldp (R + o);
+    const Pack<T> q = ldp (Qv + o);
+    T a[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) a[k] = (T) alpha[vi * W + k];
+    if constexpr (WITHX) {
+      Pack<T> x = ldp (X + o);
+      const Pack<T> p = ldp (P + o);
+#pragma unroll
+      for (int k = 0; k < W; k++) x.v[k] = fma (a[k], p.v[k], x.v[k]);
+      stp (X + o, x);
+    }
+#pragma unroll
+    for (int k = 0; k < W; k++) r.v[k] = fma (-a[k], q.v[k], r.v[k]);
+    stp (R + o, r);
+    if (R32) st32<T> (R32 + o, r);
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__ (256)
+k_pcg_out (int64_t n, int w, int ld, const T *__restrict__ X,
+           const T *__restrict__ P, int have_x, const double *__restrict__ rs,
+           T *__restrict__ Y, int ldy, const double *__restrict__ alpha, int vec)
+{
+  constexpr int W = Pack<T>::W;
+  const int nvec = (w + W - 1) / W;
+  const int64_t total = n * nvec;
+  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (int64_t) gridDim.x * blockDim.x) {
+    const int64_t i = e / nvec;
+    const int c = (int) (e - i * nvec) * W;
+    const double sc = rs ? rs[i] : 1.0;
+    Pack<T> x = have_x ? ldp (X + i * ld + c) : pzero<T> ();
+    const Pack<T> p = ldp (P + i * ld + c);
+#pragma unroll
+    for (int k = 0; k < W; k++)
+      x.v[k] = (T) (sc * (double) fma ((T) alpha[c + k], p.v[k], x.v[k]));
+    if (vec && c + W <= w) {
+      stp (Y + i * ldy + c, x);
+    } else {
+#pragma unroll
+      for (int k = 0; k < W; k++)
+        if (c + k < w) Y[i * ldy + c + k] = x.v[k];
+    }
+  }
+}
+
+/* CTAs of a streaming pass of `total` packs */
+int
+stream_grid (int64_t total)
+{
+  return (int) std::max<int64_t> (1, std::min<int64_t> (
+      (int64_t) num_sms () * 8, (total + 255) / 256));
+}
+
+/* two packs per thread at most: the sums, not the loads, set the registers */
+FlatShape
+sum_shape (int nvec, int64_t n)
+{
+  FlatShape f = flat_shape (nvec, n);
+  if (f.ch == 4 && (nvec + 1) / 2 <= FLAT_THREADS) f = flat_shape_ch (nvec, 2);
+  return f;
+}
+
+int
+sum_smem (const FlatShape &f, int ld)
+{
+  return (f.rpc * ld + FLAT_THREADS) * (int) sizeof (double);
+}
+
+int
+pcg_width (int ld, int W)
+{
+  return ld > 0 && ld % W == 0 && ld / W <= FLAT_MAXPACKS
+             ? 0
+             : set_error (LGH_ERR_SUP, "PCG pass: block width %d unsupported", ld);
+}
+
+} /* namespace */
+
+template <typename T>
+int
+launch_pcg_start (int64_t n, int w, int ld, const T *B, int ldb,
+                  const double *rs, T *R, float *R32, cudaStream_t s)
+{
+  constexpr int W = Pack<T>::W;
+  const int vec = ldb % W == 0 && (uintptr_t) B % 16 == 0;
+  k_pcg_start<T><<<stream_grid (n * (ld / W)), 256, 0, s>>> (n, w, ld, B, ldb,
+                                                            rs, R, R32, vec);
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+template <typename T, typename TZ>
+int
+launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
+                 double rtol, int iter, double *hist, const int *fresh,
+                 ZWork &ws, cudaStream_t s)
+{
+  constexpr int W = Pack<T>::W;
+  LGH_TRY (pcg_width (ld, W));
+  const int nvec = ld / W;
+  const FlatShape f = sum_shape (nvec, n);
+  const int smem = sum_smem (f, ld);
+  const int want = std::min (flat_grid (f, n), ws.nblocks);
+  const PcgCols pc{ ws.scal.p, ws.ival.p, ws.cap, w, rtol, first, iter, hist,
+                    fresh };
+  int nb = 0;
+  LGH_FLAT_DISPATCH (f.ch, {
+    if (ld <= PCG_TAIL_COLS) {
+      auto k = k_pcg_dots<T, TZ, CH_, true>;
+      k<<<fit_grid (k, want, FLAT_THREADS, smem), FLAT_THREADS, smem, s>>> (
+          n, ld, nvec, f.L, f.rpc, R, Zb, ws.partA.p, ws.partB.p,
+          ws.counters.p + 1, pc);
+    } else {
+      auto k = k_pcg_dots<T, TZ, CH_, false>;
+      nb = fit_grid (k, want, FLAT_THREADS, smem);
+      k<<<nb, FLAT_THREADS, smem, s>>> (n, ld, nvec, f.L, f.rpc, R, Zb,
+                                        ws.partA.p, ws.partB.p,
+                                        ws.counters.p + 1, pc);
+    }
+  });
+  LGH_LAUNCH_CHECK ();
+  if (nb > 0) {
+    k_pcg_columns<true><<<(ld + 7) / 8, FLAT_THREADS, 0, s>>> (
+        ws.partA.p, ws.partB.p, nb, ld, ws.counters.p + 1, pc);
+    LGH_LAUNCH_CHECK ();
+  }
+  return 0;
+}
+
+template <typename T, typename TZ>
+int
+launch_pcg_dir (int64_t n, int ld, const TZ *Zb, T *P, T *X, int flags,
+                ZWork &ws, cudaStream_t s)
+{
+  constexpr int W = Pack<T>::W;
+  const int grid = stream_grid (n * (ld / W));
+  const double *be = ws.scal.p + S_BETA * ws.cap, *al = ws.scal.p + S_ALPHA * ws.cap;
+  switch (flags) {
+  case 0:
+    k_pcg_dir<T, TZ, 0><<<grid, 256, 0, s>>> (n, ld, Zb, P, X, be, al);
+    break;
+  case PCG_P_FIRST:
+    k_pcg_dir<T, TZ, PCG_P_FIRST><<<grid, 256, 0, s>>> (n, ld, Zb, P, X, be, al);
+    break;
+  case PCG_X_FIRST:
+    k_pcg_dir<T, TZ, PCG_X_FIRST><<<grid, 256, 0, s>>> (n, ld, Zb, P, X, be, al);
+    break;
+  case PCG_X_ADD:
+    k_pcg_dir<T, TZ, PCG_X_ADD><<<grid, 256, 0, s>>> (n, ld, Zb, P, X, be, al);
+    break;
+  default:
+    return set_error (LGH_ERR_ARG_WRONG, "PCG direction: flags %d", flags);
+  }
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+template <typename T>
+int
+launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
+                 cudaStream_t s)
+{
+  constexpr int W = Pack<T>::W;
+  LGH_TRY (pcg_width (ld, W));
+  const T *vals;
+  if constexpr (std::is_same<T, double>::value) vals = Z.vals;
+  else vals = Z.vals32;
+  const int nvec = ld / W;
+  const FlatShape f = flat_shape (nvec, Z.n);
+  const int smem = sum_smem (f, ld);
+  const int want = std::min (flat_grid (f, Z.n), ws.nblocks);
+  const PcgCols pc{ ws.scal.p, ws.ival.p, ws.cap, 0, 0., 0, 0, nullptr, nullptr };
+  int nb = 0;
+  auto run = [&] (auto idx, auto ch, auto tail) -> int {
+    auto k = k_pcg_prod<T, decltype (idx), decltype (ch)::value,
+                        decltype (tail)::value>;
+    const int g = fit_grid (k, want, FLAT_THREADS, smem);
+    if (!decltype (tail)::value) nb = g;
+    k<<<g, FLAT_THREADS, smem, s>>> (Z.n, Z.rowptr, Z.colidx, vals, P, Q, ld,
+                                     nvec, f.L, f.rpc, ws.partA.p,
+                                     ws.counters.p, pc);
+    LGH_LAUNCH_CHECK ();
+    return 0;
+  };
+  const bool tail = ld <= PCG_TAIL_COLS, big = Z.nnz >= INT32_MAX;
+  LGH_FLAT_DISPATCH (f.ch, {
+    using C = std::integral_constant<int, CH_>;
+    if (big) {
+      if (tail) LGH_TRY (run (int64_t (), C (), std::true_type ()));
+      else LGH_TRY (run (int64_t (), C (), std::false_type ()));
+    } else {
+      if (tail) LGH_TRY (run (int (), C (), std::true_type ()));
+      else LGH_TRY (run (int (), C (), std::false_type ()));
+    }
+  });
+  if (nb > 0) {
+    k_pcg_columns<false><<<(ld + 7) / 8, FLAT_THREADS, 0, s>>> (
+        ws.partA.p, nullptr, nb, ld, ws.counters.p, pc);
+    LGH_LAUNCH_CHECK ();
+  }
+  return 0;
+}
+
+template <typename T>
+int
+launch_pcg_resid (int64_t n, int ld, T *R, const T *Q, float *R32, T *X,
+                  const T *P, ZWork &ws, cudaStream_t s)
+{
+  const int grid = stream_grid (n * (ld / Pack<T>::W));
+  const double *al = ws.scal.p + S_ALPHA * ws.cap;
+  if (X)
+    k_pcg_resid<T, true><<<grid, 256, 0, s>>> (n, ld, R, Q, R32, X, P, al);
+  else
+    k_pcg_resid<T, false><<<grid, 256, 0, s>>> (n, ld, R, Q, R32, X, P, al);
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+template <typename T>
+int
+launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P, int have_x,
+                const double *rs, T *Y, int ldy, ZWork &ws, cudaStream_t s)
+{
+  constexpr int W = Pack<T>::W;
+  const int vec = ldy % W == 0 && (uintptr_t) Y % 16 == 0;
+  k_pcg_out<T><<<stream_grid (n * ((w + W - 1) / W)), 256, 0, s>>> (
+      n, w, ld, X, P, have_x, rs, Y, ldy, ws.scal.p + S_ALPHA * ws.cap, vec);
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+#define LGH_PCG_INST(T)                                                      \
+  template int launch_pcg_start<T> (int64_t, int, int, const T *, int,       \
+                                    const double *, T *, float *,            \
+                                    cudaStream_t);                           \
+  template int launch_pcg_prod<T> (const Csr &, const T *, T *, int,         \
+                                   ZWork &, cudaStream_t);                   \
+  template int launch_pcg_resid<T> (int64_t, int, T *, const T *, float *,   \
+                                    T *, const T *, ZWork &, cudaStream_t);  \
+  template int launch_pcg_out<T> (int64_t, int, int, const T *, const T *,   \
+                                  int, const double *, T *, int, ZWork &,    \
+                                  cudaStream_t);
+#define LGH_PCG_INST_Z(T, TZ)                                                \
+  template int launch_pcg_dots<T, TZ> (int64_t, int, int, const T *,         \
+                                       const TZ *, int, double, int,         \
+                                       double *, const int *, ZWork &,       \
+                                       cudaStream_t);                        \
+  template int launch_pcg_dir<T, TZ> (int64_t, int, const TZ *, T *, T *,    \
+                                      int, ZWork &, cudaStream_t);
+LGH_PCG_INST (double)
+LGH_PCG_INST (float)
+LGH_PCG_INST_Z (double, double)
+LGH_PCG_INST_Z (double, float)
+LGH_PCG_INST_Z (float, float)
+#undef LGH_PCG_INST
+#undef LGH_PCG_INST_Z
+
+} /* namespace lgh */

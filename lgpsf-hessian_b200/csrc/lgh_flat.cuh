@@ -74,20 +74,20 @@ flat_grid (const FlatShape &f, int64_t n)
 template <int CH>
 struct FlatOcc
 {
-  static constexpr int v = CH == 4 ? 4 : (CH == 2 ? 6 : 8);
+  static constexpr int v = CH == 4 ? 4 : (CH == 3 ? 5 : (CH == 2 ? 6 : 8));
 };
 
 /* one row's product: acc += sum_k v_k X[c_k, :] over its entries k0, k0 +
- * step, ... below k1 (entry offsets in 32 bits: operators of fewer than
- * 2^31 entries) */
-template <typename T, int CH>
+ * step, ... below k1; I: int for operators of fewer than 2^31 entries (the
+ * wider offsets cost the registers that spill) */
+template <typename T, int CH, typename I>
 __device__ __forceinline__ void
-flat_gather (const int32_t *__restrict__ ci, const T *__restrict__ va, int k0,
-             int k1, int step, const T *__restrict__ X, int ld, int lane,
+flat_gather (const int32_t *__restrict__ ci, const T *__restrict__ va, I k0,
+             I k1, int step, const T *__restrict__ X, int ld, int lane,
              int L, int nvec, T (&acc)[CH][Pack<T>::W])
 {
   constexpr int W = Pack<T>::W;
-  for (int k = k0; k < k1; k += step) {
+  for (I k = k0; k < k1; k += step) {
     const int c = __ldg (ci + k);
     const T v = __ldg (va + k);
     const T *xr = X + (int64_t) c * ld;
@@ -103,20 +103,21 @@ flat_gather (const int32_t *__restrict__ ci, const T *__restrict__ va, int k0,
   }
 }
 
-template <typename T, int CH>
+template <typename T, int CH, int W>
 __device__ __forceinline__ void
-flat_zero (T (&acc)[CH][Pack<T>::W])
+flat_zero (T (&acc)[CH][W])
 {
 #pragma unroll
   for (int h = 0; h < CH; h++)
 #pragma unroll
-    for (int e = 0; e < Pack<T>::W; e++) acc[h][e] = T (0);
+    for (int e = 0; e < W; e++) acc[h][e] = T (0);
 }
 
 #define LGH_FLAT_DISPATCH(CHV, ...)                                          \
   switch (CHV) {                                                             \
   case 1: { constexpr int CH_ = 1; __VA_ARGS__; } break;                     \
   case 2: { constexpr int CH_ = 2; __VA_ARGS__; } break;                     \
+  case 3: { constexpr int CH_ = 3; __VA_ARGS__; } break;                     \
   default: { constexpr int CH_ = 4; __VA_ARGS__; } break;                    \
   }
 

@@ -213,10 +213,6 @@ int launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
 template <typename T>
 int launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s);
 
-/* Y = (TO) X over count elements of two blocks with the same layout */
-template <typename TI, typename TO>
-int cvt_flat (int64_t count, const TI *X, TO *Y, cudaStream_t s);
-
 /* elementwise / block helpers (k_vec.cu) */
 template <typename T>
 int launch_rowscale (int64_t n, int w, const double *scale, const T *X,

@@ -44,35 +44,27 @@
 #include "lgh_internal.h"
 #include "lgh_mg.h"
 #include "lgh_objects.h"
+#include "lgh_pcg.h"
 
 namespace lgh
 {
-
-/* kernels of zsolve.cu used by the tick (declared there) */
-template <typename T>
-int server_tick_pq (const Csr &Z, const T *Zb, const T *Pold, T *Pnew, T *Q,
-                    int ld, ZWork &ws, cudaStream_t s);
-template <typename T>
-int server_tick_upd (int64_t n, int ld, T *X, T *R, const T *Pn, const T *Q,
-                     ZWork &ws, cudaStream_t s);
-template <typename T>
-int server_tick_dots (const Csr &Z, const T *R, const T *Zb, int ld, int w,
-                      const int *fresh, double rtol, ZWork &ws, cudaStream_t s);
 
 int ensure_wz (lgh_glr_t *g);
 int launch_logdet (int kept, const double *lam, int nshift, const double *c,
                    double *out, cudaStream_t s);
 
-/* a contiguous device column into column `col` of a row-major block, with
- * an optional row scale; the same column of X and of the next direction
- * block are cleared (a fresh CG start) */
+/* a contiguous device column into column `col` of a row-major block (and
+ * its FP32 copy R32, nullable), with an optional row scale; the same column
+ * of X and of the direction block are cleared (a fresh CG start) */
 __global__ void
 k_col_place (int64_t n, const double *src, const double *scale, double *R,
-             double *X, double *P, int ld, int col)
+             float *R32, double *X, double *P, int ld, int col)
 {
   for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t) gridDim.x * blockDim.x) {
-    R[i * ld + col] = scale ? scale[i] * src[i] : src[i];
+    const double r = scale ? scale[i] * src[i] : src[i];
+    R[i * ld + col] = r;
+    if (R32) R32[i * ld + col] = (float) r;
     X[i * ld + col] = 0.;
     P[i * ld + col] = 0.;
   }
@@ -95,9 +87,10 @@ k_gather_slots (int64_t n, const double *__restrict__ X, int ld,
   }
 }
 
-/* second Z-solve of a solve request, in place: R = mass * X, X = 0, P = 0 */
+/* second Z-solve of a solve request, in place: R = mass * X (and its FP32
+ * copy), X = 0, P = 0 */
 __global__ void
-k_restage (int64_t n, double *X, double *R, double *P, int ld,
+k_restage (int64_t n, double *X, double *R, float *R32, double *P, int ld,
            const int *__restrict__ slot, int k, const double *__restrict__ mass)
 {
   const int64_t total = n * k;
@@ -105,7 +98,9 @@ k_restage (int64_t n, double *X, double *R, double *P, int ld,
        e += (int64_t) gridDim.x * blockDim.x) {
     const int64_t i = e / k;
     const int64_t o = i * ld + slot[(int) (e - i * k)];
-    R[o] = mass[i] * X[o];
+    const double r = mass[i] * X[o];
+    R[o] = r;
+    if (R32) R32[o] = (float) r;
     X[o] = 0.;
     P[o] = 0.;
   }
@@ -533,7 +528,7 @@ srv_logdet (lgh_server_t *sv, SReq *r)
  * its first run also forms, for a sample, w = U^T xi for all of its
  * columns (the copier allocated the request's staging) */
 static int
-srv_start (lgh_server_t *sv, const Adm &a, double *Pold)
+srv_start (lgh_server_t *sv, const Adm &a)
 {
   lgh_glr_t *g = sv->g;
   SReq *r = a.r;
@@ -541,6 +536,8 @@ srv_start (lgh_server_t *sv, const Adm &a, double *Pold)
   const int kept = g->kept, ldh = sv->ld;
   cudaStream_t s = sv->s;
   double *X = (double *) sv->ws.X.p, *R = (double *) sv->ws.R.p;
+  double *P = (double *) sv->ws.P0.p;
+  float *R32 = sv->pc32 ? (float *) sv->ws.R32.p : nullptr;
   if (a.j0 == 0) {
     r->cols_left = r->m;
     r->t_placed = wall ();
@@ -566,7 +563,7 @@ srv_start (lgh_server_t *sv, const Adm &a, double *Pold)
     /* first right-hand side: r (solve) or M^{1/2} xi (sample) */
     k_col_place<<<cgrid (n), 256, 0, s>>> (n, r->din.p + (size_t) j * n,
                                            r->kind == 1 ? g->prior->msqrt.p : nullptr,
-                                           R, X, Pold, sv->ld, sl);
+                                           R, R32, X, P, sv->ld, sl);
     LGH_LAUNCH_CHECK ();
     sv->fresh_h[sl] = 1;
     j++;
@@ -580,13 +577,15 @@ srv_start (lgh_server_t *sv, const Adm &a, double *Pold)
  * combination and the output column.  A request whose last column left
  * goes to the copier behind an event on the loop's stream. */
 static int
-srv_harvest (lgh_server_t *sv, const std::vector<int> &act, double *Pold)
+srv_harvest (lgh_server_t *sv, const std::vector<int> &act)
 {
   lgh_glr_t *g = sv->g;
   const int64_t n = g->n;
   const int kept = g->kept, ld = sv->ld, ldh = sv->ld;
   cudaStream_t s = sv->s;
   double *X = (double *) sv->ws.X.p, *R = (double *) sv->ws.R.p;
+  double *P = (double *) sv->ws.P0.p;
+  float *R32 = sv->pc32 ? (float *) sv->ws.R32.p : nullptr;
   Harvest &h = *sv->hv;
   int ka = 0, kb = 0;
   std::vector<SReq *> fin;
@@ -632,7 +631,7 @@ srv_harvest (lgh_server_t *sv, const std::vector<int> &act, double *Pold)
                                                               hd->wdst_a);
       LGH_LAUNCH_CHECK ();
     }
-    k_restage<<<cgrid (n * ka), 256, 0, s>>> (n, X, R, Pold, ld, hd->slot_a, ka,
+    k_restage<<<cgrid (n * ka), 256, 0, s>>> (n, X, R, R32, P, ld, hd->slot_a, ka,
                                               g->prior->mass.p);
     LGH_LAUNCH_CHECK ();
   }
@@ -676,14 +675,14 @@ srv_loop (lgh_server_t *sv)
   const int ld = sv->ld;
   cudaStream_t s = sv->s;
   double *X = (double *) sv->ws.X.p, *R = (double *) sv->ws.R.p;
-  double *P0 = (double *) sv->ws.P0.p, *P1 = (double *) sv->ws.P1.p;
+  double *P = (double *) sv->ws.P0.p;
+  float *R32 = sv->pc32 ? (float *) sv->ws.R32.p : nullptr;
   double *Q = (double *) sv->ws.Q.p, *Zb = (double *) sv->ws.Zb.p;
-  float *R32 = (float *) sv->ws.R32.p, *Z32 = (float *) sv->ws.Z32.p;
-  double *Pold = P0, *Pnew = P1;
+  float *Z32 = (float *) sv->ws.Z32.p;
   int rc = 0;
   const size_t blk = (size_t) n * ld * sizeof (double);
-  if (cudaMemsetAsync (P0, 0, blk, s) != cudaSuccess
-      || cudaMemsetAsync (P1, 0, blk, s) != cudaSuccess
+  if (cudaMemsetAsync (P, 0, blk, s) != cudaSuccess
+      || (R32 && cudaMemsetAsync (R32, 0, blk / 2, s) != cudaSuccess)
       || cudaMemsetAsync (R, 0, blk, s) != cudaSuccess
       || cudaMemsetAsync (X, 0, blk, s) != cudaSuccess
       || cudaMemsetAsync (sv->ws.ival.p, 0, sv->ws.ival.n * sizeof (int), s) != cudaSuccess
@@ -692,35 +691,40 @@ srv_loop (lgh_server_t *sv)
     return;
   }
   std::vector<int> act (sv->cap);
-  /* one PCG tick over the slot block for a given pair of direction
-   * buffers; after two eager ticks (which set up the V-cycle buffers and
-   * the launch-shape caches) each parity is captured into a CUDA graph
-   * once and replayed, so a tick costs one graph launch on the host.  A
-   * mixed-precision object's V-cycle runs in FP32 on rounded copies of the
-   * residuals (the FP64 CG scalars and iterates are unchanged). */
-  auto tick = [&] (double *Po, double *Pn) -> int {
-    if (p->mg && sv->pc32) {
-      LGH_TRY ((cvt_flat<double, float> (n * ld, R, R32, s)));
+  /* one PCG tick over the slot block; after two eager ticks (which set up
+   * the V-cycle buffers and the launch-shape caches) it is captured into a
+   * CUDA graph once and replayed, so a tick costs one graph launch on the
+   * host.  A mixed-precision object's V-cycle runs in FP32 on the FP32 copy
+   * of the residuals that the residual pass (and a column's placement)
+   * keeps; its FP32 output is widened as the dots and the direction read
+   * it (the FP64 CG scalars and iterates are unchanged). */
+  auto tick = [&] () -> int {
+    const Csr &Z = p->Z->csr;
+    if (R32) {
       LGH_TRY (mg_vcycle<float> (p->mg, R32, Z32, ld, sv->cap, s, nullptr, &sv->mgw));
-      LGH_TRY ((cvt_flat<float, double> (n * ld, Z32, Zb, s)));
-    } else if (p->mg) {
-      LGH_TRY (mg_vcycle<double> (p->mg, R, Zb, ld, sv->cap, s, nullptr, &sv->mgw));
+      LGH_TRY ((launch_pcg_dots<double, float> (n, sv->cap, ld, R, Z32, 0,
+                                                p->zcfg.rtol, 0, nullptr,
+                                                sv->fresh_d.p, sv->ws, s)));
+      LGH_TRY ((launch_pcg_dir<double, float> (n, ld, Z32, P, X, 0, sv->ws, s)));
     } else {
-      LGH_TRY (launch_rowscale<double> (n, ld, p->Z->csr.dinv, R, ld, Zb, ld, s));
+      if (p->mg)
+        LGH_TRY (mg_vcycle<double> (p->mg, R, Zb, ld, sv->cap, s, nullptr, &sv->mgw));
+      else
+        LGH_TRY (launch_rowscale<double> (n, ld, Z.dinv, R, ld, Zb, ld, s));
+      LGH_TRY ((launch_pcg_dots<double, double> (n, sv->cap, ld, R, Zb, 0,
+                                                 p->zcfg.rtol, 0, nullptr,
+                                                 sv->fresh_d.p, sv->ws, s)));
+      LGH_TRY ((launch_pcg_dir<double, double> (n, ld, Zb, P, X, 0, sv->ws, s)));
     }
-    LGH_TRY (server_tick_dots<double> (p->Z->csr, R, Zb, ld, sv->cap, sv->fresh_d.p,
-                                       p->zcfg.rtol, sv->ws, s));
-    LGH_TRY (server_tick_pq<double> (p->Z->csr, Zb, Po, Pn, Q, ld, sv->ws, s));
-    return server_tick_upd<double> (n, ld, X, R, Pn, Q, sv->ws, s);
+    LGH_TRY (launch_pcg_prod<double> (Z, P, Q, ld, sv->ws, s));
+    return launch_pcg_resid<double> (n, ld, R, Q, R32, X, P, sv->ws, s);
   };
-  cudaGraphExec_t gexec[2] = { nullptr, nullptr };
+  cudaGraphExec_t gexec = nullptr;
   bool graphs_off = false;
-  int parity = 0;   /* 0: the old direction is in P0 */
   int hold = 0;     /* ticks that converged columns have waited */
   const int batch = std::max (1, sv->cap / 8);
   auto release_graphs = [&] () {
-    for (auto &ge : gexec)
-      if (ge) { cudaGraphExecDestroy (ge); ge = nullptr; }
+    if (gexec) { cudaGraphExecDestroy (gexec); gexec = nullptr; }
   };
   double ta = 0., tt = 0., th = 0.;   /* phase seconds, published per tick */
   double occ = 0.;                    /* occupied slots summed over ticks */
@@ -730,7 +734,7 @@ srv_loop (lgh_server_t *sv)
     std::vector<Adm> adm;
     srv_admit (sv, adm);
     for (const Adm &a : adm) {
-      rc = (a.r->kind == 2) ? srv_logdet (sv, a.r) : srv_start (sv, a, Pold);
+      rc = (a.r->kind == 2) ? srv_logdet (sv, a.r) : srv_start (sv, a);
       if (rc) break;
     }
     if (!adm.empty ()) ta += wall () - w0;
@@ -752,14 +756,14 @@ srv_loop (lgh_server_t *sv)
     if (cudaMemcpyAsync (sv->fresh_d.p, sv->fresh_pin, sv->cap * sizeof (int),
                          cudaMemcpyHostToDevice, s) != cudaSuccess)
       rc = set_error (LGH_ERR_GPU, "server: fresh flags");
-    if (!rc && !graphs_off && sv->ticks >= 2 && gexec[parity] == nullptr) {
+    if (!rc && !graphs_off && sv->ticks >= 2 && gexec == nullptr) {
       cudaGraph_t gr = nullptr;
       if (cudaStreamBeginCapture (s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        const int crc = tick (Pold, Pnew);
+        const int crc = tick ();
         const cudaError_t ce = cudaStreamEndCapture (s, &gr);
         if (crc != 0 || ce != cudaSuccess || gr == nullptr
-            || cudaGraphInstantiate (&gexec[parity], gr, 0) != cudaSuccess) {
-          gexec[parity] = nullptr;
+            || cudaGraphInstantiate (&gexec, gr, 0) != cudaSuccess) {
+          gexec = nullptr;
           graphs_off = true;     /* keep ticking eagerly */
         }
         if (gr) cudaGraphDestroy (gr);
@@ -770,15 +774,13 @@ srv_loop (lgh_server_t *sv)
       clear_error ();
     }
     if (!rc) {
-      if (gexec[parity]) {
-        if (cudaGraphLaunch (gexec[parity], s) != cudaSuccess)
+      if (gexec) {
+        if (cudaGraphLaunch (gexec, s) != cudaSuccess)
           rc = set_error (LGH_ERR_GPU, "server: tick graph launch");
       } else {
-        rc = tick (Pold, Pnew);
+        rc = tick ();
       }
     }
-    std::swap (Pold, Pnew);
-    parity ^= 1;
     std::fill (sv->fresh_h.begin (), sv->fresh_h.end (), 0);
     sv->ticks++;
     /* 3. the convergence mask; converged columns are harvested in
@@ -805,7 +807,7 @@ srv_loop (lgh_server_t *sv)
       if (conv > 0) hold++;
       if (conv > 0 && (conv >= batch || conv == occ_n || hold >= 3)) {
         w0 = wall ();
-        rc = srv_harvest (sv, act, Pold);
+        rc = srv_harvest (sv, act);
         th += wall () - w0;
         hold = 0;
       }

@@ -35,6 +35,7 @@
 #include "lgh_internal.h"
 #include "lgh_ktime.h"
 #include "lgh_mg.h"
+#include "lgh_pcg.h"
 
 namespace lgh
 {
@@ -43,11 +44,6 @@ int row_grid (int64_t n, int glog);
 
 constexpr int ZS_THREADS = 256;
 constexpr int ZS_MAXCH = 8;
-
-/* per-column scalar slots in ZWork::scal (each `cap` long) */
-enum { S_RZ = 0, S_ALPHA, S_BETA, S_NORM0, S_NSLOT };
-/* int slots in ZWork::ival */
-enum { I_ACTIVE = 0, I_ITS, I_NSLOT };
 
 struct ZK
 {
@@ -443,328 +439,6 @@ k_cheb (ZK z, const T *__restrict__ vals, const T *__restrict__ vdv,
   }
 }
 
-/* ---- PCG with an explicit preconditioner z = V(r) (the AMG V-cycle):
- * p_new = z + beta p_old on the fly at neighbours, q = Z p_new, (p, q) ---- */
-template <typename T, int CH, bool GIVEN = false>
-__global__ void __launch_bounds__ (ZS_THREADS, (CH * (16 / sizeof (T)) <= 8 ? 4 : 2))
-k_pcgx_pq (ZK z, const T *__restrict__ vals, const T *__restrict__ Zb,
-           const T *__restrict__ Pold, T *__restrict__ Pnew,
-           T *__restrict__ Qv, int ld, int nvec, int glog, int first,
-           double *partA, unsigned *counter, double *scal, int *ival, int cap)
-{
-  /* GIVEN: the direction p_new is already in Pnew (formed by the
-   * streaming k_pcgx_pform); the product gathers p alone and Pnew is only
-   * read.  Otherwise p_new = z + beta p_old is formed at every neighbour
-   * row (first: p = z). */
-  /* the next row's bounds and first G (column, value) pairs are loaded
-   * while the current row's neighbours are gathered (software pipeline).
-   * The per-column beta and each lane's running (p, q) sums live in
-   * shared memory (the sums in the lane's own slots of the reduction
-   * area, added to in the same row order as register sums would be), which
-   * keeps the two-pack FP64 form within 64 registers: 4 CTAs per SM. */
-  extern __shared__ double red[];
-  ZS_GROUP_SETUP ();
-  const double *beta = scal + S_BETA * cap;
-  T *bsm = reinterpret_cast<T *> (red + (size_t) ngroups * ld);
-  for (int c = threadIdx.x; c < ld; c += blockDim.x)
-    bsm[c] = first ? T (0) : (T) beta[c];
-  double *apq = red + (size_t) group * ld;
-#pragma unroll
-  for (int h = 0; h < CH; h++) {
-    const int vi = lane + h * G;
-    if (vi < nvec)
-#pragma unroll
-      for (int e = 0; e < W; e++) apq[vi * W + e] = 0.;
-  }
-  __syncthreads ();
-  const int64_t stride = (int64_t) gridDim.x * ngroups;
-  int64_t i = (int64_t) blockIdx.x * ngroups + group;
-  int64_t k0 = 0, k1 = 0;
-  int mc = 0;
-  T mv = T (0);
-  if (i < z.n) {
-    k0 = z.rowptr[i];
-    k1 = z.rowptr[i + 1];
-    if (lane < k1 - k0) {
-      mc = z.col[k0 + lane];
-      mv = vals[k0 + lane];
-    }
-  }
-  for (; i < z.n; i += stride) {
-    const int64_t inx = i + stride;
-    int64_t k0n = 0, k1n = 0;
-    if (inx < z.n) {
-      k0n = z.rowptr[inx];
-      k1n = z.rowptr[inx + 1];
-    }
-    T acc[CH][W];
-#pragma unroll
-    for (int h = 0; h < CH; h++)
-#pragma unroll
-      for (int e = 0; e < W; e++) acc[h][e] = T (0);
-    for (int64_t kb = k0; kb < k1; kb += G) {
-      const int cnt = (int) ((k1 - kb) < G ? (k1 - kb) : G);
-      if (kb != k0) {
-        mc = 0;
-        mv = T (0);
-        if (lane < cnt) {
-          mc = z.col[kb + lane];
-          mv = vals[kb + lane];
-        }
-      }
-      for (int t = 0; t < cnt; t++) {
-        const int c = __shfl_sync (gmask, mc, t, G);
-        const T v = __shfl_sync (gmask, mv, t, G);
-#pragma unroll
-        for (int h = 0; h < CH; h++) {
-          const int vi = lane + h * G;
-          if (vi < nvec) {
-            if constexpr (GIVEN) {
-              const Pack<T> pj = ldp (Pnew + (int64_t) c * ld + vi * W);
-#pragma unroll
-              for (int e = 0; e < W; e++)
-                acc[h][e] = fma (v, pj.v[e], acc[h][e]);
-            } else {
-              Pack<T> zj = ldp (Zb + (int64_t) c * ld + vi * W);
-              Pack<T> pj = first ? pzero<T> () : ldp (Pold + (int64_t) c * ld + vi * W);
-              const Pack<T> bt = *reinterpret_cast<const Pack<T> *> (bsm + vi * W);
-#pragma unroll
-              for (int e = 0; e < W; e++)
-                acc[h][e] = fma (v, fma (bt.v[e], pj.v[e], zj.v[e]), acc[h][e]);
-            }
-          }
-        }
-      }
-    }
-    int mcn = 0;
-    T mvn = T (0);
-    if (inx < z.n && lane < k1n - k0n) {
-      mcn = z.col[k0n + lane];
-      mvn = vals[k0n + lane];
-    }
-#pragma unroll
-    for (int h = 0; h < CH; h++) {
-      const int vi = lane + h * G;
-      if (vi < nvec) {
-        Pack<T> pn, q;
-        if constexpr (GIVEN) {
-          pn = ldp (Pnew + i * ld + vi * W);
-        } else {
-          Pack<T> zi = ldp (Zb + i * ld + vi * W);
-          Pack<T> pi = first ? pzero<T> () : ldp (Pold + i * ld + vi * W);
-          const Pack<T> bt = *reinterpret_cast<const Pack<T> *> (bsm + vi * W);
-#pragma unroll
-          for (int e = 0; e < W; e++) pn.v[e] = fma (bt.v[e], pi.v[e], zi.v[e]);
-        }
-#pragma unroll
-        for (int e = 0; e < W; e++) {
-          q.v[e] = acc[h][e];
-          apq[vi * W + e] += (double) pn.v[e] * (double) q.v[e];
-        }
-        if constexpr (!GIVEN) stp (Pnew + i * ld + vi * W, pn);
-        stp (Qv + i * ld + vi * W, q);
-      }
-    }
-    k0 = k0n;
-    k1 = k1n;
-    mc = mcn;
-    mv = mvn;
-  }
-  __syncthreads ();
-  for (int c = threadIdx.x; c < ld; c += blockDim.x) {
-    double sum = 0.;
-    for (int g = 0; g < ngroups; g++) sum += red[g * ld + c];
-    partA[(size_t) c * gridDim.x + blockIdx.x] = sum;
-  }
-  const double *rz = scal + S_RZ * cap;
-  double *al = scal + S_ALPHA * cap;
-  int *act = ival + I_ACTIVE * cap;
-  last_block_reduce (partA, ld, counter, [&] (int c, double pq) {
-    if (act[c]) {
-      if (pq != 0. && isfinite (pq)) al[c] = rz[c] / pq;
-      else { al[c] = 0.; act[c] = 0; }
-    } else {
-      al[c] = 0.;
-    }
-  });
-}
-
-/* x += alpha p, r -= alpha q (no reductions) */
-template <typename T>
-__global__ void
-k_pcgx_upd (int64_t n, int ld, T *__restrict__ X, T *__restrict__ R,
-            const T *__restrict__ Pn,
-            const T *__restrict__ Qv, const double *alpha)
-{
-  constexpr int W = Pack<T>::W;
-  const int nvec = ld / W;
-  const int64_t total = n * nvec;
-  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t) gridDim.x * blockDim.x) {
-    const int64_t i = e / nvec;
-    const int vi = (int) (e - i * nvec);
-    const int64_t o = i * ld + vi * W;
-    Pack<T> x = ldp (X + o), r = ldp (R + o), p = ldp (Pn + o), q = ldp (Qv + o);
-#pragma unroll
-    for (int k = 0; k < W; k++) {
-      const T a = (T) alpha[vi * W + k];
-      x.v[k] = fma (a, p.v[k], x.v[k]);
-      r.v[k] = fma (-a, q.v[k], r.v[k]);
-    }
-    stp (X + o, x);
-    stp (R + o, r);
-  }
-}
-
-/* the direction, streamed: p_new = z + beta p_old; with it the previous
- * iteration's deferred x += alpha p_old (x is read by nothing inside an
- * iteration, so the update moves here from k_pcgx_upd; the same FMA, so
- * the same bits) */
-template <typename T>
-__global__ void
-k_pcgx_pform (int64_t n, int ld, const T *__restrict__ Zb,
-              const T *__restrict__ Pold, T *__restrict__ Pnew,
-              T *__restrict__ X, const double *beta, const double *alpha)
-{
-  constexpr int W = Pack<T>::W;
-  const int nvec = ld / W;
-  const int64_t total = n * nvec;
-  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t) gridDim.x * blockDim.x) {
-    const int64_t i = e / nvec;
-    const int vi = (int) (e - i * nvec);
-    const int64_t o = i * ld + vi * W;
-    const Pack<T> z = ldp (Zb + o), p = ldp (Pold + o);
-    Pack<T> x = ldp (X + o), pn;
-#pragma unroll
-    for (int k = 0; k < W; k++) {
-      pn.v[k] = fma ((T) beta[vi * W + k], p.v[k], z.v[k]);
-      x.v[k] = fma ((T) alpha[vi * W + k], p.v[k], x.v[k]);
-    }
-    stp (Pnew + o, pn);
-    stp (X + o, x);
-  }
-}
-
-/* r -= alpha q (the x half of the update is deferred to k_pcgx_pform) */
-template <typename T>
-__global__ void
-k_pcgx_updr (int64_t n, int ld, T *__restrict__ R, const T *__restrict__ Qv,
-             const double *alpha)
-{
-  constexpr int W = Pack<T>::W;
-  const int nvec = ld / W;
-  const int64_t total = n * nvec;
-  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t) gridDim.x * blockDim.x) {
-    const int64_t i = e / nvec;
-    const int vi = (int) (e - i * nvec);
-    const int64_t o = i * ld + vi * W;
-    Pack<T> r = ldp (R + o);
-    const Pack<T> q = ldp (Qv + o);
-#pragma unroll
-    for (int k = 0; k < W; k++) r.v[k] = fma (-(T) alpha[vi * W + k], q.v[k], r.v[k]);
-    stp (R + o, r);
-  }
-}
-
-/* the last iteration's deferred x += alpha p */
-template <typename T>
-__global__ void
-k_pcgx_xfin (int64_t n, int ld, T *__restrict__ X, const T *__restrict__ P,
-             const double *alpha)
-{
-  constexpr int W = Pack<T>::W;
-  const int nvec = ld / W;
-  const int64_t total = n * nvec;
-  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t) gridDim.x * blockDim.x) {
-    const int64_t i = e / nvec;
-    const int vi = (int) (e - i * nvec);
-    const int64_t o = i * ld + vi * W;
-    Pack<T> x = ldp (X + o);
-    const Pack<T> p = ldp (P + o);
-#pragma unroll
-    for (int k = 0; k < W; k++) x.v[k] = fma ((T) alpha[vi * W + k], p.v[k], x.v[k]);
-    stp (X + o, x);
-  }
-}
-
-/* dots (r, z), (z, z) after the preconditioner: first call sets rz, norm0
- * and the mask; later calls set beta and test convergence on ||z|| */
-template <typename T, int CH>
-__global__ void __launch_bounds__ (ZS_THREADS, (CH * (16 / sizeof (T)) <= 8 ? 3 : 2))
-k_pcgx_dots (ZK z, const T *__restrict__ R, const T *__restrict__ Zb, int ld,
-             int nvec, int glog, int w, int first, double *partA,
-             double *partB, unsigned *counter, double *scal, int *ival,
-             int cap, double rtol, int iter, double *hist,
-             const int *fresh)
-{
-  extern __shared__ double red[];
-  ZS_GROUP_SETUP ();
-  double aRZ[CH][W], aZZ[CH][W];
-#pragma unroll
-  for (int h = 0; h < CH; h++)
-#pragma unroll
-    for (int e = 0; e < W; e++) { aRZ[h][e] = 0.; aZZ[h][e] = 0.; }
-  for (int64_t i = (int64_t) blockIdx.x * ngroups + group; i < z.n;
-       i += (int64_t) gridDim.x * ngroups) {
-#pragma unroll
-    for (int h = 0; h < CH; h++) {
-      const int vi = lane + h * G;
-      if (vi < nvec) {
-        Pack<T> r = ldp (R + i * ld + vi * W), zz = ldp (Zb + i * ld + vi * W);
-#pragma unroll
-        for (int e = 0; e < W; e++) {
-          aRZ[h][e] += (double) r.v[e] * (double) zz.v[e];
-          aZZ[h][e] += (double) zz.v[e] * (double) zz.v[e];
-        }
-      }
-    }
-  }
-  block_colsum_store<T, CH> (aRZ, lane, group, G, nvec, ld, red, partA);
-  block_colsum_store<T, CH> (aZZ, lane, group, G, nvec, ld, red, partB);
-  double *rz = scal + S_RZ * cap, *be = scal + S_BETA * cap;
-  double *al_g = scal + S_ALPHA * cap, *n0 = scal + S_NORM0 * cap;
-  int *act = ival + I_ACTIVE * cap, *its = ival + I_ITS * cap;
-  bool last = last_block_reduce2 (partA, partB, ld, counter,
-      [&] (int c, double srz, double szz) {
-        if (first || (fresh != nullptr && fresh[c])) {
-          rz[c] = srz;
-          n0[c] = sqrt (szz);
-          act[c] = (c < w && szz > 0.) ? 1 : 0;
-          al_g[c] = 0.;
-          be[c] = 0.;
-          its[c] = 0;
-          return;
-        }
-        if (!act[c]) { be[c] = 0.; return; }
-        const double b = (rz[c] != 0.) ? srz / rz[c] : 0.;
-        if (hist != nullptr && c == 0 && iter < 10000) {
-          hist[2 * iter] = al_g[0];
-          hist[2 * iter + 1] = b;
-        }
-        rz[c] = srz;
-        be[c] = b;
-        /* a converged column keeps its alpha: its x update may still be
-         * pending (k_pcgx_pform or k_pcgx_xfin applies it), and the next
-         * product zeroes alpha for inactive columns */
-        if (sqrt (szz) <= rtol * n0[c] || srz == 0.) {
-          act[c] = 0;
-          be[c] = 0.;
-          its[c] = iter + 1;
-        }
-      });
-  if (last) {
-    __syncthreads ();
-    if (threadIdx.x == 0) {
-      int cnt = 0;
-      for (int c = 0; c < ld; c++) cnt += act[c];
-      ival[I_NSLOT * cap] = cnt;
-    }
-  }
-}
-
 /* Chebyshev with an explicit preconditioner: d_new = a d + b z on the fly
  * at neighbours, x += d_new, r_new = r - Z d_new */
 template <typename T, int CH>
@@ -927,13 +601,6 @@ zs_smem_bytes (int glog, int ld)
   return (ZS_THREADS >> glog) * ld * (int) sizeof (double);
 }
 
-/* k_pcgx_pq: the reduction area plus the per-column beta */
-static int
-zs_pq_smem_bytes (int glog, int ld)
-{
-  return zs_smem_bytes (glog, ld) + ld * (int) sizeof (double);
-}
-
 int
 ZWork::alloc (int64_t n_, int cap_, int is32_)
 {
@@ -1000,40 +667,6 @@ zvd (const Csr &Z)
     return set_error (LGH_ERR_SUP, "zsolve: chunking %d unsupported", CHV);  \
   }
 
-/* flat conversion of a row-major block (same leading dimension on both
- * sides), four elements per thread */
-template <typename TI, typename TO>
-__global__ void
-k_cvt_flat (int64_t count, const TI *__restrict__ X, TO *__restrict__ Y)
-{
-  const int64_t q = count / 4;
-  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < q;
-       e += (int64_t) gridDim.x * blockDim.x) {
-    const int64_t o = e * 4;
-#pragma unroll
-    for (int k = 0; k < 4; k++) Y[o + k] = (TO) X[o + k];
-  }
-  for (int64_t o = q * 4 + (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-       o < count; o += (int64_t) gridDim.x * blockDim.x)
-    Y[o] = (TO) X[o];
-}
-
-template <typename TI, typename TO>
-int
-cvt_flat (int64_t count, const TI *X, TO *Y, cudaStream_t s)
-{
-  const int grid = (int) std::max<int64_t> (1, std::min<int64_t> (
-      (int64_t) num_sms () * 8, (count / 4 + 255) / 256));
-  k_cvt_flat<TI, TO><<<grid, 256, 0, s>>> (count, X, Y);
-  LGH_LAUNCH_CHECK ();
-  return 0;
-}
-
-template int cvt_flat<double, float> (int64_t, const double *, float *,
-                                      cudaStream_t);
-template int cvt_flat<float, double> (int64_t, const float *, double *,
-                                      cudaStream_t);
-
 template <typename T>
 int
 zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
@@ -1080,30 +713,31 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
     const int cap = ws.cap;
     int *nact = ws.ival.p + I_NSLOT * cap;
 
-    ZS_DISPATCH (ch, {
-      auto kf = k_pcg_init<T, CH_>;
-      set_smem_attr (kf, smem);
-      kf<<<fit_grid (kf, grid, ZS_THREADS, smem), ZS_THREADS, smem, s>>> (zk, dinv, Xin + c0, ldx, rs_in, bX,
-                                         bR, bP0, ldt, nvec, glog, wt,
-                                         ws.partA.p, ws.partB.p,
-                                         ws.counters.p, ws.scal.p, ws.ival.p,
-                                         cap);
-    });
-    LGH_LAUNCH_CHECK ();
+    const bool mgpcg = cfg.mode <= 1 && mg != nullptr && cfg.maxit > 0;
+    if (!mgpcg) {
+      ZS_DISPATCH (ch, {
+        auto kf = k_pcg_init<T, CH_>;
+        set_smem_attr (kf, smem);
+        kf<<<fit_grid (kf, grid, ZS_THREADS, smem), ZS_THREADS, smem, s>>> (zk, dinv, Xin + c0, ldx, rs_in, bX,
+                                           bR, bP0, ldt, nvec, glog, wt,
+                                           ws.partA.p, ws.partB.p,
+                                           ws.counters.p, ws.scal.p, ws.ival.p,
+                                           cap);
+      });
+      LGH_LAUNCH_CHECK ();
+    }
 
     int iters = 0;
     T *bZ = (T *) ws.Zb.p;
-    if (cfg.mode <= 1 && mg != nullptr) {
+    if (mgpcg) {
       /* PCG with the V-cycle: z = V(r) each iteration (the reference's
        * per-column CG + PCGAMG, zsolve_impl.h:674-683, 808-818) */
-      const int egrid = std::max (1, std::min (num_sms () * 8,
-                                  (int) ((n * (ldt / W) + 255) / 256)));
       static thread_local KTrace ktr;
       KTrace *tr = timing ? &ktr : nullptr;
       const double bw = (double) n * wt * sizeof (T);
-      /* z = V(r): in T, or (cfg.pc32, FP64 iterates) an FP32 V-cycle
-       * between two conversions: the Krylov vectors and so the attainable
-       * accuracy stay FP64, the V-cycle's traffic is halved */
+      /* z = V(r): in T, or (cfg.pc32, FP64 iterates) an FP32 V-cycle on r's
+       * FP32 copy: the Krylov vectors and so the attainable accuracy stay
+       * FP64, the V-cycle's traffic is halved */
       const bool pc32 = cfg.pc32 && std::is_same<T, double>::value;
       float *R32 = nullptr, *Z32 = nullptr;
       if (pc32) {
@@ -1112,76 +746,54 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
         R32 = (float *) ws.R32.p;
         Z32 = (float *) ws.Z32.p;
       }
+      /* the direction is updated in place in bP; the first one is z itself,
+       * so its buffer and z's swap */
+      T *bP = bP0;
+      const double zw = pc32 ? sizeof (float) / (double) sizeof (T) : 1.;
+      double *hist = record_hist ? ws.hist.p : nullptr;
       auto precond = [&] () -> int {
         if (!pc32) return mg_vcycle<T> (mg, bR, bZ, ldt, wt, s, tr);
-        const int64_t cnt = n * (int64_t) ldt;
-        LGH_TRY ((cvt_flat<T, float> (cnt, bR, R32, s)));
-        LGH_TRY (mg_vcycle<float> (mg, R32, Z32, ldt, wt, s, nullptr));
-        return cvt_flat<float, T> (cnt, Z32, bZ, s);
+        return mg_vcycle<float> (mg, R32, Z32, ldt, wt, s, nullptr);
       };
+      auto dots = [&] (int first, int it) -> int {
+        if constexpr (std::is_same<T, double>::value)
+          if (pc32)
+            return launch_pcg_dots<T, float> (n, wt, ldt, bR, Z32, first,
+                                              cfg.rtol, it, hist, nullptr, ws, s);
+        return launch_pcg_dots<T, T> (n, wt, ldt, bR, bZ, first, cfg.rtol, it,
+                                      hist, nullptr, ws, s);
+      };
+      auto direction = [&] (int flags) -> int {
+        if constexpr (std::is_same<T, double>::value)
+          if (pc32)
+            return launch_pcg_dir<T, float> (n, ldt, Z32, bP, bX, flags, ws, s);
+        return launch_pcg_dir<T, T> (n, ldt, bZ, bP, bX, flags, ws, s);
+      };
+      LGH_TRY (launch_pcg_start<T> (n, wt, ldt, Xin + c0, ldx, rs_in, bR, R32, s));
       LGH_TRY (precond ());
-      ZS_DISPATCH (ch, {
-        auto kd = k_pcgx_dots<T, CH_>;
-        set_smem_attr (kd, smem);
-        kd<<<fit_grid (kd, grid, ZS_THREADS, smem), ZS_THREADS, smem, s>>> (zk, bR, bZ, ldt, nvec, glog, wt, 1,
-                                           ws.partA.p, ws.partB.p,
-                                           ws.counters.p + 1, ws.scal.p,
-                                           ws.ival.p, cap, cfg.rtol, 0, nullptr, nullptr);
-      });
-      LGH_LAUNCH_CHECK ();
-      T *Pold = bP0, *Pnew = bP1;
+      LGH_TRY (dots (1, 0));
       int h_nact = 1;
-      const double *alpha = ws.scal.p + S_ALPHA * cap;
-      const double *betap = ws.scal.p + S_BETA * cap;
       for (int it = 0; it < cfg.maxit; it++) {
-        /* iteration 0: p = z inside the product; later iterations: the
-         * direction p = z + beta p_old by a streaming pass, which also
-         * applies the previous iteration's x += alpha p_old, then the
-         * product gathers p alone */
-        if (it > 0) {
-          if (tr) LGH_TRY (tr->begin (K_PCGX_PFORM, 5. * bw, s));
-          k_pcgx_pform<T><<<egrid, 256, 0, s>>> (n, ldt, bZ, Pold, Pnew, bX,
-                                                betap, alpha);
-          LGH_LAUNCH_CHECK ();
+        if (it == 0 && !pc32) {
+          std::swap (bP, bZ);
+        } else {
+          const int flags = it == 0 ? PCG_P_FIRST
+                            : it == 1 ? PCG_X_FIRST : PCG_X_ADD;
+          if (tr) LGH_TRY (tr->begin (K_PCGX_PFORM, (it == 0 ? 1. + zw
+                                      : it == 1 ? 3. + zw : 4. + zw) * bw, s));
+          LGH_TRY (direction (flags));
           if (tr) LGH_TRY (tr->end (s));
         }
-        if (tr) LGH_TRY (tr->begin (K_PCGX_PQ, zbytes + (it == 0 ? 3. : 2.) * bw, s));
-        ZS_DISPATCH (ch, {
-          const int psm = zs_pq_smem_bytes (glog, ldt);
-          if (it == 0) {
-            auto k1 = k_pcgx_pq<T, CH_, false>;
-            set_smem_attr (k1, psm);
-            k1<<<fit_grid (k1, grid, ZS_THREADS, psm), ZS_THREADS, psm, s>>> (
-                zk, vals, bZ, Pold, Pnew, bQ, ldt, nvec, glog, 1, ws.partA.p,
-                ws.counters.p, ws.scal.p, ws.ival.p, cap);
-          } else {
-            auto k1 = k_pcgx_pq<T, CH_, true>;
-            set_smem_attr (k1, psm);
-            k1<<<fit_grid (k1, grid, ZS_THREADS, psm), ZS_THREADS, psm, s>>> (
-                zk, vals, bZ, Pold, Pnew, bQ, ldt, nvec, glog, 0, ws.partA.p,
-                ws.counters.p, ws.scal.p, ws.ival.p, cap);
-          }
-        });
-        LGH_LAUNCH_CHECK ();
+        if (tr) LGH_TRY (tr->begin (K_PCGX_PQ, zbytes + 2. * bw, s));
+        LGH_TRY (launch_pcg_prod<T> (Z, bP, bQ, ldt, ws, s));
         if (tr) LGH_TRY (tr->end (s));
-        if (tr) LGH_TRY (tr->begin (K_PCGX_UPD, 3. * bw, s));
-        k_pcgx_updr<T><<<egrid, 256, 0, s>>> (n, ldt, bR, bQ, alpha);
-        LGH_LAUNCH_CHECK ();
+        if (tr) LGH_TRY (tr->begin (K_PCGX_UPD, (pc32 ? 3. + zw : 3.) * bw, s));
+        LGH_TRY (launch_pcg_resid<T> (n, ldt, bR, bQ, R32, nullptr, nullptr, ws, s));
         if (tr) LGH_TRY (tr->end (s));
         LGH_TRY (precond ());
-        if (tr) LGH_TRY (tr->begin (K_PCGX_DOTS, 2. * bw, s));
-        ZS_DISPATCH (ch, {
-          auto kd = k_pcgx_dots<T, CH_>;
-          kd<<<fit_grid (kd, grid, ZS_THREADS, smem), ZS_THREADS, smem, s>>> (zk, bR, bZ, ldt, nvec, glog, wt, 0,
-                                             ws.partA.p, ws.partB.p,
-                                             ws.counters.p + 1, ws.scal.p,
-                                             ws.ival.p, cap, cfg.rtol, it,
-                                             record_hist ? ws.hist.p : nullptr,
-                                             nullptr);
-        });
-        LGH_LAUNCH_CHECK ();
+        if (tr) LGH_TRY (tr->begin (K_PCGX_DOTS, (1. + zw) * bw, s));
+        LGH_TRY (dots (0, it));
         if (tr) LGH_TRY (tr->end (s));
-        std::swap (Pold, Pnew);
         iters = it + 1;
         if (iters % 2 == 0 || iters == cfg.maxit || iters <= 2) {
           LGH_CUDA (cudaMemcpyAsync (&h_nact, nact, sizeof (int),
@@ -1191,10 +803,6 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
           if (h_nact == 0) break;
         }
       }
-      /* the last iteration's deferred x += alpha p (its direction is in
-       * Pold after the swap) */
-      k_pcgx_xfin<T><<<egrid, 256, 0, s>>> (n, ldt, bX, Pold, alpha);
-      LGH_LAUNCH_CHECK ();
       if (tr && !tr->ids.empty ()) {
         LGH_CUDA (cudaStreamSynchronize (s));
         LGH_TRY (tr->drain ());
@@ -1210,7 +818,12 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
         for (int c = 0; c < wt; c++) st->col_iters += act_h[c] ? iters : its_h[c];
         if (h_nact > 0) st->last_maxit_hit = 1;
         st->cols += wt;
+        st->block_iters += iters;
       }
+      /* the last iteration's deferred x += alpha p with the row scaling */
+      LGH_TRY (launch_pcg_out<T> (n, wt, ldt, bX, bP, iters > 1, rs_out, Y + c0,
+                                  ldy, ws, s));
+      continue;
     } else if (cfg.mode >= 2 && mg != nullptr) {
       /* Chebyshev around the V-cycle (modes 2/3: zsolve_impl.h:108-141
        * with the AMG / harvested-hierarchy preconditioner) */
@@ -1381,80 +994,6 @@ template int zsolve_block<float> (const Csr &, const ZsolveCfg &, Hierarchy *,
                                   ZWork &, int64_t, int, const float *, int,
                                   const double *, float *, int, const double *,
                                   ZsolveStats *, int, cudaStream_t);
-
-/* ---- one tick of the request loop's slot block (server.cu) ------------- */
-
-template <typename T>
-int
-server_tick_pq (const Csr &Z, const T *Zb, const T *Pold, T *Pnew, T *Q, int ld,
-                ZWork &ws, cudaStream_t s)
-{
-  constexpr int W = Pack<T>::W;
-  const int nvec = ld / W;
-  int glog, ch;
-  row_group_shape (nvec, glog, ch, Z.max_row_nnz);
-  const int grid = std::min (row_grid (Z.n, glog), ws.nblocks);
-  const int smem = zs_pq_smem_bytes (glog, ld);
-  ZK zk{ Z.n, Z.rowptr, Z.colidx };
-  ZS_DISPATCH (ch, {
-    auto k1 = k_pcgx_pq<T, CH_>;
-    set_smem_attr (k1, smem);
-    k1<<<fit_grid (k1, grid, ZS_THREADS, smem), ZS_THREADS, smem, s>>> (zk, zvals<T> (Z), Zb, Pold, Pnew, Q, ld,
-                                       nvec, glog, 0, ws.partA.p,
-                                       ws.counters.p, ws.scal.p, ws.ival.p,
-                                       ws.cap);
-  });
-  LGH_LAUNCH_CHECK ();
-  return 0;
-}
-
-template <typename T>
-int
-server_tick_upd (int64_t n, int ld, T *X, T *R, const T *Pn, const T *Q,
-                 ZWork &ws, cudaStream_t s)
-{
-  constexpr int W = Pack<T>::W;
-  const int egrid = std::max (1, std::min (num_sms () * 8,
-                              (int) ((n * (ld / W) + 255) / 256)));
-  k_pcgx_upd<T><<<egrid, 256, 0, s>>> (n, ld, X, R, Pn, Q,
-                                       ws.scal.p + S_ALPHA * ws.cap);
-  LGH_LAUNCH_CHECK ();
-  return 0;
-}
-
-template <typename T>
-int
-server_tick_dots (const Csr &Z, const T *R, const T *Zb, int ld, int w,
-                  const int *fresh, double rtol, ZWork &ws, cudaStream_t s)
-{
-  constexpr int W = Pack<T>::W;
-  const int nvec = ld / W;
-  int glog, ch;
-  row_group_shape (nvec, glog, ch, Z.max_row_nnz);
-  const int grid = std::min (row_grid (Z.n, glog), ws.nblocks);
-  const int smem = zs_smem_bytes (glog, ld);
-  ZK zk{ Z.n, Z.rowptr, Z.colidx };
-  ZS_DISPATCH (ch, {
-    auto kd = k_pcgx_dots<T, CH_>;
-    set_smem_attr (kd, smem);
-    kd<<<fit_grid (kd, grid, ZS_THREADS, smem), ZS_THREADS, smem, s>>> (zk, R, Zb, ld, nvec, glog, w, 0,
-                                       ws.partA.p, ws.partB.p,
-                                       ws.counters.p + 1, ws.scal.p, ws.ival.p,
-                                       ws.cap, rtol, 0, nullptr, fresh);
-  });
-  LGH_LAUNCH_CHECK ();
-  return 0;
-}
-
-template int server_tick_pq<double> (const Csr &, const double *, const double *,
-                                     double *, double *, int, ZWork &,
-                                     cudaStream_t);
-template int server_tick_upd<double> (int64_t, int, double *, double *,
-                                      const double *, const double *, ZWork &,
-                                      cudaStream_t);
-template int server_tick_dots<double> (const Csr &, const double *,
-                                       const double *, int, int, const int *,
-                                       double, ZWork &, cudaStream_t);
 
 /* L2 bytes the smoother's neighbour reuse may span: a row's r and d rows
  * are gathered again by the rows up to the bandwidth away, so the band of
