@@ -71,7 +71,7 @@ struct ShiftPlan
   int64_t n = 0;
   int m = 0, kept = 0, cap_shift = 0;
   /* workspace of the batched operation (stable addresses for the graph) */
-  DBuf<double> R, Xs, Y0, Wc, work, g, fc, cdev;
+  DBuf<double> R, Xs, Y0, Wc, S, work, g, fc, cdev;
   DBuf<char> pdev;
   Params *ph = nullptr;   /* pinned */
   double *cph = nullptr;  /* pinned shifts */
@@ -113,7 +113,7 @@ struct ShiftPlan
     }
   }
 
-  int ensure (int64_t n_, int m_, int kept_, int nshift)
+  int ensure (int64_t n_, int m_, int kept_, int nshift, bool fp64)
   {
     if (n_ != n || m_ > m || kept_ != kept) {
       drop_graph ();
@@ -136,6 +136,13 @@ struct ShiftPlan
       if (cph) cudaFreeHost (cph);
       cph = nullptr;
       LGH_CUDA (cudaMallocHost ((void **) &cph, cap_shift * sizeof (double)));
+    }
+    /* the scaled coefficient block of the FP64 form (the tensor-core form
+     * of mixed objects splits its own) */
+    const size_t sn = (size_t) std::max (kept, 1) * nshift * m_;
+    if (fp64 && sn > S.n) {
+      drop_graph ();
+      LGH_TRY (S.alloc (sn));
     }
     if (!ph) {
       LGH_CUDA (cudaMallocHost ((void **) &ph, sizeof (Params)));
@@ -228,7 +235,7 @@ enqueue_tail (ShiftPlan &P, lgh_glr_t *g, int kind, int nshift, int variant,
                                       P.err.p, s);
   }
   return launch_shift_combine_variant (variant, P.n, P.kept, m, nshift, g->Wz.p,
-                                       g->ldu, P.Wc.p, P.g.p, P.fc.p, P.Y0.p,
+                                       g->ldu, P.Wc.p, P.g.p, P.S.p, P.fc.p, P.Y0.p,
                                        round_ld (m), &pd->out, &pd->ldo, s);
 }
 
@@ -237,7 +244,9 @@ shift_plan_get (lgh_glr_t *g, int64_t n, int m, int kept, int nshift,
                 ShiftPlan **out)
 {
   if (!g->splan) g->splan = new ShiftPlan ();
-  LGH_TRY (g->splan->ensure (n, m, kept, nshift));
+  LGH_TRY (g->splan->ensure (n, m, kept, nshift,
+                             g->exec.precision != LGH_PREC_MIXED || kept == 0
+                                 || !umma_supported ()));
   *out = g->splan;
   return 0;
 }

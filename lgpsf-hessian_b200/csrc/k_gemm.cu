@@ -13,17 +13,26 @@
  *
  *   dense_apply  Y = A^{-1} B on the multigrid's dense coarse level.
  *
- * All three run on the FP64 tensor cores: a CTA of 4 warps owns a 64 x 64
- * output tile, each warp a 32 x 32 quarter of 4 x 4 mma.sync m8n8k4 f64
- * tiles; operands are staged k-major in shared memory 16 k-values at a
- * time (rows padded to 68 doubles so that a fragment load touches 16
- * distinct bank pairs), and the next stage is read into registers while
- * the current one is multiplied.  Float blocks (mixed path) are widened to
- * FP64 as they are staged; every product accumulates in FP64.  These
- * products are O(n ell^2) and bounded by the FP64 tensor pipe.
- */
+ * The tall products run on the FP64 tensor cores (mma.sync m8n8k4): a CTA of
+ * 4 (or 8) warps owns a 64 (128) x 64 output tile, each warp a 32 x 32 part
+ * of 4 x 4 fragments.  Operands come into shared memory 16 k-values at a
+ * time with cp.async in a ring of three stages, in their own layout: a block
+ * whose columns are the output's rows (A^T B) stays k-major, one whose
+ * columns are summed over (X M) stays row-major; the row strides (68 and 20
+ * doubles, 72 and 20 floats) put the 16 values of a fragment load's
+ * half-warp in distinct banks either way.  Float blocks (mixed path) are
+ * widened to FP64 as the fragments are read; every product accumulates in
+ * FP64.  Fragments past the operands' edges are not multiplied (220 columns
+ * are 27.5 fragments, not the 32 of four whole tiles), and the Gram X^T X
+ * forms the tiles on and above its diagonal alone.  At 262144 x 220 x 220
+ * the scalar register staging this replaces took 1.42 ms a product (17.9
+ * TFLOP/s, the load pipe 76-88 % busy with 8-byte accesses); see the launch
+ * functions for what they take now. */
 
 #include <algorithm>
+#include <mutex>
+#include <set>
+#include <type_traits>
 
 #include "lgh_batch.h"
 #include "lgh_device.cuh"
@@ -32,34 +41,164 @@
 namespace lgh
 {
 
-constexpr int GB = 64, GK = 16;
-constexpr int SLD = GB + 4;   /* shared row stride, doubles */
+constexpr int GB = 64, GK = 16, GSTAGES = 3;
 
-/* one staged k block: As[k][i] (k-major), Bs[k][j]; warp (wm, wn) adds
- * its 32 x 32 quarter.  m8n8k4 f64 fragments: A (8 x 4, row) holds
- * A[lane / 4][lane % 4], B (4 x 8, col) holds B[lane % 4][lane / 4],
- * C holds C[lane / 4][2 (lane % 4) + {0, 1}]. */
+/* CB bytes from global to shared memory, the last CB - bytes zero */
+template <int CB>
 __device__ __forceinline__ void
-dmma_block (const double (*As)[SLD], const double (*Bs)[SLD], int wm, int wn,
-            int lane, double (&acc)[4][4][2])
+cp_async (void *smem, const void *src, int bytes)
+{
+  const unsigned d = (unsigned) __cvta_generic_to_shared (smem);
+  if constexpr (CB == 16)
+    asm volatile ("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d),
+                  "l"(src), "r"(bytes) : "memory");
+  else if constexpr (CB == 8)
+    asm volatile ("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d),
+                  "l"(src), "r"(bytes) : "memory");
+  else
+    asm volatile ("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d),
+                  "l"(src), "r"(bytes) : "memory");
+}
+
+/* one operand's stage: BX values of x by GK of k.  KM: element (x, k) at
+ * k * ld + x in memory and [k][x] in shared memory; else x * ld + k and
+ * [x][k]. */
+template <typename T, bool KM, int BX>
+struct GOp
+{
+  static constexpr int S = KM ? (sizeof (T) == 8 ? BX + 4 : BX + 8) : GK + 4;
+  static constexpr int ROWS = KM ? GK : BX;
+  static constexpr int ELEMS = ROWS * S;
+
+  template <int CB, int NT>
+  static __device__ __forceinline__ void
+  load (T *sm, const T *g, int64_t ld, int64_t x0, int64_t k0, int64_t xmax,
+        int64_t kmax, int tid)
+  {
+    constexpr int E = CB / (int) sizeof (T);
+    constexpr int CPR = (KM ? BX : GK) / E;       /* copies per row */
+    constexpr int RPP = NT / CPR > 0 ? NT / CPR : 1;
+    static_assert (NT % CPR == 0 && ROWS % RPP == 0, "copy split");
+    const int c = (tid % CPR) * E, r0 = tid / CPR;
+    if constexpr (KM) {
+      const int64_t left = xmax - x0 - c;         /* columns from here on */
+      /* whole fragments past the edge are never read */
+      if (left <= -8) return;
+      const int eb = (int) (left >= E ? E : (left > 0 ? left : 0)) * (int) sizeof (T);
+#pragma unroll
+      for (int r = r0; r < ROWS; r += RPP) {
+        const int64_t k = k0 + r;
+        const int bytes = k < kmax ? eb : 0;
+        cp_async<CB> (sm + r * S + c, bytes ? g + k * ld + x0 + c : g, bytes);
+      }
+    } else {
+      const int64_t left = kmax - k0 - c;
+      const int eb = (int) (left >= E ? E : (left > 0 ? left : 0)) * (int) sizeof (T);
+#pragma unroll
+      for (int r = r0; r < ROWS; r += RPP) {
+        const int64_t x = x0 + r;
+        if (x >= xmax + 8) break;
+        const int bytes = x < xmax ? eb : 0;
+        cp_async<CB> (sm + r * S + c, bytes ? g + x * ld + k0 + c : g, bytes);
+      }
+    }
+  }
+
+  static __device__ __forceinline__ double
+  frag (const T *sm, int x, int k)
+  {
+    return (double) sm[KM ? k * S + x : x * S + k];
+  }
+};
+
+/* acc += the product over k in [k0, k1) of the CTA's tile: BM x 64 output
+ * values, BM / 16 warps.  ma, nb: fragments of this warp that hold output
+ * (warp-uniform).  m8n8k4 f64 fragments: A (8 x 4, row) holds A[lane / 4]
+ * [lane % 4], B (4 x 8, col) holds B[lane % 4][lane / 4], C holds
+ * C[lane / 4][2 (lane % 4) + {0, 1}]. */
+template <typename TA, bool AKM, int CA, typename TB, bool BKM, int CBB, int BM>
+__device__ __forceinline__ void
+gemm_tile (const TA *A, int64_t lda, int64_t i0, int64_t imax, const TB *B,
+           int64_t ldb, int64_t j0, int64_t jmax, int64_t k0, int64_t k1, int ma,
+           int nb, unsigned char *smem, double (&acc)[4][4][2])
+{
+  using OA = GOp<TA, AKM, BM>;
+  using OB = GOp<TB, BKM, GB>;
+  constexpr int NT = BM * 2;
+  constexpr int ABYTES = OA::ELEMS * (int) sizeof (TA);
+  constexpr int SBYTES = ABYTES + OB::ELEMS * (int) sizeof (TB);
+  static_assert (ABYTES % 16 == 0 && SBYTES % 16 == 0, "stage alignment");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = warp >> 1, wn = warp & 1;
+  auto stage = [&] (int st) { return smem + st * SBYTES; };
+  auto fetch = [&] (int st, int64_t k) {
+    unsigned char *p = stage (st);
+    OA::template load<CA, NT> ((TA *) p, A, lda, i0, k, imax, k1, tid);
+    OB::template load<CBB, NT> ((TB *) (p + ABYTES), B, ldb, j0, k, jmax, k1, tid);
+  };
+  const int64_t nk = (k1 - k0 + GK - 1) / GK;
+#pragma unroll
+  for (int q = 0; q < GSTAGES - 1; q++) {
+    if (q < nk) fetch (q, k0 + q * GK);
+    asm volatile ("cp.async.commit_group;" ::: "memory");
+  }
+  int st = 0;
+  for (int64_t q = 0; q < nk; q++) {
+    asm volatile ("cp.async.wait_group %0;" ::"n"(GSTAGES - 2) : "memory");
+    __syncthreads ();
+    const int sn = st + GSTAGES - 1 >= GSTAGES ? st - 1 : st + GSTAGES - 1;
+    if (q + GSTAGES - 1 < nk) fetch (sn, k0 + (q + GSTAGES - 1) * GK);
+    asm volatile ("cp.async.commit_group;" ::: "memory");
+    const TA *As = (const TA *) stage (st);
+    const TB *Bs = (const TB *) (stage (st) + ABYTES);
+    if (ma > 0 && nb > 0) {
+#pragma unroll
+      for (int kk = 0; kk < GK; kk += 4) {
+        double a[4], b[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          a[t] = t < ma ? OA::frag (As, wm * 32 + t * 8 + (lane >> 2), kk + (lane & 3)) : 0.;
+          b[t] = t < nb ? OB::frag (Bs, wn * 32 + t * 8 + (lane >> 2), kk + (lane & 3)) : 0.;
+        }
+#pragma unroll
+        for (int ti = 0; ti < 4; ti++)
+          if (ti < ma)
+#pragma unroll
+            for (int tj = 0; tj < 4; tj++)
+              if (tj < nb)
+                asm volatile ("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
+                              "{%0, %1}, {%2}, {%3}, {%0, %1};"
+                              : "+d"(acc[ti][tj][0]), "+d"(acc[ti][tj][1])
+                              : "d"(a[ti]), "d"(b[tj]));
+      }
+    }
+    st = st + 1 == GSTAGES ? 0 : st + 1;
+  }
+  asm volatile ("cp.async.wait_group 0;" ::: "memory");
+}
+
+template <typename TA, bool AKM, typename TB, bool BKM, int BM>
+constexpr int
+gemm_smem ()
+{
+  return GSTAGES * (GOp<TA, AKM, BM>::ELEMS * (int) sizeof (TA)
+                    + GOp<TB, BKM, GB>::ELEMS * (int) sizeof (TB));
+}
+
+/* fragments of a warp's 32 values from x that lie below xmax */
+__device__ __forceinline__ int
+gemm_frags (int64_t x, int64_t xmax)
+{
+  return xmax <= x ? 0 : (int) (xmax - x >= 32 ? 4 : (xmax - x + 7) / 8);
+}
+
+__device__ __forceinline__ void
+gemm_zero (double (&acc)[4][4][2])
 {
 #pragma unroll
-  for (int kk = 0; kk < GK; kk += 4) {
-    double a[4], b[4];
+  for (int a = 0; a < 4; a++)
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      a[t] = As[kk + (lane & 3)][wm * 32 + t * 8 + (lane >> 2)];
-      b[t] = Bs[kk + (lane & 3)][wn * 32 + t * 8 + (lane >> 2)];
-    }
-#pragma unroll
-    for (int ti = 0; ti < 4; ti++)
-#pragma unroll
-      for (int tj = 0; tj < 4; tj++)
-        asm volatile ("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
-                      "{%0, %1}, {%2}, {%3}, {%0, %1};"
-                      : "+d"(acc[ti][tj][0]), "+d"(acc[ti][tj][1])
-                      : "d"(a[ti]), "d"(b[tj]));
-  }
+    for (int b = 0; b < 4; b++) acc[a][b][0] = acc[a][b][1] = 0.;
 }
 
 /* the C element of acc[ti][tj][c] inside the CTA tile */
@@ -75,51 +214,67 @@ dmma_col (int wn, int tj, int c, int lane)
   return wn * 32 + tj * 8 + (lane & 3) * 2 + c;
 }
 
-/* partial C = A^T B over rows [kb0, kb1) of row-major A (n x m1), B
- * (n x m2), into work[z] (column-major m1 x m2) */
+/* bytes per copy that an operand's base and leading dimension allow */
 template <typename T>
-__global__ void __launch_bounds__ (128)
+static int
+copy_bytes (const T *p, int64_t ld)
+{
+  const uintptr_t a = (uintptr_t) p;
+  const size_t l = (size_t) ld * sizeof (T);
+  if (a % 16 == 0 && l % 16 == 0) return 16;
+  if (sizeof (T) == 8 || (a % 8 == 0 && l % 8 == 0)) return 8;
+  return 4;
+}
+
+/* opt kernel k into its dynamic shared memory (above 48 KB), once */
+template <typename K>
+static int
+gemm_smem_attr (K k, int bytes)
+{
+  static std::mutex mu;
+  static std::set<const void *> done;
+  std::lock_guard<std::mutex> lk (mu);
+  if (done.count ((const void *) k)) return 0;
+  LGH_CUDA (cudaFuncSetAttribute ((const void *) k,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  bytes));
+  done.insert ((const void *) k);
+  return 0;
+}
+
+/* partial C = A^T B over rows [kb0, kb1) of row-major A (n x m1), B
+ * (n x m2), into work[z] (column-major m1 x m2).  sym (A = B): blockIdx.x
+ * counts the tiles on and above the diagonal, column by column. */
+template <typename T, int CA, int CB>
+__global__ void __launch_bounds__ (128, 4)
 k_gemm_tn_part (int64_t n, int m1, int m2, const T *__restrict__ A, int lda,
                 const T *__restrict__ B, int ldb, double *__restrict__ work,
-                int64_t kchunk)
+                int64_t kchunk, int sym)
 {
-  __shared__ double As[GK][SLD], Bs[GK][SLD];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  extern __shared__ __align__ (16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = warp >> 1, wn = warp & 1;
-  const int i0 = blockIdx.x * GB, j0 = blockIdx.y * GB;
-  const int64_t kb0 = (int64_t) blockIdx.z * kchunk;
-  int64_t kb1 = kb0 + kchunk;
-  if (kb1 > n) kb1 = n;
-  double acc[4][4][2];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b][0] = acc[a][b][1] = 0.;
-  /* staging: thread -> k row (tid / 8), 8 consecutive columns */
-  const int lk = tid >> 3, lc = (tid & 7) * 8;
-  double ra[8], rb[8];
-  auto fetch = [&] (int64_t k0) {
-    const int64_t kr = k0 + lk;
-    const bool rin = kr < kb1;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      const int ci = i0 + lc + e, cj = j0 + lc + e;
-      ra[e] = (rin && ci < m1) ? (double) A[kr * lda + ci] : 0.;
-      rb[e] = (rin && cj < m2) ? (double) B[kr * ldb + cj] : 0.;
-    }
-  };
-  if (kb0 < kb1) fetch (kb0);
-  for (int64_t k0 = kb0; k0 < kb1; k0 += GK) {
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      As[lk][lc + e] = ra[e];
-      Bs[lk][lc + e] = rb[e];
-    }
-    __syncthreads ();
-    if (k0 + GK < kb1) fetch (k0 + GK);   /* next stage behind the mma */
-    dmma_block (As, Bs, wm, wn, lane, acc);
-    __syncthreads ();
+  int ti0, tj0;
+  if (sym) {
+    tj0 = 0;
+    int t = blockIdx.x;
+    while (t > tj0) t -= ++tj0;
+    ti0 = t;
+  } else {
+    const int tm = (m1 + GB - 1) / GB;
+    tj0 = blockIdx.x / tm;
+    ti0 = blockIdx.x - tj0 * tm;
   }
+  const int i0 = ti0 * GB, j0 = tj0 * GB;
+  const int64_t kb0 = (int64_t) blockIdx.z * kchunk;
+  const int64_t kb1 = kb0 + kchunk < n ? kb0 + kchunk : n;
+  double acc[4][4][2];
+  gemm_zero (acc);
+  int ma = gemm_frags (i0 + wm * 32, m1), nb = gemm_frags (j0 + wn * 32, m2);
+  if (sym && i0 + wm * 32 > j0 + wn * 32) ma = 0;   /* below the diagonal */
+  if (kb0 < kb1)
+    gemm_tile<T, true, CA, T, true, CB, GB> (A, lda, i0, m1, B, ldb, j0, m2,
+                                             kb0, kb1, ma, nb, smem, acc);
   double *wz = work + (size_t) blockIdx.z * m1 * m2;
 #pragma unroll
   for (int ti = 0; ti < 4; ti++)
@@ -128,37 +283,43 @@ k_gemm_tn_part (int64_t n, int m1, int m2, const T *__restrict__ A, int lda,
 #pragma unroll
       for (int c = 0; c < 2; c++) {
         const int i = i0 + dmma_row (wm, ti, lane), j = j0 + dmma_col (wn, tj, c, lane);
-        if (i < m1 && j < m2) wz[i + (size_t) j * m1] = acc[ti][tj][c];
+        if (i < m1 && j < m2 && (!sym || i <= j)) wz[i + (size_t) j * m1] = acc[ti][tj][c];
       }
 }
 
+/* C = the sum of the slices in slice order; upper: the slices hold the
+ * entries on and above the diagonal of a symmetric product */
 __global__ void
 k_gemm_tn_reduce (int m1, int m2, int nsplit, const double *__restrict__ work,
-                  double *C, int ldc, int sym)
+                  double *C, int ldc, int sym, int upper)
 {
   const int64_t total = (int64_t) m1 * m2;
+  auto sum = [&] (int64_t e) {
+    double s[4] = { 0., 0., 0., 0. };
+    for (int z = 0; z < nsplit; z += 4)
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (z + q < nsplit) s[q] += work[(size_t) (z + q) * total + e];
+    return (s[0] + s[1]) + (s[2] + s[3]);
+  };
   for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (int64_t) gridDim.x * blockDim.x) {
     const int i = (int) (e % m1), j = (int) (e / m1);
-    double s = 0.;
-    for (int z = 0; z < nsplit; z++) s += work[(size_t) z * total + e];
-    if (sym) {
-      double s2 = 0.;
-      const int64_t et = (int64_t) j + (int64_t) i * m1;
-      for (int z = 0; z < nsplit; z++) s2 += work[(size_t) z * total + et];
-      s = 0.5 * (s + s2);
-    }
+    if (upper && i > j) continue;
+    double s = sum (e);
+    if (sym && !upper) s = 0.5 * (s + sum ((int64_t) j + (int64_t) i * m1));
     C[i + (size_t) j * ldc] = s;
+    if (upper) C[j + (size_t) i * ldc] = s;
   }
 }
 
 static int
 tn_splits (int64_t n, int m1, int m2)
 {
-  /* about 4 resident 4-warp CTAs per SM over all tiles and slices (the
-   * bound of gemm_tn_work_max follows this rule) */
+  /* one wave of 4 resident 4-warp CTAs per SM over all tiles and slices
+   * (gemm_tn_work_max follows this rule) */
   const int tiles = ((m1 + GB - 1) / GB) * ((m2 + GB - 1) / GB);
-  int want = (4 * num_sms () + tiles - 1) / tiles;
+  int want = 4 * num_sms () / tiles;
   int64_t maxs = (n + 255) / 256;
   if (want > maxs) want = (int) maxs;
   if (want < 1) want = 1;
@@ -182,6 +343,39 @@ gemm_tn_work_max (int m1max, int m2max)
   return (4 * (size_t) num_sms () + tmax) * GB * GB;
 }
 
+/* nsplit slices (their partial tiles in work), then the sum */
+template <typename T>
+static int
+gemm_tn_run (int64_t n, int m1, int m2, const T *A, int lda, const T *B, int ldb,
+             double *C, int ldc, int sym, double *work, int nsplit, bool upper,
+             cudaStream_t s)
+{
+  int64_t kchunk = (n + nsplit - 1) / nsplit;
+  kchunk = (kchunk + GK - 1) / GK * GK;
+  const int tm = (m1 + GB - 1) / GB, tn = (m2 + GB - 1) / GB;
+  dim3 grid ((unsigned) (upper ? tm * (tm + 1) / 2 : tm * tn), 1, (unsigned) nsplit);
+  constexpr int smem = gemm_smem<T, true, T, true, GB> ();
+  auto run = [&] (auto ca, auto cb) -> int {
+    auto k = k_gemm_tn_part<T, decltype (ca)::value, decltype (cb)::value>;
+    LGH_TRY (gemm_smem_attr (k, smem));
+    k<<<grid, 128, smem, s>>> (n, m1, m2, A, lda, B, ldb, work, kchunk, upper);
+    LGH_LAUNCH_CHECK ();
+    return 0;
+  };
+  using C16 = std::integral_constant<int, 16>;
+  using CS = std::integral_constant<int, sizeof (T)>;
+  const bool a16 = copy_bytes (A, lda) == 16, b16 = copy_bytes (B, ldb) == 16;
+  if (a16 && b16) LGH_TRY (run (C16 (), C16 ()));
+  else if (a16) LGH_TRY (run (C16 (), CS ()));
+  else if (b16) LGH_TRY (run (CS (), C16 ()));
+  else LGH_TRY (run (CS (), CS ()));
+  const int64_t total = (int64_t) m1 * m2;
+  int rg = (int) std::min<int64_t> ((total + 255) / 256, num_sms () * 8);
+  k_gemm_tn_reduce<<<rg, 256, 0, s>>> (m1, m2, nsplit, work, C, ldc, sym, upper);
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
 template <typename T>
 int
 launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
@@ -190,20 +384,20 @@ launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
 {
   if (m1 == 0 || m2 == 0) return 0;
   LGH_CHECK (!sym || m1 == m2, LGH_ERR_ARG_SIZ, "gemm_tn: sym needs square");
-  const int ns = tn_splits (n, m1, m2);
+  int ns = tn_splits (n, m1, m2);
   LGH_CHECK ((size_t) ns * m1 * m2 <= work_elems, LGH_ERR_ARG_SIZ,
              "gemm_tn: workspace too small");
-  int64_t kchunk = (n + ns - 1) / ns;
-  kchunk = (kchunk + GK - 1) / GK * GK;
-  dim3 grid ((m1 + GB - 1) / GB, (m2 + GB - 1) / GB, ns);
-  k_gemm_tn_part<T><<<grid, 128, 0, s>>> (n, m1, m2, A, lda, B, ldb, work,
-                                          kchunk);
-  LGH_LAUNCH_CHECK ();
-  const int64_t total = (int64_t) m1 * m2;
-  int rg = (int) std::min<int64_t> ((total + 255) / 256, num_sms () * 8);
-  k_gemm_tn_reduce<<<rg, 256, 0, s>>> (m1, m2, ns, work, C, ldc, sym);
-  LGH_LAUNCH_CHECK ();
-  return 0;
+  /* X^T X: its upper tiles alone, over as many more slices as fit */
+  const bool upper = (const void *) A == (const void *) B && lda == ldb && m1 == m2;
+  if (upper) {
+    const int tm = (m1 + GB - 1) / GB;
+    const int64_t want = std::max (1, 4 * num_sms () / (tm * (tm + 1) / 2));
+    ns = (int) std::min<int64_t> (std::min<int64_t> (want, 256),
+                                  std::min<int64_t> ((n + 255) / 256,
+                                                     (int64_t) (work_elems / ((size_t) m1 * m2))));
+    ns = std::max (ns, 1);
+  }
+  return gemm_tn_run<T> (n, m1, m2, A, lda, B, ldb, C, ldc, sym, work, ns, upper, s);
 }
 
 /* the same product with an explicit split count and caller-provided
@@ -215,17 +409,8 @@ launch_gemm_tn_fixed (int64_t n, int m1, int m2, const double *A, int lda,
 {
   if (m1 == 0 || m2 == 0) return 0;
   if (nsplit < 1) nsplit = 1;
-  int64_t kchunk = (n + nsplit - 1) / nsplit;
-  kchunk = (kchunk + GK - 1) / GK * GK;
-  dim3 grid ((m1 + GB - 1) / GB, (m2 + GB - 1) / GB, nsplit);
-  k_gemm_tn_part<double><<<grid, 128, 0, s>>> (n, m1, m2, A, lda, B, ldb,
-                                               work, kchunk);
-  LGH_LAUNCH_CHECK ();
-  const int64_t total = (int64_t) m1 * m2;
-  int rg = (int) std::min<int64_t> ((total + 255) / 256, num_sms () * 8);
-  k_gemm_tn_reduce<<<rg, 256, 0, s>>> (m1, m2, nsplit, work, C, ldc, 0);
-  LGH_LAUNCH_CHECK ();
-  return 0;
+  return gemm_tn_run<double> (n, m1, m2, A, lda, B, ldb, C, ldc, 0, work, nsplit,
+                              A == B && lda == ldb && m1 == m2, s);
 }
 
 int
@@ -241,48 +426,26 @@ template int launch_gemm_tn<float> (int64_t, int, int, const float *, int,
                                     const float *, int, double *, int, int,
                                     double *, size_t, cudaStream_t);
 
-/* Y = alpha X M + beta Y0: X row-major n x k, M column-major k x m2 */
-template <typename T>
-__global__ void __launch_bounds__ (128)
+/* Y = alpha X M + beta Y0: X row-major n x k, M column-major k x m2.
+ * Column tiles run fastest, so the CTAs resident at once share a band of X
+ * rows in L2 (rows fastest read X from HBM once per column tile). */
+template <typename T, int CA, int CB>
+__global__ void __launch_bounds__ (128, 3)
 k_gemm_nn (int64_t n, int k, int m2, double alpha, const T *__restrict__ X,
            int ldx, const double *__restrict__ M, int ldm, double beta,
-           const T *Y0, int ldy0, T *Y, int ldy)
+           const T *Y0, int ldy0, T *Y, int ldy, int tn)
 {
-  __shared__ double As[GK][SLD], Bs[GK][SLD];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  extern __shared__ __align__ (16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = warp >> 1, wn = warp & 1;
-  const int64_t i0 = (int64_t) blockIdx.x * GB;
-  const int j0 = blockIdx.y * GB;
+  const int64_t rt = blockIdx.x / tn;
+  const int64_t i0 = rt * GB;
+  const int j0 = (int) (blockIdx.x - rt * tn) * GB;
   double acc[4][4][2];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b][0] = acc[a][b][1] = 0.;
-  /* staging: thread -> tile row / column (tid / 2), 8 consecutive k */
-  const int lr = tid >> 1, lk = (tid & 1) * 8;
-  double ra[8], rb[8];
-  auto fetch = [&] (int k0) {
-    const int64_t gi = i0 + lr;
-    const int gj = j0 + lr;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      const int kk = k0 + lk + e;
-      ra[e] = (gi < n && kk < k) ? (double) X[gi * ldx + kk] : 0.;
-      rb[e] = (gj < m2 && kk < k) ? M[kk + (size_t) gj * ldm] : 0.;
-    }
-  };
-  if (k > 0) fetch (0);
-  for (int k0 = 0; k0 < k; k0 += GK) {
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      As[lk + e][lr] = ra[e];
-      Bs[lk + e][lr] = rb[e];
-    }
-    __syncthreads ();
-    if (k0 + GK < k) fetch (k0 + GK);
-    dmma_block (As, Bs, wm, wn, lane, acc);
-    __syncthreads ();
-  }
+  gemm_zero (acc);
+  gemm_tile<T, false, CA, double, false, CB, GB> (
+      X, ldx, i0, n, M, ldm, j0, m2, 0, k, gemm_frags (i0 + wm * 32, n),
+      gemm_frags (j0 + wn * 32, m2), smem, acc);
 #pragma unroll
   for (int ti = 0; ti < 4; ti++)
 #pragma unroll
@@ -302,91 +465,33 @@ k_gemm_nn (int64_t n, int k, int m2, double alpha, const T *__restrict__ X,
 /* The Woodbury combination of many shifts in one launch (the batched
  * solve / sample of the shift-independent form x_c = f(c) y0 + W D_c U^T r,
  * glr_common_impl.h:910-929 applied per shift):
- *   out[:, J] = fc[si] Y0[:, j] + W (g[si, :] .* C[:, j]),  J = si m + j,
- * W n x kept row-major (the shift-independent W = Z^{-1} M^{1/2} U), C
- * kept x m column-major (U^T r), g kept x nshift column-major (g[k, si] =
- * f(lam_k + c_si) - f(c_si)), Y0 n x m row-major, out column-major with
- * leading dimension *ldo at *out (the output pointer is read from device
- * memory so that a captured graph serves every call).  One GEMM of n x
- * (nshift m) x kept on the FP64 tensor cores: the shift coefficient is
- * folded into the staging of the B operand, and the epilogue adds f(c) y0
- * and writes the caller's column-major result directly.  Column tiles run
- * fastest, so the CTAs resident at once share a band of W rows in L2. */
-/* one staged k block of a BM-row A tile (row stride BM + 4) */
-template <int BM>
-__device__ __forceinline__ void
-dmma_block_rows (const double (*As)[BM + 4], const double (*Bs)[SLD], int wm,
-                 int wn, int lane, double (&acc)[4][4][2])
-{
-#pragma unroll
-  for (int kk = 0; kk < GK; kk += 4) {
-    double a[4], b[4];
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-      a[t] = As[kk + (lane & 3)][wm * 32 + t * 8 + (lane >> 2)];
-      b[t] = Bs[kk + (lane & 3)][wn * 32 + t * 8 + (lane >> 2)];
-    }
-#pragma unroll
-    for (int ti = 0; ti < 4; ti++)
-#pragma unroll
-      for (int tj = 0; tj < 4; tj++)
-        asm volatile ("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
-                      "{%0, %1}, {%2}, {%3}, {%0, %1};"
-                      : "+d"(acc[ti][tj][0]), "+d"(acc[ti][tj][1])
-                      : "d"(a[ti]), "d"(b[tj]));
-  }
-}
-
-/* BM = 64 (4 warps, 2 x 2 quarters of 32 x 32) or 128 (8 warps, 4 x 2) */
-template <typename T, int BM>
-__global__ void __launch_bounds__ (BM * 2)
-k_shift_combine (int64_t n, int kept, int m, int nshift,
-                 const T *__restrict__ W, int ldw, const double *__restrict__ C,
-                 const double *__restrict__ g, const double *__restrict__ fc,
-                 const T *__restrict__ Y0, int ldy0,
+ *   out[:, J] = fc[si] Y0[:, j] + W S[:, J],  J = si m + j,
+ * W n x kept row-major (the shift-independent W = Z^{-1} M^{1/2} U), S kept
+ * x (nshift m) column-major (k_shift_scale: g[:, si] .* (U^T r)[:, j] with
+ * g[k, si] = f(lam_k + c_si) - f(c_si)), Y0 n x m row-major, out
+ * column-major with leading dimension *ldo at *out (the output pointer is
+ * read from device memory so that a captured graph serves every call).
+ * One GEMM on the FP64 tensor cores, whose epilogue adds f(c) y0 and writes
+ * the caller's column-major result.  Column tiles run fastest, so the CTAs
+ * resident at once share a band of W rows in L2. */
+template <int BM, int CA, int CB>
+__global__ void __launch_bounds__ (BM * 2, BM == 128 ? 2 : 3)
+k_shift_combine (int64_t n, int kept, int m, int ncol,
+                 const double *__restrict__ W, int ldw,
+                 const double *__restrict__ S, const double *__restrict__ fc,
+                 const double *__restrict__ Y0, int ldy0,
                  double *const *__restrict__ out, const int64_t *__restrict__ ldo)
 {
-  __shared__ double As[GK][BM + 4], Bs[GK][SLD];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  extern __shared__ __align__ (16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = warp >> 1, wn = warp & 1;
-  const int ncol = nshift * m;
   const int64_t i0 = (int64_t) blockIdx.y * BM;
   const int j0 = blockIdx.x * GB;
   double acc[4][4][2];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b][0] = acc[a][b][1] = 0.;
-  /* staging: thread -> A tile row tid / 2 (all threads) and B tile column
-   * tid / 2 (the first 128 threads), 8 consecutive k each */
-  const int lr = tid >> 1, lk = (tid & 1) * 8;
-  const bool bthr = lr < GB;
-  const int Jr = j0 + lr;
-  const bool bcol = bthr && Jr < ncol;
-  const int sr = bcol ? Jr / m : 0, jr = bcol ? Jr - sr * m : 0;
-  double ra[8], rb[8];
-  auto fetch = [&] (int k0) {
-    const int64_t gi = i0 + lr;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      const int kk = k0 + lk + e;
-      ra[e] = (gi < n && kk < kept) ? (double) W[gi * ldw + kk] : 0.;
-      rb[e] = (bcol && kk < kept)
-              ? g[kk + (size_t) sr * kept] * C[kk + (size_t) jr * kept] : 0.;
-    }
-  };
-  if (kept > 0) fetch (0);
-  for (int k0 = 0; k0 < kept; k0 += GK) {
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      As[lk + e][lr] = ra[e];
-      if (bthr) Bs[lk + e][lr] = rb[e];
-    }
-    __syncthreads ();
-    if (k0 + GK < kept) fetch (k0 + GK);
-    dmma_block_rows<BM> (As, Bs, wm, wn, lane, acc);
-    __syncthreads ();
-  }
+  gemm_zero (acc);
+  gemm_tile<double, false, CA, double, false, CB, BM> (
+      W, ldw, i0, n, S, kept, j0, ncol, 0, kept, gemm_frags (i0 + wm * 32, n),
+      gemm_frags (j0 + wn * 32, ncol), smem, acc);
   double *const o = *out;
   const int64_t ld = *ldo;
 #pragma unroll
@@ -401,15 +506,33 @@ k_shift_combine (int64_t n, int kept, int m, int nshift,
       for (int ti = 0; ti < 4; ti++) {
         const int64_t i = i0 + dmma_row (wm, ti, lane);
         if (i < n)
-          o[i + (int64_t) J * ld] = acc[ti][tj][c] + f * (double) Y0[i * ldy0 + j];
+          o[i + (int64_t) J * ld] = acc[ti][tj][c] + f * Y0[i * ldy0 + j];
       }
     }
 }
 
+/* S[k + J kept] = g[k, si] C[k, j], J = si m + j */
+__global__ void
+k_shift_scale (int kept, int m, int64_t ncol, const double *__restrict__ C,
+               const double *__restrict__ g, double *__restrict__ S)
+{
+  const int64_t total = (int64_t) kept * ncol;
+  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (int64_t) gridDim.x * blockDim.x) {
+    const int64_t J = e / kept;
+    const int k = (int) (e - J * kept);
+    const int64_t si = J / m;
+    S[e] = g[k + si * kept] * C[k + (J - si * m) * kept];
+  }
+}
+
+/* 128-row tiles (8 warps) or 64-row tiles (4 warps), as the autotuner picks
+ * (262144 rows x 200 kept, 16 shifts x 96 columns: 8.5 ms with the scalar
+ * staging, 18.9 TFLOP/s) */
 int
 launch_shift_combine_variant (int variant, int64_t n, int kept, int m,
                               int nshift, const double *W, int ldw,
-                              const double *C, const double *g,
+                              const double *C, const double *g, double *S,
                               const double *fc, const double *Y0, int ldy0,
                               double *const *out, const int64_t *ldo,
                               cudaStream_t s)
@@ -421,15 +544,33 @@ launch_shift_combine_variant (int variant, int64_t n, int kept, int m,
   LGH_CHECK (ncol < INT32_MAX && rt < 65536, LGH_ERR_ARG_OUTOFRANGE,
              "shift combine: %lld rows x %lld columns exceed the grid",
              (long long) n, (long long) ncol);
+  if (kept > 0) {
+    const int sg = (int) std::min<int64_t> (((int64_t) kept * ncol + 255) / 256,
+                                            num_sms () * 8);
+    k_shift_scale<<<sg, 256, 0, s>>> (kept, m, ncol, C, g, S);
+    LGH_LAUNCH_CHECK ();
+  }
   dim3 grid ((unsigned) ((ncol + GB - 1) / GB), (unsigned) rt);
+  auto run = [&] (auto bm, auto cb) -> int {
+    constexpr int BM_ = decltype (bm)::value;
+    constexpr int smem = gemm_smem<double, false, double, false, BM_> ();
+    /* W's rows are padded to 4 values at a 256-byte base */
+    auto k = k_shift_combine<BM_, 16, decltype (cb)::value>;
+    LGH_TRY (gemm_smem_attr (k, smem));
+    k<<<grid, BM_ * 2, smem, s>>> (n, kept, m, (int) ncol, W, ldw, S, fc, Y0,
+                                   ldy0, out, ldo);
+    LGH_LAUNCH_CHECK ();
+    return 0;
+  };
+  LGH_CHECK (kept == 0 || copy_bytes (W, ldw) == 16, LGH_ERR_ARG_WRONG,
+             "shift combine: W must be 16-byte aligned");
+  using std::integral_constant;
+  const bool b16 = copy_bytes (S, kept) == 16;
   if (variant == 1)
-    k_shift_combine<double, 128><<<grid, 256, 0, s>>> (
-        n, kept, m, nshift, W, ldw, C, g, fc, Y0, ldy0, out, ldo);
-  else
-    k_shift_combine<double, 64><<<grid, 128, 0, s>>> (
-        n, kept, m, nshift, W, ldw, C, g, fc, Y0, ldy0, out, ldo);
-  LGH_LAUNCH_CHECK ();
-  return 0;
+    return b16 ? run (integral_constant<int, 128> (), integral_constant<int, 16> ())
+               : run (integral_constant<int, 128> (), integral_constant<int, 8> ());
+  return b16 ? run (integral_constant<int, 64> (), integral_constant<int, 16> ())
+             : run (integral_constant<int, 64> (), integral_constant<int, 8> ());
 }
 
 /* Y = A^{-1} B on the dense coarse level: A^{-1} n0 x n0 column-major (and
@@ -542,11 +683,24 @@ launch_gemm_nn (int64_t n, int k, int m2, double alpha, const T *X, int ldx,
                 T *Y, int ldy, cudaStream_t s)
 {
   if (n == 0 || m2 == 0) return 0;
-  dim3 grid ((unsigned) ((n + GB - 1) / GB), (unsigned) ((m2 + GB - 1) / GB));
-  k_gemm_nn<T><<<grid, 128, 0, s>>> (n, k, m2, alpha, X, ldx, M, ldm, beta,
-                                     Y0, ldy0, Y, ldy);
-  LGH_LAUNCH_CHECK ();
-  return 0;
+  const int tn = (m2 + GB - 1) / GB;
+  const int64_t tiles = (n + GB - 1) / GB * tn;
+  LGH_CHECK (tiles < INT32_MAX, LGH_ERR_ARG_OUTOFRANGE, "gemm_nn: too many tiles");
+  constexpr int smem = gemm_smem<T, false, double, false, GB> ();
+  auto run = [&] (auto ca, auto cb) -> int {
+    auto f = k_gemm_nn<T, decltype (ca)::value, decltype (cb)::value>;
+    LGH_TRY (gemm_smem_attr (f, smem));
+    f<<<(unsigned) tiles, 128, smem, s>>> (n, k, m2, alpha, X, ldx, M, ldm, beta,
+                                           Y0, ldy0, Y, ldy, tn);
+    LGH_LAUNCH_CHECK ();
+    return 0;
+  };
+  using C16 = std::integral_constant<int, 16>;
+  using CT = std::integral_constant<int, sizeof (T)>;
+  using C8 = std::integral_constant<int, 8>;
+  const bool a16 = copy_bytes (X, ldx) == 16, b16 = copy_bytes (M, ldm) == 16;
+  if (a16) return b16 ? run (C16 (), C16 ()) : run (C16 (), C8 ());
+  return b16 ? run (CT (), C16 ()) : run (CT (), C8 ());
 }
 
 template int launch_gemm_nn<double> (int64_t, int, int, double,

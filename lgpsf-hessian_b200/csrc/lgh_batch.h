@@ -51,9 +51,10 @@ constexpr int kUmmaVariants = 4;
 /* tcgen05 variant u = variant - kShiftVariants: tile width and stages */
 inline int umma_variant_tn (int u) { return (u & 1) ? 256 : 128; }
 inline int umma_variant_stages (int u) { return u >= 2 ? 1 : 2; }
+/* S: kept x (nshift m) scratch for the scaled coefficient block */
 int launch_shift_combine_variant (int variant, int64_t n, int kept, int m,
                                   int nshift, const double *W, int ldw,
-                                  const double *C, const double *g,
+                                  const double *C, const double *g, double *S,
                                   const double *fc, const double *Y0,
                                   int ldy0, double *const *out,
                                   const int64_t *ldo, cudaStream_t s);
