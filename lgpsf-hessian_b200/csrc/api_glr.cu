@@ -161,7 +161,7 @@ sgrid (int64_t total)
 struct Small
 {
   int n = 0;
-  DBuf<double> G, G0, M, T, A2, V, V2, w, C, work, sel, lam;
+  DBuf<double> G, G0, M, T, V, w, C, work, sel, lam;
   DBuf<int> order, info;
   int alloc (int n_, int64_t rows, int maxw)
   {
@@ -171,9 +171,7 @@ struct Small
     LGH_TRY (G0.alloc (nn));
     LGH_TRY (M.alloc (nn));
     LGH_TRY (T.alloc (nn));
-    LGH_TRY (A2.alloc (nn));
     LGH_TRY (V.alloc (nn));
-    LGH_TRY (V2.alloc (nn));
     LGH_TRY (w.alloc (n));
     LGH_TRY (C.alloc (nn));
     /* split-K workspace: enough for every (m1, m2) <= (maxw, maxw) shape */
@@ -308,8 +306,7 @@ rayleigh_ritz (lgh_glr_t *g, int ell, const T *Q, int ldq, const double *Araw,
   k_symmetrize<<<sgrid ((int64_t) ell * ell), 256, 0, s>>> (ell, Araw, sm.T.p);
   LGH_LAUNCH_CHECK ();
   int sweeps = 0;
-  LGH_TRY (launch_syev_jacobi (ell, sm.T.p, sm.V.p, sm.w.p, sm.A2.p, sm.V2.p,
-                               &sweeps, s));
+  LGH_TRY (launch_syev_jacobi (ell, sm.T.p, sm.V.p, sm.w.p, &sweeps, s));
   LGH_TRY (launch_select (ell, sm.w.p, sm.V.p, g->opts.trunc_abs,
                           g->opts.trunc_rel, (int) g->opts.treat, sm.order.p,
                           sm.sel.p, sm.lam.p, sm.C.p, s));

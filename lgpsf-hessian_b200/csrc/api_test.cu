@@ -318,14 +318,11 @@ int
 lgh_test_syev (int n, const double *A, double *w, double *V, int *sweeps)
 {
   LGH_TRY (ensure_init ());
-  DBuf<double> da, da2, dv, dv2, dw;
+  DBuf<double> da, dv, dw;
   LGH_TRY (up (da, A, (size_t) n * n));
-  LGH_TRY (da2.alloc ((size_t) n * n));
   LGH_TRY (dv.alloc ((size_t) n * n));
-  LGH_TRY (dv2.alloc ((size_t) n * n));
   LGH_TRY (dw.alloc (n));
-  LGH_TRY (launch_syev_jacobi (n, da.p, dv.p, dw.p, da2.p, dv2.p, sweeps,
-                               stream ()));
+  LGH_TRY (launch_syev_jacobi (n, da.p, dv.p, dw.p, sweeps, stream ()));
   LGH_TRY (down (w, dw, n));
   return down (V, dv, (size_t) n * n);
 }

@@ -219,7 +219,7 @@ upload_idx (const std::vector<int> &h, DBuf<int> &d)
  * solver's order (index i of vals is column i of vecs) */
 struct SmallEig
 {
-  DBuf<double> a, a2, vecs, v2, w;
+  DBuf<double> a, vecs, w;
   std::vector<double> vals;
   int n = 0;
   int run (int n_, const double *A)
@@ -230,13 +230,11 @@ struct SmallEig
     const size_t nn = (size_t) n * n;
     cudaStream_t s = stream ();
     LGH_TRY (a.alloc (nn));
-    LGH_TRY (a2.alloc (nn));
     LGH_TRY (vecs.alloc (nn));
-    LGH_TRY (v2.alloc (nn));
     LGH_TRY (w.alloc (n));
     LGH_CUDA (cudaMemcpyAsync (a.p, A, nn * sizeof (double),
                                cudaMemcpyDeviceToDevice, s));
-    LGH_TRY (launch_syev_jacobi (n, a.p, vecs.p, w.p, a2.p, v2.p, nullptr, s));
+    LGH_TRY (launch_syev_jacobi (n, a.p, vecs.p, w.p, nullptr, s));
     LGH_CUDA (cudaMemcpyAsync (vals.data (), w.p, n * sizeof (double),
                                cudaMemcpyDeviceToHost, s));
     LGH_CUDA (cudaStreamSynchronize (s));

@@ -9,19 +9,13 @@
  *           transposed so that X L^{-T} is a plain GEMM (the DTRSM of
  *           glr_common_impl.h:402).
  *   syev    DSYEVD("V","U") of the projected T (glr_common_impl.h:496-514):
- *           cyclic two-sided Jacobi in round-robin parallel order.  One
- *           cooperative launch; every CTA computes all rotations of a round
- *           from the same matrix (so all CTAs agree on convergence without
- *           communication), applies them to its slice of A and V, and meets
- *           the others at a bounded grid barrier.  Relative-accuracy
- *           rotation threshold, at most 40 sweeps.
+ *           cyclic two-sided block Jacobi in round-robin parallel order,
+ *           relative-accuracy rotation threshold, at most 40 sweeps.
  *   select  ordering by |lambda| descending, the cut max(trunc_abs,
  *           trunc_rel max|lambda|), treatment FLIP/RELU/NONE and the report
  *           fields (glr_common_impl.h:517-559; glr_scalapack_impl.h:375-425),
  *           plus the gathered eigenvector columns C_kept.
  */
-
-#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cmath>
@@ -185,188 +179,314 @@ launch_trtri_lower (int n, const double *L, double *Linv, int transpose,
 
 /* ------------------------------------------------------------- jacobi -- */
 
-struct JacobiCtl
-{
-  unsigned count, gen;
-  int err, sweeps;
-};
+/* Block Jacobi: the matrix in blocks of JB rows, paired round-robin.  A
+ * round diagonalises the 2 JB x 2 JB submatrix of every block pair by one
+ * cyclic sweep in shared memory (k_jacobi_pairs, one CTA per pair, the
+ * accumulated rotations W kept) and applies the W's to the rest of A and to
+ * V as small tensor-core products (k_jacobi_apply, one CTA per tile).  A
+ * sweep is nblk - 1 rounds of two launches, 13 at n = 220, where the scalar
+ * ordering needs n - 1 rounds, each with a barrier over the whole grid and
+ * an update of every entry (5.2 us a round, bound by the barrier and the L2
+ * latency behind it: 10.3 ms at n = 220, 2.0 ms at n = 60).  Blocks of 16:
+ * the sweep inside a pair is the longest chain of a round, and a 32 x 32
+ * submatrix is also one tile of the products. */
+constexpr int JB = 16, JT = 2 * JB, JS = JT + 4;   /* block, tile, row stride */
 
 /* index at position `pos` in round r of the round-robin over np entries */
-__device__ __forceinline__ int
+__host__ __device__ __forceinline__ int
 rr_index (int pos, int r, int np)
 {
   return pos == 0 ? 0 : 1 + ((pos - 1 + r) % (np - 1));
 }
 
-__global__ void __launch_bounds__ (256)
-k_jacobi (int n, int np, double *A, double *A2, double *V, double *V2,
-          JacobiCtl *ctl, int max_sweeps)
+/* the matrix index of row i of block pair k in round r (n or more: padding) */
+__device__ __forceinline__ int
+jacobi_row (int i, int k, int r, int nblk)
 {
-  extern __shared__ double sh[];
-  const int npair = np / 2;
-  double *cs = sh;                  /* c per pair    */
-  double *sn = cs + npair;          /* s per pair    */
-  double *tt = sn + npair;          /* t per pair    */
-  int *pp = (int *) (tt + npair);   /* p per pair    */
-  int *qq = pp + npair;             /* q per pair    */
-  int *pr = qq + npair;             /* pair of index */
-  __shared__ int any_rot;
-  const int64_t nn = (int64_t) n * n;
-  const int64_t gtid = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t gstride = (int64_t) gridDim.x * blockDim.x;
-  /* V = I */
-  for (int64_t e = gtid; e < nn; e += gstride)
-    V[e] = ((e % n) == (e / n)) ? 1. : 0.;
-  if (!grid_barrier (&ctl->count, &ctl->gen, &ctl->err)) return;
-  int done = 0;
-  for (int sweep = 0; sweep < max_sweeps; sweep++) {
-    if (threadIdx.x == 0) any_rot = 0;
+  const int b = rr_index (i < JB ? k : nblk - 1 - k, r, nblk);
+  return b * JB + (i & (JB - 1));
+}
+
+/* 2^-e for the exponent e of x (x normal and below 2^1023) */
+__device__ __forceinline__ double
+exponent_scale (double x)
+{
+  const int e = (__double2hiint (x) >> 20) & 0x7ff;
+  return __hiloint2double ((2046 - e) << 20, 0);
+}
+
+/* the rotation that annihilates apq: tan t = s / c with |t| <= 1, from the
+ * double angle, d = aqq - app, b = 2 apq: cos 2a = |d| / r, c^2 = (1 + cos
+ * 2a) / 2, s = b / (2 r c), r^2 = d^2 + b^2.  Two reciprocal square roots
+ * long where t, c from the quotient d / b take three divisions and two
+ * square roots one after the other (a round of k_jacobi_pairs: 1.3 us); both
+ * are scaled by a power of two first, so nothing overflows.  False (no
+ * rotation) below the relative threshold 1e-15 sqrt |app aqq|. */
+__device__ __forceinline__ bool
+jacobi_rotation (double app, double aqq, double apq, double &c, double &s,
+                 double &t)
+{
+  c = 1.;
+  s = t = 0.;
+  if (!(fabs (apq) > 1e-300)) return false;
+  const double f = exponent_scale (apq), x = apq * f;
+  if (!(x * x > 1e-30 * ((fabs (app) * f) * (fabs (aqq) * f)))) return false;
+  double d = aqq - app, b = 2. * apq;
+  const double g = exponent_scale (fmax (fabs (d), fabs (b)));
+  d *= g;
+  b *= g;
+  const double ri = rsqrt (fma (d, d, b * b));
+  const double c2 = fma (0.5 * fabs (d), ri, 0.5);
+  const double ci = rsqrt (c2);
+  c = c2 * ci;
+  s = (d < 0. ? -0.5 : 0.5) * b * ri * ci;
+  t = s * ci;
+  return true;
+}
+
+/* the 2 JB x 2 JB submatrix of each pair: up to `sweeps` cyclic sweeps
+ * (stopping at one without a rotation); the diagonalised submatrix goes back
+ * to A, the rotations to W (row-major), whether there were any to rot[pair],
+ * and any_rot / done (sweeps run) record the round */
+__global__ void __launch_bounds__ (256)
+k_jacobi_pairs (int n, int nblk, int r, int sweeps, double *A, double *Wg,
+                int *rot, int *any_rot, int *done)
+{
+  __shared__ double S[JT][JS], W[JT][JS];
+  __shared__ double cs[JB], sn[JB], tt[JB];
+  __shared__ int pp[JB], qq[JB];
+  __shared__ int rotated, ever;
+  const int tid = threadIdx.x, k = blockIdx.x;
+  for (int e = tid; e < JT * JT; e += 256) {
+    const int i = e % JT, j = e / JT;
+    const int gi = jacobi_row (i, k, r, nblk), gj = jacobi_row (j, k, r, nblk);
+    S[i][j] = (gi < n && gj < n) ? A[gi + (size_t) gj * n] : 0.;
+    W[i][j] = i == j ? 1. : 0.;
+  }
+  if (tid == 0) ever = 0;
+  int sw = 0;
+  for (; sw < sweeps; sw++) {
+    if (tid == 0) rotated = 0;
     __syncthreads ();
-    for (int r = 0; r < np - 1; r++) {
-      for (int k = threadIdx.x; k < npair; k += blockDim.x) {
-        int p = rr_index (k, r, np), q = rr_index (np - 1 - k, r, np);
-        if (p > q) { int t = p; p = q; q = t; }
-        double c = 1., s = 0., t = 0.;
-        if (q < n) {
-          const double apq = A[p + (size_t) q * n];
-          const double app = A[p + (size_t) p * n];
-          const double aqq = A[q + (size_t) q * n];
-          if (fabs (apq) > 1e-300
-              && fabs (apq) > 1e-15 * sqrt (fabs (app) * fabs (aqq))) {
-            const double th = (aqq - app) / (2. * apq);
-            t = (th >= 0. ? 1. : -1.) / (fabs (th) + sqrt (1. + th * th));
-            c = 1. / sqrt (1. + t * t);
-            s = t * c;
-            any_rot = 1;
-          }
-        }
-        cs[k] = c; sn[k] = s; tt[k] = t; pp[k] = p; qq[k] = q;
-        if (p < np) pr[p] = k;
-        if (q < np) pr[q] = k;
+    for (int q = 0; q < JT - 1; q++) {
+      if (tid < JB) {
+        const int a = rr_index (tid, q, JT), b = rr_index (JT - 1 - tid, q, JT);
+        const int pi = a < b ? a : b, qi = a < b ? b : a;
+        double c, s, t;
+        if (jacobi_rotation (S[pi][pi], S[qi][qi], S[pi][qi], c, s, t)) rotated = 1;
+        cs[tid] = c;
+        sn[tid] = s;
+        tt[tid] = t;
+        pp[tid] = pi;
+        qq[tid] = qi;
       }
       __syncthreads ();
-      for (int64_t e = gtid; e < nn; e += gstride) {
-        const int i = (int) (e % n), j = (int) (e / n);
-        const int ki = pr[i], kj = pr[j];
-        /* a pair with the padding index (odd n) never rotates: clamp its
-         * partner to itself so every load stays inside the n x n matrix */
-        const int pi = pp[ki], pj = pp[kj];
-        const int qi = (qq[ki] < n) ? qq[ki] : pi;
-        const int qj = (qq[kj] < n) ? qq[kj] : pj;
-        double v;
-        if (ki == kj && i != j) {
-          /* the annihilated pair (kept as is when the rotation was skipped) */
-          v = (sn[ki] != 0.) ? 0. : A[e];
-        } else if (ki == kj) {
-          const double apq = A[pi + (size_t) qi * n];
-          v = (i == pi) ? A[i + (size_t) i * n] - tt[ki] * apq
-                        : A[i + (size_t) i * n] + tt[ki] * apq;
-        } else {
-          /* weights of rows/cols: index == p -> (c, -s); == q -> (s, c) */
-          const double ci = cs[ki], si = sn[ki], cj = cs[kj], sj = sn[kj];
-          const double wi0 = (i == pi) ? ci : si, wi1 = (i == pi) ? -si : ci;
-          const double wj0 = (j == pj) ? cj : sj, wj1 = (j == pj) ? -sj : cj;
-          const double a00 = A[pi + (size_t) pj * n], a01 = A[pi + (size_t) qj * n];
-          const double a10 = A[qi + (size_t) pj * n], a11 = A[qi + (size_t) qj * n];
-          v = wi0 * (a00 * wj0 + a01 * wj1) + wi1 * (a10 * wj0 + a11 * wj1);
+      {
+        /* one 2 x 2 block of S per thread, a half-warp along one row pair */
+        const int a = tid / JB, b = tid & (JB - 1);
+        const int pa = pp[a], qa = qq[a], pb = pp[b], qb = qq[b];
+        const double ca = cs[a], sa = sn[a], cb = cs[b], sb = sn[b];
+        if (a == b) {
+          if (sa != 0.) {
+            const double apq = S[pa][qa], t = tt[a];
+            S[pa][pa] -= t * apq;
+            S[qa][qa] += t * apq;
+            S[pa][qa] = 0.;
+            S[qa][pa] = 0.;
+          }
+        } else if (sa != 0. || sb != 0.) {
+          const double x00 = S[pa][pb], x01 = S[pa][qb];
+          const double x10 = S[qa][pb], x11 = S[qa][qb];
+          const double y00 = cb * x00 - sb * x01, y01 = sb * x00 + cb * x01;
+          const double y10 = cb * x10 - sb * x11, y11 = sb * x10 + cb * x11;
+          S[pa][pb] = ca * y00 - sa * y10;
+          S[pa][qb] = ca * y01 - sa * y11;
+          S[qa][pb] = sa * y00 + ca * y10;
+          S[qa][qb] = sa * y01 + ca * y11;
         }
-        A2[e] = v;
-        /* V' = V J : column j mixes V(:, pj), V(:, qj) */
-        {
-          const double cj = cs[kj], sj = sn[kj];
-          const double wj0 = (j == pj) ? cj : sj, wj1 = (j == pj) ? -sj : cj;
-          V2[e] = V[i + (size_t) pj * n] * wj0 + V[i + (size_t) qj * n] * wj1;
+        /* two rows of W's columns pb, qb */
+        if (sb != 0.) {
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int i = a + h * JB;
+            const double w0 = W[i][pb], w1 = W[i][qb];
+            W[i][pb] = cb * w0 - sb * w1;
+            W[i][qb] = sb * w0 + cb * w1;
+          }
         }
       }
-      if (!grid_barrier (&ctl->count, &ctl->gen, &ctl->err)) return;
-      { double *t = A; A = A2; A2 = t; }
-      { double *t = V; V = V2; V2 = t; }
+      __syncthreads ();
     }
+    if (!rotated) break;
+    if (tid == 0) ever = 1;
     __syncthreads ();
-    done++;
-    if (!any_rot) break;
   }
-  /* the result sits in whichever buffers the last round wrote; the host
-   * locates it from the number of completed sweeps */
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->sweeps = done;
+  __syncthreads ();
+  if (tid == 0) {
+    rot[k] = ever;
+    if (ever) *any_rot = 1;
+    if (k == 0) *done = sw + 1 < sweeps ? sw + 1 : sweeps;
+  }
+  if (!ever) return;
+  for (int e = tid; e < JT * JT; e += 256) {
+    const int i = e % JT, j = e / JT;
+    const int gi = jacobi_row (i, k, r, nblk), gj = jacobi_row (j, k, r, nblk);
+    if (gi < n && gj < n) A[gi + (size_t) gj * n] = S[i][j];
+    Wg[(size_t) k * JT * JT + e] = W[e / JT][e % JT];
+  }
+}
+
+/* D = op (P) Q for 32 x 32 shared tiles, 8 warps: warp w makes row fragment
+ * w / 2 and column fragments 2 (w % 2) + {0, 1}; TP: P is transposed */
+template <bool TP>
+__device__ __forceinline__ void
+jacobi_mma (const double (*Pm)[JS], const double (*Qm)[JS], double (&acc)[2][2])
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i0 = (warp >> 1) * 8, j0 = (warp & 1) * 16;
+#pragma unroll
+  for (int t = 0; t < 2; t++) acc[t][0] = acc[t][1] = 0.;
+#pragma unroll
+  for (int kk = 0; kk < JT; kk += 4) {
+    const int k = kk + (lane & 3), x = lane >> 2;
+    const double a = TP ? Pm[k][i0 + x] : Pm[i0 + x][k];
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      const double b = Qm[k][j0 + t * 8 + x];
+      asm volatile ("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
+                    "{%0, %1}, {%2}, {%3}, {%0, %1};"
+                    : "+d"(acc[t][0]), "+d"(acc[t][1])
+                    : "d"(a), "d"(b));
+    }
+  }
+}
+
+/* blockIdx.y < npair: tile (x, y) of A, x < y: W_x^T A W_y, with its mirror;
+ * above: 32 rows of V times W_x */
+__global__ void __launch_bounds__ (256)
+k_jacobi_apply (int n, int nblk, int r, double *A, double *V,
+                const double *__restrict__ Wg, const int *__restrict__ rot)
+{
+  __shared__ double T[JT][JS], WP[JT][JS], WQ[JT][JS];
+  const int npair = nblk / 2, tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  const int fi = (warp >> 1) * 8 + (lane >> 2), fj = (warp & 1) * 16 + (lane & 3) * 2;
+  const bool isv = (int) blockIdx.y >= npair;
+  const int kq = isv ? blockIdx.x : blockIdx.y, kp = isv ? 0 : blockIdx.x;
+  const int v0 = isv ? ((int) blockIdx.y - npair) * JT : 0;
+  double acc[2][2];
+  if (isv) {
+    if (!rot[kq]) return;
+  } else if (kp >= kq || (!rot[kp] && !rot[kq])) {
+    return;
+  }
+  for (int e = tid; e < JT * JT; e += 256) {
+    const int i = e % JT, j = e / JT;
+    const int gj = jacobi_row (j, kq, r, nblk);
+    const int gi = isv ? v0 + i : jacobi_row (i, kp, r, nblk);
+    const double *src = isv ? V : A;
+    T[i][j] = (gi < n && gj < n) ? src[gi + (size_t) gj * n] : 0.;
+    const int wi = e / JT, wj = e % JT;
+    WQ[wi][wj] = rot[kq] ? Wg[(size_t) kq * JT * JT + e] : (wi == wj ? 1. : 0.);
+    if (!isv)
+      WP[wi][wj] = rot[kp] ? Wg[(size_t) kp * JT * JT + e] : (wi == wj ? 1. : 0.);
+  }
+  __syncthreads ();
+  jacobi_mma<false> (T, WQ, acc);
+  if (!isv) {
+    __syncthreads ();
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) T[fi][fj + t * 8 + c] = acc[t][c];
+    __syncthreads ();
+    jacobi_mma<true> (WP, T, acc);
+  }
+  __syncthreads ();
+#pragma unroll
+  for (int t = 0; t < 2; t++)
+#pragma unroll
+    for (int c = 0; c < 2; c++) T[fi][fj + t * 8 + c] = acc[t][c];
+  __syncthreads ();
+  for (int e = tid; e < JT * JT; e += 256) {
+    const int i = e % JT, j = e / JT;
+    const int gj = jacobi_row (j, kq, r, nblk);
+    const int gi = isv ? v0 + i : jacobi_row (i, kp, r, nblk);
+    if (gi < n && gj < n) (isv ? V : A)[gi + (size_t) gj * n] = T[i][j];
+    if (!isv) {
+      /* the mirror tile, again along its columns */
+      const int mi = jacobi_row (i, kq, r, nblk), mj = jacobi_row (j, kp, r, nblk);
+      if (mi < n && mj < n) A[mi + (size_t) mj * n] = T[j][i];
+    }
+  }
 }
 
 __global__ void
-k_jacobi_finish (int n, const double *A, const double *V, double *Vout,
-                 double *w)
+k_jacobi_start (int n, double *V, int *flags, int nflags)
 {
   const int64_t nn = (int64_t) n * n;
   for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < nn;
-       e += (int64_t) gridDim.x * blockDim.x) {
-    if (Vout != V) Vout[e] = V[e];
-    const int i = (int) (e % n), j = (int) (e / n);
-    if (i == j) w[i] = A[e];
-  }
+       e += (int64_t) gridDim.x * blockDim.x)
+    V[e] = ((e % n) == (e / n)) ? 1. : 0.;
+  if (blockIdx.x == 0)
+    for (int e = threadIdx.x; e < nflags; e += blockDim.x) flags[e] = 0;
+}
+
+__global__ void
+k_jacobi_diag (int n, const double *A, double *w)
+{
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += gridDim.x * blockDim.x)
+    w[i] = A[i + (size_t) i * n];
 }
 
 int
-launch_syev_jacobi (int n, double *A, double *V, double *w, double *A2,
-                    double *V2, int *sweeps, cudaStream_t s)
+launch_syev_jacobi (int n, double *A, double *V, double *w, int *sweeps,
+                    cudaStream_t s)
 {
   if (n <= 0) return 0;
   LGH_CHECK (n <= 2048, LGH_ERR_SUP, "syev: n=%d > 2048", n);
-  if (n == 1) {
-    LGH_CUDA (cudaMemcpyAsync (w, A, sizeof (double), cudaMemcpyDeviceToDevice, s));
-    double one = 1.;
-    LGH_CUDA (cudaMemcpyAsync (V, &one, sizeof (double), cudaMemcpyHostToDevice, s));
-    LGH_CUDA (cudaStreamSynchronize (s));
-    if (sweeps) *sweeps = 0;
-    return 0;
-  }
-  const int np = n + (n & 1);
-  const int npair = np / 2;
-  const int smem = npair * 3 * (int) sizeof (double) + (2 * npair + np) * (int) sizeof (int);
-  LGH_CUDA (cudaFuncSetAttribute (k_jacobi,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  smem));
-  int per_sm = 0;
-  LGH_CUDA (cudaOccupancyMaxActiveBlocksPerMultiprocessor (&per_sm, k_jacobi,
-                                                           256, smem));
-  LGH_CHECK (per_sm >= 1, LGH_ERR_GPU, "syev: kernel cannot be resident");
-  /* two CTAs per SM (within what is resident, as the cooperative launch
-   * needs): a round's element updates are the larger part of its time, so
-   * more CTAs shorten it despite the wider barrier (measured at n = 220:
-   * 15.7 ms on 48 CTAs, 11.6 ms on 296; at n = 520: 65 ms on 148 CTAs,
-   * 51 ms on 296); the result does not depend on the grid.  Small
-   * problems keep about one CTA per 128 matrix entries (n = 220 still
-   * gets 296), so that a 10 x 10 eigensolve does not pay a 296-CTA
-   * barrier every round. */
-  const int64_t by_size = std::max<int64_t> (1, ((int64_t) n * n + 127) / 128);
-  int grid = (int) std::min<int64_t> (std::min<int64_t> (2 * (int64_t) num_sms (),
-                                                         (int64_t) num_sms () * per_sm),
-                                      by_size);
-  JacobiCtl *ctl;
-  LGH_TRY (dalloc ((void **) &ctl, sizeof (JacobiCtl)));
-  cudaMemsetAsync (ctl, 0, sizeof (JacobiCtl), s);
-  int max_sweeps = 40;
-  void *args[] = { &n, (void *) &np, &A, &A2, &V, &V2, &ctl, &max_sweeps };
-  cudaError_t e = cudaLaunchCooperativeKernel ((const void *) k_jacobi, grid,
-                                               256, args, smem, s);
-  if (e != cudaSuccess) {
-    dfree (ctl);
-    return set_error (LGH_ERR_GPU, "syev: cooperative launch: %s",
-                      cudaGetErrorString (e));
-  }
-  JacobiCtl h;
-  e = cudaMemcpyAsync (&h, ctl, sizeof (JacobiCtl), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize (s);
-  dfree (ctl);
-  if (e != cudaSuccess)
-    return set_error (LGH_ERR_GPU, "syev: %s", cudaGetErrorString (e));
-  LGH_CHECK (h.err == 0, LGH_ERR_GPU, "syev: grid barrier timed out");
-  /* rounds per sweep = np - 1; each round swaps the buffers */
-  const long swaps = (long) h.sweeps * (np - 1);
-  const double *Af = (swaps & 1) ? A2 : A;
-  const double *Vf = (swaps & 1) ? V2 : V;
-  k_jacobi_finish<<<std::max (1, std::min (num_sms () * 4, (n * n + 255) / 256)),
-                    256, 0, s>>> (n, Af, Vf, V, w);
+  constexpr int MAXS = 40;
+  const int npair = (n + JT - 1) / JT, nblk = 2 * npair;
+  DBuf<double> Wg;
+  DBuf<int> flags;     /* rot[npair], any_rot[MAXS], done */
+  LGH_TRY (Wg.alloc ((size_t) npair * JT * JT));
+  LGH_TRY (flags.alloc (npair + MAXS + 1));
+  int *rot = flags.p, *any = rot + npair, *done = any + MAXS;
+  k_jacobi_start<<<std::max (1, std::min (num_sms () * 4, (n * n + 255) / 256)),
+                   256, 0, s>>> (n, V, flags.p, npair + MAXS + 1);
   LGH_LAUNCH_CHECK ();
-  if (sweeps) *sweeps = h.sweeps;
+  int ran = 0;
+  const dim3 tiles ((unsigned) npair, (unsigned) (npair + npair));
+  if (npair == 1) {
+    /* the whole matrix in one CTA, to convergence */
+    k_jacobi_pairs<<<1, 256, 0, s>>> (n, nblk, 0, MAXS, A, Wg.p, rot, any, done);
+    LGH_LAUNCH_CHECK ();
+    k_jacobi_apply<<<tiles, 256, 0, s>>> (n, nblk, 0, A, V, Wg.p, rot);
+    LGH_LAUNCH_CHECK ();
+    LGH_CUDA (cudaMemcpyAsync (&ran, done, sizeof (int), cudaMemcpyDeviceToHost, s));
+    LGH_CUDA (cudaStreamSynchronize (s));
+  } else {
+    for (; ran < MAXS; ) {
+      for (int r = 0; r < nblk - 1; r++) {
+        k_jacobi_pairs<<<npair, 256, 0, s>>> (n, nblk, r, 1, A, Wg.p, rot,
+                                              any + ran, done);
+        k_jacobi_apply<<<tiles, 256, 0, s>>> (n, nblk, r, A, V, Wg.p, rot);
+      }
+      LGH_LAUNCH_CHECK ();
+      ran++;
+      /* four sweeps before the first look at convergence */
+      if (ran < 4) continue;
+      int more = 0;
+      LGH_CUDA (cudaMemcpyAsync (&more, any + ran - 1, sizeof (int),
+                                 cudaMemcpyDeviceToHost, s));
+      LGH_CUDA (cudaStreamSynchronize (s));
+      if (!more) break;
+    }
+  }
+  k_jacobi_diag<<<std::max (1, (n + 255) / 256), 256, 0, s>>> (n, A, w);
+  LGH_LAUNCH_CHECK ();
+  if (sweeps) *sweeps = std::max (ran, 1);
   return 0;
 }
 
@@ -455,15 +575,13 @@ device_tridiag_extremes (int m, const double *alpha, const double *beta,
       T[k + 1 + (size_t) k * m] = e;
     }
   }
-  DBuf<double> A, A2, V, V2, w;
+  DBuf<double> A, V, w;
   LGH_TRY (A.alloc ((size_t) m * m));
-  LGH_TRY (A2.alloc ((size_t) m * m));
   LGH_TRY (V.alloc ((size_t) m * m));
-  LGH_TRY (V2.alloc ((size_t) m * m));
   LGH_TRY (w.alloc (m));
   LGH_CUDA (cudaMemcpyAsync (A.p, T.data (), T.size () * sizeof (double),
                              cudaMemcpyHostToDevice, s));
-  LGH_TRY (launch_syev_jacobi (m, A.p, V.p, w.p, A2.p, V2.p, nullptr, s));
+  LGH_TRY (launch_syev_jacobi (m, A.p, V.p, w.p, nullptr, s));
   std::vector<double> wh (m);
   LGH_CUDA (cudaMemcpyAsync (wh.data (), w.p, m * sizeof (double),
                              cudaMemcpyDeviceToHost, s));

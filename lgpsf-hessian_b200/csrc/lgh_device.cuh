@@ -202,34 +202,6 @@ block_colsum_store (const double (&acc)[CH][Pack<T>::W], int lane, int group,
   }
 }
 
-/* bounded grid barrier for cooperative launches (co-residency guaranteed
- * by the launch); returns false if the wait ran out (error flag set). */
-__device__ __forceinline__ bool
-grid_barrier (unsigned *count, unsigned *gen, int *err)
-{
-  __syncthreads ();
-  if (threadIdx.x == 0) {
-    volatile unsigned *vgen = gen;
-    unsigned g = *vgen;
-    __threadfence ();
-    unsigned arrived = atomicAdd (count, 1u);
-    if (arrived == gridDim.x - 1) {
-      *count = 0u;
-      __threadfence ();
-      atomicAdd (gen, 1u);
-    } else {
-      long spins = 0;
-      while (*vgen == g) {
-        if (++spins > (1L << 25)) { atomicExch (err, 1); break; }
-        __nanosleep (32);
-      }
-    }
-    __threadfence ();
-  }
-  __syncthreads ();
-  return *((volatile int *) err) == 0;
-}
-
 } /* namespace lgh */
 
 #endif /* LGH_DEVICE_CUH */

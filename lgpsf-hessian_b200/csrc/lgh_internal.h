@@ -276,8 +276,8 @@ int launch_potrf (int n, double *G, double *G0, int jitter_mode, int *info,
 int launch_trtri_lower (int n, const double *L, double *Linv, int transpose,
                         cudaStream_t s);
 /* symmetric eigensolve: A (destroyed) -> w (unordered), V (column-major) */
-int launch_syev_jacobi (int n, double *A, double *V, double *w, double *A2,
-                        double *V2, int *sweeps, cudaStream_t s);
+int launch_syev_jacobi (int n, double *A, double *V, double *w, int *sweeps,
+                        cudaStream_t s);
 /* order by |w| desc; cut = max(trunc_abs, trunc_rel*max|w|); fills
  * order[n], sel[6] = {kept, absmax, next_abs, raw_min, raw_max, nneg},
  * lam[kept] treated; C (n x kept col-major) = V[:, order[0:kept]] */
