@@ -1049,6 +1049,13 @@ lgh_glr_apply (lgh_glr_t *glr, double c, lgh_Vec v, lgh_Vec y)
   lgh_prior_t *p = glr->prior;
   cudaStream_t s = stream ();
   LGH_TRY (mat_mult_vec (glr->B, v->d, y->d));
+  if (p->is_mat && !p->Z->rows) {
+    /* the mass division and the sum in the two Z products' stores */
+    LGH_TRY (launch_spmv_div (p->Z->csr, v->d, p->mass.p, glr->w2.p, s));
+    LGH_TRY (launch_spmv_add (p->Z->csr, glr->w2.p, c, y->d, s));
+    LGH_CUDA (cudaStreamSynchronize (s));
+    return 0;
+  }
   LGH_TRY (prior_applyZ (p, v->d, glr->w1.p));
   LGH_TRY (launch_vec_div (glr->n, glr->w1.p, p->mass.p, glr->w2.p, s));
   LGH_TRY (prior_applyZ (p, glr->w2.p, glr->w1.p));

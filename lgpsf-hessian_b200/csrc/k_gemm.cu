@@ -313,6 +313,23 @@ k_gemm_tn_reduce (int m1, int m2, int nsplit, const double *__restrict__ work,
   }
 }
 
+/* the same sum with one warp per entry, for products of few entries in many
+ * slices (the 200 coefficients of one vector: one CTA of serial sums took
+ * 16 us) */
+__global__ void __launch_bounds__ (256)
+k_gemm_tn_reduce_warp (int64_t total, int m1, int nsplit,
+                       const double *__restrict__ work, double *C, int ldc)
+{
+  const int lane = threadIdx.x & 31;
+  for (int64_t e = (int64_t) blockIdx.x * 8 + (threadIdx.x >> 5); e < total;
+       e += (int64_t) gridDim.x * 8) {
+    double s = 0.;
+    for (int z = lane; z < nsplit; z += 32) s += work[(size_t) z * total + e];
+    s = warp_sum (s);
+    if (lane == 0) C[e % m1 + (size_t) (e / m1) * ldc] = s;
+  }
+}
+
 static int
 tn_splits (int64_t n, int m1, int m2)
 {
@@ -343,6 +360,132 @@ gemm_tn_work_max (int m1max, int m2max)
   return (4 * (size_t) num_sms () + tmax) * GB * GB;
 }
 
+/* C from nsplit slices of partial sums in work */
+static int
+gemm_tn_sum (int m1, int m2, int nsplit, const double *work, double *C, int ldc,
+             int sym, int upper, cudaStream_t s)
+{
+  const int64_t total = (int64_t) m1 * m2;
+  if (!sym && !upper && nsplit >= 16 && total <= 8192) {
+    k_gemm_tn_reduce_warp<<<(int) ((total + 7) / 8), 256, 0, s>>> (
+        total, m1, nsplit, work, C, ldc);
+  } else {
+    const int rg = (int) std::min<int64_t> ((total + 255) / 256, num_sms () * 8);
+    k_gemm_tn_reduce<<<rg, 256, 0, s>>> (m1, m2, nsplit, work, C, ldc, sym, upper);
+  }
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+/* work[z] = the part of A^T x in this CTA's rows (A n x m1 row-major, x a
+ * strided vector): two packs of a row per thread, 512 / L rows of a CTA at
+ * once, four rows of a thread in flight.  HBM streams A once; the 64-column
+ * output tiles of k_gemm_tn_part read it at 2 TB/s for one column. */
+constexpr int GV_THREADS = 512;
+
+template <typename T>
+__global__ void __launch_bounds__ (GV_THREADS)
+k_gemv_t (int64_t n, int m1, const T *__restrict__ A, int lda,
+          const T *__restrict__ x, int ldx, double *__restrict__ work, int L,
+          int rpc)
+{
+  constexpr int W = Pack<T>::W, CH = 2, U = 4;
+  extern __shared__ double red[];          /* [rpc][nvec * W] */
+  const int nvec = (m1 + W - 1) / W;
+  const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
+  const int64_t stride = (int64_t) gridDim.x * rpc;
+  double acc[CH][W];
+#pragma unroll
+  for (int h = 0; h < CH; h++)
+#pragma unroll
+    for (int e = 0; e < W; e++) acc[h][e] = 0.;
+  if (rl < rpc)
+    for (int64_t i = (int64_t) blockIdx.x * rpc + rl; i < n; i += U * stride) {
+      Pack<T> a[U][CH];
+      double xv[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int64_t r = i + u * stride;
+        xv[u] = r < n ? (double) x[r * ldx] : 0.;
+#pragma unroll
+        for (int h = 0; h < CH; h++) {
+          const int vi = lane + h * L;
+          a[u][h] = (r < n && vi < nvec) ? ldp (A + r * lda + vi * W) : pzero<T> ();
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int h = 0; h < CH; h++)
+#pragma unroll
+          for (int e = 0; e < W; e++)
+            acc[h][e] = fma ((double) a[u][h].v[e], xv[u], acc[h][e]);
+    }
+  const int mw = nvec * W;
+  if (rl < rpc)
+#pragma unroll
+    for (int h = 0; h < CH; h++) {
+      const int vi = lane + h * L;
+      if (vi < nvec)
+#pragma unroll
+        for (int e = 0; e < W; e++) red[rl * mw + vi * W + e] = acc[h][e];
+    }
+  __syncthreads ();
+  for (int c = threadIdx.x; c < m1; c += GV_THREADS) {
+    double sum = 0.;
+    for (int r = 0; r < rpc; r++) sum += red[r * mw + c];
+    work[(size_t) blockIdx.x * m1 + c] = sum;
+  }
+}
+
+/* y = alpha X m + beta y0 for one column: a warp per row, two rows in
+ * flight, m in shared memory */
+template <typename T>
+__global__ void __launch_bounds__ (256)
+k_gemv_n (int64_t n, int k, double alpha, const T *__restrict__ X, int ldx,
+          const double *__restrict__ M, double beta, const T *Y0, int ldy0,
+          T *Y, int ldy)
+{
+  constexpr int W = Pack<T>::W;
+  extern __shared__ __align__ (16) unsigned char smem[];
+  double *m = reinterpret_cast<double *> (smem);
+  for (int e = threadIdx.x; e < k; e += 256) m[e] = M[e];
+  __syncthreads ();
+  const int lane = threadIdx.x & 31, nfull = k / W;
+  const int64_t nw = (int64_t) gridDim.x * 8;
+  for (int64_t i = (int64_t) blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += 2 * nw) {
+    const int64_t i1 = i + nw;
+    const bool two = i1 < n;
+    const T *x0 = X + i * ldx, *x1 = X + (two ? i1 : i) * ldx;
+    double s0 = 0., s1 = 0.;
+#pragma unroll 4
+    for (int v = lane; v < nfull; v += 32) {
+      const Pack<T> a = ldp (x0 + v * W), b = ldp (x1 + v * W);
+#pragma unroll
+      for (int e = 0; e < W; e++) {
+        const double mv = m[v * W + e];
+        s0 = fma ((double) a.v[e], mv, s0);
+        s1 = fma ((double) b.v[e], mv, s1);
+      }
+    }
+    const int t = nfull * W + lane;
+    if (t < k) {
+      s0 = fma ((double) x0[t], m[t], s0);
+      s1 = fma ((double) x1[t], m[t], s1);
+    }
+    s0 = alpha * warp_sum (s0);
+    s1 = alpha * warp_sum (s1);
+    if (lane == 0) {
+      if (beta != 0.) s0 += beta * (double) Y0[i * ldy0];
+      Y[i * ldy] = (T) s0;
+      if (two) {
+        if (beta != 0.) s1 += beta * (double) Y0[i1 * ldy0];
+        Y[i1 * ldy] = (T) s1;
+      }
+    }
+  }
+}
+
 /* nsplit slices (their partial tiles in work), then the sum */
 template <typename T>
 static int
@@ -369,12 +512,9 @@ gemm_tn_run (int64_t n, int m1, int m2, const T *A, int lda, const T *B, int ldb
   else if (a16) LGH_TRY (run (C16 (), CS ()));
   else if (b16) LGH_TRY (run (CS (), C16 ()));
   else LGH_TRY (run (CS (), CS ()));
-  const int64_t total = (int64_t) m1 * m2;
-  int rg = (int) std::min<int64_t> ((total + 255) / 256, num_sms () * 8);
-  k_gemm_tn_reduce<<<rg, 256, 0, s>>> (m1, m2, nsplit, work, C, ldc, sym, upper);
-  LGH_LAUNCH_CHECK ();
-  return 0;
+  return gemm_tn_sum (m1, m2, nsplit, work, C, ldc, sym, upper, s);
 }
+
 
 template <typename T>
 int
@@ -387,6 +527,18 @@ launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
   int ns = tn_splits (n, m1, m2);
   LGH_CHECK ((size_t) ns * m1 * m2 <= work_elems, LGH_ERR_ARG_SIZ,
              "gemm_tn: workspace too small");
+  constexpr int W = Pack<T>::W;
+  if (m2 == 1 && m1 > 1 && copy_bytes (A, lda) == 16 && (m1 + W - 1) / W <= 2 * GV_THREADS) {
+    const int nvec = (m1 + W - 1) / W, L = (nvec + 1) / 2, rpc = GV_THREADS / L;
+    const int64_t tiles = (n + rpc - 1) / rpc;
+    const int nb = (int) std::max<int64_t> (1, std::min<int64_t> (
+        std::min<int64_t> (2 * num_sms (), (tiles + 3) / 4),
+        (int64_t) (work_elems / (size_t) m1)));
+    const int smem = rpc * nvec * W * (int) sizeof (double);
+    k_gemv_t<T><<<nb, GV_THREADS, smem, s>>> (n, m1, A, lda, B, ldb, work, L, rpc);
+    LGH_LAUNCH_CHECK ();
+    return gemm_tn_sum (m1, 1, nb, work, C, ldc, 0, 0, s);
+  }
   /* X^T X: its upper tiles alone, over as many more slices as fit */
   const bool upper = (const void *) A == (const void *) B && lda == ldb && m1 == m2;
   if (upper) {
@@ -683,6 +835,15 @@ launch_gemm_nn (int64_t n, int k, int m2, double alpha, const T *X, int ldx,
                 T *Y, int ldy, cudaStream_t s)
 {
   if (n == 0 || m2 == 0) return 0;
+  if (m2 == 1 && k > 0 && k <= 2048 && copy_bytes (X, ldx) == 16) {
+    const int want = (int) std::min<int64_t> ((n + 15) / 16, 1 << 20);
+    const int smem = k * (int) sizeof (double);
+    auto f = k_gemv_n<T>;
+    f<<<fit_grid (f, std::max (want, 1), 256, smem), 256, smem, s>>> (
+        n, k, alpha, X, ldx, M, beta, Y0, ldy0, Y, ldy);
+    LGH_LAUNCH_CHECK ();
+    return 0;
+  }
   const int tn = (m2 + GB - 1) / GB;
   const int64_t tiles = (n + GB - 1) / GB * tn;
   LGH_CHECK (tiles < INT32_MAX, LGH_ERR_ARG_OUTOFRANGE, "gemm_nn: too many tiles");

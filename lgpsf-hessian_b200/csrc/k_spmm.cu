@@ -11,6 +11,7 @@
  * nnz (s_v + 4) + 8 (N + 1) + 2 N w s_x.
  */
 
+#include <algorithm>
 #include <type_traits>
 
 #include "lgh_device.cuh"
@@ -119,31 +120,71 @@ k_spmm (int64_t n, const int64_t *__restrict__ rowptr,
   }
 }
 
+/* what becomes of a row's product: / div_i (nullable), then stored, or
+ * (add) scaled and added to Y */
+template <typename T>
+struct SpvEp
+{
+  const T *div;
+  T scale;
+  int add;
+};
+
 /* Scalar form for single vectors and unaligned views (ld not a multiple
  * of the 16-byte vector, or an offset base): G lanes split a row's
- * nonzeros (CSR-vector), reduce with shuffles; columns in a loop. */
-template <typename T, typename TV>
+ * nonzeros (CSR-vector), reduce with shuffles; columns in a loop.  A lane
+ * issues U entries' column and value loads, then U gathers of x (which L2
+ * holds), so that a row of 183 entries is two rounds of loads for a warp
+ * instead of 23 dependent steps for 8 lanes: HBM streams the operator.  G:
+ * a warp for rows of more than 32 entries, 8 lanes from 8 up, 4 below
+ * (5-point rows leave 3 of 8 lanes idle). */
+template <typename T, typename TV, int G, int U>
 __global__ void __launch_bounds__ (256)
 k_spmm_scalar (int64_t n, const int64_t *__restrict__ rowptr,
                const int32_t *__restrict__ colidx, const TV *__restrict__ vals,
                const T *__restrict__ X, int ldx, T *__restrict__ Y, int ldy,
-               int w)
+               int w, SpvEp<T> ep)
 {
-  constexpr int G = 8;
   const int lane = threadIdx.x & (G - 1);
-  const unsigned gmask = 0xffu << ((threadIdx.x & 31) & ~(G - 1));
+  const unsigned gmask = G == 32 ? 0xffffffffu
+                         : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
   const int64_t row0 = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / G;
   const int64_t rstride = ((int64_t) gridDim.x * blockDim.x) / G;
+  int64_t k0n = 0, k1n = 0;
+  if (row0 < n) {
+    k0n = rowptr[row0];
+    k1n = rowptr[row0 + 1];
+  }
   for (int64_t i = row0; i < n; i += rstride) {
-    const int64_t k0 = rowptr[i], k1 = rowptr[i + 1];
+    const int64_t k0 = k0n, k1 = k1n;
+    if (i + rstride < n) {   /* the next row's bounds, behind this one's loads */
+      k0n = rowptr[i + rstride];
+      k1n = rowptr[i + rstride + 1];
+    }
     for (int c = 0; c < w; c++) {
       T acc = T (0);
-      for (int64_t k = k0 + lane; k < k1; k += G)
-        acc = fma ((T) vals[k], X[(int64_t) colidx[k] * ldx + c], acc);
+      for (int64_t k = k0 + lane; k < k1; k += G * U) {
+        int32_t j[U];
+        T v[U], x[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const bool in = k + u * G < k1;
+          j[u] = in ? __ldcs (colidx + k + u * G) : 0;
+          v[u] = in ? (T) __ldcs (vals + k + u * G) : T (0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          x[u] = k + u * G < k1 ? X[(int64_t) j[u] * ldx + c] : T (0);
+#pragma unroll
+        for (int u = 0; u < U; u++) acc = fma (v[u], x[u], acc);
+      }
 #pragma unroll
       for (int o = G / 2; o > 0; o >>= 1)
         acc += __shfl_xor_sync (gmask, acc, o, G);
-      if (lane == 0) Y[i * ldy + c] = acc;
+      if (lane == 0) {
+        if (ep.div) acc /= ep.div[i];
+        Y[i * ldy + c] = ep.add ? fma (ep.scale, acc, Y[i * ldy + c]) : acc;
+      }
     }
   }
 }
@@ -180,6 +221,50 @@ row_grid (int64_t n, int glog)
 
 template <typename T, typename TV>
 static int
+spmv_dispatch (const Csr &A, const TV *vals, const T *X, int ldx, T *Y, int ldy,
+               int w, SpvEp<T> ep, cudaStream_t s)
+{
+  const int64_t avg = A.n > 0 ? A.nnz / A.n : 0;
+  auto run = [&] (auto gl, auto un) {
+    constexpr int G = decltype (gl)::value, U = decltype (un)::value;
+    auto k = k_spmm_scalar<T, TV, G, U>;
+    const int want = (int) std::max<int64_t> (1, std::min<int64_t> (
+        (A.n * G + 255) / 256, 1 << 20));
+    k<<<fit_grid (k, want, 256, 0), 256, 0, s>>> (A.n, A.rowptr, A.colidx, vals,
+                                                 X, ldx, Y, ldy, w, ep);
+  };
+  using std::integral_constant;
+  if (avg > 128)
+    run (integral_constant<int, 32> (), integral_constant<int, 8> ());
+  else if (avg > 32)
+    run (integral_constant<int, 32> (), integral_constant<int, 4> ());
+  else if (avg >= 8)
+    run (integral_constant<int, 8> (), integral_constant<int, 4> ());
+  else
+    run (integral_constant<int, 4> (), integral_constant<int, 2> ());
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+/* y = (A x) ./ div, or y += scale A x (div null) of single FP64 vectors */
+int
+launch_spmv_div (const Csr &A, const double *x, const double *div, double *y,
+                 cudaStream_t s)
+{
+  return spmv_dispatch<double, double> (A, A.vals, x, 1, y, 1, 1,
+                                        SpvEp<double>{ div, 0., 0 }, s);
+}
+
+int
+launch_spmv_add (const Csr &A, const double *x, double scale, double *y,
+                 cudaStream_t s)
+{
+  return spmv_dispatch<double, double> (A, A.vals, x, 1, y, 1, 1,
+                                        SpvEp<double>{ nullptr, scale, 1 }, s);
+}
+
+template <typename T, typename TV>
+static int
 spmm_dispatch (const Csr &A, const TV *vals, const T *X, int ldx, T *Y,
                int ldy, int w, cudaStream_t s, int mode = 0,
                const T *Bm = nullptr, int ldb = 0)
@@ -193,13 +278,8 @@ spmm_dispatch (const Csr &A, const TV *vals, const T *X, int ldx, T *Y,
     if (mode != 0)
       return set_error (LGH_ERR_ARG_WRONG, "spmm: accumulate/residual forms "
                         "need 16-byte aligned row-major blocks");
-    int64_t g = (A.n * 8 + 255) / 256;
-    if (g > (int64_t) num_sms () * 16) g = (int64_t) num_sms () * 16;
-    if (g < 1) g = 1;
-    k_spmm_scalar<T, TV><<<(int) g, 256, 0, s>>> (A.n, A.rowptr, A.colidx,
-                                                  vals, X, ldx, Y, ldy, w);
-    LGH_LAUNCH_CHECK ();
-    return 0;
+    return spmv_dispatch<T, TV> (A, vals, X, ldx, Y, ldy, w,
+                                 SpvEp<T>{ nullptr, T (0), 0 }, s);
   }
   /* column chunks of at most 32 lanes * MAXCH vectors */
   for (int c0 = 0; c0 < w; c0 += 32 * MAXCH * W) {

@@ -166,6 +166,12 @@ template <typename T>
 int launch_spmm (const Csr &A, const T *X, int ldx, T *Y, int ldy, int w,
                  cudaStream_t s);
 
+/* single FP64 vectors: y = (A x) ./ div;  y += scale A x */
+int launch_spmv_div (const Csr &A, const double *x, const double *div, double *y,
+                     cudaStream_t s);
+int launch_spmv_add (const Csr &A, const double *x, double scale, double *y,
+                     cudaStream_t s);
+
 /* lanes per row (2^glog) and 16-byte packs per lane (ch) of the row-group
  * kernels for a block of nvec packs; kmax > 0 (the operator's longest row)
  * lets a narrow block use half the lanes with two packs each */

@@ -704,7 +704,10 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
 
   for (int c0 = 0; c0 < w; c0 += tile) {
     const int wt = std::min (tile, w - c0);
-    const int ldt = round_ld (wt);
+    const bool mgpcg = cfg.mode <= 1 && mg != nullptr && cfg.maxit > 0;
+    /* one FP64 column around the FP64 V-cycle: rows of one 16-byte pack */
+    const int ldt = (mgpcg && wt == 1 && sizeof (T) == 8 && !cfg.pc32)
+                        ? 2 : round_ld (wt);
     const int nvec = ldt / W;
     int glog, ch;
     row_group_shape (nvec, glog, ch, Z.max_row_nnz);
@@ -713,7 +716,6 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
     const int cap = ws.cap;
     int *nact = ws.ival.p + I_NSLOT * cap;
 
-    const bool mgpcg = cfg.mode <= 1 && mg != nullptr && cfg.maxit > 0;
     if (!mgpcg) {
       ZS_DISPATCH (ch, {
         auto kf = k_pcg_init<T, CH_>;

@@ -70,3 +70,44 @@ def test_shift_combination(cuda_device, rank, m, ns):
             ref = one(cs[s], R[:, m - 1])
             err = np.linalg.norm(out[s][:, m - 1] - ref)
             assert err < 1e-8 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("nx,ny,rank", [(40, 31, 5), (64, 64, 50),
+                                        (33, 47, 41)])
+def test_single_vector_operations(cuda_device, nx, ny, rank):
+    """The one-column products U^T x and U w through the filter f(x) = x:
+    out = f_c in + U diag(f - f_c) U^T in."""
+    n = nx * ny
+    rng = np.random.default_rng(rank)
+    z = 1.0 + rng.random(n)
+    A = rng.standard_normal((n, rank))
+    Z = L.Mat(P.diag_csr(z))
+    prior = L.Prior(Z=Z, mass=np.ones(n), pc="jacobi")
+    g = L.Glr(L.Mat(dense=A @ A.T / n), prior,
+              L.glr_opts(ell=rank + 3, trunc_rel=0.0),
+              exec=L.exec_opts(rank_cap=rank))
+    U, x = g.U(), rng.standard_normal(n)
+    f = rng.standard_normal(rank)
+    y = g.filter(f, 0.25, x)
+    ref = 0.25 * x + U @ ((f - 0.25) * (U.T @ x))
+    assert np.linalg.norm(y - ref) < 1e-13 * n ** 0.5 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [7, 100, 4097])
+@pytest.mark.parametrize("nnz", [1, 5, 9, 40, 200])
+def test_matvec(cuda_device, n, nnz):
+    """The single-vector product at each split of a row, with empty and
+    uneven rows."""
+    rng = np.random.default_rng(n + nnz)
+    cnt = rng.integers(0, 2 * nnz + 1, n)
+    cnt[0] = 0
+    cnt = np.minimum(cnt, n)
+    rp = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int64)
+    ci = np.concatenate([rng.choice(n, c, replace=False) for c in cnt]
+                        ).astype(np.int32) if rp[-1] else np.zeros(0, np.int32)
+    A = dict(n=n, rowptr=rp, colidx=ci, vals=rng.standard_normal(rp[-1]))
+    x = rng.standard_normal(n)
+    y = L.Mat(A).mult(x)
+    ref = P.csr_matvec(A, x)
+    mag = P.csr_matvec(dict(A, vals=np.abs(A["vals"])), np.abs(x))
+    assert np.all(np.abs(y - ref) <= 1e-14 * mag + 0.0)
