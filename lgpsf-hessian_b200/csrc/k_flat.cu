@@ -35,6 +35,7 @@ k_flat_resid (int64_t n, const int64_t *__restrict__ rowptr,
               const T *__restrict__ X, const T *__restrict__ B,
               T *__restrict__ Y, int ld, int nvec, int L, int rpc)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
   const int64_t stride = (int64_t) gridDim.x * rpc;
@@ -77,6 +78,7 @@ k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
                T *__restrict__ R2, int ld, int nvec, int L, int rpc, T a2,
                T s2)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
   const int64_t stride = (int64_t) gridDim.x * rpc;
@@ -125,6 +127,7 @@ k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
                const T *__restrict__ Xc, T *__restrict__ Z, int ld, int nvec,
                int L, int rpc, T g, T b2)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
   const int64_t stride = (int64_t) gridDim.x * rpc;
@@ -186,6 +189,7 @@ k_flat_mult (int64_t n, const int64_t *__restrict__ rowptr,
              const T *__restrict__ X, T *__restrict__ Y, int ld, int nvec,
              int L, int rows, int S)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   extern __shared__ __align__ (16) unsigned char smem[];
   T *part = reinterpret_cast<T *> (smem);   /* [rows * S][nvec * W] */
@@ -296,9 +300,10 @@ launch_vc_first (const Csr &F1, const T *R0, T *R1, int ld, cudaStream_t s)
     const FlatShape f = flat_shape (nv, F1.n);
     LGH_FLAT_DISPATCH (f.ch, {
       auto k = k_flat_resid<T, CH_>;
-      k<<<fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
-          s>>> (F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
-                R0 + v0 * W, R1 + v0 * W, ld, nv, f.L, f.rpc);
+      LGH_CUDA (launch_pdl (k,
+          fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
+          s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
+          R0 + v0 * W, R1 + v0 * W, ld, nv, f.L, f.rpc));
     });
     LGH_LAUNCH_CHECK ();
     return 0;
@@ -316,9 +321,10 @@ launch_vc_second (const Csr &F1, const T *R0, const T *R1, T *R2, int ld,
     const FlatShape f = flat_shape (nv, F1.n);
     LGH_FLAT_DISPATCH (f.ch, {
       auto k = k_flat_second<T, CH_>;
-      k<<<fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
-          s>>> (F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
-                R1 + v0 * W, R2 + v0 * W, ld, nv, f.L, f.rpc, (T) a2, (T) s2);
+      LGH_CUDA (launch_pdl (k,
+          fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
+          s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
+          R1 + v0 * W, R2 + v0 * W, ld, nv, f.L, f.rpc, (T) a2, (T) s2));
     });
     LGH_LAUNCH_CHECK ();
     return 0;
@@ -349,10 +355,11 @@ launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
       f = flat_shape_ch (nv, 3);
     LGH_FLAT_DISPATCH (f.ch, {
       auto k = k_flat_finish<T, CH_>;
-      k<<<fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
-          s>>> (F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), Q.rowptr, Q.colidx,
-                fvals<T> (Q), dinv, R0 + v0 * W, R1 + v0 * W, R2 + v0 * W,
-                Xc + v0 * W, Z + v0 * W, ld, nv, f.L, f.rpc, (T) g, (T) b2);
+      LGH_CUDA (launch_pdl (k,
+          fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
+          s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), Q.rowptr, Q.colidx,
+          fvals<T> (Q), dinv, R0 + v0 * W, R1 + v0 * W, R2 + v0 * W,
+          Xc + v0 * W, Z + v0 * W, ld, nv, f.L, f.rpc, (T) g, (T) b2));
     });
     LGH_LAUNCH_CHECK ();
     return 0;
@@ -382,14 +389,14 @@ launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s)
     LGH_FLAT_DISPATCH (f.ch, {
       if (S > 1) {
         auto k = k_flat_mult<T, CH_, true>;
-        k<<<fit_grid (k, want, FLAT_THREADS, smem), FLAT_THREADS, smem, s>>> (
-            A.n, A.rowptr, A.colidx, fvals<T> (A), X + v0 * W, Y + v0 * W, ld,
-            nv, f.L, rows, S);
+        LGH_CUDA (launch_pdl (k, fit_grid (k, want, FLAT_THREADS, smem),
+            FLAT_THREADS, smem, s, A.n, A.rowptr, A.colidx, fvals<T> (A),
+            X + v0 * W, Y + v0 * W, ld, nv, f.L, rows, S));
       } else {
         auto k = k_flat_mult<T, CH_, false>;
-        k<<<fit_grid (k, want, FLAT_THREADS, 0), FLAT_THREADS, 0, s>>> (
-            A.n, A.rowptr, A.colidx, fvals<T> (A), X + v0 * W, Y + v0 * W, ld,
-            nv, f.L, rows, 1);
+        LGH_CUDA (launch_pdl (k, fit_grid (k, want, FLAT_THREADS, 0),
+            FLAT_THREADS, 0, s, A.n, A.rowptr, A.colidx, fvals<T> (A),
+            X + v0 * W, Y + v0 * W, ld, nv, f.L, rows, 1));
       }
     });
     LGH_LAUNCH_CHECK ();

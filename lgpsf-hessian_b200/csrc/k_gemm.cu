@@ -520,7 +520,7 @@ template <typename T>
 int
 launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
                 int ldb, double *C, int ldc, int sym, double *work,
-                size_t work_elems, cudaStream_t s)
+                size_t work_elems, cudaStream_t s, int tiles)
 {
   if (m1 == 0 || m2 == 0) return 0;
   LGH_CHECK (!sym || m1 == m2, LGH_ERR_ARG_SIZ, "gemm_tn: sym needs square");
@@ -528,7 +528,7 @@ launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
   LGH_CHECK ((size_t) ns * m1 * m2 <= work_elems, LGH_ERR_ARG_SIZ,
              "gemm_tn: workspace too small");
   constexpr int W = Pack<T>::W;
-  if (m2 == 1 && m1 > 1 && copy_bytes (A, lda) == 16 && (m1 + W - 1) / W <= 2 * GV_THREADS) {
+  if (!tiles && m2 == 1 && m1 > 1 && copy_bytes (A, lda) == 16 && (m1 + W - 1) / W <= 2 * GV_THREADS) {
     const int nvec = (m1 + W - 1) / W, L = (nvec + 1) / 2, rpc = GV_THREADS / L;
     const int64_t tiles = (n + rpc - 1) / rpc;
     const int nb = (int) std::max<int64_t> (1, std::min<int64_t> (
@@ -573,10 +573,10 @@ gemm_tn_splits (int64_t n, int m1, int m2)
 
 template int launch_gemm_tn<double> (int64_t, int, int, const double *, int,
                                      const double *, int, double *, int, int,
-                                     double *, size_t, cudaStream_t);
+                                     double *, size_t, cudaStream_t, int);
 template int launch_gemm_tn<float> (int64_t, int, int, const float *, int,
                                     const float *, int, double *, int, int,
-                                    double *, size_t, cudaStream_t);
+                                    double *, size_t, cudaStream_t, int);
 
 /* Y = alpha X M + beta Y0: X row-major n x k, M column-major k x m2.
  * Column tiles run fastest, so the CTAs resident at once share a band of X
@@ -741,6 +741,7 @@ __global__ void __launch_bounds__ (NW * 32)
 k_dense_apply (int n0, const double *__restrict__ Ainv, const T *__restrict__ B,
                T *__restrict__ Y, int w, int ld)
 {
+  pdl_wait ();
   constexpr int TM = 8 * MT, TN = 8 * NT;
   extern __shared__ double red[];              /* [NW][TM * TN] */
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -805,7 +806,8 @@ dense_apply_tile (int n0, const double *Ainv, const T *B, T *Y, int w, int ld,
   static_assert (NW * 64 * MT * NT * 8 <= 48 * 1024, "static shared limit");
   dim3 grid ((unsigned) ((n0 + 8 * MT - 1) / (8 * MT)),
              (unsigned) ((ld + 8 * NT - 1) / (8 * NT)));
-  k_dense_apply<T, MT, NT, NW><<<grid, NW * 32, smem, s>>> (n0, Ainv, B, Y, w, ld);
+  LGH_CUDA (launch_pdl (k_dense_apply<T, MT, NT, NW>, grid, NW * 32, smem, s, n0,
+                        Ainv, B, Y, w, ld));
   LGH_LAUNCH_CHECK ();
   return 0;
 }
@@ -832,10 +834,10 @@ template <typename T>
 int
 launch_gemm_nn (int64_t n, int k, int m2, double alpha, const T *X, int ldx,
                 const double *M, int ldm, double beta, const T *Y0, int ldy0,
-                T *Y, int ldy, cudaStream_t s)
+                T *Y, int ldy, cudaStream_t s, int tiles_only)
 {
   if (n == 0 || m2 == 0) return 0;
-  if (m2 == 1 && k > 0 && k <= 2048 && copy_bytes (X, ldx) == 16) {
+  if (!tiles_only && m2 == 1 && k > 0 && k <= 2048 && copy_bytes (X, ldx) == 16) {
     const int want = (int) std::min<int64_t> ((n + 15) / 16, 1 << 20);
     const int smem = k * (int) sizeof (double);
     auto f = k_gemv_n<T>;
@@ -867,10 +869,10 @@ launch_gemm_nn (int64_t n, int k, int m2, double alpha, const T *X, int ldx,
 template int launch_gemm_nn<double> (int64_t, int, int, double,
                                      const double *, int, const double *, int,
                                      double, const double *, int, double *,
-                                     int, cudaStream_t);
+                                     int, cudaStream_t, int);
 template int launch_gemm_nn<float> (int64_t, int, int, double, const float *,
                                     int, const double *, int, double,
                                     const float *, int, float *, int,
-                                    cudaStream_t);
+                                    cudaStream_t, int);
 
 } /* namespace lgh */

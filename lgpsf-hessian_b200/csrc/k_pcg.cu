@@ -221,6 +221,7 @@ __global__ void __launch_bounds__ (FLAT_THREADS)
 k_pcg_columns (const double *partA, const double *partB, int nb, int ld,
                unsigned *counter, PcgCols pc)
 {
+  pdl_wait ();
   pcg_columns<DOTS> (partA, partB, nb,
                      (int) (blockIdx.x * (FLAT_THREADS / 32) + (threadIdx.x >> 5)),
                      (int) (gridDim.x * (FLAT_THREADS / 32)), ld, pc);
@@ -238,6 +239,7 @@ k_pcg_start (int64_t n, int w, int ld, const T *__restrict__ B, int ldb,
              const double *__restrict__ rs, T *__restrict__ R,
              float *__restrict__ R32, int vec)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   const int nvec = ld / W;
   const int64_t total = n * nvec;
@@ -267,6 +269,7 @@ k_pcg_dots (int64_t n, int ld, int nvec, int L, int rpc, const T *__restrict__ R
             const TZ *__restrict__ Zb, double *partA, double *partB,
             unsigned *counter, PcgCols pc)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   extern __shared__ double red[];
   const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
@@ -301,6 +304,7 @@ k_pcg_dir (int64_t n, int ld, const TZ *__restrict__ Zb, T *__restrict__ P,
            T *__restrict__ X, const double *__restrict__ beta,
            const double *__restrict__ alpha)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   const int nvec = ld / W;
   const int64_t total = n * nvec;
@@ -337,6 +341,7 @@ k_pcg_prod (int64_t n, const int64_t *__restrict__ rowptr,
             const T *__restrict__ P, T *__restrict__ Q, int ld, int nvec, int L,
             int rpc, double *partA, unsigned *counter, PcgCols pc)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   extern __shared__ double red[];
   const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
@@ -384,6 +389,7 @@ k_pcg_resid (int64_t n, int ld, T *__restrict__ R, const T *__restrict__ Qv,
              float *__restrict__ R32, T *__restrict__ X,
              const T *__restrict__ P, const double *__restrict__ alpha)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   const int nvec = ld / W;
   const int64_t total = n * nvec;
@@ -417,6 +423,7 @@ k_pcg_out (int64_t n, int w, int ld, const T *__restrict__ X,
            const T *__restrict__ P, int have_x, const double *__restrict__ rs,
            T *__restrict__ Y, int ldy, const double *__restrict__ alpha, int vec)
 {
+  pdl_wait ();
   constexpr int W = Pack<T>::W;
   const int nvec = (w + W - 1) / W;
   const int64_t total = n * nvec;
@@ -480,8 +487,8 @@ launch_pcg_start (int64_t n, int w, int ld, const T *B, int ldb,
 {
   constexpr int W = Pack<T>::W;
   const int vec = ldb % W == 0 && (uintptr_t) B % 16 == 0;
-  k_pcg_start<T><<<stream_grid (n * (ld / W)), 256, 0, s>>> (n, w, ld, B, ldb,
-                                                            rs, R, R32, vec);
+  LGH_CUDA (launch_pdl (k_pcg_start<T>, stream_grid (n * (ld / W)), 256, 0, s,
+      n, w, ld, B, ldb, rs, R, R32, vec));
   LGH_LAUNCH_CHECK ();
   return 0;
 }
@@ -504,21 +511,20 @@ launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
   LGH_FLAT_DISPATCH (f.ch, {
     if (ld <= PCG_TAIL_COLS) {
       auto k = k_pcg_dots<T, TZ, CH_, true>;
-      k<<<fit_grid (k, want, FLAT_THREADS, smem), FLAT_THREADS, smem, s>>> (
-          n, ld, nvec, f.L, f.rpc, R, Zb, ws.partA.p, ws.partB.p,
-          ws.counters.p + 1, pc);
+      LGH_CUDA (launch_pdl (k, fit_grid (k, want, FLAT_THREADS, smem),
+          FLAT_THREADS, smem, s, n, ld, nvec, f.L, f.rpc, R, Zb, ws.partA.p,
+          ws.partB.p, ws.counters.p + 1, pc));
     } else {
       auto k = k_pcg_dots<T, TZ, CH_, false>;
       nb = fit_grid (k, want, FLAT_THREADS, smem);
-      k<<<nb, FLAT_THREADS, smem, s>>> (n, ld, nvec, f.L, f.rpc, R, Zb,
-                                        ws.partA.p, ws.partB.p,
-                                        ws.counters.p + 1, pc);
+      LGH_CUDA (launch_pdl (k, nb, FLAT_THREADS, smem, s, n, ld, nvec, f.L,
+          f.rpc, R, Zb, ws.partA.p, ws.partB.p, ws.counters.p + 1, pc));
     }
   });
   LGH_LAUNCH_CHECK ();
   if (nb > 0) {
-    k_pcg_columns<true><<<(ld + 7) / 8, FLAT_THREADS, 0, s>>> (
-        ws.partA.p, ws.partB.p, nb, ld, ws.counters.p + 1, pc);
+    LGH_CUDA (launch_pdl (k_pcg_columns<true>, (ld + 7) / 8, FLAT_THREADS, 0,
+        s, ws.partA.p, ws.partB.p, nb, ld, ws.counters.p + 1, pc));
     LGH_LAUNCH_CHECK ();
   }
   return 0;
@@ -534,16 +540,20 @@ launch_pcg_dir (int64_t n, int ld, const TZ *Zb, T *P, T *X, int flags,
   const double *be = ws.scal.p + S_BETA * ws.cap, *al = ws.scal.p + S_ALPHA * ws.cap;
   switch (flags) {
   case 0:
-    k_pcg_dir<T, TZ, 0><<<grid, 256, 0, s>>> (n, ld, Zb, P, X, be, al);
+    LGH_CUDA (launch_pdl (k_pcg_dir<T, TZ, 0>, grid, 256, 0, s, n, ld, Zb, P,
+        X, be, al));
     break;
   case PCG_P_FIRST:
-    k_pcg_dir<T, TZ, PCG_P_FIRST><<<grid, 256, 0, s>>> (n, ld, Zb, P, X, be, al);
+    LGH_CUDA (launch_pdl (k_pcg_dir<T, TZ, PCG_P_FIRST>, grid, 256, 0, s, n,
+        ld, Zb, P, X, be, al));
     break;
   case PCG_X_FIRST:
-    k_pcg_dir<T, TZ, PCG_X_FIRST><<<grid, 256, 0, s>>> (n, ld, Zb, P, X, be, al);
+    LGH_CUDA (launch_pdl (k_pcg_dir<T, TZ, PCG_X_FIRST>, grid, 256, 0, s, n,
+        ld, Zb, P, X, be, al));
     break;
   case PCG_X_ADD:
-    k_pcg_dir<T, TZ, PCG_X_ADD><<<grid, 256, 0, s>>> (n, ld, Zb, P, X, be, al);
+    LGH_CUDA (launch_pdl (k_pcg_dir<T, TZ, PCG_X_ADD>, grid, 256, 0, s, n, ld,
+        Zb, P, X, be, al));
     break;
   default:
     return set_error (LGH_ERR_ARG_WRONG, "PCG direction: flags %d", flags);
@@ -573,9 +583,9 @@ launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
                         decltype (tail)::value>;
     const int g = fit_grid (k, want, FLAT_THREADS, smem);
     if (!decltype (tail)::value) nb = g;
-    k<<<g, FLAT_THREADS, smem, s>>> (Z.n, Z.rowptr, Z.colidx, vals, P, Q, ld,
-                                     nvec, f.L, f.rpc, ws.partA.p,
-                                     ws.counters.p, pc);
+    LGH_CUDA (launch_pdl (k, g, FLAT_THREADS, smem, s, Z.n, Z.rowptr,
+        Z.colidx, vals, P, Q, ld, nvec, f.L, f.rpc, ws.partA.p, ws.counters.p,
+        pc));
     LGH_LAUNCH_CHECK ();
     return 0;
   };
@@ -591,8 +601,8 @@ launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
     }
   });
   if (nb > 0) {
-    k_pcg_columns<false><<<(ld + 7) / 8, FLAT_THREADS, 0, s>>> (
-        ws.partA.p, nullptr, nb, ld, ws.counters.p, pc);
+    LGH_CUDA (launch_pdl (k_pcg_columns<false>, (ld + 7) / 8, FLAT_THREADS, 0,
+        s, ws.partA.p, nullptr, nb, ld, ws.counters.p, pc));
     LGH_LAUNCH_CHECK ();
   }
   return 0;
@@ -606,9 +616,11 @@ launch_pcg_resid (int64_t n, int ld, T *R, const T *Q, float *R32, T *X,
   const int grid = stream_grid (n * (ld / Pack<T>::W));
   const double *al = ws.scal.p + S_ALPHA * ws.cap;
   if (X)
-    k_pcg_resid<T, true><<<grid, 256, 0, s>>> (n, ld, R, Q, R32, X, P, al);
+    LGH_CUDA (launch_pdl (k_pcg_resid<T, true>, grid, 256, 0, s, n, ld, R, Q,
+        R32, X, P, al));
   else
-    k_pcg_resid<T, false><<<grid, 256, 0, s>>> (n, ld, R, Q, R32, X, P, al);
+    LGH_CUDA (launch_pdl (k_pcg_resid<T, false>, grid, 256, 0, s, n, ld, R, Q,
+        R32, X, P, al));
   LGH_LAUNCH_CHECK ();
   return 0;
 }
@@ -620,8 +632,9 @@ launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P, int have_x,
 {
   constexpr int W = Pack<T>::W;
   const int vec = ldy % W == 0 && (uintptr_t) Y % 16 == 0;
-  k_pcg_out<T><<<stream_grid (n * ((w + W - 1) / W)), 256, 0, s>>> (
-      n, w, ld, X, P, have_x, rs, Y, ldy, ws.scal.p + S_ALPHA * ws.cap, vec);
+  LGH_CUDA (launch_pdl (k_pcg_out<T>, stream_grid (n * ((w + W - 1) / W)),
+      256, 0, s, n, w, ld, X, P, have_x, rs, Y, ldy,
+      ws.scal.p + S_ALPHA * ws.cap, vec));
   LGH_LAUNCH_CHECK ();
   return 0;
 }

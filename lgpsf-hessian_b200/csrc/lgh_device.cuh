@@ -9,6 +9,16 @@
 namespace lgh
 {
 
+/* a kernel launched with launch_pdl: wait until the previous kernel of the
+ * stream has completed (its writes visible), then let the next one's CTAs
+ * come up; nothing to do in an ordinary launch */
+__device__ __forceinline__ void
+pdl_wait ()
+{
+  cudaGridDependencySynchronize ();
+  cudaTriggerProgrammaticLaunchCompletion ();
+}
+
 /* 16-byte vector of T: 2 doubles or 4 floats */
 template <typename T>
 struct __align__ (16) Pack

@@ -13,6 +13,7 @@
 #ifndef LGH_INTERNAL_H
 #define LGH_INTERNAL_H
 
+#include <utility>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -66,6 +67,30 @@ extern RuntimeCounters g_rt;
       return ::lgh::set_error (LGH_ERR_GPU, "%s:%d launch: %s", __FILE__,    \
                                __LINE__, cudaGetErrorString (e_));           \
   } while (0)
+
+/* Launch with programmatic stream serialisation: the kernel's CTAs may
+ * become resident while the previous kernel of the stream drains, and the
+ * kernel waits for that one itself (pdl_wait in lgh_device.cuh, before its
+ * first global access).  For the chains of short passes of a Z-solve, where
+ * the gap between two launches, 1 to 2 us, is a third of a pass.  A kernel
+ * that does not wait must not be launched this way. */
+template <typename... KArgs, typename... Args>
+inline cudaError_t
+launch_pdl (void (*kern) (KArgs...), dim3 grid, int threads, int smem,
+            cudaStream_t s, Args &&...args)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3 ((unsigned) threads);
+  cfg.dynamicSmemBytes = (size_t) smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx (&cfg, kern, std::forward<Args> (args)...);
+}
 
 /* ---- runtime ------------------------------------------------------------ */
 
@@ -250,17 +275,22 @@ int launch_vec_axpby (int64_t n, double a, const double *x, double b,
                       const double *y, double *out, cudaStream_t s);
 
 /* dense (k_gemm.cu): C = A^T B over n rows (split-K, FP64 accumulate),
- * C is m1 x m2 column-major with leading dim ldc; sym: 1 => C = (C + C^T)/2 */
+ * C is m1 x m2 column-major with leading dim ldc; sym: 1 => C = (C + C^T)/2.
+ * One column takes a streaming kernel of its own unless tiles (and
+ * tiles_only below) is set: the request loop's columns get the same bits at
+ * every batch width from the tiled form alone. */
 template <typename T>
 int launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda,
                     const T *B, int ldb, double *C, int ldc, int sym,
-                    double *work, size_t work_elems, cudaStream_t s);
+                    double *work, size_t work_elems, cudaStream_t s,
+                    int tiles = 0);
 /* Y = alpha X M + beta Y0; X n x k row-major, M k x m2 column-major FP64
  * (leading dim ldm); Y, Y0 row-major */
 template <typename T>
 int launch_gemm_nn (int64_t n, int k, int m2, double alpha, const T *X,
                     int ldx, const double *M, int ldm, double beta,
-                    const T *Y0, int ldy0, T *Y, int ldy, cudaStream_t s);
+                    const T *Y0, int ldy0, T *Y, int ldy, cudaStream_t s,
+                    int tiles_only = 0);
 size_t gemm_tn_work_elems (int64_t n, int m1, int m2);
 
 /* partial-sum elements enough for every gemm_tn shape up to m1max x m2max */

@@ -548,7 +548,7 @@ srv_start (lgh_server_t *sv, const Adm &a)
                                               sv->H.p, ldh, nullptr, s));
         LGH_TRY (launch_gemm_tn<double> (n, kept, mc, g->U.p, g->ldu, sv->H.p, ldh,
                                          r->wcoef.p + (size_t) c0 * kept, kept, 0,
-                                         sv->gemmwork.p, sv->gemmwork.n, s));
+                                         sv->gemmwork.p, sv->gemmwork.n, s, 1));
       }
     }
   }
@@ -626,7 +626,7 @@ srv_harvest (lgh_server_t *sv, const std::vector<int> &act)
       LGH_LAUNCH_CHECK ();
       LGH_TRY (launch_gemm_tn<double> (n, kept, ka, g->U.p, g->ldu, sv->H.p, ldh,
                                        sv->coef.p, kept, 0, sv->gemmwork.p,
-                                       sv->gemmwork.n, s));
+                                       sv->gemmwork.n, s, 1));
       k_put_coef<<<cgrid ((int64_t) kept * ka), 256, 0, s>>> (kept, ka, sv->coef.p,
                                                               hd->wdst_a);
       LGH_LAUNCH_CHECK ();
@@ -646,7 +646,7 @@ srv_harvest (lgh_server_t *sv, const std::vector<int> &act)
                                                                hd->wsrc_b, sv->coef.p);
       LGH_LAUNCH_CHECK ();
       LGH_TRY (launch_gemm_nn<double> (n, kept, kb, 1.0, g->Wz.p, g->ldu, sv->coef.p,
-                                       kept, 1.0, sv->H.p, ldh, sv->H.p, ldh, s));
+                                       kept, 1.0, sv->H.p, ldh, sv->H.p, ldh, s, 1));
     }
     k_scatter_cols<<<cgrid (n * kb), 256, 0, s>>> (n, sv->H.p, ldh, kb, hd->out_b);
     LGH_LAUNCH_CHECK ();
