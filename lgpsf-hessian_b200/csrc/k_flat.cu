@@ -295,12 +295,13 @@ int
 launch_vc_first (const Csr &F1, const T *R0, T *R1, int ld, cudaStream_t s)
 {
   constexpr int W = Pack<T>::W;
+  const int64_t bytes = F1.n * ld * (int64_t) sizeof (T);
   LGH_TRY (flat_check<T> (F1, R0, R1, nullptr, ld));
   return flat_slices (F1.n, F1.bandwidth, ld, ld / W, sizeof (T), [&] (int v0, int nv) {
     const FlatShape f = flat_shape (nv, F1.n);
     LGH_FLAT_DISPATCH (f.ch, {
       auto k = k_flat_resid<T, CH_>;
-      LGH_CUDA (launch_pdl (k,
+      LGH_CUDA (launch_pdl (bytes, k,
           fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
           s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
           R0 + v0 * W, R1 + v0 * W, ld, nv, f.L, f.rpc));
@@ -316,12 +317,13 @@ launch_vc_second (const Csr &F1, const T *R0, const T *R1, T *R2, int ld,
                   double a2, double s2, cudaStream_t s)
 {
   constexpr int W = Pack<T>::W;
+  const int64_t bytes = F1.n * ld * (int64_t) sizeof (T);
   LGH_TRY (flat_check<T> (F1, R0, R1, R2, ld));
   return flat_slices (F1.n, F1.bandwidth, ld, ld / W, sizeof (T), [&] (int v0, int nv) {
     const FlatShape f = flat_shape (nv, F1.n);
     LGH_FLAT_DISPATCH (f.ch, {
       auto k = k_flat_second<T, CH_>;
-      LGH_CUDA (launch_pdl (k,
+      LGH_CUDA (launch_pdl (bytes, k,
           fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
           s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
           R1 + v0 * W, R2 + v0 * W, ld, nv, f.L, f.rpc, (T) a2, (T) s2));
@@ -338,6 +340,7 @@ launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
                   double b2, cudaStream_t s)
 {
   constexpr int W = Pack<T>::W;
+  const int64_t bytes = F1.n * ld * (int64_t) sizeof (T);
   LGH_TRY (flat_check<T> (F1, R0, R1, R2, ld));
   LGH_TRY (flat_check<T> (Q, Xc, Z, nullptr, ld));
   LGH_CHECK (dinv && Q.n == F1.n, LGH_ERR_ARG_WRONG, "V-cycle finish: operators");
@@ -355,7 +358,7 @@ launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
       f = flat_shape_ch (nv, 3);
     LGH_FLAT_DISPATCH (f.ch, {
       auto k = k_flat_finish<T, CH_>;
-      LGH_CUDA (launch_pdl (k,
+      LGH_CUDA (launch_pdl (bytes, k,
           fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
           s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), Q.rowptr, Q.colidx,
           fvals<T> (Q), dinv, R0 + v0 * W, R1 + v0 * W, R2 + v0 * W,
@@ -371,6 +374,7 @@ int
 launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s)
 {
   constexpr int W = Pack<T>::W;
+  const int64_t bytes = A.ncols * ld * (int64_t) sizeof (T);
   LGH_TRY (flat_check<T> (A, X, Y, nullptr, ld));
   /* one launch holds at most FLAT_MAXPACKS packs of a row */
   return flat_slices (0, 0, ld, ld / W, sizeof (T), [&] (int v0, int nv) {
@@ -389,12 +393,12 @@ launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s)
     LGH_FLAT_DISPATCH (f.ch, {
       if (S > 1) {
         auto k = k_flat_mult<T, CH_, true>;
-        LGH_CUDA (launch_pdl (k, fit_grid (k, want, FLAT_THREADS, smem),
+        LGH_CUDA (launch_pdl (bytes, k, fit_grid (k, want, FLAT_THREADS, smem),
             FLAT_THREADS, smem, s, A.n, A.rowptr, A.colidx, fvals<T> (A),
             X + v0 * W, Y + v0 * W, ld, nv, f.L, rows, S));
       } else {
         auto k = k_flat_mult<T, CH_, false>;
-        LGH_CUDA (launch_pdl (k, fit_grid (k, want, FLAT_THREADS, 0),
+        LGH_CUDA (launch_pdl (bytes, k, fit_grid (k, want, FLAT_THREADS, 0),
             FLAT_THREADS, 0, s, A.n, A.rowptr, A.colidx, fvals<T> (A),
             X + v0 * W, Y + v0 * W, ld, nv, f.L, rows, 1));
       }

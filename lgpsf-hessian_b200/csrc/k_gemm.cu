@@ -806,7 +806,7 @@ dense_apply_tile (int n0, const double *Ainv, const T *B, T *Y, int w, int ld,
   static_assert (NW * 64 * MT * NT * 8 <= 48 * 1024, "static shared limit");
   dim3 grid ((unsigned) ((n0 + 8 * MT - 1) / (8 * MT)),
              (unsigned) ((ld + 8 * NT - 1) / (8 * NT)));
-  LGH_CUDA (launch_pdl (k_dense_apply<T, MT, NT, NW>, grid, NW * 32, smem, s, n0,
+  LGH_CUDA (launch_pdl (0, k_dense_apply<T, MT, NT, NW>, grid, NW * 32, smem, s, n0,
                         Ainv, B, Y, w, ld));
   LGH_LAUNCH_CHECK ();
   return 0;

@@ -485,9 +485,10 @@ int
 launch_pcg_start (int64_t n, int w, int ld, const T *B, int ldb,
                   const double *rs, T *R, float *R32, cudaStream_t s)
 {
+  const int64_t bytes = n * ld * (int64_t) sizeof (T);
   constexpr int W = Pack<T>::W;
   const int vec = ldb % W == 0 && (uintptr_t) B % 16 == 0;
-  LGH_CUDA (launch_pdl (k_pcg_start<T>, stream_grid (n * (ld / W)), 256, 0, s,
+  LGH_CUDA (launch_pdl (bytes, k_pcg_start<T>, stream_grid (n * (ld / W)), 256, 0, s,
       n, w, ld, B, ldb, rs, R, R32, vec));
   LGH_LAUNCH_CHECK ();
   return 0;
@@ -499,6 +500,7 @@ launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
                  double rtol, int iter, double *hist, const int *fresh,
                  ZWork &ws, cudaStream_t s)
 {
+  const int64_t bytes = n * ld * (int64_t) sizeof (T);
   constexpr int W = Pack<T>::W;
   LGH_TRY (pcg_width (ld, W));
   const int nvec = ld / W;
@@ -511,19 +513,19 @@ launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
   LGH_FLAT_DISPATCH (f.ch, {
     if (ld <= PCG_TAIL_COLS) {
       auto k = k_pcg_dots<T, TZ, CH_, true>;
-      LGH_CUDA (launch_pdl (k, fit_grid (k, want, FLAT_THREADS, smem),
+      LGH_CUDA (launch_pdl (bytes, k, fit_grid (k, want, FLAT_THREADS, smem),
           FLAT_THREADS, smem, s, n, ld, nvec, f.L, f.rpc, R, Zb, ws.partA.p,
           ws.partB.p, ws.counters.p + 1, pc));
     } else {
       auto k = k_pcg_dots<T, TZ, CH_, false>;
       nb = fit_grid (k, want, FLAT_THREADS, smem);
-      LGH_CUDA (launch_pdl (k, nb, FLAT_THREADS, smem, s, n, ld, nvec, f.L,
+      LGH_CUDA (launch_pdl (bytes, k, nb, FLAT_THREADS, smem, s, n, ld, nvec, f.L,
           f.rpc, R, Zb, ws.partA.p, ws.partB.p, ws.counters.p + 1, pc));
     }
   });
   LGH_LAUNCH_CHECK ();
   if (nb > 0) {
-    LGH_CUDA (launch_pdl (k_pcg_columns<true>, (ld + 7) / 8, FLAT_THREADS, 0,
+    LGH_CUDA (launch_pdl (0, k_pcg_columns<true>, (ld + 7) / 8, FLAT_THREADS, 0,
         s, ws.partA.p, ws.partB.p, nb, ld, ws.counters.p + 1, pc));
     LGH_LAUNCH_CHECK ();
   }
@@ -535,24 +537,25 @@ int
 launch_pcg_dir (int64_t n, int ld, const TZ *Zb, T *P, T *X, int flags,
                 ZWork &ws, cudaStream_t s)
 {
+  const int64_t bytes = n * ld * (int64_t) sizeof (T);
   constexpr int W = Pack<T>::W;
   const int grid = stream_grid (n * (ld / W));
   const double *be = ws.scal.p + S_BETA * ws.cap, *al = ws.scal.p + S_ALPHA * ws.cap;
   switch (flags) {
   case 0:
-    LGH_CUDA (launch_pdl (k_pcg_dir<T, TZ, 0>, grid, 256, 0, s, n, ld, Zb, P,
+    LGH_CUDA (launch_pdl (bytes, k_pcg_dir<T, TZ, 0>, grid, 256, 0, s, n, ld, Zb, P,
         X, be, al));
     break;
   case PCG_P_FIRST:
-    LGH_CUDA (launch_pdl (k_pcg_dir<T, TZ, PCG_P_FIRST>, grid, 256, 0, s, n,
+    LGH_CUDA (launch_pdl (bytes, k_pcg_dir<T, TZ, PCG_P_FIRST>, grid, 256, 0, s, n,
         ld, Zb, P, X, be, al));
     break;
   case PCG_X_FIRST:
-    LGH_CUDA (launch_pdl (k_pcg_dir<T, TZ, PCG_X_FIRST>, grid, 256, 0, s, n,
+    LGH_CUDA (launch_pdl (bytes, k_pcg_dir<T, TZ, PCG_X_FIRST>, grid, 256, 0, s, n,
         ld, Zb, P, X, be, al));
     break;
   case PCG_X_ADD:
-    LGH_CUDA (launch_pdl (k_pcg_dir<T, TZ, PCG_X_ADD>, grid, 256, 0, s, n, ld,
+    LGH_CUDA (launch_pdl (bytes, k_pcg_dir<T, TZ, PCG_X_ADD>, grid, 256, 0, s, n, ld,
         Zb, P, X, be, al));
     break;
   default:
@@ -567,6 +570,7 @@ int
 launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
                  cudaStream_t s)
 {
+  const int64_t bytes = Z.n * ld * (int64_t) sizeof (T);
   constexpr int W = Pack<T>::W;
   LGH_TRY (pcg_width (ld, W));
   const T *vals;
@@ -583,7 +587,7 @@ launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
                         decltype (tail)::value>;
     const int g = fit_grid (k, want, FLAT_THREADS, smem);
     if (!decltype (tail)::value) nb = g;
-    LGH_CUDA (launch_pdl (k, g, FLAT_THREADS, smem, s, Z.n, Z.rowptr,
+    LGH_CUDA (launch_pdl (bytes, k, g, FLAT_THREADS, smem, s, Z.n, Z.rowptr,
         Z.colidx, vals, P, Q, ld, nvec, f.L, f.rpc, ws.partA.p, ws.counters.p,
         pc));
     LGH_LAUNCH_CHECK ();
@@ -601,7 +605,7 @@ launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
     }
   });
   if (nb > 0) {
-    LGH_CUDA (launch_pdl (k_pcg_columns<false>, (ld + 7) / 8, FLAT_THREADS, 0,
+    LGH_CUDA (launch_pdl (0, k_pcg_columns<false>, (ld + 7) / 8, FLAT_THREADS, 0,
         s, ws.partA.p, nullptr, nb, ld, ws.counters.p, pc));
     LGH_LAUNCH_CHECK ();
   }
@@ -613,13 +617,14 @@ int
 launch_pcg_resid (int64_t n, int ld, T *R, const T *Q, float *R32, T *X,
                   const T *P, ZWork &ws, cudaStream_t s)
 {
+  const int64_t bytes = n * ld * (int64_t) sizeof (T);
   const int grid = stream_grid (n * (ld / Pack<T>::W));
   const double *al = ws.scal.p + S_ALPHA * ws.cap;
   if (X)
-    LGH_CUDA (launch_pdl (k_pcg_resid<T, true>, grid, 256, 0, s, n, ld, R, Q,
+    LGH_CUDA (launch_pdl (bytes, k_pcg_resid<T, true>, grid, 256, 0, s, n, ld, R, Q,
         R32, X, P, al));
   else
-    LGH_CUDA (launch_pdl (k_pcg_resid<T, false>, grid, 256, 0, s, n, ld, R, Q,
+    LGH_CUDA (launch_pdl (bytes, k_pcg_resid<T, false>, grid, 256, 0, s, n, ld, R, Q,
         R32, X, P, al));
   LGH_LAUNCH_CHECK ();
   return 0;
@@ -630,9 +635,10 @@ int
 launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P, int have_x,
                 const double *rs, T *Y, int ldy, ZWork &ws, cudaStream_t s)
 {
+  const int64_t bytes = n * ld * (int64_t) sizeof (T);
   constexpr int W = Pack<T>::W;
   const int vec = ldy % W == 0 && (uintptr_t) Y % 16 == 0;
-  LGH_CUDA (launch_pdl (k_pcg_out<T>, stream_grid (n * ((w + W - 1) / W)),
+  LGH_CUDA (launch_pdl (bytes, k_pcg_out<T>, stream_grid (n * ((w + W - 1) / W)),
       256, 0, s, n, w, ld, X, P, have_x, rs, Y, ldy,
       ws.scal.p + S_ALPHA * ws.cap, vec));
   LGH_LAUNCH_CHECK ();

@@ -72,12 +72,16 @@ extern RuntimeCounters g_rt;
  * become resident while the previous kernel of the stream drains, and the
  * kernel waits for that one itself (pdl_wait in lgh_device.cuh, before its
  * first global access).  For the chains of short passes of a Z-solve, where
- * the gap between two launches, 1 to 2 us, is a third of a pass.  A kernel
- * that does not wait must not be launched this way. */
+ * the gap between two launches, 1 to 2 us, is a third of a pass.  block:
+ * bytes of the pass's block; above 128 MB (the L2) the launch is an ordinary
+ * one: passes of 100 us and more lose more to the early CTAs than the gap
+ * (512^2 job of 220 columns 222 ms with them, 218 without; the 132-column
+ * mixed job, blocks of 105 MB, 78.4 and 80.6).  A kernel that does not wait
+ * must not be launched this way. */
 template <typename... KArgs, typename... Args>
 inline cudaError_t
-launch_pdl (void (*kern) (KArgs...), dim3 grid, int threads, int smem,
-            cudaStream_t s, Args &&...args)
+launch_pdl (int64_t block, void (*kern) (KArgs...), dim3 grid, int threads,
+            int smem, cudaStream_t s, Args &&...args)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -88,7 +92,7 @@ launch_pdl (void (*kern) (KArgs...), dim3 grid, int threads, int smem,
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = block <= ((int64_t) 128 << 20) ? 1 : 0;
   return cudaLaunchKernelEx (&cfg, kern, std::forward<Args> (args)...);
 }
 
