@@ -231,6 +231,46 @@ dfree (void *p)
   rt_add (g_rt.free_s, g_rt.frees, wall () - t0);
 }
 
+/* ---- polled host flags ---------------------------------------------------- */
+
+namespace
+{
+constexpr int FLAG_SLOTS = 64, FLAG_STRIDE = 16;   /* ints: a line each */
+std::mutex g_flag_mu;
+int *g_flag_page = nullptr;
+bool g_flag_tried = false;
+uint64_t g_flag_used = 0;
+} /* namespace */
+
+void
+HostFlag::take ()
+{
+  if (p) return;
+  std::lock_guard<std::mutex> lk (g_flag_mu);
+  if (!g_flag_tried) {
+    g_flag_tried = true;
+    void *q = nullptr;
+    if (cudaHostAlloc (&q, FLAG_SLOTS * FLAG_STRIDE * sizeof (int),
+                       cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess)
+      g_flag_page = (int *) q;
+    else
+      cudaGetLastError ();
+  }
+  if (!g_flag_page || g_flag_used == ~(uint64_t) 0) return;
+  const int k = __builtin_ctzll (~g_flag_used);
+  g_flag_used |= (uint64_t) 1 << k;
+  p = g_flag_page + k * FLAG_STRIDE;
+  *p = -1;
+}
+
+HostFlag::~HostFlag ()
+{
+  if (!p) return;
+  std::lock_guard<std::mutex> lk (g_flag_mu);
+  g_flag_used &= ~((uint64_t) 1 << ((p - g_flag_page) / FLAG_STRIDE));
+  p = nullptr;
+}
+
 /* ---- CSR helpers --------------------------------------------------------- */
 
 __global__ void

@@ -124,6 +124,8 @@ struct PcgCols
   int first, iter;
   double *hist;
   const int *fresh;
+  volatile int *host;   /* polled by the host: seq << 16 | active columns */
+  int seq;
 
   /* alpha from (p, q) */
   __device__ void prod (int c, double pq) const
@@ -178,7 +180,13 @@ struct PcgCols
     for (int c = threadIdx.x; c - (int) threadIdx.x < ld; c += blockDim.x)
       cnt += __syncthreads_count (
           c < ld && ((volatile int *) ival)[I_ACTIVE * cap + c] != 0);
-    if (threadIdx.x == 0) ival[I_NSLOT * cap] = cnt;
+    if (threadIdx.x == 0) {
+      ival[I_NSLOT * cap] = cnt;
+      if (host) {
+        *host = (int) (((unsigned) seq << 16) | (unsigned) cnt);
+        __threadfence_system ();
+      }
+    }
   }
 };
 
@@ -498,7 +506,7 @@ template <typename T, typename TZ>
 int
 launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
                  double rtol, int iter, double *hist, const int *fresh,
-                 ZWork &ws, cudaStream_t s)
+                 ZWork &ws, cudaStream_t s, int report)
 {
   const int64_t bytes = n * ld * (int64_t) sizeof (T);
   constexpr int W = Pack<T>::W;
@@ -507,8 +515,9 @@ launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
   const FlatShape f = sum_shape (nvec, n);
   const int smem = sum_smem (f, ld);
   const int want = std::min (flat_grid (f, n), ws.nblocks);
+  if (report) ws.nact.seq = (ws.nact.seq + 1) & 0x7fff;
   const PcgCols pc{ ws.scal.p, ws.ival.p, ws.cap, w, rtol, first, iter, hist,
-                    fresh };
+                    fresh, report ? ws.nact.p : nullptr, ws.nact.seq };
   int nb = 0;
   LGH_FLAT_DISPATCH (f.ch, {
     if (ld <= PCG_TAIL_COLS) {
@@ -580,7 +589,8 @@ launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
   const FlatShape f = flat_shape (nvec, Z.n);
   const int smem = sum_smem (f, ld);
   const int want = std::min (flat_grid (f, Z.n), ws.nblocks);
-  const PcgCols pc{ ws.scal.p, ws.ival.p, ws.cap, 0, 0., 0, 0, nullptr, nullptr };
+  const PcgCols pc{ ws.scal.p, ws.ival.p, ws.cap, 0, 0., 0, 0, nullptr, nullptr,
+                    nullptr, 0 };
   int nb = 0;
   auto run = [&] (auto idx, auto ch, auto tail) -> int {
     auto k = k_pcg_prod<T, decltype (idx), decltype (ch)::value,
@@ -645,6 +655,40 @@ launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P, int have_x,
   return 0;
 }
 
+/* the active columns of the last reported dots: the host spins on the flag
+ * that its kernel writes, a few us after the write; a copy of the count and
+ * a synchronisation left the device idle for 31 us a look.  Now and then it
+ * asks the stream, so that a failed launch ends the wait. */
+int
+pcg_wait_count (ZWork &ws, cudaStream_t s, int *count)
+{
+  if (!ws.nact.p) {
+    LGH_CUDA (cudaMemcpyAsync (count, ws.ival.p + I_NSLOT * ws.cap, sizeof (int),
+                               cudaMemcpyDeviceToHost, s));
+    LGH_CUDA (cudaStreamSynchronize (s));
+    return 0;
+  }
+  auto seen = [&] () {
+    const unsigned v = (unsigned) *ws.nact.p;
+    if ((int) (v >> 16) != ws.nact.seq) return false;
+    *count = (int) (v & 0xffffu);
+    return true;
+  };
+  for (long spin = 1;; spin++) {
+    if (seen ()) return 0;
+    if (spin % 4096 == 0) {
+      const cudaError_t e = cudaStreamQuery (s);
+      if (e == cudaSuccess) {
+        if (seen ()) return 0;
+        return set_error (LGH_ERR_GPU, "zsolve: the column count did not arrive");
+      }
+      if (e != cudaErrorNotReady)
+        return set_error (LGH_ERR_GPU, "zsolve: %s", cudaGetErrorString (e));
+      cudaGetLastError ();
+    }
+  }
+}
+
 #define LGH_PCG_INST(T)                                                      \
   template int launch_pcg_start<T> (int64_t, int, int, const T *, int,       \
                                     const double *, T *, float *,            \
@@ -660,7 +704,7 @@ launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P, int have_x,
   template int launch_pcg_dots<T, TZ> (int64_t, int, int, const T *,         \
                                        const TZ *, int, double, int,         \
                                        double *, const int *, ZWork &,       \
-                                       cudaStream_t);                        \
+                                       cudaStream_t, int);                        \
   template int launch_pcg_dir<T, TZ> (int64_t, int, const TZ *, T *, T *,    \
                                       int, ZWork &, cudaStream_t);
 LGH_PCG_INST (double)

@@ -352,6 +352,20 @@ struct ZsolveStats
   int last_maxit_hit = 0;
 };
 
+/* One int of pinned host memory that the device writes and the host polls
+ * (api_core.cu): slots of one page, taken once per process; p is null when
+ * none is left. */
+struct HostFlag
+{
+  volatile int *p = nullptr;
+  int seq = 0;              /* the last sequence number handed out */
+  HostFlag () = default;
+  HostFlag (const HostFlag &) = delete;
+  HostFlag &operator= (const HostFlag &) = delete;
+  ~HostFlag ();
+  void take ();
+};
+
 /* Workspace for blocked solves of width <= cap. */
 struct ZWork
 {
@@ -365,6 +379,7 @@ struct ZWork
   DBuf<int> ival;              /* active flags / counts */
   DBuf<unsigned> counters;
   DBuf<double> hist;           /* alpha/beta history for Lanczos */
+  HostFlag nact;               /* active columns after each iteration */
   int nblocks = 0;
   int alloc (int64_t n, int cap, int is32);
 };

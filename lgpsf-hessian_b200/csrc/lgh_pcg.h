@@ -25,7 +25,11 @@ int launch_pcg_start (int64_t n, int w, int ld, const T *B, int ldb,
 template <typename T, typename TZ>
 int launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb,
                      int first, double rtol, int iter, double *hist,
-                     const int *fresh, ZWork &ws, cudaStream_t s);
+                     const int *fresh, ZWork &ws, cudaStream_t s,
+                     int report = 0);
+/* report: the count of active columns also goes to the host, where this
+ * waits for it */
+int pcg_wait_count (ZWork &ws, cudaStream_t s, int *count);
 
 /* the direction, in place: p = z (PCG_P_FIRST), p = z + beta p; with it the
  * previous iteration's deferred x = alpha p_old (PCG_X_FIRST) or x += alpha

@@ -624,6 +624,7 @@ ZWork::alloc (int64_t n_, int cap_, int is32_)
   LGH_TRY (ival.alloc ((size_t) cap * I_NSLOT + 8));
   LGH_TRY (counters.alloc (8));
   LGH_TRY (hist.alloc (2 * 10000 + 16));
+  nact.take ();
   LGH_CUDA (cudaMemset (counters.p, 0, 8 * sizeof (unsigned)));
   LGH_CUDA (cudaMemset (ival.p, 0, ((size_t) cap * I_NSLOT + 8) * sizeof (int)));
   return 0;
@@ -757,13 +758,14 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
         if (!pc32) return mg_vcycle<T> (mg, bR, bZ, ldt, wt, s, tr);
         return mg_vcycle<float> (mg, R32, Z32, ldt, wt, s, nullptr);
       };
-      auto dots = [&] (int first, int it) -> int {
+      auto dots = [&] (int first, int it, int report) -> int {
         if constexpr (std::is_same<T, double>::value)
           if (pc32)
             return launch_pcg_dots<T, float> (n, wt, ldt, bR, Z32, first,
-                                              cfg.rtol, it, hist, nullptr, ws, s);
+                                              cfg.rtol, it, hist, nullptr, ws, s,
+                                              report);
         return launch_pcg_dots<T, T> (n, wt, ldt, bR, bZ, first, cfg.rtol, it,
-                                      hist, nullptr, ws, s);
+                                      hist, nullptr, ws, s, report);
       };
       auto direction = [&] (int flags) -> int {
         if constexpr (std::is_same<T, double>::value)
@@ -773,7 +775,7 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
       };
       LGH_TRY (launch_pcg_start<T> (n, wt, ldt, Xin + c0, ldx, rs_in, bR, R32, s));
       LGH_TRY (precond ());
-      LGH_TRY (dots (1, 0));
+      LGH_TRY (dots (1, 0, 0));
       int h_nact = 1;
       for (int it = 0; it < cfg.maxit; it++) {
         if (it == 0 && !pc32) {
@@ -794,37 +796,42 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
         if (tr) LGH_TRY (tr->end (s));
         LGH_TRY (precond ());
         if (tr) LGH_TRY (tr->begin (K_PCGX_DOTS, (1. + zw) * bw, s));
-        LGH_TRY (dots (0, it));
-        if (tr) LGH_TRY (tr->end (s));
+        /* look at the active columns at 1, 2, 4 and from 6 iterations on:
+         * an iteration past the last column's is lost */
         iters = it + 1;
-        if (iters % 2 == 0 || iters == cfg.maxit || iters <= 2) {
-          LGH_CUDA (cudaMemcpyAsync (&h_nact, nact, sizeof (int),
-                                     cudaMemcpyDeviceToHost, s));
-          LGH_CUDA (cudaStreamSynchronize (s));
-          if (tr) LGH_TRY (tr->drain ());
+        const int look = iters <= 2 || iters == 4 || iters >= 6
+                         || iters == cfg.maxit;
+        LGH_TRY (dots (0, it, look));
+        if (tr) LGH_TRY (tr->end (s));
+        if (look) {
+          LGH_TRY (pcg_wait_count (ws, s, &h_nact));
+          if (tr) {
+            LGH_CUDA (cudaStreamSynchronize (s));
+            LGH_TRY (tr->drain ());
+          }
           if (h_nact == 0) break;
         }
       }
+      /* the last iteration's deferred x += alpha p with the row scaling */
+      LGH_TRY (launch_pcg_out<T> (n, wt, ldt, bX, bP, iters > 1, rs_out, Y + c0,
+                                  ldy, ws, s));
       if (tr && !tr->ids.empty ()) {
         LGH_CUDA (cudaStreamSynchronize (s));
         LGH_TRY (tr->drain ());
       }
       if (st) {
-        its_h.resize (ldt);
-        std::vector<int> act_h (ldt);
-        LGH_CUDA (cudaMemcpyAsync (its_h.data (), ws.ival.p + I_ITS * cap,
-                                   ldt * sizeof (int), cudaMemcpyDeviceToHost, s));
-        LGH_CUDA (cudaMemcpyAsync (act_h.data (), ws.ival.p + I_ACTIVE * cap,
-                                   ldt * sizeof (int), cudaMemcpyDeviceToHost, s));
+        /* I_ACTIVE and I_ITS are neighbours: one copy */
+        its_h.resize (2 * cap);
+        LGH_CUDA (cudaMemcpyAsync (its_h.data (), ws.ival.p, 2 * cap * sizeof (int),
+                                   cudaMemcpyDeviceToHost, s));
         LGH_CUDA (cudaStreamSynchronize (s));
-        for (int c = 0; c < wt; c++) st->col_iters += act_h[c] ? iters : its_h[c];
+        const int *act_h = its_h.data () + I_ACTIVE * cap;
+        const int *col_h = its_h.data () + I_ITS * cap;
+        for (int c = 0; c < wt; c++) st->col_iters += act_h[c] ? iters : col_h[c];
         if (h_nact > 0) st->last_maxit_hit = 1;
         st->cols += wt;
         st->block_iters += iters;
       }
-      /* the last iteration's deferred x += alpha p with the row scaling */
-      LGH_TRY (launch_pcg_out<T> (n, wt, ldt, bX, bP, iters > 1, rs_out, Y + c0,
-                                  ldy, ws, s));
       continue;
     } else if (cfg.mode >= 2 && mg != nullptr) {
       /* Chebyshev around the V-cycle (modes 2/3: zsolve_impl.h:108-141
