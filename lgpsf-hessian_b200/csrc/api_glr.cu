@@ -725,7 +725,16 @@ batch_op (lgh_glr_t *g, int kind, int nshift, const double *c, int m,
              "batch: a row-sharded object runs the per-shift operations");
   LGH_CHECK (m > 0 && nshift > 0 && ldr >= n && ldx >= n, LGH_ERR_ARG_SIZ, "batch: size");
   std::vector<double> ch (nshift);
-  LGH_CUDA (cudaMemcpy (ch.data (), c, nshift * sizeof (double), cudaMemcpyDefault));
+  /* the shifts may lie on either side; a copy from ordinary host memory is
+   * the host's own (cudaMemcpyDefault took 330 us for it) */
+  cudaPointerAttributes pa;
+  if (cudaPointerGetAttributes (&pa, c) == cudaSuccess
+      && (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged)) {
+    LGH_CUDA (cudaMemcpy (ch.data (), c, nshift * sizeof (double), cudaMemcpyDefault));
+  } else {
+    cudaGetLastError ();
+    memcpy (ch.data (), c, nshift * sizeof (double));
+  }
   for (int i = 0; i < nshift; i++) LGH_TRY (check_shift (g, ch[i], "batch"));
   /* one shift and no W yet: the per-call formula of glr_common_impl.h:
    * 1007-1024 / 1084-1091 (the same Z-solves of width m, no W) */

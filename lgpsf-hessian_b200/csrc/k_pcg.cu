@@ -455,6 +455,90 @@ k_pcg_out (int64_t n, int w, int ld, const T *__restrict__ X,
   }
 }
 
+/* One step of the fixed-count iteration around an explicit preconditioner:
+ * x += b z, r -= b Z z (first: x = b z).  The step lengths are the
+ * Chebyshev recurrence's; its direction term a d is not part of the
+ * iteration, so no direction block is kept and r is updated in place, row
+ * by row, from the gathered z: 5 block transfers (7 with an x, d and r
+ * written beside the old ones: 37 us at 257 x 255 x 48 columns). */
+template <typename T, typename I, int CH, bool FIRST>
+__global__ void __launch_bounds__ (FLAT_THREADS, FlatOcc<CH>::v)
+k_pcg_cheb (int64_t n, const int64_t *__restrict__ rowptr,
+            const int32_t *__restrict__ colidx, const T *__restrict__ vals,
+            const T *__restrict__ Zb, T *__restrict__ R, T *__restrict__ X,
+            int ld, int nvec, int L, int rpc, T b)
+{
+  pdl_wait ();
+  constexpr int W = Pack<T>::W;
+  const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
+  const int64_t stride = (int64_t) gridDim.x * rpc;
+  int64_t i = (int64_t) blockIdx.x * rpc + rl;
+  if (rl >= rpc || i >= n) return;
+  I k0 = (I) rowptr[i], k1 = (I) rowptr[i + 1];
+  for (; i < n; i += stride) {
+    I k0n = 0, k1n = 0;
+    if (i + stride < n) {
+      k0n = (I) rowptr[i + stride];
+      k1n = (I) rowptr[i + stride + 1];
+    }
+    T acc[CH][W];
+    flat_zero<T, CH, W> (acc);
+    flat_gather<T, CH> (colidx, vals, k0, k1, 1, Zb, ld, lane, L, nvec, acc);
+#pragma unroll
+    for (int h = 0; h < CH; h++) {
+      const int vi = lane + h * L;
+      if (h < CH - 1 || vi < nvec) {
+        const int64_t o = i * ld + vi * W;
+        const Pack<T> z = ldp (Zb + o);
+        Pack<T> r = ldp (R + o), x = FIRST ? pzero<T> () : ldp (X + o);
+#pragma unroll
+        for (int e = 0; e < W; e++) {
+          x.v[e] = fma (b, z.v[e], x.v[e]);
+          r.v[e] = fma (-b, acc[h][e], r.v[e]);
+        }
+        stp (X + o, x);
+        stp (R + o, r);
+      }
+    }
+    k0 = k0n;
+    k1 = k1n;
+  }
+}
+
+/* the last step with the row scaling, Y = S (x + b z) over the w columns:
+ * its residual is not needed, so there is no product.  only: it is also
+ * the first (x = 0). */
+template <typename T>
+__global__ void __launch_bounds__ (256)
+k_pcg_cheb_out (int64_t n, int w, int ld, const T *__restrict__ Zb,
+                const T *__restrict__ X, T b, int only,
+                const double *__restrict__ rs, T *__restrict__ Y, int ldy,
+                int vec)
+{
+  pdl_wait ();
+  constexpr int W = Pack<T>::W;
+  const int nvec = (w + W - 1) / W;
+  const int64_t total = n * nvec;
+  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (int64_t) gridDim.x * blockDim.x) {
+    const int64_t i = e / nvec;
+    const int c = (int) (e - i * nvec) * W;
+    const double sc = rs ? rs[i] : 1.0;
+    const Pack<T> z = ldp (Zb + i * ld + c);
+    Pack<T> x = only ? pzero<T> () : ldp (X + i * ld + c);
+#pragma unroll
+    for (int k = 0; k < W; k++)
+      x.v[k] = (T) (sc * (double) fma (b, z.v[k], x.v[k]));
+    if (vec && c + W <= w) {
+      stp (Y + i * ldy + c, x);
+    } else {
+#pragma unroll
+      for (int k = 0; k < W; k++)
+        if (c + k < w) Y[i * ldy + c + k] = x.v[k];
+    }
+  }
+}
+
 /* CTAs of a streaming pass of `total` packs */
 int
 stream_grid (int64_t total)
@@ -655,6 +739,57 @@ launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P, int have_x,
   return 0;
 }
 
+template <typename T>
+int
+launch_pcg_cheb (const Csr &Z, const T *Zb, T *R, T *X, int ld, double b,
+                 int first, cudaStream_t s)
+{
+  constexpr int W = Pack<T>::W;
+  LGH_TRY (pcg_width (ld, W));
+  const int64_t bytes = Z.n * ld * (int64_t) sizeof (T);
+  const T *vals;
+  if constexpr (std::is_same<T, double>::value) vals = Z.vals;
+  else vals = Z.vals32;
+  const int nvec = ld / W;
+  const FlatShape f = flat_shape (nvec, Z.n);
+  auto run = [&] (auto idx, auto ch, auto fst) -> int {
+    auto k = k_pcg_cheb<T, decltype (idx), decltype (ch)::value,
+                        decltype (fst)::value>;
+    LGH_CUDA (launch_pdl (bytes, k,
+        fit_grid (k, flat_grid (f, Z.n), FLAT_THREADS, 0), FLAT_THREADS, 0, s,
+        Z.n, Z.rowptr, Z.colidx, vals, Zb, R, X, ld, nvec, f.L, f.rpc, (T) b));
+    LGH_LAUNCH_CHECK ();
+    return 0;
+  };
+  const bool big = Z.nnz >= INT32_MAX;
+  LGH_FLAT_DISPATCH (f.ch, {
+    using C = std::integral_constant<int, CH_>;
+    if (big) {
+      if (first) LGH_TRY (run (int64_t (), C (), std::true_type ()));
+      else LGH_TRY (run (int64_t (), C (), std::false_type ()));
+    } else {
+      if (first) LGH_TRY (run (int (), C (), std::true_type ()));
+      else LGH_TRY (run (int (), C (), std::false_type ()));
+    }
+  });
+  return 0;
+}
+
+template <typename T>
+int
+launch_pcg_cheb_out (int64_t n, int w, int ld, const T *Zb, const T *X, double b,
+                     int only, const double *rs, T *Y, int ldy, cudaStream_t s)
+{
+  constexpr int W = Pack<T>::W;
+  const int64_t bytes = n * ld * (int64_t) sizeof (T);
+  const int vec = ldy % W == 0 && (uintptr_t) Y % 16 == 0;
+  LGH_CUDA (launch_pdl (bytes, k_pcg_cheb_out<T>,
+      stream_grid (n * ((w + W - 1) / W)), 256, 0, s, n, w, ld, Zb, X, (T) b,
+      only, rs, Y, ldy, vec));
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
 /* the active columns of the last reported dots: the host spins on the flag
  * that its kernel writes, a few us after the write; a copy of the count and
  * a synchronisation left the device idle for 31 us a look.  Now and then it
@@ -700,6 +835,16 @@ pcg_wait_count (ZWork &ws, cudaStream_t s, int *count)
   template int launch_pcg_out<T> (int64_t, int, int, const T *, const T *,   \
                                   int, const double *, T *, int, ZWork &,    \
                                   cudaStream_t);
+#define LGH_PCG_INST_C(T)                                                    \
+  template int launch_pcg_cheb<T> (const Csr &, const T *, T *, T *, int,    \
+                                   double, int, cudaStream_t);               \
+  template int launch_pcg_cheb_out<T> (int64_t, int, int, const T *,         \
+                                       const T *, double, int,               \
+                                       const double *, T *, int,             \
+                                       cudaStream_t);
+LGH_PCG_INST_C (double)
+LGH_PCG_INST_C (float)
+#undef LGH_PCG_INST_C
 #define LGH_PCG_INST_Z(T, TZ)                                                \
   template int launch_pcg_dots<T, TZ> (int64_t, int, int, const T *,         \
                                        const TZ *, int, double, int,         \

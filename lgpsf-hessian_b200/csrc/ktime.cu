@@ -24,7 +24,7 @@ static double g_bytes[K_NKERN];
 
 static const char *g_names[K_NKERN] = {
   "k_pcg_pq", "k_pcg_upd", "k_cheb", "k_spmm", "k_pcg_init",
-  "k_pcg_prod", "k_pcg_resid", "k_pcg_dots", "k_chebx",
+  "k_pcg_prod", "k_pcg_resid", "k_pcg_dots", "k_pcg_cheb",
   "k_cheb@vcycle", "k_spmm<resid>@vcycle", "k_flat_mult@restrict",
   "k_spmm<acc>@prolong", "k_dense_apply@coarse", "k_cheb_tail@vcycle",
   "k_pcg_dir", "k_flat_resid@vcycle", "k_flat_second@vcycle",

@@ -57,6 +57,16 @@ int launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P,
                     int have_x, const double *rs, T *Y, int ldy, ZWork &ws,
                     cudaStream_t s);
 
+/* the fixed-count iteration around z = V(r): a step x += b z, r -= b Z z
+ * (first: x = b z), and the last step's x with the row scaling */
+template <typename T>
+int launch_pcg_cheb (const Csr &Z, const T *Zb, T *R, T *X, int ld, double b,
+                     int first, cudaStream_t s);
+template <typename T>
+int launch_pcg_cheb_out (int64_t n, int w, int ld, const T *Zb, const T *X,
+                         double b, int only, const double *rs, T *Y, int ldy,
+                         cudaStream_t s);
+
 } /* namespace lgh */
 
 #endif /* LGH_PCG_H */

@@ -439,71 +439,6 @@ k_cheb (ZK z, const T *__restrict__ vals, const T *__restrict__ vdv,
   }
 }
 
-/* Chebyshev with an explicit preconditioner: d_new = a d + b z on the fly
- * at neighbours, x += d_new, r_new = r - Z d_new */
-template <typename T, int CH>
-__global__ void __launch_bounds__ (ZS_THREADS, (CH * (16 / sizeof (T)) <= 8 ? 3 : 2))
-k_chebx (ZK z, const T *__restrict__ vals, const T *__restrict__ Zb,
-         T *__restrict__ X,
-         const T *__restrict__ Rold, T *__restrict__ Rnew,
-         const T *__restrict__ Dold, T *__restrict__ Dnew, int ld, int nvec,
-         int glog, T a, T b, int first)
-{
-  ZS_GROUP_SETUP ();
-  for (int64_t i = (int64_t) blockIdx.x * ngroups + group; i < z.n;
-       i += (int64_t) gridDim.x * ngroups) {
-    T acc[CH][W];
-#pragma unroll
-    for (int h = 0; h < CH; h++)
-#pragma unroll
-      for (int e = 0; e < W; e++) acc[h][e] = T (0);
-    const int64_t k0 = z.rowptr[i], k1 = z.rowptr[i + 1];
-    for (int64_t kb = k0; kb < k1; kb += G) {
-      const int cnt = (int) ((k1 - kb) < G ? (k1 - kb) : G);
-      int mc = 0;
-      T mv = T (0);
-      if (lane < cnt) {
-        mc = z.col[kb + lane];
-        mv = vals[kb + lane];
-      }
-      for (int t = 0; t < cnt; t++) {
-        const int c = __shfl_sync (gmask, mc, t, G);
-        const T v = __shfl_sync (gmask, mv, t, G);
-#pragma unroll
-        for (int h = 0; h < CH; h++) {
-          const int vi = lane + h * G;
-          if (vi < nvec) {
-            Pack<T> zj = ldp (Zb + (int64_t) c * ld + vi * W);
-            Pack<T> dj = first ? pzero<T> () : ldp (Dold + (int64_t) c * ld + vi * W);
-#pragma unroll
-            for (int e = 0; e < W; e++)
-              acc[h][e] = fma (v, fma (b, zj.v[e], a * dj.v[e]), acc[h][e]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < CH; h++) {
-      const int vi = lane + h * G;
-      if (vi < nvec) {
-        const int64_t o = i * ld + vi * W;
-        Pack<T> ri = ldp (Rold + o), x = ldp (X + o), zi = ldp (Zb + o);
-        Pack<T> di = first ? pzero<T> () : ldp (Dold + o);
-        Pack<T> dn, rn;
-#pragma unroll
-        for (int e = 0; e < W; e++) {
-          dn.v[e] = fma (b, zi.v[e], a * di.v[e]);
-          x.v[e] += dn.v[e];
-          rn.v[e] = ri.v[e] - acc[h][e];
-        }
-        stp (X + o, x);
-        stp (Dnew + o, dn);
-        stp (Rnew + o, rn);
-      }
-    }
-  }
-}
-
 /* ---- FP64 residual, R = S B - Z X (pads zero), per-column ||D^{-1} R|| and
  * ||D^{-1} S B|| (tests) ------------------------------------------------- */
 template <typename TO, int CH>
@@ -717,7 +652,8 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
     const int cap = ws.cap;
     int *nact = ws.ival.p + I_NSLOT * cap;
 
-    if (!mgpcg) {
+    const bool mgcheb = cfg.mode >= 2 && mg != nullptr && cfg.nit > 0;
+    if (!mgpcg && !mgcheb) {
       ZS_DISPATCH (ch, {
         auto kf = k_pcg_init<T, CH_>;
         set_smem_attr (kf, smem);
@@ -833,46 +769,44 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
         st->block_iters += iters;
       }
       continue;
-    } else if (cfg.mode >= 2 && mg != nullptr) {
-      /* Chebyshev around the V-cycle (modes 2/3: zsolve_impl.h:108-141
-       * with the AMG / harvested-hierarchy preconditioner) */
+    } else if (mgcheb) {
+      /* fixed count around the V-cycle (modes 2/3: zsolve_impl.h:108-141
+       * with the AMG / harvested-hierarchy preconditioner), at the step
+       * lengths b of the Chebyshev recurrence */
       const double theta = 0.5 * (cfg.lmax + cfg.lmin);
       const double delta = 0.5 * (cfg.lmax - cfg.lmin);
       const double sigma1 = theta / delta;
       double rho_old = 1.0 / sigma1;
-      T *Ro = bR, *Rn = bQ, *Do = bP0, *Dn = bP1;
+      LGH_TRY (launch_pcg_start<T> (n, wt, ldt, Xin + c0, ldx, rs_in, bR, nullptr, s));
       for (int k = 1; k <= cfg.nit; k++) {
-        double a, b;
-        if (k == 1) { a = 0.; b = 1.0 / theta; }
-        else {
+        double b = 1.0 / theta;
+        if (k > 1) {
           const double rho = 1.0 / (2.0 * sigma1 - rho_old);
-          a = rho * rho_old;
           b = 2.0 * rho / delta;
           rho_old = rho;
         }
         static thread_local KTrace ktc;
         KTrace *tc = (timing && k % 4 == 0) ? &ktc : nullptr;
-        LGH_TRY (mg_vcycle<T> (mg, Ro, bZ, ldt, wt, s, tc));
-        if (tc) LGH_TRY (tc->begin (K_CHEBX, zbytes + 7. * (double) n * wt * sizeof (T), s));
-        ZS_DISPATCH (ch, {
-          k_chebx<T, CH_><<<fit_grid (k_chebx<T, CH_>, grid, ZS_THREADS, 0),
-                                           ZS_THREADS, 0, s>>> (zk, vals, bZ, bX, Ro, Rn,
-                                                       Do, Dn, ldt, nvec, glog,
-                                                       (T) a, (T) b,
-                                                      (k == 1 ? CHEB_FIRST : 0)
-                                                      | CHEB_STORE_D);
-        });
-        LGH_LAUNCH_CHECK ();
+        LGH_TRY (mg_vcycle<T> (mg, bR, bZ, ldt, wt, s, tc));
+        if (k == cfg.nit) {
+          LGH_TRY (launch_pcg_cheb_out<T> (n, wt, ldt, bZ, bX, b, k == 1, rs_out,
+                                           Y + c0, ldy, s));
+        } else {
+          if (tc) LGH_TRY (tc->begin (K_CHEBX, zbytes + 5. * (double) n * wt * sizeof (T), s));
+          LGH_TRY (launch_pcg_cheb<T> (Z, bZ, bR, bX, ldt, b, k == 1, s));
+          if (tc) LGH_TRY (tc->end (s));
+        }
         if (tc) {
-          LGH_TRY (tc->end (s));
           LGH_CUDA (cudaStreamSynchronize (s));
           LGH_TRY (tc->drain ());
         }
-        std::swap (Ro, Rn);
-        std::swap (Do, Dn);
       }
-      iters = cfg.nit;
-      if (st) { st->col_iters += (long) iters * wt; st->cols += wt; }
+      if (st) {
+        st->col_iters += (long) cfg.nit * wt;
+        st->cols += wt;
+        st->block_iters += cfg.nit;
+      }
+      continue;
     } else if (cfg.mode <= 1) {
       T *Pold = bP0, *Pnew = bP1;
       int h_nact = 1;

@@ -89,3 +89,33 @@ def test_coarse_only(cuda_device, n, w):
     assert np.linalg.norm(Y - ref) < 1e-11 * np.linalg.norm(ref)
     Y, _ = L.test_vcycle(prior, X, fp32=True)
     assert np.linalg.norm(Y - ref) < 1e-5 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("w", [1, 3, 5, 33, 66, 131])
+@pytest.mark.parametrize("rtol", [0.5, 1e-2, 1e-6])
+@pytest.mark.parametrize("mode", [2, 3])
+def test_fixed_count(problems, mode, rtol, w):
+    """The fixed-count iteration, from two steps (the first and the last
+    step's own forms) to a dozen, against its steps x += b_k z, r -= b_k Z z
+    in numpy around the library's V-cycle, b_k the Chebyshev recurrence's
+    step lengths.  Rounding only: 1e-12."""
+    _, X, _ = problems["2d"]
+    Z = CASES["2d"]()
+    X = X[:, :w]
+    prior = L.Prior(Z=L.Mat(Z), mass=np.ones(Z["n"]),
+                    opts=L.prior_opts(blocked_mode=mode, cheb_rtol=rtol))
+    info = prior.info()
+    lo, hi, nit = info["lmin"], info["lmax"], info["nit"]
+    A = P.csr_to_dense(Z)
+    theta, delta = 0.5 * (hi + lo), 0.5 * (hi - lo)
+    s1 = theta / delta
+    b, rho = 1.0 / theta, 1.0 / s1
+    x, r = np.zeros_like(X), X.copy()
+    for k in range(nit):
+        if k > 0:
+            rho = 1.0 / (2.0 * s1 - rho)
+            b = 2.0 * rho / delta
+        z = L.test_vcycle(prior, r)[0]
+        x, r = x + b * z, r - b * (A @ z)
+    Y = prior.solve_block(X)
+    assert np.linalg.norm(Y - x) < 1e-12 * np.linalg.norm(x)
