@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "lgh_device.cuh"
+#include "lgh_flat.cuh"
 #include "lgh_internal.h"
 #include "lgh_strip.h"
 
@@ -124,109 +125,236 @@ k_scan_counts (int64_t m, const int64_t *__restrict__ counts,
   }
 }
 
-/* Y (rows r0 .. r0 + R) = strip s times X over the packs of this warp's
- * column slice: lane l owns packs l + 32 h, h < CH, of the slice starting
- * at pack 32 CH blockIdx.y.  The gathers are latency-bound, so the kernel
- * is built for bytes in flight: a warp stages the columns and values of 32
- * union entries in shared memory with coalesced loads, then issues the X
- * gathers of D entries (D CH = 8 packs per lane) before any of their FMAs,
- * reading the values back as shared-memory broadcasts. */
-template <typename T, typename TV, int R, int CH>
-__global__ void __launch_bounds__ (256, 2)
-k_strip_spmm (int64_t n, int64_t nstrips, const int64_t *__restrict__ sptr,
-              const int32_t *__restrict__ scol, const TV *__restrict__ sval,
-              const T *__restrict__ X, int ldx, T *__restrict__ Y, int ldy,
-              int nvec)
+/* FP64 blocks, strips of 8 rows: an 8-row strip times 8 columns of X is the
+ * m8n8k4 product of the tensor cores, four union entries at a time.  The A
+ * fragment is the entries' values as they lie (4 entries x 8 rows, 256
+ * contiguous bytes), the B fragment the gathered X rows (8 columns of each,
+ * whole sectors), so nothing is staged.  A warp takes one strip and NT x 8
+ * columns, U steps of loads in flight; the warps of a CTA are neighbouring
+ * column slices of the same strips.  The vector form of this (a warp per
+ * strip and 128 columns, values staged in shared memory, 16 FMAs per
+ * gathered pack) was bound by FP64 issue and the load pipe: 2.49 ms at
+ * 512^2 x 220 columns, now 1.42 (1.0 at the FP64 rate with the strips'
+ * zeros).  w: columns, a multiple of 2. */
+template <int NT, int U, int MINB>
+__global__ void __launch_bounds__ (256, MINB)
+k_strip_mma (int64_t n, int64_t items, int ncs, const int64_t *__restrict__ sptr,
+             const int32_t *__restrict__ scol, const double *__restrict__ sval,
+             const double *__restrict__ X, int ldx, double *__restrict__ Y,
+             int ldy, int w)
 {
-  constexpr int W = Pack<T>::W;
-  constexpr int D = (8 / CH) > 0 ? 8 / CH : 1;
-  __shared__ __align__ (16) TV sv_s[8][32 * R];
-  __shared__ int sc_s[8][32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t s = (int64_t) blockIdx.x * (blockDim.x >> 5) + wid;
-  if (s >= nstrips) return;
-  const int pbase = blockIdx.y * 32 * CH;
-  T acc[R][CH][W];
+  const int lane = threadIdx.x & 31;
+  const int64_t item = (int64_t) blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (item >= items) return;
+  const int64_t s = item / ncs;
+  const int c0 = (int) (item - s * ncs) * NT * 8;
+  const int kl = lane & 3, x = lane >> 2;
+  const int64_t k0 = sptr[s];
+  const int cnt = (int) (sptr[s + 1] - k0);
+  const int32_t *sc = scol + k0;
+  const double *sv = sval + k0 * 8;
+  double acc[NT][2];
 #pragma unroll
-  for (int r = 0; r < R; r++)
+  for (int t = 0; t < NT; t++) acc[t][0] = acc[t][1] = 0.;
+  for (int k = 0; k < cnt; k += 4 * U) {
+    double a[U], b[U][NT];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int kk = k + 4 * u + kl;
+      const bool in = kk < cnt;
+      const int c = in ? __ldg (sc + kk) : 0;
+      a[u] = in ? __ldg (sv + (size_t) kk * 8 + x) : 0.;
+      const double *xr = X + (int64_t) c * ldx + c0 + x;
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+        b[u][t] = (in && c0 + t * 8 + x < w) ? __ldg (xr + t * 8) : 0.;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+        asm volatile ("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
+                      "{%0, %1}, {%2}, {%3}, {%0, %1};"
+                      : "+d"(acc[t][0]), "+d"(acc[t][1])
+                      : "d"(a[u]), "d"(b[u][t]));
+  }
+  const int64_t i = s * 8 + x;
+  if (i >= n) return;
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    const int c = c0 + t * 8 + kl * 2;
+    double *y = Y + i * ldy + c;
+    if (c < w) {              /* w is even */
+      Pack<double> o;
+      o.v[0] = acc[t][0];
+      o.v[1] = acc[t][1];
+      stp (y, o);
+    }
+  }
+}
+
+/* two FP32 fused multiply-adds in one instruction, each rounded as fmaf */
+__device__ __forceinline__ void
+fma_f32x2 (unsigned long long &d, unsigned long long a, unsigned long long b)
+{
+  asm ("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+/* the product of U entries from the k-th (see k_strip_f32) */
+template <int CH, int U>
+__device__ __forceinline__ void
+strip_step_f32 (int k, const int32_t *__restrict__ sc,
+                const ulonglong2 *__restrict__ sv,
+                const float *__restrict__ X, int ldx, int lane, int L,
+                int nvec, unsigned long long (&acc)[4][CH][4])
+{
+  ulonglong2 v[U][2];
+  Pack<float> x[U][CH];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const float *xr = X + (int64_t) __ldg (sc + k + u) * ldx;
+#pragma unroll
+    for (int q = 0; q < 2; q++) v[u][q] = __ldg (sv + (size_t) (k + u) * 2 + q);
+#pragma unroll
+    for (int h = 0; h < CH; h++) {
+      const int vi = lane + h * L;
+      if (h < CH - 1 || vi < nvec) x[u][h] = ldp (xr + vi * 4);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++)
+#pragma unroll
+    for (int h = 0; h < CH; h++)
+      if (h < CH - 1 || lane + h * L < nvec)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const unsigned b = __float_as_uint (x[u][h].v[e]);
+          const unsigned long long bb = ((unsigned long long) b << 32) | b;
+          fma_f32x2 (acc[0][h][e], v[u][0].x, bb);
+          fma_f32x2 (acc[1][h][e], v[u][0].y, bb);
+          fma_f32x2 (acc[2][h][e], v[u][1].x, bb);
+          fma_f32x2 (acc[3][h][e], v[u][1].y, bb);
+        }
+}
+
+/* FP32 blocks, strips of 8 rows, in the flat mapping of lgh_flat.cuh over
+ * strips: a thread holds CH packs of all 8 rows, as 4 pairs of rows (the
+ * values lie in pairs; an X element is repeated once for four FMAs of two),
+ * U entries in flight.  The accumulators take 32 CH registers, so at 2
+ * packs two CTAs are resident and two entries in flight hide the gathers;
+ * one entry at 4 CTAs of single packs was bound by issue.  256^2 (118 union
+ * entries per strip), us at 131 / 220 columns: a warp per 64 packs 140 /
+ * 155, one pack 113 / 199, two packs with one entry 112 / 191, with two 88 /
+ * 146 (96 / 165 without the paired FMAs); 389 x 511 of 286 entries at 131
+ * columns 866 and 608. */
+template <int CH, int U>
+__global__ void __launch_bounds__ (FLAT_THREADS, 2)
+k_strip_f32 (int64_t n, int64_t nstrips, const int64_t *__restrict__ sptr,
+             const int32_t *__restrict__ scol, const float *__restrict__ sval,
+             const float *__restrict__ X, int ldx, float *__restrict__ Y,
+             int ldy, int nvec, int L, int rpc)
+{
+  const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
+  const int64_t s = (int64_t) blockIdx.x * rpc + rl;
+  if (rl >= rpc || s >= nstrips) return;
+  const int64_t k0 = sptr[s];
+  const int cnt = (int) (sptr[s + 1] - k0);
+  const int32_t *sc = scol + k0;
+  const ulonglong2 *sv = reinterpret_cast<const ulonglong2 *> (sval + k0 * 8);
+  unsigned long long acc[4][CH][4];
+#pragma unroll
+  for (int r = 0; r < 4; r++)
 #pragma unroll
     for (int h = 0; h < CH; h++)
 #pragma unroll
-      for (int e = 0; e < W; e++) acc[r][h][e] = T (0);
-  const int64_t k0 = sptr[s], k1 = sptr[s + 1];
-  TV *sv = sv_s[wid];
-  int *sc = sc_s[wid];
-  for (int64_t kb = k0; kb < k1; kb += 32) {
-    const int cnt = (int) ((k1 - kb) < 32 ? (k1 - kb) : 32);
-    /* stage: lane l takes entry kb + l (its column and R values) */
-    sc[lane] = lane < cnt ? scol[kb + lane] : 0;
+      for (int e = 0; e < 4; e++) acc[r][h][e] = 0;
+  int k = 0;
+  for (; k + U <= cnt; k += U)
+    strip_step_f32<CH, U> (k, sc, sv, X, ldx, lane, L, nvec, acc);
+  for (; k < cnt; k++)
+    strip_step_f32<CH, 1> (k, sc, sv, X, ldx, lane, L, nvec, acc);
+  const int64_t r0 = s * 8;
 #pragma unroll
-    for (int r = 0; r < R; r++)
-      sv[lane * R + r] = lane < cnt ? __ldg (sval + (kb + lane) * R + r) : TV (0);
-    __syncwarp ();
-    for (int t0 = 0; t0 < cnt; t0 += D) {
-      Pack<T> x[D][CH];
+  for (int r = 0; r < 8; r++) {
+    if (r0 + r >= n) break;
 #pragma unroll
-      for (int d = 0; d < D; d++) {
-        const int t = t0 + d;
-        const T *xr = X + (int64_t) sc[t < cnt ? t : 0] * ldx;
+    for (int h = 0; h < CH; h++) {
+      const int vi = lane + h * L;
+      if (h < CH - 1 || vi < nvec) {
+        Pack<float> o;
 #pragma unroll
-        for (int h = 0; h < CH; h++) {
-          const int vi = pbase + lane + 32 * h;
-          x[d][h] = (t < cnt && vi < nvec) ? ldp_nc (xr + vi * W) : pzero<T> ();
+        for (int e = 0; e < 4; e++)
+          o.v[e] = __uint_as_float ((unsigned) (acc[r / 2][h][e] >> (r & 1) * 32));
+        stp (Y + (r0 + r) * ldy + vi * 4, o);
+      }
+    }
+  }
+}
+
+/* strips of 2 or 4 rows (operators whose rows share few columns): the flat
+ * mapping over strips, a thread holding CH packs of all R rows.  FP64 at 56
+ * entries per row, 256^2 x 60 / 131 / 220 columns, R = 4: a warp per 128
+ * columns 208 / 228 / 246 us, here 99 / 177 / 269; R = 2: 343 / 373 / 398
+ * and 94 / 177 / 277. */
+template <typename T, int R, int CH>
+__global__ void __launch_bounds__ (FLAT_THREADS, sizeof (T) == 8 ? 3 : 4)
+k_strip_flat (int64_t n, int64_t nstrips, const int64_t *__restrict__ sptr,
+              const int32_t *__restrict__ scol, const T *__restrict__ sval,
+              const T *__restrict__ X, int ldx, T *__restrict__ Y, int ldy,
+              int nvec, int L, int rpc)
+{
+  constexpr int W = Pack<T>::W, VW = R < W ? R : W;
+  const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
+  if (rl >= rpc) return;
+  for (int64_t s = (int64_t) blockIdx.x * rpc + rl; s < nstrips;
+       s += (int64_t) gridDim.x * rpc) {
+    const int64_t k0 = sptr[s];
+    const int cnt = (int) (sptr[s + 1] - k0);
+    const int32_t *sc = scol + k0;
+    const T *sv = sval + k0 * R;
+    T acc[R][CH][W];
+#pragma unroll
+    for (int r = 0; r < R; r++) flat_zero<T, CH, W> (acc[r]);
+    for (int k = 0; k < cnt; k++) {
+      const T *xr = X + (int64_t) __ldg (sc + k) * ldx;
+      T v[R];
+      if constexpr (VW == W) {
+#pragma unroll
+        for (int r = 0; r < R; r += W) {
+          const Pack<T> p = ldp_nc (sv + (size_t) k * R + r);
+#pragma unroll
+          for (int e = 0; e < W; e++) v[r + e] = p.v[e];
         }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = __ldg (sv + (size_t) k * R + r);
       }
 #pragma unroll
-      for (int d = 0; d < D; d++) {
-        const int t = t0 + d;
-        if (t < cnt) {
-          /* the entry's R values as 16-byte shared broadcasts */
-          T v[R];
-          if constexpr (sizeof (TV) == 8) {
-#pragma unroll
-            for (int r = 0; r < R; r += 2) {
-              const double2 u = *reinterpret_cast<const double2 *> (sv + t * R + r);
-              v[r] = (T) u.x;
-              v[r + 1] = (T) u.y;
-            }
-          } else if constexpr (R % 4 == 0) {
-#pragma unroll
-            for (int r = 0; r < R; r += 4) {
-              const float4 u = *reinterpret_cast<const float4 *> (sv + t * R + r);
-              v[r] = (T) u.x;
-              v[r + 1] = (T) u.y;
-              v[r + 2] = (T) u.z;
-              v[r + 3] = (T) u.w;
-            }
-          } else {
-#pragma unroll
-            for (int r = 0; r < R; r++) v[r] = (T) sv[t * R + r];
-          }
+      for (int h = 0; h < CH; h++) {
+        const int vi = lane + h * L;
+        if (h < CH - 1 || vi < nvec) {
+          const Pack<T> x = ldp (xr + vi * W);
 #pragma unroll
           for (int r = 0; r < R; r++)
 #pragma unroll
-            for (int h = 0; h < CH; h++)
-#pragma unroll
-              for (int e = 0; e < W; e++)
-                acc[r][h][e] = fma (v[r], x[d][h].v[e], acc[r][h][e]);
+            for (int e = 0; e < W; e++)
+              acc[r][h][e] = fma (v[r], x.v[e], acc[r][h][e]);
         }
       }
     }
-    __syncwarp ();
-  }
-  const int64_t r0 = s * R;
+    const int64_t r0 = s * R;
 #pragma unroll
-  for (int r = 0; r < R; r++) {
-    if (r0 + r >= n) break;
-    T *yr = Y + (r0 + r) * ldy;
+    for (int r = 0; r < R; r++) {
+      if (r0 + r >= n) break;
 #pragma unroll
-    for (int h = 0; h < CH; h++) {
-      const int vi = pbase + lane + 32 * h;
-      if (vi < nvec) {
-        Pack<T> o;
+      for (int h = 0; h < CH; h++) {
+        const int vi = lane + h * L;
+        if (h < CH - 1 || vi < nvec) {
+          Pack<T> o;
 #pragma unroll
-        for (int e = 0; e < W; e++) o.v[e] = acc[r][h][e];
-        stp (yr + vi * W, o);
+          for (int e = 0; e < W; e++) o.v[e] = acc[r][h][e];
+          stp (Y + (r0 + r) * ldy + vi * W, o);
+        }
       }
     }
   }
@@ -349,24 +477,63 @@ strip_build (const Csr &A, int force_R, StripForm &S)
   return 0;
 }
 
-template <typename T, typename TV, int R>
+template <int NT, int U, int MINB>
 static int
-strip_dispatch (const StripForm &S, const TV *sval, const T *X, int ldx, T *Y,
-                int ldy, int nvec, cudaStream_t s)
+strip_mma (const StripForm &S, const double *X, int ldx, double *Y, int ldy,
+           int w, cudaStream_t s)
 {
-  /* one warp per strip and slice of 32 CH packs: R x CH = 16 accumulator
-   * packs and 8 packs of gathers in flight per lane within 128 registers
-   * (two CTAs of 8 warps per SM) */
-  constexpr int CH = 16 / R;
-  const int slices = (nvec + 32 * CH - 1) / (32 * CH);
-  const int64_t ctas = (S.nstrips + 7) / 8;
-  LGH_CHECK (ctas < (int64_t) INT32_MAX && slices < 65536, LGH_ERR_ARG_OUTOFRANGE,
+  const int ncs = (w + NT * 8 - 1) / (NT * 8);
+  const int64_t items = S.nstrips * ncs, ctas = (items + 7) / 8;
+  LGH_CHECK (ctas < (int64_t) INT32_MAX, LGH_ERR_ARG_OUTOFRANGE,
              "strip product: grid too large");
-  dim3 grid ((unsigned) ctas, (unsigned) slices);
-  k_strip_spmm<T, TV, R, CH><<<grid, 256, 0, s>>> (S.n, S.nstrips, S.sptr,
-                                                   S.scol, sval, X, ldx, Y,
-                                                   ldy, nvec);
+  k_strip_mma<NT, U, MINB><<<(unsigned) ctas, 256, 0, s>>> (
+      S.n, items, ncs, S.sptr, S.scol, S.sval, X, ldx, Y, ldy, w);
   LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+/* strip rows of 2 and 4; two packs per thread where there are that many */
+template <typename T, int R>
+static int
+strip_flat (const StripForm &S, const T *sval, const T *X, int ldx, T *Y,
+            int ldy, int nvec, cudaStream_t s)
+{
+  constexpr int W = Pack<T>::W;
+  for (int p0 = 0; p0 < nvec; p0 += FLAT_THREADS * 2) {
+    const int nv = std::min (nvec - p0, FLAT_THREADS * 2);
+    const FlatShape f = flat_shape_ch (nv, nv > 2 ? 2 : 1);
+    auto kern = f.ch == 2 ? k_strip_flat<T, R, 2> : k_strip_flat<T, R, 1>;
+    kern<<<flat_grid (f, S.nstrips), FLAT_THREADS, 0, s>>> (
+        S.n, S.nstrips, S.sptr, S.scol, sval, X + p0 * W, ldx, Y + p0 * W,
+        ldy, nv, f.L, f.rpc);
+    LGH_LAUNCH_CHECK ();
+  }
+  return 0;
+}
+
+/* FP32, 8 rows: two packs per thread, one where there are no more than two
+ * (256^2 x 5 columns: 75 us and 32) or some SM would not get its two CTAs
+ * (64^2 x 60: 68 us and 42; 256^2 x 131, 547 CTAs: 88 us and 116) */
+static int
+strip_f32 (const StripForm &S, const float *X, int ldx, float *Y, int ldy,
+           int nvec, cudaStream_t s)
+{
+  for (int p0 = 0; p0 < nvec; p0 += FLAT_THREADS) {
+    const int nv = std::min (nvec - p0, FLAT_THREADS);
+    FlatShape f = flat_shape_ch (nv, 2);
+    int64_t ctas = (S.nstrips + f.rpc - 1) / f.rpc;
+    if (nv <= 2 || ctas < 2 * num_sms ()) {
+      f = flat_shape_ch (nv, 1);
+      ctas = (S.nstrips + f.rpc - 1) / f.rpc;
+    }
+    LGH_CHECK (ctas < (int64_t) INT32_MAX, LGH_ERR_ARG_OUTOFRANGE,
+               "strip product: grid too large");
+    auto kern = f.ch == 2 ? k_strip_f32<2, 2> : k_strip_f32<1, 4>;
+    kern<<<(unsigned) ctas, FLAT_THREADS, 0, s>>> (
+        S.n, S.nstrips, S.sptr, S.scol, S.sval32, X + p0 * 4, ldx,
+        Y + p0 * 4, ldy, nv, f.L, f.rpc);
+    LGH_LAUNCH_CHECK ();
+  }
   return 0;
 }
 
@@ -385,9 +552,22 @@ launch_strip_spmm (const StripForm &S, const T *X, int ldx, T *Y, int ldy,
   const T *sv;
   if constexpr (sizeof (T) == 4) sv = S.sval32;
   else sv = S.sval;
-  if (S.R == 2) return strip_dispatch<T, T, 2> (S, sv, X, ldx, Y, ldy, nvec, s);
-  if (S.R == 4) return strip_dispatch<T, T, 4> (S, sv, X, ldx, Y, ldy, nvec, s);
-  return strip_dispatch<T, T, 8> (S, sv, X, ldx, Y, ldy, nvec, s);
+  if (S.R == 2) return strip_flat<T, 2> (S, sv, X, ldx, Y, ldy, nvec, s);
+  if (S.R == 4) return strip_flat<T, 4> (S, sv, X, ldx, Y, ldy, nvec, s);
+  if constexpr (sizeof (T) == 4) {
+    return strip_f32 (S, X, ldx, Y, ldy, nvec, s);
+  } else {
+    /* 112 columns per warp (the strip's columns and values read twice at
+     * 220 columns) against 32: 1.42 ms and 1.68 at 512^2 x 220, so the wide
+     * tile unless it pads a fifth more columns or leaves an SM with fewer
+     * than 16 warps (64^2 x 60 columns: 36 us and 17.5).  Whole packs are
+     * computed and stored, as everywhere. */
+    const int wp = nvec * W, n14 = (wp + 111) / 112, n4 = (wp + 31) / 32;
+    if (n14 * 112 * 5 > n4 * 32 * 6
+        || S.nstrips * n14 < (int64_t) num_sms () * 16)
+      return strip_mma<4, 2, 4> (S, X, ldx, Y, ldy, wp, s);
+    return strip_mma<14, 2, 2> (S, X, ldx, Y, ldy, wp, s);
+  }
 }
 
 template int launch_strip_spmm<double> (const StripForm &, const double *, int,
