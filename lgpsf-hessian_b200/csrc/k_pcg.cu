@@ -11,7 +11,9 @@
  * order, one warp per column.  Up to 32 columns the last CTA to finish does
  * that; wider blocks leave it to a small launch of one warp per column,
  * since one CTA takes 40 us over the 592 partials of 220 columns and the
- * launch 4 us (the whole product pass: 347 us with the last-CTA sum).
+ * launch 4 us (the whole product pass: 347 us with the last-CTA sum).  A
+ * column's scalars load while its partials do, and the partials all at
+ * once.
  *
  * The preconditioner's output may be FP32 (a mixed solve's float V-cycle):
  * the passes that read z widen it as they load it, which gives the values a
@@ -57,62 +59,81 @@ st32 (float *p, const Pack<T> &r)
     stp (p, r);
 }
 
-/* a thread's pack sums -> this CTA's column sums -> part[c * grid + block].
- * red: rpc * ld doubles and, behind them, 256 more. */
-template <typename T, int CH>
+/* a thread's pack sums (NS of them) -> this CTA's column sums ->
+ * part[q][c * grid + block].  red: NS rpc ld doubles and, behind them, 256
+ * more. */
+template <typename T, int CH, int NS>
 __device__ __forceinline__ void
-flat_colsum (const double (&acc)[CH][Pack<T>::W], int rl, int lane, int L,
-             int rpc, int nvec, int ld, double *red, double *part)
+flat_colsum (const double (&acc)[NS][CH][Pack<T>::W], int rl, int lane, int L,
+             int rpc, int nvec, int ld, double *red, double *partA,
+             double *partB)
 {
   constexpr int W = Pack<T>::W;
-  __syncthreads ();
+  const int cols = NS * ld;
   if (rl < rpc) {
 #pragma unroll
-    for (int h = 0; h < CH; h++) {
-      const int vi = lane + h * L;
-      if (h < CH - 1 || vi < nvec)
+    for (int q = 0; q < NS; q++)
 #pragma unroll
-        for (int e = 0; e < W; e++) red[rl * ld + vi * W + e] = acc[h][e];
-    }
+      for (int h = 0; h < CH; h++) {
+        const int vi = lane + h * L;
+        if (h < CH - 1 || vi < nvec)
+#pragma unroll
+          for (int e = 0; e < W; e++)
+            red[rl * cols + q * ld + vi * W + e] = acc[q][h][e];
+      }
   }
   __syncthreads ();
+  auto put = [&] (int c, double v) {
+    double *part = NS == 1 || c < ld ? partA + (size_t) c * gridDim.x
+                                     : partB + (size_t) (c - ld) * gridDim.x;
+    part[blockIdx.x] = v;
+  };
   /* narrow blocks hold many rows per CTA: nseg threads share a column */
   int nseg = 1;
-  while (nseg < 16 && 2 * nseg * ld <= FLAT_THREADS) nseg *= 2;
+  while (nseg < 16 && 2 * nseg * cols <= FLAT_THREADS) nseg *= 2;
   if (nseg == 1) {
-    for (int c = threadIdx.x; c < ld; c += FLAT_THREADS) {
+    for (int c = threadIdx.x; c < cols; c += FLAT_THREADS) {
       double s = 0.;
-      for (int r = 0; r < rpc; r++) s += red[r * ld + c];
-      part[(size_t) c * gridDim.x + blockIdx.x] = s;
+#pragma unroll 4
+      for (int r = 0; r < rpc; r++) s += red[r * cols + c];
+      put (c, s);
     }
     return;
   }
-  double *red2 = red + rpc * ld;
-  const int seg = threadIdx.x / ld, c = threadIdx.x - seg * ld;
+  double *red2 = red + rpc * cols;
+  const int seg = threadIdx.x / cols, c = threadIdx.x - seg * cols;
   if (seg < nseg) {
     double s = 0.;
-    for (int r = seg; r < rpc; r += nseg) s += red[r * ld + c];
-    red2[seg * ld + c] = s;
+#pragma unroll 4
+    for (int r = seg; r < rpc; r += nseg) s += red[r * cols + c];
+    red2[seg * cols + c] = s;
   }
   __syncthreads ();
-  if (threadIdx.x < ld) {
+  if (threadIdx.x < cols) {
     double s = 0.;
-    for (int q = 0; q < nseg; q++) s += red2[q * ld + threadIdx.x];
-    part[(size_t) threadIdx.x * gridDim.x + blockIdx.x] = s;
+    for (int q = 0; q < nseg; q++) s += red2[q * cols + threadIdx.x];
+    put (threadIdx.x, s);
   }
 }
 
-/* the sum of one column's nb partials by one warp, in a fixed order */
+/* the sum of one column's nb partials by one warp, in a fixed order; the
+ * loads of 512 partials go out together */
 __device__ __forceinline__ double
 part_sum (const double *part, int nb, int lane)
 {
-  double s[4] = { 0., 0., 0., 0. };
-  for (int b = lane; b < nb; b += 128) {
+  double s = 0.;
+  for (int b = lane; b < nb; b += 512) {
+    double v[16];
 #pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (b + 32 * q < nb) s[q] += __ldcg (part + b + 32 * q);
+    for (int q = 0; q < 16; q++)
+      v[q] = b + 32 * q < nb ? __ldcg (part + b + 32 * q) : 0.;
+#pragma unroll
+    for (int d = 8; d > 0; d /= 2)
+#pragma unroll
+      for (int q = 0; q < d; q++) v[q] += v[q + d];
+    s += v[0];
   }
-  return warp_sum ((s[0] + s[1]) + (s[2] + s[3]));
+  return warp_sum (s);
 }
 
 struct PcgCols
@@ -127,86 +148,111 @@ struct PcgCols
   volatile int *host;   /* polled by the host: seq << 16 | active columns */
   int seq;
 
-  /* alpha from (p, q) */
-  __device__ void prod (int c, double pq) const
+  /* a column's scalars, loaded before its partials are summed */
+  struct Old
   {
-    double *al = scal + S_ALPHA * cap;
-    int *act = ival + I_ACTIVE * cap;
-    if (act[c]) {
-      if (pq != 0. && isfinite (pq)) al[c] = scal[S_RZ * cap + c] / pq;
-      else { al[c] = 0.; act[c] = 0; }
-    } else {
-      al[c] = 0.;
+    int act, fresh;
+    double rz, n0;
+  };
+  __device__ Old load (int c, bool dots) const
+  {
+    Old o{ ival[I_ACTIVE * cap + c], 0, scal[S_RZ * cap + c], 0. };
+    if (dots) {
+      o.n0 = scal[S_NORM0 * cap + c];
+      o.fresh = fresh != nullptr ? fresh[c] : 0;
     }
+    return o;
   }
 
-  /* the start of a column, or beta and the convergence test */
-  __device__ void dots (int c, double srz, double szz) const
+  /* alpha from (p, q) */
+  __device__ int prod (int c, double pq, const Old &o) const
+  {
+    double al = 0.;
+    if (o.act) {
+      if (pq != 0. && isfinite (pq)) al = o.rz / pq;
+      else ival[I_ACTIVE * cap + c] = 0;
+    }
+    scal[S_ALPHA * cap + c] = al;
+    return 0;
+  }
+
+  /* the start of a column, or beta and the convergence test; returns
+   * whether the column is active */
+  __device__ int dots (int c, double srz, double szz, const Old &o) const
   {
     double *rz = scal + S_RZ * cap, *be = scal + S_BETA * cap;
     double *al = scal + S_ALPHA * cap, *n0 = scal + S_NORM0 * cap;
     int *act = ival + I_ACTIVE * cap, *its = ival + I_ITS * cap;
-    if (first || (fresh != nullptr && fresh[c])) {
+    if (first || o.fresh) {
+      const int on = (c < w && szz > 0.) ? 1 : 0;
       rz[c] = srz;
       n0[c] = sqrt (szz);
-      act[c] = (c < w && szz > 0.) ? 1 : 0;
+      act[c] = on;
       al[c] = 0.;
       be[c] = 0.;
       its[c] = 0;
-      return;
+      return on;
     }
-    if (!act[c]) { be[c] = 0.; return; }
-    const double b = (rz[c] != 0.) ? srz / rz[c] : 0.;
+    if (!o.act) { be[c] = 0.; return 0; }
+    const double b = (o.rz != 0.) ? srz / o.rz : 0.;
     if (hist != nullptr && c == 0 && iter < 10000) {
       hist[2 * iter] = al[0];
       hist[2 * iter + 1] = b;
     }
     rz[c] = srz;
-    be[c] = b;
     /* a converged column keeps its alpha: its x update may still be
      * pending (launch_pcg_dir or launch_pcg_out applies it), and the next
      * product zeroes alpha for inactive columns */
-    if (sqrt (szz) <= rtol * n0[c] || srz == 0.) {
+    if (sqrt (szz) <= rtol * o.n0 || srz == 0.) {
       act[c] = 0;
       be[c] = 0.;
       its[c] = iter + 1;
+      return 0;
     }
+    be[c] = b;
+    return 1;
   }
 
-  /* the active columns, counted by the whole CTA */
-  __device__ void count (int ld) const
+  /* the count of active columns, to the device's slot and the host's */
+  __device__ void report (int cnt) const
   {
-    int cnt = 0;
-    for (int c = threadIdx.x; c - (int) threadIdx.x < ld; c += blockDim.x)
-      cnt += __syncthreads_count (
-          c < ld && ((volatile int *) ival)[I_ACTIVE * cap + c] != 0);
-    if (threadIdx.x == 0) {
-      ival[I_NSLOT * cap] = cnt;
-      if (host) {
-        *host = (int) (((unsigned) seq << 16) | (unsigned) cnt);
-        __threadfence_system ();
-      }
-    }
+    ival[I_NSLOT * cap] = cnt;
+    if (host) *host = (int) (((unsigned) seq << 16) | (unsigned) cnt);
   }
 };
 
 /* columns up to which the last CTA sums the partials */
 constexpr int PCG_TAIL_COLS = 32;
 
+/* columns c0, c0 + cstep, ... of one warp; returns its active ones (lane 0) */
 template <bool DOTS>
-__device__ __forceinline__ void
+__device__ __forceinline__ int
 pcg_columns (const double *partA, const double *partB, int nb, int c0, int cstep,
              int ld, const PcgCols &pc)
 {
   const int lane = threadIdx.x & 31;
+  int on = 0;
   for (int c = c0; c < ld; c += cstep) {
+    const PcgCols::Old o = pc.load (c, DOTS);
     const double a = part_sum (partA + (size_t) c * nb, nb, lane);
     const double b = DOTS ? part_sum (partB + (size_t) c * nb, nb, lane) : 0.;
-    if (lane == 0) {
-      if (DOTS) pc.dots (c, a, b);
-      else pc.prod (c, a);
-    }
+    if (lane == 0) on += DOTS ? pc.dots (c, a, b, o) : pc.prod (c, a, o);
   }
+  return on;
+}
+
+/* the sum of the warps' lane 0 values, in thread 0 */
+__device__ __forceinline__ int
+warps_total (int v)
+{
+  __shared__ int sh[FLAT_THREADS / 32];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads ();
+  int t = 0;
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < FLAT_THREADS / 32; q++) t += sh[q];
+  return t;
 }
 
 template <bool DOTS>
@@ -215,28 +261,37 @@ pcg_tail (const double *partA, const double *partB, int ld, unsigned *counter,
           const PcgCols &pc)
 {
   if (!last_block_ticket (counter)) return;
-  pcg_columns<DOTS> (partA, partB, gridDim.x, threadIdx.x >> 5,
-                     FLAT_THREADS / 32, ld, pc);
-  __syncthreads ();
-  if (DOTS) pc.count (ld);
+  const int on = pcg_columns<DOTS> (partA, partB, gridDim.x, threadIdx.x >> 5,
+                                    FLAT_THREADS / 32, ld, pc);
+  if (DOTS) {
+    const int cnt = warps_total (on);
+    if (threadIdx.x == 0) pc.report (cnt);
+  }
   if (threadIdx.x == 0) *counter = 0u;
 }
 
-/* the partials of a wide block: one warp per column over all CTAs; the
- * last CTA counts the active columns */
+/* the partials of a wide block: one warp per column over all CTAs.  The
+ * active columns are counted in the ticket itself (tickets above bit 16,
+ * columns below), so the last CTA reads nothing back. */
 template <bool DOTS>
 __global__ void __launch_bounds__ (FLAT_THREADS)
 k_pcg_columns (const double *partA, const double *partB, int nb, int ld,
                unsigned *counter, PcgCols pc)
 {
   pdl_wait ();
-  pcg_columns<DOTS> (partA, partB, nb,
-                     (int) (blockIdx.x * (FLAT_THREADS / 32) + (threadIdx.x >> 5)),
-                     (int) (gridDim.x * (FLAT_THREADS / 32)), ld, pc);
+  const int on = pcg_columns<DOTS> (
+      partA, partB, nb,
+      (int) (blockIdx.x * (FLAT_THREADS / 32) + (threadIdx.x >> 5)),
+      (int) (gridDim.x * (FLAT_THREADS / 32)), ld, pc);
   if (!DOTS) return;
-  if (!last_block_ticket (counter)) return;
-  pc.count (ld);
-  if (threadIdx.x == 0) *counter = 0u;
+  const int cnt = warps_total (on);
+  if (threadIdx.x == 0) {
+    const unsigned t = atomicAdd (counter, (1u << 16) + (unsigned) cnt);
+    if (t >> 16 == gridDim.x - 1) {
+      *counter = 0u;
+      pc.report ((int) (t & 0xffffu) + cnt);
+    }
+  }
 }
 
 /* ---- the passes ----------------------------------------------------------- */
@@ -281,9 +336,9 @@ k_pcg_dots (int64_t n, int ld, int nvec, int L, int rpc, const T *__restrict__ R
   constexpr int W = Pack<T>::W;
   extern __shared__ double red[];
   const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
-  double arz[CH][W], azz[CH][W];
-  flat_zero<double, CH, W> (arz);
-  flat_zero<double, CH, W> (azz);
+  double acc[2][CH][W];   /* (r, z), (z, z) */
+  flat_zero<double, CH, W> (acc[0]);
+  flat_zero<double, CH, W> (acc[1]);
   if (rl < rpc)
     for (int64_t i = (int64_t) blockIdx.x * rpc + rl; i < n;
          i += (int64_t) gridDim.x * rpc) {
@@ -295,14 +350,13 @@ k_pcg_dots (int64_t n, int ld, int nvec, int L, int rpc, const T *__restrict__ R
           const Pack<T> z = ldz<T, TZ> (Zb + i * ld + vi * W);
 #pragma unroll
           for (int e = 0; e < W; e++) {
-            arz[h][e] += (double) r.v[e] * (double) z.v[e];
-            azz[h][e] += (double) z.v[e] * (double) z.v[e];
+            acc[0][h][e] += (double) r.v[e] * (double) z.v[e];
+            acc[1][h][e] += (double) z.v[e] * (double) z.v[e];
           }
         }
       }
     }
-  flat_colsum<T, CH> (arz, rl, lane, L, rpc, nvec, ld, red, partA);
-  flat_colsum<T, CH> (azz, rl, lane, L, rpc, nvec, ld, red, partB);
+  flat_colsum<T, CH, 2> (acc, rl, lane, L, rpc, nvec, ld, red, partA, partB);
   if (TAIL) pcg_tail<true> (partA, partB, ld, counter, pc);
 }
 
@@ -354,8 +408,8 @@ k_pcg_prod (int64_t n, const int64_t *__restrict__ rowptr,
   extern __shared__ double red[];
   const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
   const int64_t stride = (int64_t) gridDim.x * rpc;
-  double apq[CH][W];
-  flat_zero<double, CH, W> (apq);
+  double apq[1][CH][W];
+  flat_zero<double, CH, W> (apq[0]);
   int64_t i = (int64_t) blockIdx.x * rpc + rl;
   if (rl < rpc && i < n) {
     I k0 = (I) rowptr[i], k1 = (I) rowptr[i + 1];
@@ -378,7 +432,7 @@ k_pcg_prod (int64_t n, const int64_t *__restrict__ rowptr,
 #pragma unroll
           for (int e = 0; e < W; e++) {
             q.v[e] = acc[h][e];
-            apq[h][e] += (double) p.v[e] * (double) q.v[e];
+            apq[0][h][e] += (double) p.v[e] * (double) q.v[e];
           }
           stp (Q + o, q);
         }
@@ -387,7 +441,7 @@ k_pcg_prod (int64_t n, const int64_t *__restrict__ rowptr,
       k1 = k1n;
     }
   }
-  flat_colsum<T, CH> (apq, rl, lane, L, rpc, nvec, ld, red, partA);
+  flat_colsum<T, CH, 1> (apq, rl, lane, L, rpc, nvec, ld, red, partA, nullptr);
   if (TAIL) pcg_tail<false> (partA, nullptr, ld, counter, pc);
 }
 
@@ -557,9 +611,9 @@ sum_shape (int nvec, int64_t n)
 }
 
 int
-sum_smem (const FlatShape &f, int ld)
+sum_smem (const FlatShape &f, int cols)
 {
-  return (f.rpc * ld + FLAT_THREADS) * (int) sizeof (double);
+  return (f.rpc * cols + FLAT_THREADS) * (int) sizeof (double);
 }
 
 int
@@ -597,7 +651,7 @@ launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
   LGH_TRY (pcg_width (ld, W));
   const int nvec = ld / W;
   const FlatShape f = sum_shape (nvec, n);
-  const int smem = sum_smem (f, ld);
+  const int smem = sum_smem (f, 2 * ld);
   const int want = std::min (flat_grid (f, n), ws.nblocks);
   if (report) ws.nact.seq = (ws.nact.seq + 1) & 0x7fff;
   const PcgCols pc{ ws.scal.p, ws.ival.p, ws.cap, w, rtol, first, iter, hist,
@@ -611,6 +665,9 @@ launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
           ws.partB.p, ws.counters.p + 1, pc));
     } else {
       auto k = k_pcg_dots<T, TZ, CH_, false>;
+      if (smem > 48 * 1024)   /* FP32 blocks of over 2900 columns */
+        LGH_CUDA (cudaFuncSetAttribute (
+            k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       nb = fit_grid (k, want, FLAT_THREADS, smem);
       LGH_CUDA (launch_pdl (bytes, k, nb, FLAT_THREADS, smem, s, n, ld, nvec, f.L,
           f.rpc, R, Zb, ws.partA.p, ws.partB.p, ws.counters.p + 1, pc));
@@ -687,7 +744,7 @@ launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
     LGH_LAUNCH_CHECK ();
     return 0;
   };
-  const bool tail = ld <= PCG_TAIL_COLS, big = Z.nnz >= INT32_MAX;
+  const bool tail = ld <= PCG_TAIL_COLS, big = Z.nnz >= FLAT_NNZ_MAX;
   LGH_FLAT_DISPATCH (f.ch, {
     using C = std::integral_constant<int, CH_>;
     if (big) {
@@ -761,7 +818,7 @@ launch_pcg_cheb (const Csr &Z, const T *Zb, T *R, T *X, int ld, double b,
     LGH_LAUNCH_CHECK ();
     return 0;
   };
-  const bool big = Z.nnz >= INT32_MAX;
+  const bool big = Z.nnz >= FLAT_NNZ_MAX;
   LGH_FLAT_DISPATCH (f.ch, {
     using C = std::integral_constant<int, CH_>;
     if (big) {

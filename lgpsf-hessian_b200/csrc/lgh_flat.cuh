@@ -12,7 +12,12 @@
  * the kernels are bound by L1 wavefronts and by how many warps are
  * resident, so registers spent on more entries in flight cost more than
  * they hide (first smoothing step, 512^2 x 220 columns FP64: 180 us with
- * one entry in flight at 4 CTAs per SM, 206 with two, 275 with five).
+ * one entry in flight at 4 CTAs per SM, 206 with two, 275 with five).  One
+ * pack per thread is the other regime, narrow blocks or few rows on a chip
+ * that is not full: there five entries go out at once (one solve of one
+ * column at 512^2: 3.18 ms with one, 2.92 with four at 6 CTAs per SM, 2.83
+ * at 5, 2.76 with five at 5, 2.93 with eight at 4; 64^2 x 1: 0.53, 0.48,
+ * 0.47, 0.46, 0.47).
  * Packs per thread: 4 above 32 packs, 2 down to 3, 1 below (4 columns
  * FP64); fewer where the grid would not reach two CTAs per SM.  At 64
  * columns FP64, 2 packs 59 us, 4 packs 62, 1 pack 72; at 4 columns, 1 pack
@@ -30,6 +35,7 @@ namespace lgh
 {
 
 constexpr int FLAT_THREADS = 256;
+constexpr int FLAT_BATCH = 5;           /* entries in flight at one pack */
 constexpr int FLAT_MAXPACKS = FLAT_THREADS * 4;   /* packs of one launch */
 
 /* threads per row, packs per thread, rows per CTA */
@@ -70,11 +76,12 @@ flat_grid (const FlatShape &f, int64_t n)
 }
 
 /* CTAs per SM each shape is built for: 4 packs fit 64 registers, 2 packs
- * 42, 1 pack 32 (without spills in the single-gather kernels) */
+ * 42 (without spills in the single-gather kernels), 1 pack with its batch
+ * 48 */
 template <int CH>
 struct FlatOcc
 {
-  static constexpr int v = CH == 4 ? 4 : (CH == 3 ? 5 : (CH == 2 ? 6 : 8));
+  static constexpr int v = CH == 4 ? 4 : (CH == 3 ? 5 : (CH == 2 ? 6 : 5));
 };
 
 /* one row's product: acc += sum_k v_k X[c_k, :] over its entries k0, k0 +
@@ -87,6 +94,32 @@ flat_gather (const int32_t *__restrict__ ci, const T *__restrict__ va, I k0,
              int L, int nvec, T (&acc)[CH][Pack<T>::W])
 {
   constexpr int W = Pack<T>::W;
+  if constexpr (CH == 1) {
+    /* bound by latency: a batch of entries' loads go out together.  Past
+     * the row's end an entry of the row is loaded again and not used, so
+     * the sum is the one of the loop below */
+    for (I k = k0; k < k1; k += FLAT_BATCH * step) {
+      int c[FLAT_BATCH];
+      T v[FLAT_BATCH];
+      Pack<T> x[FLAT_BATCH];
+#pragma unroll
+      for (int u = 0; u < FLAT_BATCH; u++) {
+        const I ku = k + u * step < k1 ? k + u * step : k;
+        c[u] = __ldg (ci + ku);
+        v[u] = __ldg (va + ku);
+      }
+#pragma unroll
+      for (int u = 0; u < FLAT_BATCH; u++)
+        x[u] = ldp (X + (int64_t) c[u] * ld + lane * W);
+#pragma unroll
+      for (int u = 0; u < FLAT_BATCH; u++)
+        if (k + u * step < k1)
+#pragma unroll
+          for (int e = 0; e < W; e++)
+            acc[0][e] = fma (v[u], x[u].v[e], acc[0][e]);
+    }
+    return;
+  }
   for (I k = k0; k < k1; k += step) {
     const int c = __ldg (ci + k);
     const T v = __ldg (va + k);

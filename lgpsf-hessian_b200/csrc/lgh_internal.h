@@ -221,6 +221,10 @@ fit_grid (K kern, int want, int threads, int smem)
   return (r > 0 && r < want) ? r : want;
 }
 
+/* entries up to which 32-bit entry offsets hold, with a batch's step past a
+ * row's end (lgh_flat.cuh) */
+constexpr int64_t FLAT_NNZ_MAX = INT32_MAX - 8192;
+
 /* Y += A X (mode 1) or Y = B - A X (mode 2) */
 template <typename T>
 int launch_spmm_mode (const Csr &A, const T *X, int ldx, T *Y, int ldy, int w,

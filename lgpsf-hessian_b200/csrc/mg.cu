@@ -897,7 +897,7 @@ row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
                                cudaMemcpyDeviceToHost, s) != cudaSuccess
               || cudaStreamSynchronize (s) != cudaSuccess))
     rc = set_error (LGH_ERR_GPU, "mg: sparse product sizes");
-  if (!rc && out.nnz >= INT32_MAX) *fits = 0;
+  if (!rc && out.nnz >= FLAT_NNZ_MAX) *fits = 0;
   if (!rc && *fits) {
     rc = dalloc ((void **) &out.colidx, (size_t) out.nnz * sizeof (int32_t) + 16);
     if (!rc) rc = dalloc ((void **) &out.vals, (size_t) out.nnz * sizeof (double) + 16);
@@ -913,7 +913,8 @@ row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
 static int
 smoothed_correction (MgLevel &lv)
 {
-  if (lv.A.nnz >= INT32_MAX || lv.P.nnz >= INT32_MAX || lv.R.nnz >= INT32_MAX)
+  if (lv.A.nnz >= FLAT_NNZ_MAX || lv.P.nnz >= FLAT_NNZ_MAX
+      || lv.R.nnz >= FLAT_NNZ_MAX)
     return 0;
   double b1, a2, b2;
   cheb2_coeffs (lv, &b1, &a2, &b2);
