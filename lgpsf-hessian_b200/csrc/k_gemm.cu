@@ -735,9 +735,9 @@ launch_shift_combine_variant (int variant, int64_t n, int kept, int m,
  * several k steps in flight; the warps' partial tiles are added in warp
  * order through shared memory.  A 64 x 64 tile with one serial pass over n0
  * left 9 to 36 CTAs on the chip: 45 us at n0 = 559 x 220 columns and 46 us
- * at 704 x 1; now see the launch rule below. */
-template <typename T, int MT, int NT, int NW>
-__global__ void __launch_bounds__ (NW * 32)
+ * at 704 x 1, now 10.6 and 4.3 (back to back launches alone take 4). */
+template <typename T, int MT, int NT, int NW, int U>
+__global__ void __launch_bounds__ (NW * 32, NT > 1 ? 2 : 1)
 k_dense_apply (int n0, const double *__restrict__ Ainv, const T *__restrict__ B,
                T *__restrict__ Y, int w, int ld)
 {
@@ -756,7 +756,7 @@ k_dense_apply (int n0, const double *__restrict__ Ainv, const T *__restrict__ B,
   for (int a = 0; a < MT; a++)
 #pragma unroll
     for (int b = 0; b < NT; b++) acc[a][b][0] = acc[a][b][1] = 0.;
-#pragma unroll 4
+#pragma unroll U
   for (int s = s0; s < s1; s++) {
     const int k = 4 * s + kl;
     double a[MT], b[NT];
@@ -797,16 +797,16 @@ k_dense_apply (int n0, const double *__restrict__ Ainv, const T *__restrict__ B,
   }
 }
 
-template <typename T, int MT, int NT, int NW>
+template <typename T, int MT, int NT, int NW, int U>
 static int
 dense_apply_tile (int n0, const double *Ainv, const T *B, T *Y, int w, int ld,
                   cudaStream_t s)
 {
   const int smem = NW * 64 * MT * NT * (int) sizeof (double);
-  static_assert (NW * 64 * MT * NT * 8 <= 48 * 1024, "static shared limit");
+  static_assert (NW * 64 * MT * NT * 8 <= 48 * 1024, "default shared limit");
   dim3 grid ((unsigned) ((n0 + 8 * MT - 1) / (8 * MT)),
              (unsigned) ((ld + 8 * NT - 1) / (8 * NT)));
-  LGH_CUDA (launch_pdl (0, k_dense_apply<T, MT, NT, NW>, grid, NW * 32, smem, s, n0,
+  LGH_CUDA (launch_pdl (0, k_dense_apply<T, MT, NT, NW, U>, grid, NW * 32, smem, s, n0,
                         Ainv, B, Y, w, ld));
   LGH_LAUNCH_CHECK ();
   return 0;
@@ -817,12 +817,17 @@ int
 launch_dense_apply (int n0, const double *Ainv, const T *B, T *Y, int w, int ld,
                     cudaStream_t s)
 {
-  /* narrow blocks: 16 rows x 8 columns over 16 warps, so that n0 = 560
-   * still makes 35 CTAs and a warp's share of the terms stays near 10
-   * steps; wide ones: 32 x 32 over 4 warps (126 CTAs at 559 x 220) */
-  if (ld <= 8) return dense_apply_tile<T, 2, 1, 16> (n0, Ainv, B, Y, w, ld, s);
-  if (ld <= 64) return dense_apply_tile<T, 2, 2, 16> (n0, Ainv, B, Y, w, ld, s);
-  return dense_apply_tile<T, 4, 4, 4> (n0, Ainv, B, Y, w, ld, s);
+  /* one tile of columns: 8 rows over 16 warps while that is one wave
+   * (n0 = 704: 4.3 us, 6.3 with 16 rows; 1500: 8.1 and 6.3).  Up to 64
+   * columns 16 x 16 over 16 warps (32 KB of partials), wider 32 x 16 over 8:
+   * us in FP64 of the two, and of 32 x 32 over 4 warps, at 704 x 33 columns
+   * 6.3, 8.3, 14.5; 1500 x 60 16.5, 18.6, 24.7; 559 x 132 11.4, 10.4, 12.5;
+   * 559 x 220 12.5, 10.6, 12.8; FP32 at 1500 x 90 20.6, 18.6, 35.0 */
+  if (ld <= 8 && n0 <= 8 * num_sms ())
+    return dense_apply_tile<T, 1, 1, 16, 8> (n0, Ainv, B, Y, w, ld, s);
+  if (ld <= 8) return dense_apply_tile<T, 2, 1, 16, 4> (n0, Ainv, B, Y, w, ld, s);
+  if (ld <= 64) return dense_apply_tile<T, 2, 2, 16, 2> (n0, Ainv, B, Y, w, ld, s);
+  return dense_apply_tile<T, 4, 2, 8, 4> (n0, Ainv, B, Y, w, ld, s);
 }
 
 template int launch_dense_apply<double> (int, const double *, const double *,
