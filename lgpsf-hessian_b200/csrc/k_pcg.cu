@@ -378,13 +378,11 @@ k_pcg_dir (int64_t n, int ld, const TZ *__restrict__ Zb, T *__restrict__ P,
     Pack<T> z = ldz<T, TZ> (Zb + o);
     if constexpr (!(FLAGS & PCG_P_FIRST)) {
       const Pack<T> p = ldp (P + o);
-      if constexpr (FLAGS & (PCG_X_FIRST | PCG_X_ADD)) {
-        Pack<T> x = (FLAGS & PCG_X_ADD) ? ldp (X + o) : pzero<T> ();
+      Pack<T> x = (FLAGS & PCG_X_ADD) ? ldp (X + o) : pzero<T> ();
 #pragma unroll
-        for (int k = 0; k < W; k++)
-          x.v[k] = fma ((T) alpha[vi * W + k], p.v[k], x.v[k]);
-        stp (X + o, x);
-      }
+      for (int k = 0; k < W; k++)
+        x.v[k] = fma ((T) alpha[vi * W + k], p.v[k], x.v[k]);
+      stp (X + o, x);
 #pragma unroll
       for (int k = 0; k < W; k++)
         z.v[k] = fma ((T) beta[vi * W + k], p.v[k], z.v[k]);
@@ -445,11 +443,10 @@ k_pcg_prod (int64_t n, const int64_t *__restrict__ rowptr,
   if (TAIL) pcg_tail<false> (partA, nullptr, ld, counter, pc);
 }
 
-template <typename T, bool WITHX>
+template <typename T>
 __global__ void __launch_bounds__ (256)
 k_pcg_resid (int64_t n, int ld, T *__restrict__ R, const T *__restrict__ Qv,
-             float *__restrict__ R32, T *__restrict__ X,
-             const T *__restrict__ P, const double *__restrict__ alpha)
+             float *__restrict__ R32, const double *__restrict__ alpha)
 {
   pdl_wait ();
   constexpr int W = Pack<T>::W;
@@ -462,18 +459,9 @@ k_pcg_resid (int64_t n, int ld, T *__restrict__ R, const T *__restrict__ Qv,
     const int64_t o = i * ld + vi * W;
     Pack<T> r = ldp (R + o);
     const Pack<T> q = ldp (Qv + o);
-    T a[W];
 #pragma unroll
-    for (int k = 0; k < W; k++) a[k] = (T) alpha[vi * W + k];
-    if constexpr (WITHX) {
-      Pack<T> x = ldp (X + o);
-      const Pack<T> p = ldp (P + o);
-#pragma unroll
-      for (int k = 0; k < W; k++) x.v[k] = fma (a[k], p.v[k], x.v[k]);
-      stp (X + o, x);
-    }
-#pragma unroll
-    for (int k = 0; k < W; k++) r.v[k] = fma (-a[k], q.v[k], r.v[k]);
+    for (int k = 0; k < W; k++)
+      r.v[k] = fma (-(T) alpha[vi * W + k], q.v[k], r.v[k]);
     stp (R + o, r);
     if (R32) st32<T> (R32 + o, r);
   }
@@ -692,10 +680,6 @@ launch_pcg_dir (int64_t n, int ld, const TZ *Zb, T *P, T *X, int flags,
   const int grid = stream_grid (n * (ld / W));
   const double *be = ws.scal.p + S_BETA * ws.cap, *al = ws.scal.p + S_ALPHA * ws.cap;
   switch (flags) {
-  case 0:
-    LGH_CUDA (launch_pdl (bytes, k_pcg_dir<T, TZ, 0>, grid, 256, 0, s, n, ld, Zb, P,
-        X, be, al));
-    break;
   case PCG_P_FIRST:
     LGH_CUDA (launch_pdl (bytes, k_pcg_dir<T, TZ, PCG_P_FIRST>, grid, 256, 0, s, n,
         ld, Zb, P, X, be, al));
@@ -765,18 +749,14 @@ launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
 
 template <typename T>
 int
-launch_pcg_resid (int64_t n, int ld, T *R, const T *Q, float *R32, T *X,
-                  const T *P, ZWork &ws, cudaStream_t s)
+launch_pcg_resid (int64_t n, int ld, T *R, const T *Q, float *R32, ZWork &ws,
+                  cudaStream_t s)
 {
   const int64_t bytes = n * ld * (int64_t) sizeof (T);
   const int grid = stream_grid (n * (ld / Pack<T>::W));
   const double *al = ws.scal.p + S_ALPHA * ws.cap;
-  if (X)
-    LGH_CUDA (launch_pdl (bytes, k_pcg_resid<T, true>, grid, 256, 0, s, n, ld, R, Q,
-        R32, X, P, al));
-  else
-    LGH_CUDA (launch_pdl (bytes, k_pcg_resid<T, false>, grid, 256, 0, s, n, ld, R, Q,
-        R32, X, P, al));
+  LGH_CUDA (launch_pdl (bytes, k_pcg_resid<T>, grid, 256, 0, s, n, ld, R, Q, R32,
+      al));
   LGH_LAUNCH_CHECK ();
   return 0;
 }
@@ -888,7 +868,7 @@ pcg_wait_count (ZWork &ws, cudaStream_t s, int *count)
   template int launch_pcg_prod<T> (const Csr &, const T *, T *, int,         \
                                    ZWork &, cudaStream_t);                   \
   template int launch_pcg_resid<T> (int64_t, int, T *, const T *, float *,   \
-                                    T *, const T *, ZWork &, cudaStream_t);  \
+                                    ZWork &, cudaStream_t);                  \
   template int launch_pcg_out<T> (int64_t, int, int, const T *, const T *,   \
                                   int, const double *, T *, int, ZWork &,    \
                                   cudaStream_t);

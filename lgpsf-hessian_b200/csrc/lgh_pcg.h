@@ -44,11 +44,10 @@ template <typename T>
 int launch_pcg_prod (const Csr &Z, const T *P, T *Q, int ld, ZWork &ws,
                      cudaStream_t s);
 
-/* r -= alpha q, and the FP32 copy of r where R32 is given; with X also
- * x += alpha p */
+/* r -= alpha q, and the FP32 copy of r where R32 is given */
 template <typename T>
-int launch_pcg_resid (int64_t n, int ld, T *R, const T *Q, float *R32, T *X,
-                      const T *P, ZWork &ws, cudaStream_t s);
+int launch_pcg_resid (int64_t n, int ld, T *R, const T *Q, float *R32,
+                      ZWork &ws, cudaStream_t s);
 
 /* Y = S (x + alpha p) over the w columns (have_x 0: x is zero): the last
  * iteration's deferred update with the solution's row scaling */

@@ -53,20 +53,53 @@ int ensure_wz (lgh_glr_t *g);
 int launch_logdet (int kept, const double *lam, int nshift, const double *c,
                    double *out, cudaStream_t s);
 
-/* a contiguous device column into column `col` of a row-major block (and
- * its FP32 copy R32, nullable), with an optional row scale; the same column
- * of X and of the direction block are cleared (a fresh CG start) */
-__global__ void
-k_col_place (int64_t n, const double *src, const double *scale, double *R,
-             float *R32, double *X, double *P, int ld, int col)
+/* slots of one placement launch */
+constexpr int PLACE_COLS = 32;
+struct PlaceSlots
 {
-  for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t) gridDim.x * blockDim.x) {
-    const double r = scale ? scale[i] * src[i] : src[i];
-    R[i * ld + col] = r;
-    if (R32) R32[i * ld + col] = (float) r;
-    X[i * ld + col] = 0.;
-    P[i * ld + col] = 0.;
+  int v[PLACE_COLS];
+};
+
+/* columns src + t n (t < k) -> columns slot[t] of the row-major residual
+ * block R (and of its FP32 copy R32, nullable), with an optional row scale;
+ * the same columns of X and of the direction block are cleared (a fresh CG
+ * start).  A column alone dirties a whole sector of three blocks per row
+ * (31 us at 512^2 whatever its width of 8 bytes), so a request's columns
+ * are placed together: 32 rows are transposed through shared memory and
+ * neighbouring slots written in one go. */
+__global__ void __launch_bounds__ (256)
+k_col_place (int64_t n, const double *__restrict__ src,
+             const double *__restrict__ scale, double *__restrict__ R,
+             float *__restrict__ R32, double *__restrict__ X,
+             double *__restrict__ P, int ld, PlaceSlots slot, int k)
+{
+  __shared__ double tile[PLACE_COLS][33];
+  __shared__ int col[PLACE_COLS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int t = 0; t < PLACE_COLS; t++)
+    if (threadIdx.x == t) col[t] = slot.v[t];
+  for (int64_t i0 = (int64_t) blockIdx.x * 32; i0 < n;
+       i0 += (int64_t) gridDim.x * 32) {
+    const int rows = (int) min ((int64_t) 32, n - i0);
+    __syncthreads ();
+    if (lane < rows) {
+      const double sc = scale ? scale[i0 + lane] : 1.;
+      for (int t = warp; t < k; t += 8) {
+        const double v = src[(size_t) t * n + i0 + lane];
+        tile[t][lane] = scale ? sc * v : v;
+      }
+    }
+    __syncthreads ();
+    for (int e = threadIdx.x; e < rows * k; e += 256) {
+      const int r = e / k, t = e - r * k;
+      const int64_t o = (i0 + r) * ld + col[t];
+      const double v = tile[t][r];
+      R[o] = v;
+      if (R32) R32[o] = (float) v;
+      X[o] = 0.;
+      P[o] = 0.;
+    }
   }
 }
 
@@ -554,20 +587,30 @@ srv_start (lgh_server_t *sv, const Adm &a)
   }
   int j = a.j0;
   const int jend = a.j0 + a.take;
+  PlaceSlots ps{};
+  int k = 0;
+  /* first right-hand sides: r (solve) or M^{1/2} xi (sample) */
+  auto place = [&] () -> int {
+    const int g1 = (int) std::min<int64_t> ((n + 31) / 32, num_sms () * 8);
+    k_col_place<<<std::max (g1, 1), 256, 0, s>>> (
+        n, r->din.p + (size_t) (j - k) * n,
+        r->kind == 1 ? g->prior->msqrt.p : nullptr, R, R32, X, P, sv->ld, ps, k);
+    LGH_LAUNCH_CHECK ();
+    k = 0;
+    return 0;
+  };
   for (int sl = 0; sl < sv->cap && j < jend; sl++) {
     Slot &S = sv->slots[sl];
     if (S.req) continue;
     S.req = r;
     S.col = j;
     S.stage = 1;
-    /* first right-hand side: r (solve) or M^{1/2} xi (sample) */
-    k_col_place<<<cgrid (n), 256, 0, s>>> (n, r->din.p + (size_t) j * n,
-                                           r->kind == 1 ? g->prior->msqrt.p : nullptr,
-                                           R, R32, X, P, sv->ld, sl);
-    LGH_LAUNCH_CHECK ();
     sv->fresh_h[sl] = 1;
+    ps.v[k++] = sl;
     j++;
+    if (k == PLACE_COLS) LGH_TRY (place ());
   }
+  if (k > 0) LGH_TRY (place ());
   LGH_CHECK (j == jend, LGH_ERR_ARG_WRONG, "server: admitted without free slots");
   return 0;
 }
@@ -697,7 +740,11 @@ srv_loop (lgh_server_t *sv)
    * host.  A mixed-precision object's V-cycle runs in FP32 on the FP32 copy
    * of the residuals that the residual pass (and a column's placement)
    * keeps; its FP32 output is widened as the dots and the direction read
-   * it (the FP64 CG scalars and iterates are unchanged). */
+   * it (the FP64 CG scalars and iterates are unchanged).  x += alpha p
+   * rides on the direction pass of the next tick, which reads p anyway: a
+   * column that a tick's dots find converged keeps its alpha until that
+   * tick's direction has used it, so its x is complete when the tick
+   * ends. */
   auto tick = [&] () -> int {
     const Csr &Z = p->Z->csr;
     if (R32) {
@@ -705,7 +752,7 @@ srv_loop (lgh_server_t *sv)
       LGH_TRY ((launch_pcg_dots<double, float> (n, sv->cap, ld, R, Z32, 0,
                                                 p->zcfg.rtol, 0, nullptr,
                                                 sv->fresh_d.p, sv->ws, s)));
-      LGH_TRY ((launch_pcg_dir<double, float> (n, ld, Z32, P, X, 0, sv->ws, s)));
+      LGH_TRY ((launch_pcg_dir<double, float> (n, ld, Z32, P, X, PCG_X_ADD, sv->ws, s)));
     } else {
       if (p->mg)
         LGH_TRY (mg_vcycle<double> (p->mg, R, Zb, ld, sv->cap, s, nullptr, &sv->mgw));
@@ -714,10 +761,10 @@ srv_loop (lgh_server_t *sv)
       LGH_TRY ((launch_pcg_dots<double, double> (n, sv->cap, ld, R, Zb, 0,
                                                  p->zcfg.rtol, 0, nullptr,
                                                  sv->fresh_d.p, sv->ws, s)));
-      LGH_TRY ((launch_pcg_dir<double, double> (n, ld, Zb, P, X, 0, sv->ws, s)));
+      LGH_TRY ((launch_pcg_dir<double, double> (n, ld, Zb, P, X, PCG_X_ADD, sv->ws, s)));
     }
     LGH_TRY (launch_pcg_prod<double> (Z, P, Q, ld, sv->ws, s));
-    return launch_pcg_resid<double> (n, ld, R, Q, R32, X, P, sv->ws, s);
+    return launch_pcg_resid<double> (n, ld, R, Q, R32, sv->ws, s);
   };
   cudaGraphExec_t gexec = nullptr;
   bool graphs_off = false;

@@ -728,7 +728,7 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
         LGH_TRY (launch_pcg_prod<T> (Z, bP, bQ, ldt, ws, s));
         if (tr) LGH_TRY (tr->end (s));
         if (tr) LGH_TRY (tr->begin (K_PCGX_UPD, (pc32 ? 3. + zw : 3.) * bw, s));
-        LGH_TRY (launch_pcg_resid<T> (n, ldt, bR, bQ, R32, nullptr, nullptr, ws, s));
+        LGH_TRY (launch_pcg_resid<T> (n, ldt, bR, bQ, R32, ws, s));
         if (tr) LGH_TRY (tr->end (s));
         LGH_TRY (precond ());
         if (tr) LGH_TRY (tr->begin (K_PCGX_DOTS, (1. + zw) * bw, s));
