@@ -340,6 +340,7 @@ k_pcg_dots (int64_t n, int ld, int nvec, int L, int rpc, const T *__restrict__ R
   flat_zero<double, CH, W> (acc[0]);
   flat_zero<double, CH, W> (acc[1]);
   if (rl < rpc)
+#pragma unroll (CH == 1 ? 4 : 1)
     for (int64_t i = (int64_t) blockIdx.x * rpc + rl; i < n;
          i += (int64_t) gridDim.x * rpc) {
 #pragma unroll
@@ -483,10 +484,13 @@ k_pcg_out (int64_t n, int w, int ld, const T *__restrict__ X,
     const int c = (int) (e - i * nvec) * W;
     const double sc = rs ? rs[i] : 1.0;
     Pack<T> x = have_x ? ldp (X + i * ld + c) : pzero<T> ();
-    const Pack<T> p = ldp (P + i * ld + c);
+    if (P != nullptr) {
+      const Pack<T> p = ldp (P + i * ld + c);
 #pragma unroll
-    for (int k = 0; k < W; k++)
-      x.v[k] = (T) (sc * (double) fma ((T) alpha[c + k], p.v[k], x.v[k]));
+      for (int k = 0; k < W; k++) x.v[k] = fma ((T) alpha[c + k], p.v[k], x.v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < W; k++) x.v[k] = (T) (sc * (double) x.v[k]);
     if (vec && c + W <= w) {
       stp (Y + i * ldy + c, x);
     } else {
@@ -640,7 +644,10 @@ launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
   const int nvec = ld / W;
   const FlatShape f = sum_shape (nvec, n);
   const int smem = sum_smem (f, 2 * ld);
-  const int want = std::min (flat_grid (f, n), ws.nblocks);
+  /* one pack per thread and the last CTA's sum: two CTAs per SM, four rows
+   * in flight each, leave it few partials */
+  const int want = std::min (flat_grid (f, n), f.ch == 1 && ld <= PCG_TAIL_COLS
+                                                   ? 2 * num_sms () : ws.nblocks);
   if (report) ws.nact.seq = (ws.nact.seq + 1) & 0x7fff;
   const PcgCols pc{ ws.scal.p, ws.ival.p, ws.cap, w, rtol, first, iter, hist,
                     fresh, report ? ws.nact.p : nullptr, ws.nact.seq };

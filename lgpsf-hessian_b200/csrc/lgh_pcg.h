@@ -49,8 +49,9 @@ template <typename T>
 int launch_pcg_resid (int64_t n, int ld, T *R, const T *Q, float *R32,
                       ZWork &ws, cudaStream_t s);
 
-/* Y = S (x + alpha p) over the w columns (have_x 0: x is zero): the last
- * iteration's deferred update with the solution's row scaling */
+/* Y = S (x + alpha p) over the w columns (have_x 0: x is zero; P null: no
+ * alpha p): the last iteration's deferred update with the solution's row
+ * scaling */
 template <typename T>
 int launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P,
                     int have_x, const double *rs, T *Y, int ldy, ZWork &ws,

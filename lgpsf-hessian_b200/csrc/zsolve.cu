@@ -603,6 +603,13 @@ zvd (const Csr &Z)
     return set_error (LGH_ERR_SUP, "zsolve: chunking %d unsupported", CHV);  \
   }
 
+/* block bytes up to which the next direction and product are queued before
+ * the host has seen the active count: it saves the 6 us that the device
+ * idles at each look and costs one more direction and product per solve
+ * (8 us at 64^2 x 60 columns, 2 MB; 30 at 32 MB), and most solves look 5 to
+ * 20 times */
+constexpr double PCG_AHEAD = 32. * 1048576.;
+
 template <typename T>
 int
 zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
@@ -713,7 +720,8 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
       LGH_TRY (precond ());
       LGH_TRY (dots (1, 0, 0));
       int h_nact = 1;
-      for (int it = 0; it < cfg.maxit; it++) {
+      bool ahead = false;     /* the next direction and product are queued */
+      auto dir_prod = [&] (int it) -> int {
         if (it == 0 && !pc32) {
           std::swap (bP, bZ);
         } else {
@@ -727,6 +735,10 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
         if (tr) LGH_TRY (tr->begin (K_PCGX_PQ, zbytes + 2. * bw, s));
         LGH_TRY (launch_pcg_prod<T> (Z, bP, bQ, ldt, ws, s));
         if (tr) LGH_TRY (tr->end (s));
+        return 0;
+      };
+      for (int it = 0; it < cfg.maxit; it++) {
+        if (!ahead) LGH_TRY (dir_prod (it));
         if (tr) LGH_TRY (tr->begin (K_PCGX_UPD, (pc32 ? 3. + zw : 3.) * bw, s));
         LGH_TRY (launch_pcg_resid<T> (n, ldt, bR, bQ, R32, ws, s));
         if (tr) LGH_TRY (tr->end (s));
@@ -739,6 +751,11 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
                          || iters == cfg.maxit;
         LGH_TRY (dots (0, it, look));
         if (tr) LGH_TRY (tr->end (s));
+        /* small blocks: the device does not wait for the host's look.  The
+         * next direction and product only complete x when every column has
+         * converged (its alpha is still set for the first and zero after) */
+        ahead = look && !tr && iters < cfg.maxit && bw <= PCG_AHEAD;
+        if (ahead) LGH_TRY (dir_prod (iters));
         if (look) {
           LGH_TRY (pcg_wait_count (ws, s, &h_nact));
           if (tr) {
@@ -748,9 +765,10 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
           if (h_nact == 0) break;
         }
       }
-      /* the last iteration's deferred x += alpha p with the row scaling */
-      LGH_TRY (launch_pcg_out<T> (n, wt, ldt, bX, bP, iters > 1, rs_out, Y + c0,
-                                  ldy, ws, s));
+      /* the last iteration's deferred x += alpha p (unless the queued
+       * direction did it) with the row scaling */
+      LGH_TRY (launch_pcg_out<T> (n, wt, ldt, bX, ahead ? nullptr : bP,
+                                  ahead || iters > 1, rs_out, Y + c0, ldy, ws, s));
       if (tr && !tr->ids.empty ()) {
         LGH_CUDA (cudaStreamSynchronize (s));
         LGH_TRY (tr->drain ());
