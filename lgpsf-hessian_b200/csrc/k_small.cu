@@ -29,15 +29,24 @@ namespace lgh
 
 /* ---------------------------------------------------------------- potrf -- */
 
-__global__ void __launch_bounds__ (1024)
-k_potrf (int n, double *G, const double *G0, int jitter_mode, int *info,
-         int nb)
+/* One CTA, panels of NB columns.  The panel's NB x NB diagonal block is
+ * factored by one warp with a row per lane in registers, the rows below it
+ * by a thread each with theirs in registers; the arithmetic and its order
+ * are those of a column at a time.  A column at a time over the whole panel
+ * cost three barriers of 1024 threads for each, 0.8 us a column (n = 60: 47
+ * us, now 41; 220: 328 and 237; 800: 6.2 and 5.2 ms); what is left is the chain of a square root and a division per
+ * column.  The trailing update is m8n8k4 products of the panel, a warp per
+ * 8 x 8 tile.  16 columns: the rows fit the registers of 512 threads. */
+constexpr int NB = 16;
+
+__global__ void __launch_bounds__ (512)
+k_potrf (int n, double *G, const double *G0, int jitter_mode, int *info)
 {
-  extern __shared__ double P[];     /* (n - k0) x (nb + 1) panel */
+  extern __shared__ double P[];     /* (n - k0) x (NB + 1) panel */
   __shared__ int fail;
   __shared__ double jit;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int ps = nb + 1;
+  constexpr int ps = NB + 1;
   if (tid == 0) { info[0] = 0; info[1] = 0; }
   for (int attempt = 0; attempt < 2; attempt++) {
     if (attempt == 1) {
@@ -63,46 +72,86 @@ k_potrf (int n, double *G, const double *G0, int jitter_mode, int *info,
     }
     if (tid == 0) fail = 0;
     __syncthreads ();
-    for (int k0 = 0; k0 < n && !fail; k0 += nb) {
-      const int kb = min (nb, n - k0);
+    for (int k0 = 0; k0 < n && !fail; k0 += NB) {
+      const int kb = min (NB, n - k0);
       const int m = n - k0;
       for (int e = tid; e < m * kb; e += nt) {
         const int r = e % m, kk = e / m;
         P[r * ps + kk] = G[(k0 + r) + (size_t) (k0 + kk) * n];
       }
       __syncthreads ();
-      for (int kk = 0; kk < kb; kk++) {
-        if (tid == 0) {
-          const double d = P[kk * ps + kk];
-          if (!(d > 0.) || !isfinite (d)) fail = 1;
-          else P[kk * ps + kk] = sqrt (d);
+      if (tid < 32) {
+        /* lane r: row r of the diagonal block; columns kb .. NB - 1 of a
+         * last panel are never reached */
+        double a[NB];
+#pragma unroll
+        for (int j = 0; j < NB; j++) a[j] = (tid < kb && j < kb) ? P[tid * ps + j] : 0.;
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < NB; k++) {
+          if (k < kb && ok) {
+            const double d = __shfl_sync (0xffffffffu, a[k], k);
+            ok = d > 0. && isfinite (d);
+            if (ok) {
+              const double dk = sqrt (d);
+              if (tid == k) a[k] = dk;
+              if (tid > k) a[k] /= dk;
+#pragma unroll
+              for (int j = k + 1; j < NB; j++) {
+                const double l = __shfl_sync (0xffffffffu, a[k], j);
+                if (tid >= j) a[j] -= a[k] * l;
+              }
+            }
+          }
         }
-        __syncthreads ();
-        if (fail) break;
-        const double dk = P[kk * ps + kk];
-        for (int r = kk + 1 + tid; r < m; r += nt) P[r * ps + kk] /= dk;
-        __syncthreads ();
-        const int rem = kb - kk - 1;
-        for (int e = tid; e < m * rem; e += nt) {
-          const int r = e % m, jj = kk + 1 + e / m;
-          if (r >= jj) P[r * ps + jj] -= P[r * ps + kk] * P[jj * ps + kk];
-        }
-        __syncthreads ();
+        if (tid < kb)
+#pragma unroll
+          for (int j = 0; j < NB; j++)
+            if (j <= tid) P[tid * ps + j] = a[j];
+        if (tid == 0 && !ok) fail = 1;
       }
+      __syncthreads ();
       if (fail) break;
+      if (kb == NB) {               /* a shorter panel is the last one */
+        for (int r = NB + tid; r < m; r += nt) {
+          double x[NB];
+#pragma unroll
+          for (int j = 0; j < NB; j++) x[j] = P[r * ps + j];
+#pragma unroll
+          for (int k = 0; k < NB; k++) {
+            x[k] /= P[k * ps + k];
+#pragma unroll
+            for (int j = k + 1; j < NB; j++) x[j] -= x[k] * P[j * ps + k];
+          }
+#pragma unroll
+          for (int j = 0; j < NB; j++) P[r * ps + j] = x[j];
+        }
+      }
+      __syncthreads ();
       for (int e = tid; e < m * kb; e += nt) {
         const int r = e % m, kk = e / m;
         if (r >= kk) G[(k0 + r) + (size_t) (k0 + kk) * n] = P[r * ps + kk];
       }
       /* trailing update G(i, j) -= P(i, :) P(j, :)^T, i >= j >= k0 + kb */
-      const int mt = m - kb;
-      for (int e = tid; e < mt * mt; e += nt) {
-        const int ii = e % mt, jj = e / mt;
-        if (ii < jj) continue;
-        const int ri = kb + ii, rj = kb + jj;
-        double s = 0.;
-        for (int kk = 0; kk < kb; kk++) s = fma (P[ri * ps + kk], P[rj * ps + kk], s);
-        G[(k0 + ri) + (size_t) (k0 + rj) * n] -= s;
+      const int mt = m - kb, nt8 = (mt + 7) / 8;
+      const int lane = tid & 31, kl = lane & 3, ml = lane >> 2;
+      for (int t = tid >> 5; t < nt8 * nt8; t += nt / 32) {
+        const int ti = t % nt8, tj = t / nt8;
+        if (ti < tj) continue;
+        const int ri = ti * 8 + ml, rj = tj * 8 + ml;
+        double c0 = 0., c1 = 0.;
+#pragma unroll
+        for (int k = 0; k < NB; k += 4) {
+          const double a = ri < mt ? P[(kb + ri) * ps + k + kl] : 0.;
+          const double b = rj < mt ? P[(kb + rj) * ps + k + kl] : 0.;
+          asm volatile ("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
+                        "{%0, %1}, {%2}, {%3}, {%0, %1};"
+                        : "+d"(c0), "+d"(c1) : "d"(a), "d"(b));
+        }
+        const int cj = tj * 8 + kl * 2;
+        double *g = G + (k0 + kb + ri) + (size_t) (k0 + kb + cj) * n;
+        if (ri < mt && cj <= ri) g[0] -= c0;
+        if (ri < mt && cj + 1 <= ri) g[n] -= c1;
       }
       __syncthreads ();
     }
@@ -123,15 +172,14 @@ launch_potrf (int n, double *G, double *G0, int jitter_mode, int *info,
               cudaStream_t s)
 {
   if (n <= 0) return 0;
-  const int nb = (n <= 800) ? 32 : 16;
-  const int smem = n * (nb + 1) * (int) sizeof (double);
+  const int smem = n * (NB + 1) * (int) sizeof (double);
   LGH_CHECK (smem <= 220 * 1024, LGH_ERR_SUP, "potrf: n=%d too large", n);
   if (G0) LGH_CUDA (cudaMemcpyAsync (G0, G, (size_t) n * n * sizeof (double),
                                      cudaMemcpyDeviceToDevice, s));
   LGH_CUDA (cudaFuncSetAttribute (k_potrf,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   smem));
-  k_potrf<<<1, 1024, smem, s>>> (n, G, G0, jitter_mode, info, nb);
+  k_potrf<<<1, 512, smem, s>>> (n, G, G0, jitter_mode, info);
   LGH_LAUNCH_CHECK ();
   return 0;
 }
@@ -163,11 +211,63 @@ k_trtri_lower (int n, const double *__restrict__ L, double *__restrict__ out,
   }
 }
 
+/* the same with the column in registers, row i in lane i % 32: up to 32 T
+ * rows.  Through shared memory a step cost two warp barriers and a round
+ * trip, 0.5 us a row; here it is a shuffle, the division and a multiply-add
+ * (n = 60: 29.3 us and 16.0; 220: 206 and 62; 500: 851 and 153). */
+template <int T>
+__global__ void __launch_bounds__ (128)
+k_trtri_regs (int n, const double *__restrict__ L, double *__restrict__ out,
+              int transpose)
+{
+  const int lane = threadIdx.x & 31;
+  const int j = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (j >= n) return;
+  double x[T];
+#pragma unroll
+  for (int t = 0; t < T; t++) x[t] = 32 * t + lane == j ? 1. : 0.;
+#pragma unroll
+  for (int t = 0; t < T; t++) {
+    const int kend = min (32, n - 32 * t);
+    for (int kk = max (0, j - 32 * t); kk < kend; kk++) {
+      const int k = 32 * t + kk;
+      const double *c = L + (size_t) k * n;
+      double l[T];
+#pragma unroll
+      for (int q = t; q < T; q++) {
+        const int i = 32 * q + lane;
+        l[q] = i > k && i < n ? __ldg (c + i) : 0.;
+      }
+      const double xk = __shfl_sync (0xffffffffu, x[t], kk) / __ldg (c + k);
+      if (lane == kk) x[t] = xk;
+#pragma unroll
+      for (int q = t; q < T; q++)
+        if (q > t || lane > kk) x[q] -= l[q] * xk;
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < T; t++) {
+    const int i = 32 * t + lane;
+    if (i >= n) break;
+    const double v = i >= j ? x[t] : 0.;
+    if (transpose) out[j + (size_t) i * n] = v;
+    else out[i + (size_t) j * n] = v;
+  }
+}
+
 int
 launch_trtri_lower (int n, const double *L, double *Linv, int transpose,
                     cudaStream_t s)
 {
   if (n <= 0) return 0;
+  /* columns of up to 512 rows in registers */
+  if (n <= 512) {
+    auto k = n <= 64 ? k_trtri_regs<2> : n <= 128 ? k_trtri_regs<4>
+             : n <= 256 ? k_trtri_regs<8> : k_trtri_regs<16>;
+    k<<<(n + 3) / 4, 128, 0, s>>> (n, L, Linv, transpose);
+    LGH_LAUNCH_CHECK ();
+    return 0;
+  }
   const int smem = 8 * n * (int) sizeof (double);
   LGH_CUDA (cudaFuncSetAttribute (k_trtri_lower,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
