@@ -347,7 +347,10 @@ tn_splits (int64_t n, int m1, int m2)
 size_t
 gemm_tn_work_elems (int64_t n, int m1, int m2)
 {
-  return (size_t) tn_splits (n, m1, m2) * m1 * m2;
+  /* one column: two CTAs of k_gemv_t per SM (one: 134 us at 512^2 x 220,
+   * two: 83) */
+  const int ns = tn_splits (n, m1, m2);
+  return (size_t) (m2 == 1 ? std::max (ns, 2 * num_sms ()) : ns) * m1 * m2;
 }
 
 /* a workspace bound for every shape m1 <= m1max, m2 <= m2max: with t tiles
