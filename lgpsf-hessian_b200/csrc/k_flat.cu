@@ -15,9 +15,11 @@
  * residual after it is ever stored, and each pass gathers one fine block:
  * in the second step A d2 = a2 A d1 + b2 A D^{-1} r1, and A d1 = r0 - r1
  * is at hand, so r1 alone is gathered where d2 = a2 d1 + b2 D^{-1} r1 was.
- * Block passes at 512^2: 2 + 3 + 4 (and the coarse blocks), against 2 + 4
- * + 2 + 3 with the stored iterate; measured at 220 columns FP64 on the
- * finest level, all in one V-cycle: see each kernel. */
+ * Block passes: 2 + 3 + 4 (and the coarse blocks), against 2 + 4 + 2 + 3
+ * with the stored iterate.  All four are bound by L1 wavefronts at the
+ * residency their registers allow (lgh_flat.cuh); each kernel gives its
+ * time at 512^2 x 220 columns FP64 on the finest level, its floor at the
+ * measured HBM rate and what the passes it replaces took. */
 
 #include <type_traits>
 
@@ -27,7 +29,8 @@
 namespace lgh
 {
 
-/* Y = B - A X (first step: X = B = r0) */
+/* Y = B - A X (first step: X = B = r0): 180 us, floor 141; a row per power
+ * of two of lanes with shuffled entries 247 */
 template <typename T, int CH>
 __global__ void __launch_bounds__ (FLAT_THREADS, FlatOcc<CH>::v)
 k_flat_resid (int64_t n, const int64_t *__restrict__ rowptr,
@@ -69,7 +72,8 @@ k_flat_resid (int64_t n, const int64_t *__restrict__ rowptr,
 }
 
 /* r2 = r1 - a2 (r0 - r1) - s2 F1 r1 (s2 = b2 / b1): reads r1 (gathered)
- * and r0, writes r2 */
+ * and r0, writes r2.  280 us, floor 211; with d and x re-formed from two
+ * gathered blocks 580 */
 template <typename T, int CH>
 __global__ void __launch_bounds__ (FLAT_THREADS, FlatOcc<CH>::v)
 k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
@@ -115,7 +119,8 @@ k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
 }
 
 /* z = dinv (g (r0 + r2) + b2 (r1 + r2 - F1 r2)) + Q xc: reads r0, r1, r2
- * (gathered) and the coarse block (gathered), writes z */
+ * (gathered) and the coarse block (gathered), writes z.  487 us, floor 297;
+ * the post residual and the two post-smoothing steps took 787 */
 template <typename T, int CH>
 __global__ void __launch_bounds__ (FLAT_THREADS, CH == 2 ? 5 : (CH == 3 ? 4 : FlatOcc<CH>::v))
 k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
@@ -181,7 +186,8 @@ k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
 /* Y = A X for the restriction P^T: its rows hold 15 (2D) to 230 (3D)
  * entries and there are few of them on the lower levels, so a row's
  * entries are dealt out to S neighbouring thread groups of the CTA, whose
- * sums are added in group order through shared memory */
+ * sums are added in group order through shared memory.  128 us for the
+ * finest level's, 154 with a warp group per row */
 template <typename T, int CH, bool SPLIT>
 __global__ void __launch_bounds__ (FLAT_THREADS, FlatOcc<CH>::v)
 k_flat_mult (int64_t n, const int64_t *__restrict__ rowptr,

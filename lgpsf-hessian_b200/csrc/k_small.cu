@@ -287,7 +287,8 @@ launch_trtri_lower (int n, const double *L, double *Linv, int transpose,
  * sweep is nblk - 1 rounds of two launches, 13 at n = 220, where the scalar
  * ordering needs n - 1 rounds, each with a barrier over the whole grid and
  * an update of every entry (5.2 us a round, bound by the barrier and the L2
- * latency behind it: 10.3 ms at n = 220, 2.0 ms at n = 60).  Blocks of 16:
+ * latency behind it: 10.3 ms at n = 220, 2.0 ms at n = 60; now 3.3 and
+ * 0.56).  Blocks of 16:
  * the sweep inside a pair is the longest chain of a round, and a 32 x 32
  * submatrix is also one tile of the products. */
 constexpr int JB = 16, JT = 2 * JB, JS = JT + 4;   /* block, tile, row stride */

@@ -9,10 +9,10 @@
  *             alpha/beta and a per-column convergence mask;
  *   mode 2    fixed-count Chebyshev (zsolve_impl.h:94-141), nit from the
  *             margined spectral interval.
- * The preconditioner is Jacobi (the reference's PCGAMG is replaced; the
- * aggregation V-cycle of mode 3 lives in mg.cu).
+ * The preconditioner is the aggregation V-cycle (mg.cu; the iteration's own
+ * passes are those of k_pcg.cu) or Jacobi, whose kernels are here.
  *
- * Each CG iteration is two fused kernels:
+ * Each CG iteration with Jacobi is two fused kernels:
  *   k_pcg_pq   p_new = D^{-1} r + beta p_old, computed on the fly at every
  *              neighbour row, q = Z p_new, and the per-column dot (p, q);
  *              the last CTA (atomic ticket) reduces the per-CTA partials in
