@@ -145,6 +145,7 @@ k_spmm_scalar (int64_t n, const int64_t *__restrict__ rowptr,
                const T *__restrict__ X, int ldx, T *__restrict__ Y, int ldy,
                int w, SpvEp<T> ep)
 {
+  pdl_wait ();
   const int lane = threadIdx.x & (G - 1);
   const unsigned gmask = G == 32 ? 0xffffffffu
                          : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
@@ -230,18 +231,22 @@ spmv_dispatch (const Csr &A, const TV *vals, const T *X, int ldx, T *Y, int ldy,
     auto k = k_spmm_scalar<T, TV, G, U>;
     const int want = (int) std::max<int64_t> (1, std::min<int64_t> (
         (A.n * G + 255) / 256, 1 << 20));
-    k<<<fit_grid (k, want, 256, 0), 256, 0, s>>> (A.n, A.rowptr, A.colidx, vals,
-                                                 X, ldx, Y, ldy, w, ep);
+    /* H v is three products of 12, 124 and 12 us at 512^2: the next one's
+     * CTAs are in place when the last of the previous one leave */
+    LGH_CUDA (launch_pdl (A.n * (int64_t) sizeof (T), k,
+                          fit_grid (k, want, 256, 0), 256, 0, s, A.n, A.rowptr,
+                          A.colidx, vals, X, ldx, Y, ldy, w, ep));
+    return 0;
   };
   using std::integral_constant;
   if (avg > 128)
-    run (integral_constant<int, 32> (), integral_constant<int, 8> ());
+    LGH_TRY (run (integral_constant<int, 32> (), integral_constant<int, 8> ()));
   else if (avg > 32)
-    run (integral_constant<int, 32> (), integral_constant<int, 4> ());
+    LGH_TRY (run (integral_constant<int, 32> (), integral_constant<int, 4> ()));
   else if (avg >= 8)
-    run (integral_constant<int, 8> (), integral_constant<int, 4> ());
+    LGH_TRY (run (integral_constant<int, 8> (), integral_constant<int, 4> ()));
   else
-    run (integral_constant<int, 4> (), integral_constant<int, 2> ());
+    LGH_TRY (run (integral_constant<int, 4> (), integral_constant<int, 2> ()));
   LGH_LAUNCH_CHECK ();
   return 0;
 }
