@@ -134,10 +134,7 @@ struct SpvEp
  * of the 16-byte vector, or an offset base): G lanes split a row's
  * nonzeros (CSR-vector), reduce with shuffles; columns in a loop.  A lane
  * issues U entries' column and value loads, then U gathers of x (which L2
- * holds), so that a row of 183 entries is two rounds of loads for a warp
- * instead of 23 dependent steps for 8 lanes: HBM streams the operator.  G:
- * a warp for rows of more than 32 entries, 8 lanes from 8 up, 4 below
- * (5-point rows leave 3 of 8 lanes idle). */
+ * holds): HBM streams the operator.  G and U: see spmv_dispatch. */
 template <typename T, typename TV, int G, int U>
 __global__ void __launch_bounds__ (256)
 k_spmm_scalar (int64_t n, const int64_t *__restrict__ rowptr,
@@ -225,30 +222,50 @@ static int
 spmv_dispatch (const Csr &A, const TV *vals, const T *X, int ldx, T *Y, int ldy,
                int w, SpvEp<T> ep, cudaStream_t s)
 {
-  const int64_t avg = A.n > 0 ? A.nnz / A.n : 0;
-  auto run = [&] (auto gl, auto un) {
+  auto run = [&] (auto gl, auto un) -> int {
     constexpr int G = decltype (gl)::value, U = decltype (un)::value;
     auto k = k_spmm_scalar<T, TV, G, U>;
     const int want = (int) std::max<int64_t> (1, std::min<int64_t> (
         (A.n * G + 255) / 256, 1 << 20));
-    /* H v is three products of 12, 124 and 12 us at 512^2: the next one's
+    /* H v is three products of 6, 104 and 6 us at 512^2: the next one's
      * CTAs are in place when the last of the previous one leave */
     LGH_CUDA (launch_pdl (A.n * (int64_t) sizeof (T), k,
                           fit_grid (k, want, 256, 0), 256, 0, s, A.n, A.rowptr,
                           A.colidx, vals, X, ldx, Y, ldy, w, ep));
+    LGH_LAUNCH_CHECK ();
     return 0;
   };
   using std::integral_constant;
-  if (avg > 128)
-    LGH_TRY (run (integral_constant<int, 32> (), integral_constant<int, 8> ()));
-  else if (avg > 32)
-    LGH_TRY (run (integral_constant<int, 32> (), integral_constant<int, 4> ()));
-  else if (avg >= 8)
-    LGH_TRY (run (integral_constant<int, 8> (), integral_constant<int, 4> ()));
-  else
-    LGH_TRY (run (integral_constant<int, 4> (), integral_constant<int, 2> ()));
-  LGH_LAUNCH_CHECK ();
-  return 0;
+#define LGH_SPV(G, U) return run (integral_constant<int, G> (), integral_constant<int, U> ())
+  if (w > 1) {
+    /* columns of an unaligned view: the entries are read again for each */
+    const int64_t avg = A.n > 0 ? A.nnz / A.n : 0;
+    if (avg > 128) LGH_SPV (32, 8);
+    if (avg > 32) LGH_SPV (32, 4);
+    if (avg >= 8) LGH_SPV (8, 4);
+    LGH_SPV (4, 2);
+  }
+  /* One vector: the fewest lanes whose G U entries cover the mean row in
+   * one round of loads, as idle slots cost issue and a second round costs a
+   * round trip.  262144 rows, us with this rule / with 4 x 2 below 8
+   * entries, 8 x 4 to 32, 32 x 4 to 128, 32 x 8 above: 3 entries 10 / 16, 5
+   * 11 / 16, 7 12 / 16, 9 14 / 25, 19 20 / 31, 27 25 / 37, 40 33 / 76, 57 45
+   * / 82, 81 59 / 96, 100 76 / 102, 150 102 / 125, 183 111 / 131 (floor 90),
+   * 220 and 256 the same; 300 141 / 160, 400 145 / 145.  Rows of 8 times
+   * what a round covers take the next shape. */
+  auto fits = [&] (int cover) {
+    return A.nnz <= cover * A.n && A.max_row_nnz <= 8 * cover;
+  };
+  if (fits (5)) LGH_SPV (1, 5);
+  if (fits (10)) LGH_SPV (1, 8);
+  if (fits (28)) LGH_SPV (4, 7);
+  if (fits (48)) LGH_SPV (8, 6);
+  if (fits (64)) LGH_SPV (8, 8);
+  if (fits (96)) LGH_SPV (16, 6);
+  if (fits (128)) LGH_SPV (16, 8);
+  if (!fits (192) && fits (256)) LGH_SPV (32, 8);
+  LGH_SPV (32, 6);
+#undef LGH_SPV
 }
 
 /* y = (A x) ./ div, or y += scale A x (div null) of single FP64 vectors */
