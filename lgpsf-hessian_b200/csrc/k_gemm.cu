@@ -331,6 +331,31 @@ k_gemm_tn_reduce_warp (int64_t total, int m1, int nsplit,
   }
 }
 
+/* the sum of k_gemm_tn_reduce_warp, in its order, with one thread per
+ * entry: the same bits for products of many entries, whose slices a warp
+ * per entry would read a sector at a time.  For the request loop, whose
+ * columns must not depend on how many of them are harvested together. */
+__global__ void __launch_bounds__ (128)
+k_gemm_tn_reduce_same (int64_t total, int m1, int nsplit,
+                       const double *__restrict__ work, double *C, int ldc)
+{
+  for (int64_t e = (int64_t) blockIdx.x * 128 + threadIdx.x; e < total;
+       e += (int64_t) gridDim.x * 128) {
+    double s[32];
+#pragma unroll
+    for (int q = 0; q < 32; q++) s[q] = 0.;
+    for (int z = 0; z < nsplit; z += 32)
+#pragma unroll
+      for (int q = 0; q < 32; q++)
+        if (z + q < nsplit) s[q] += work[(size_t) (z + q) * total + e];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < o; q++) s[q] += s[q + o];
+    C[e % m1 + (size_t) (e / m1) * ldc] = s[0];
+  }
+}
+
 static int
 tn_splits (int64_t n, int m1, int m2)
 {
@@ -364,15 +389,27 @@ gemm_tn_work_max (int m1max, int m2max)
   return (4 * (size_t) num_sms () + tmax) * GB * GB;
 }
 
-/* C from nsplit slices of partial sums in work */
+/* the tiled form takes as many slices as one column does at every width
+ * (launch_gemm_tn with tiles set): this many partial sums */
+size_t
+gemm_tn_work_tiles (int64_t n, int m1, int m2max)
+{
+  return (size_t) tn_splits (n, m1, 1) * m1 * m2max;
+}
+
+/* C from nsplit slices of partial sums in work; tiles: each entry's sum in
+ * an order that does not depend on m2 */
 static int
 gemm_tn_sum (int m1, int m2, int nsplit, const double *work, double *C, int ldc,
-             int sym, int upper, cudaStream_t s)
+             int sym, int upper, cudaStream_t s, int tiles = 0)
 {
   const int64_t total = (int64_t) m1 * m2;
   if (!sym && !upper && nsplit >= 16 && total <= 8192) {
     k_gemm_tn_reduce_warp<<<(int) ((total + 7) / 8), 256, 0, s>>> (
         total, m1, nsplit, work, C, ldc);
+  } else if (!sym && !upper && nsplit >= 16 && tiles) {
+    const int rg = (int) std::min<int64_t> ((total + 127) / 128, num_sms () * 8);
+    k_gemm_tn_reduce_same<<<rg, 128, 0, s>>> (total, m1, nsplit, work, C, ldc);
   } else {
     const int rg = (int) std::min<int64_t> ((total + 255) / 256, num_sms () * 8);
     k_gemm_tn_reduce<<<rg, 256, 0, s>>> (m1, m2, nsplit, work, C, ldc, sym, upper);
@@ -495,7 +532,7 @@ template <typename T>
 static int
 gemm_tn_run (int64_t n, int m1, int m2, const T *A, int lda, const T *B, int ldb,
              double *C, int ldc, int sym, double *work, int nsplit, bool upper,
-             cudaStream_t s)
+             cudaStream_t s, int tiles = 0)
 {
   int64_t kchunk = (n + nsplit - 1) / nsplit;
   kchunk = (kchunk + GK - 1) / GK * GK;
@@ -516,9 +553,8 @@ gemm_tn_run (int64_t n, int m1, int m2, const T *A, int lda, const T *B, int ldb
   else if (a16) LGH_TRY (run (C16 (), CS ()));
   else if (b16) LGH_TRY (run (CS (), C16 ()));
   else LGH_TRY (run (CS (), CS ()));
-  return gemm_tn_sum (m1, m2, nsplit, work, C, ldc, sym, upper, s);
+  return gemm_tn_sum (m1, m2, nsplit, work, C, ldc, sym, upper, s, tiles);
 }
-
 
 template <typename T>
 int
@@ -528,7 +564,7 @@ launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
 {
   if (m1 == 0 || m2 == 0) return 0;
   LGH_CHECK (!sym || m1 == m2, LGH_ERR_ARG_SIZ, "gemm_tn: sym needs square");
-  int ns = tn_splits (n, m1, m2);
+  int ns = tn_splits (n, m1, tiles ? 1 : m2);
   LGH_CHECK ((size_t) ns * m1 * m2 <= work_elems, LGH_ERR_ARG_SIZ,
              "gemm_tn: workspace too small");
   constexpr int W = Pack<T>::W;
@@ -544,7 +580,8 @@ launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
     return gemm_tn_sum (m1, 1, nb, work, C, ldc, 0, 0, s);
   }
   /* X^T X: its upper tiles alone, over as many more slices as fit */
-  const bool upper = (const void *) A == (const void *) B && lda == ldb && m1 == m2;
+  const bool upper = !tiles && (const void *) A == (const void *) B && lda == ldb
+                     && m1 == m2;
   if (upper) {
     const int tm = (m1 + GB - 1) / GB;
     const int64_t want = std::max (1, 4 * num_sms () / (tm * (tm + 1) / 2));
@@ -553,7 +590,8 @@ launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
                                                      (int64_t) (work_elems / ((size_t) m1 * m2))));
     ns = std::max (ns, 1);
   }
-  return gemm_tn_run<T> (n, m1, m2, A, lda, B, ldb, C, ldc, sym, work, ns, upper, s);
+  return gemm_tn_run<T> (n, m1, m2, A, lda, B, ldb, C, ldc, sym, work, ns, upper, s,
+                         tiles);
 }
 
 /* the same product with an explicit split count and caller-provided

@@ -285,8 +285,9 @@ int launch_vec_axpby (int64_t n, double a, const double *x, double b,
 /* dense (k_gemm.cu): C = A^T B over n rows (split-K, FP64 accumulate),
  * C is m1 x m2 column-major with leading dim ldc; sym: 1 => C = (C + C^T)/2.
  * One column takes a streaming kernel of its own unless tiles (and
- * tiles_only below) is set: the request loop's columns get the same bits at
- * every batch width from the tiled form alone. */
+ * tiles_only below) is set: the request loop's columns must get the same
+ * bits at every batch width, so with tiles the row slices and the order of
+ * their sum do not depend on m2 either (workspace: gemm_tn_work_tiles). */
 template <typename T>
 int launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda,
                     const T *B, int ldb, double *C, int ldc, int sym,
@@ -300,6 +301,7 @@ int launch_gemm_nn (int64_t n, int k, int m2, double alpha, const T *X,
                     const T *Y0, int ldy0, T *Y, int ldy, cudaStream_t s,
                     int tiles_only = 0);
 size_t gemm_tn_work_elems (int64_t n, int m1, int m2);
+size_t gemm_tn_work_tiles (int64_t n, int m1, int m2max);
 
 /* partial-sum elements enough for every gemm_tn shape up to m1max x m2max */
 size_t gemm_tn_work_max (int m1max, int m2max);
