@@ -31,6 +31,9 @@ struct MgLevel
    * coarse solution (k_flat.cu; owned, empty on the coarsest level and at
    * other smoother degrees) */
   Csr Q;
+  /* A P, where Q is not formed (rows of more than 1022 entries): the
+   * residual after the coarse correction is r2 - (A P) xc (owned) */
+  Csr AP;
 };
 
 struct MgWork

@@ -677,6 +677,7 @@ Hierarchy::~Hierarchy ()
     dfree (l.f1v);
     dfree (l.f1v32);
     csr_free (l.Q);
+    csr_free (l.AP);
   }
 }
 
@@ -848,9 +849,13 @@ k_row_sum (int64_t n, Sum op, int64_t *counts, const int64_t *ptr,
   }
 }
 
+/* lists of a row that k_row_sum takes: 32 per lane */
+constexpr int ROW_SUM_LISTS = 1024;
+
 /* the result as a device Csr of n rows and m columns (rowptr, colidx and
  * vals alone; csr_finish adds the rest); maxlists: the most lists of a row;
- * *fits = 0 (and no result) if they exceed 32 per lane or the entries 2^31 */
+ * *fits = 0 (and no result) if they exceed ROW_SUM_LISTS or the entries
+ * 2^31 */
 template <typename Sum>
 static int
 row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
@@ -884,7 +889,7 @@ row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
       return run (integral_constant<int, 32> (), integral_constant<int, 3> ());
     if (maxlists <= 256)
       return run (integral_constant<int, 32> (), integral_constant<int, 8> ());
-    if (maxlists <= 1024)
+    if (maxlists <= ROW_SUM_LISTS)
       return run (integral_constant<int, 32> (), integral_constant<int, 32> ());
     *fits = 0;
     return 0;
@@ -907,11 +912,13 @@ row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
   return rc;
 }
 
-/* lv.Q from the level's device operators (A, F1, P).  Left empty, and the
- * level on the correction form, where an operator's entries pass 32 bits
- * or a row of A holds more than 1022. */
+/* lv.Q from the level's device operators (A, F1, P).  Where a row of A
+ * holds more than 1022 entries the merge does not fit a group's lists: the
+ * level keeps A P instead (hAP, the Galerkin step's).  Both are left empty,
+ * and the level on the correction form, where an operator's entries pass
+ * 32 bits. */
 static int
-smoothed_correction (MgLevel &lv)
+smoothed_correction (MgLevel &lv, const HCsr &hAP)
 {
   if (lv.A.nnz >= FLAT_NNZ_MAX || lv.P.nnz >= FLAT_NNZ_MAX
       || lv.R.nnz >= FLAT_NNZ_MAX)
@@ -921,6 +928,8 @@ smoothed_correction (MgLevel &lv)
   const int64_t m = lv.P.ncols;
   int fits = 0;
   Csr AP;
+  if (lv.A.max_row_nnz + 2 > ROW_SUM_LISTS)
+    return hAP.rp[hAP.n] < FLAT_NNZ_MAX ? csr_upload (hAP, lv.AP) : 0;
   LGH_TRY (row_sum (lv.n, m, lv.A.max_row_nnz, SumAP{ lv.A, lv.P }, AP, &fits));
   if (!fits) return 0;
   const SumQ q{ lv.F1, lv.P, AP, lv.A.dinv, b2, b1 * (1. + a2) + b2 };
@@ -936,11 +945,11 @@ mg_destroy (Hierarchy *h)
   delete h;
 }
 
-/* smoothed-aggregation hierarchy of Z (level 0 borrows Z's device arrays) */
-/* the Galerkin step of one level: R = P^T, A P and Ac = P^T (A P), symmetrised against rounding: every entry
- * (i, j) averaged with its mirror (j, i), found in row j's sorted columns
- * (the pattern of P^T A P is symmetric); the averages go to a copy so that
- * each pair reads the unsymmetrised values */
+/* the Galerkin step of one level: R = P^T, A P and Ac = P^T (A P),
+ * symmetrised against rounding: every entry (i, j) averaged with its mirror
+ * (j, i), found in row j's sorted columns (the pattern of P^T A P is
+ * symmetric); the averages go to a copy so that each pair reads the
+ * unsymmetrised values */
 static void
 galerkin (const HCsr &A, const HCsr &P, HCsr &R, HCsr &AP, HCsr &Ac)
 {
@@ -1026,6 +1035,7 @@ mg_host_galerkin (int64_t n, const int64_t *rowptr, const int32_t *colidx,
   return 0;
 }
 
+/* smoothed-aggregation hierarchy of Z (level 0 borrows Z's device arrays) */
 int
 mg_build (const Csr &Z, int tile, double smoother_top, int nu, Hierarchy **out)
 {
@@ -1128,7 +1138,7 @@ mg_build (const Csr &Z, int tile, double smoother_top, int nu, Hierarchy **out)
     lap (3);
     rc = csr_upload (P, lv.P);
     if (!rc) rc = csr_upload (R, lv.R);
-    if (!rc && lv.f1v) rc = smoothed_correction (lv);
+    if (!rc && lv.f1v) rc = smoothed_correction (lv, AP);
     if (rc) { delete h; return rc; }
     h->lev.push_back (lv);
     A = std::move (Ac);
@@ -1150,7 +1160,7 @@ mg_build (const Csr &Z, int tile, double smoother_top, int nu, Hierarchy **out)
 static bool
 two_step (const MgLevel &lv)
 {
-  return lv.nu == 2 && lv.f1v != nullptr && lv.Q.n == lv.n;
+  return lv.nu == 2 && lv.f1v != nullptr && (lv.Q.n == lv.n || lv.AP.n == lv.n);
 }
 
 template <typename T>
@@ -1169,14 +1179,14 @@ mg_work (Hierarchy *h, int ld, MgWork **w0, std::vector<MgWork> *own)
       LGH_TRY (w.X.alloc (bytes));
     }
     /* the coarsest level solves densely from B into X; the two-step
-     * smoother keeps no direction blocks (only other degrees use D0, D1) */
+     * smoother keeps no direction blocks (other degrees use D0 and D1, a
+     * two-step level without Q has its third residual in D0) */
     if (l + 1 < h->lev.size ()) {
+      const MgLevel &lv = h->lev[l];
       LGH_TRY (w.R0.alloc (bytes));
       LGH_TRY (w.R1.alloc (bytes));
-      if (!two_step (h->lev[l])) {
-        LGH_TRY (w.D0.alloc (bytes));
-        LGH_TRY (w.D1.alloc (bytes));
-      }
+      if (!two_step (lv) || lv.Q.n != lv.n) LGH_TRY (w.D0.alloc (bytes));
+      if (!two_step (lv)) LGH_TRY (w.D1.alloc (bytes));
     }
     w.cap = ld;
   }
@@ -1283,10 +1293,23 @@ vcycle_level (Hierarchy *h, MgWork *W, size_t l, const T *B, T *X, int ld,
     LGH_TRY (launch_flat_mult<T> (lv.R, Ra, Bc, ld, s));
     if (tr) LGH_TRY (tr->end (s));
     LGH_TRY (vcycle_level<T> (h, W, l + 1, Bc, Xc, ld, w, s, trace));
+    /* without Q: z = S r0 + S r3 + P xc with the corrected residual r3 =
+     * r2 - (A P) xc, the same form in r3 and P.  A solve at 4000 rows of
+     * 1201 entries, 1 / 64 / 220 columns: 21, 17, 45 ms; 64, 42, 107 with
+     * the correction form */
+    const bool q = lv.Q.n == n;
+    const Csr &C = q ? lv.Q : lv.P;
+    if (!q) {
+      if (tr) LGH_TRY (tr->begin (K_MG_RESID, 2. * blk + cb
+                                  + (4. + sizeof (T)) * lv.AP.nnz, s));
+      LGH_TRY (launch_spmm_mode<T> (lv.AP, Xc, ld, D0, ld, ld, 2, Ra, ld, s));
+      if (tr) LGH_TRY (tr->end (s));
+      Ra = D0;
+    }
     if (tr) LGH_TRY (tr->begin (K_MG_FINISH, mb + 4. * blk + cb
-                                + (4. + sizeof (T)) * lv.Q.nnz + 8. * (n + 1)
+                                + (4. + sizeof (T)) * C.nnz + 8. * (n + 1)
                                 + (double) n * sizeof (T), s));
-    LGH_TRY (launch_vc_finish<T> (lv.F1, lv.Q, zdinv_of<T> (lv.A), B, R, Ra, Xc,
+    LGH_TRY (launch_vc_finish<T> (lv.F1, C, zdinv_of<T> (lv.A), B, R, Ra, Xc,
                                   X, ld, b1 * (1. + a2), b2, s));
     if (tr) LGH_TRY (tr->end (s));
     return 0;
