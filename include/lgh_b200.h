@@ -721,6 +721,11 @@ int lgh_test_zsolve (lgh_prior_t *prior, int w, const double *X, double *Y,
  * the level count and smax (cap entries) each level's lambda_max estimate */
 int lgh_test_vcycle (lgh_prior_t *prior, int w, const double *X, double *Y,
                      int fp32, double *smax, int cap, int *nlev);
+/* the finest level's passes of that V-cycle alone, with the restricted
+ * residual itself as the coarse solution and fixed coefficients; wide != 0:
+ * with the 64-bit entry offsets that operators of 2^31 entries take */
+int lgh_test_vc_level (lgh_prior_t *prior, int w, const double *X, double *Y,
+                       int fp32, int wide);
 /* one Chebyshev-Jacobi smoothing step of a square CSR Mat (n x w row-major
  * host blocks) with the smoother's kernel: X in place, Rout = Ro - A d_new,
  * Dout = d_new (flags & 4), d_new = a Do + b D^{-1} Ro (flags & 1: a Do

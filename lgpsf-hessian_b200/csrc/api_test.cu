@@ -97,7 +97,55 @@ test_vcycle (lgh_prior_t *p, int w, const double *X, double *Y)
   return 0;
 }
 
+/* the finest level's four passes alone: z from r = X with the restricted
+ * second residual itself as the coarse solution */
+template <typename T>
+static int
+test_vc_level (lgh_prior_t *p, int w, const double *X, double *Y, int wide)
+{
+  const MgLevel &lv = p->mg->lev[0];
+  const int64_t n = p->n;
+  const int ld = round_ld (w);
+  cudaStream_t s = stream ();
+  const Csr &Q = lv.Q.n == n ? lv.Q : lv.P;
+  const T *dinv;
+  if constexpr (sizeof (T) == 8) dinv = lv.A.dinv;
+  else dinv = lv.A.dinv32;
+  std::vector<T> h ((size_t) n * ld, T (0));
+  for (int64_t i = 0; i < n; i++)
+    for (int j = 0; j < w; j++) h[i * ld + j] = (T) X[i * w + j];
+  DBuf<T> r0, r1, r2, xc, z;
+  LGH_TRY (up (r0, h.data (), h.size ()));
+  LGH_TRY (r1.alloc (h.size ()));
+  LGH_TRY (r2.alloc (h.size ()));
+  LGH_TRY (xc.alloc ((size_t) lv.R.n * ld));
+  LGH_TRY (z.alloc (h.size ()));
+  LGH_TRY (launch_vc_first<T> (lv.F1, r0.p, r1.p, ld, s, wide));
+  LGH_TRY (launch_vc_second<T> (lv.F1, r0.p, r1.p, r2.p, ld, 0.25, 0.75, s, wide));
+  LGH_TRY (launch_flat_mult<T> (lv.R, r2.p, xc.p, ld, s, wide));
+  LGH_TRY (launch_vc_finish<T> (lv.F1, Q, dinv, r0.p, r1.p, r2.p, xc.p, z.p, ld,
+                                0.5, 0.375, s, wide));
+  LGH_CUDA (cudaStreamSynchronize (s));
+  LGH_TRY (down (h.data (), z, h.size ()));
+  for (int64_t i = 0; i < n; i++)
+    for (int j = 0; j < w; j++) Y[i * w + j] = (double) h[i * ld + j];
+  return 0;
+}
+
 extern "C" {
+
+int
+lgh_test_vc_level (lgh_prior_t *prior, int w, const double *X, double *Y,
+                   int fp32, int wide)
+{
+  LGH_TRY (ensure_init ());
+  LGH_CHECK (prior && X && Y && w > 0, LGH_ERR_ARG_NULL, "lgh_test_vc_level: NULL");
+  LGH_CHECK (prior->mg && !prior->rows && prior->mg->lev.size () > 1
+                 && prior->mg->lev[0].f1v, LGH_ERR_SUP,
+             "lgh_test_vc_level: the prior has no two-step level");
+  return fp32 ? test_vc_level<float> (prior, w, X, Y, wide)
+              : test_vc_level<double> (prior, w, X, Y, wide);
+}
 
 int
 lgh_test_vcycle (lgh_prior_t *prior, int w, const double *X, double *Y,

@@ -17,7 +17,8 @@
  * is at hand, so r1 alone is gathered where d2 = a2 d1 + b2 D^{-1} r1 was.
  * Block passes: 2 + 3 + 4 (and the coarse blocks), against 2 + 4 + 2 + 3
  * with the stored iterate.  All four are bound by L1 wavefronts at the
- * residency their registers allow (lgh_flat.cuh); each kernel gives its
+ * residency their registers allow (lgh_flat.cuh); I is the type of entry
+ * offsets, 64 bits only for operators of 2^31 entries; each kernel gives its
  * time at 512^2 x 220 columns FP64 on the finest level, its floor at the
  * measured HBM rate and what the passes it replaces took. */
 
@@ -31,7 +32,7 @@ namespace lgh
 
 /* Y = B - A X (first step: X = B = r0): 180 us, floor 141; a row per power
  * of two of lanes with shuffled entries 247 */
-template <typename T, int CH>
+template <typename T, typename I, int CH>
 __global__ void __launch_bounds__ (FLAT_THREADS, FlatOcc<CH>::v)
 k_flat_resid (int64_t n, const int64_t *__restrict__ rowptr,
               const int32_t *__restrict__ colidx, const T *__restrict__ vals,
@@ -44,13 +45,13 @@ k_flat_resid (int64_t n, const int64_t *__restrict__ rowptr,
   const int64_t stride = (int64_t) gridDim.x * rpc;
   int64_t i = (int64_t) blockIdx.x * rpc + rl;
   if (rl >= rpc || i >= n) return;
-  int k0 = (int) rowptr[i], k1 = (int) rowptr[i + 1];
+  I k0 = (I) rowptr[i], k1 = (I) rowptr[i + 1];
   for (; i < n; i += stride) {
     /* the next row's bounds load during this row's gathers */
-    int k0n = 0, k1n = 0;
+    I k0n = 0, k1n = 0;
     if (i + stride < n) {
-      k0n = (int) rowptr[i + stride];
-      k1n = (int) rowptr[i + stride + 1];
+      k0n = (I) rowptr[i + stride];
+      k1n = (I) rowptr[i + stride + 1];
     }
     T acc[CH][W];
     flat_zero<T, CH, W> (acc);
@@ -74,7 +75,7 @@ k_flat_resid (int64_t n, const int64_t *__restrict__ rowptr,
 /* r2 = r1 - a2 (r0 - r1) - s2 F1 r1 (s2 = b2 / b1): reads r1 (gathered)
  * and r0, writes r2.  280 us, floor 211; with d and x re-formed from two
  * gathered blocks 580 */
-template <typename T, int CH>
+template <typename T, typename I, int CH>
 __global__ void __launch_bounds__ (FLAT_THREADS, FlatOcc<CH>::v)
 k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
                const int32_t *__restrict__ colidx, const T *__restrict__ vals,
@@ -88,12 +89,12 @@ k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
   const int64_t stride = (int64_t) gridDim.x * rpc;
   int64_t i = (int64_t) blockIdx.x * rpc + rl;
   if (rl >= rpc || i >= n) return;
-  int k0 = (int) rowptr[i], k1 = (int) rowptr[i + 1];
+  I k0 = (I) rowptr[i], k1 = (I) rowptr[i + 1];
   for (; i < n; i += stride) {
-    int k0n = 0, k1n = 0;
+    I k0n = 0, k1n = 0;
     if (i + stride < n) {
-      k0n = (int) rowptr[i + stride];
-      k1n = (int) rowptr[i + stride + 1];
+      k0n = (I) rowptr[i + stride];
+      k1n = (I) rowptr[i + stride + 1];
     }
     T acc[CH][W];
     flat_zero<T, CH, W> (acc);
@@ -121,7 +122,7 @@ k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
 /* z = dinv (g (r0 + r2) + b2 (r1 + r2 - F1 r2)) + Q xc: reads r0, r1, r2
  * (gathered) and the coarse block (gathered), writes z.  487 us, floor 297;
  * the post residual and the two post-smoothing steps took 787 */
-template <typename T, int CH>
+template <typename T, typename I, int CH>
 __global__ void __launch_bounds__ (FLAT_THREADS, CH == 2 ? 5 : (CH == 3 ? 4 : FlatOcc<CH>::v))
 k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
                const int32_t *__restrict__ fci, const T *__restrict__ fv,
@@ -138,15 +139,15 @@ k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
   const int64_t stride = (int64_t) gridDim.x * rpc;
   int64_t i = (int64_t) blockIdx.x * rpc + rl;
   if (rl >= rpc || i >= n) return;
-  int k0 = (int) frp[i], k1 = (int) frp[i + 1];
-  int q0 = (int) qrp[i], q1 = (int) qrp[i + 1];
+  I k0 = (I) frp[i], k1 = (I) frp[i + 1];
+  I q0 = (I) qrp[i], q1 = (I) qrp[i + 1];
   for (; i < n; i += stride) {
-    int k0n = 0, k1n = 0, q0n = 0, q1n = 0;
+    I k0n = 0, k1n = 0, q0n = 0, q1n = 0;
     if (i + stride < n) {
-      k0n = (int) frp[i + stride];
-      k1n = (int) frp[i + stride + 1];
-      q0n = (int) qrp[i + stride];
-      q1n = (int) qrp[i + stride + 1];
+      k0n = (I) frp[i + stride];
+      k1n = (I) frp[i + stride + 1];
+      q0n = (I) qrp[i + stride];
+      q1n = (I) qrp[i + stride + 1];
     }
     T acc[CH][W];
     flat_zero<T, CH, W> (acc);
@@ -188,7 +189,7 @@ k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
  * entries are dealt out to S neighbouring thread groups of the CTA, whose
  * sums are added in group order through shared memory.  128 us for the
  * finest level's, 154 with a warp group per row */
-template <typename T, int CH, bool SPLIT>
+template <typename T, typename I, int CH, bool SPLIT>
 __global__ void __launch_bounds__ (FLAT_THREADS, FlatOcc<CH>::v)
 k_flat_mult (int64_t n, const int64_t *__restrict__ rowptr,
              const int32_t *__restrict__ colidx, const T *__restrict__ vals,
@@ -208,7 +209,7 @@ k_flat_mult (int64_t n, const int64_t *__restrict__ rowptr,
     T acc[CH][W];
     flat_zero<T, CH, W> (acc);
     if (on) {
-      flat_gather<T, CH> (colidx, vals, (int) rowptr[i] + sp, (int) rowptr[i + 1],
+      flat_gather<T, CH> (colidx, vals, (I) rowptr[i] + sp, (I) rowptr[i + 1],
                           SPLIT ? S : 1, X, ld, lane, L, nvec, acc);
     }
     if constexpr (SPLIT) {
@@ -298,19 +299,25 @@ flat_check (const Csr &A, const void *a, const void *b, const void *c, int ld)
 
 template <typename T>
 int
-launch_vc_first (const Csr &F1, const T *R0, T *R1, int ld, cudaStream_t s)
+launch_vc_first (const Csr &F1, const T *R0, T *R1, int ld, cudaStream_t s,
+                 int wide)
 {
   constexpr int W = Pack<T>::W;
+  const bool big = wide || F1.nnz >= FLAT_NNZ_MAX;
   const int64_t bytes = F1.n * ld * (int64_t) sizeof (T);
   LGH_TRY (flat_check<T> (F1, R0, R1, nullptr, ld));
   return flat_slices (F1.n, F1.bandwidth, ld, ld / W, sizeof (T), [&] (int v0, int nv) {
     const FlatShape f = flat_shape (nv, F1.n);
     LGH_FLAT_DISPATCH (f.ch, {
-      auto k = k_flat_resid<T, CH_>;
-      LGH_CUDA (launch_pdl (bytes, k,
-          fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
-          s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
-          R0 + v0 * W, R1 + v0 * W, ld, nv, f.L, f.rpc));
+      auto run = [&] (auto idx) -> int {
+        auto k = k_flat_resid<T, decltype (idx), CH_>;
+        LGH_CUDA (launch_pdl (bytes, k,
+            fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
+            s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
+            R0 + v0 * W, R1 + v0 * W, ld, nv, f.L, f.rpc));
+        return 0;
+      };
+      LGH_TRY (big ? run (int64_t ()) : run (int ()));
     });
     LGH_LAUNCH_CHECK ();
     return 0;
@@ -320,19 +327,24 @@ launch_vc_first (const Csr &F1, const T *R0, T *R1, int ld, cudaStream_t s)
 template <typename T>
 int
 launch_vc_second (const Csr &F1, const T *R0, const T *R1, T *R2, int ld,
-                  double a2, double s2, cudaStream_t s)
+                  double a2, double s2, cudaStream_t s, int wide)
 {
   constexpr int W = Pack<T>::W;
+  const bool big = wide || F1.nnz >= FLAT_NNZ_MAX;
   const int64_t bytes = F1.n * ld * (int64_t) sizeof (T);
   LGH_TRY (flat_check<T> (F1, R0, R1, R2, ld));
   return flat_slices (F1.n, F1.bandwidth, ld, ld / W, sizeof (T), [&] (int v0, int nv) {
     const FlatShape f = flat_shape (nv, F1.n);
     LGH_FLAT_DISPATCH (f.ch, {
-      auto k = k_flat_second<T, CH_>;
-      LGH_CUDA (launch_pdl (bytes, k,
-          fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
-          s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
-          R1 + v0 * W, R2 + v0 * W, ld, nv, f.L, f.rpc, (T) a2, (T) s2));
+      auto run = [&] (auto idx) -> int {
+        auto k = k_flat_second<T, decltype (idx), CH_>;
+        LGH_CUDA (launch_pdl (bytes, k,
+            fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
+            s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), R0 + v0 * W,
+            R1 + v0 * W, R2 + v0 * W, ld, nv, f.L, f.rpc, (T) a2, (T) s2));
+        return 0;
+      };
+      LGH_TRY (big ? run (int64_t ()) : run (int ()));
     });
     LGH_LAUNCH_CHECK ();
     return 0;
@@ -343,9 +355,10 @@ template <typename T>
 int
 launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
                   const T *R1, const T *R2, const T *Xc, T *Z, int ld, double g,
-                  double b2, cudaStream_t s)
+                  double b2, cudaStream_t s, int wide)
 {
   constexpr int W = Pack<T>::W;
+  const bool big = wide || F1.nnz >= FLAT_NNZ_MAX || Q.nnz >= FLAT_NNZ_MAX;
   const int64_t bytes = F1.n * ld * (int64_t) sizeof (T);
   LGH_TRY (flat_check<T> (F1, R0, R1, R2, ld));
   LGH_TRY (flat_check<T> (Q, Xc, Z, nullptr, ld));
@@ -363,12 +376,16 @@ launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
         && (lng || (nv % 3 == 0 && nv <= 64)))
       f = flat_shape_ch (nv, 3);
     LGH_FLAT_DISPATCH (f.ch, {
-      auto k = k_flat_finish<T, CH_>;
-      LGH_CUDA (launch_pdl (bytes, k,
-          fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
-          s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), Q.rowptr, Q.colidx,
-          fvals<T> (Q), dinv, R0 + v0 * W, R1 + v0 * W, R2 + v0 * W,
-          Xc + v0 * W, Z + v0 * W, ld, nv, f.L, f.rpc, (T) g, (T) b2));
+      auto run = [&] (auto idx) -> int {
+        auto k = k_flat_finish<T, decltype (idx), CH_>;
+        LGH_CUDA (launch_pdl (bytes, k,
+            fit_grid (k, flat_grid (f, F1.n), FLAT_THREADS, 0), FLAT_THREADS, 0,
+            s, F1.n, F1.rowptr, F1.colidx, fvals<T> (F1), Q.rowptr, Q.colidx,
+            fvals<T> (Q), dinv, R0 + v0 * W, R1 + v0 * W, R2 + v0 * W,
+            Xc + v0 * W, Z + v0 * W, ld, nv, f.L, f.rpc, (T) g, (T) b2));
+        return 0;
+      };
+      LGH_TRY (big ? run (int64_t ()) : run (int ()));
     });
     LGH_LAUNCH_CHECK ();
     return 0;
@@ -377,9 +394,11 @@ launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
 
 template <typename T>
 int
-launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s)
+launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s,
+                  int wide)
 {
   constexpr int W = Pack<T>::W;
+  const bool big = wide || A.nnz >= FLAT_NNZ_MAX;
   const int64_t bytes = A.ncols * ld * (int64_t) sizeof (T);
   LGH_TRY (flat_check<T> (A, X, Y, nullptr, ld));
   /* one launch holds at most FLAT_MAXPACKS packs of a row */
@@ -397,17 +416,20 @@ launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s)
     const int want = (int) std::max<int64_t> (1, std::min<int64_t> (tiles, 1 << 20));
     const int smem = S > 1 ? rows * S * nv * 16 : 0;
     LGH_FLAT_DISPATCH (f.ch, {
-      if (S > 1) {
-        auto k = k_flat_mult<T, CH_, true>;
+      auto run = [&] (auto idx, auto split) -> int {
+        constexpr bool SPLIT = decltype (split)::value;
+        auto k = k_flat_mult<T, decltype (idx), CH_, SPLIT>;
         LGH_CUDA (launch_pdl (bytes, k, fit_grid (k, want, FLAT_THREADS, smem),
             FLAT_THREADS, smem, s, A.n, A.rowptr, A.colidx, fvals<T> (A),
             X + v0 * W, Y + v0 * W, ld, nv, f.L, rows, S));
-      } else {
-        auto k = k_flat_mult<T, CH_, false>;
-        LGH_CUDA (launch_pdl (bytes, k, fit_grid (k, want, FLAT_THREADS, 0),
-            FLAT_THREADS, 0, s, A.n, A.rowptr, A.colidx, fvals<T> (A),
-            X + v0 * W, Y + v0 * W, ld, nv, f.L, rows, 1));
-      }
+        return 0;
+      };
+      if (S > 1)
+        LGH_TRY (big ? run (int64_t (), std::true_type ())
+                     : run (int (), std::true_type ()));
+      else
+        LGH_TRY (big ? run (int64_t (), std::false_type ())
+                     : run (int (), std::false_type ()));
     });
     LGH_LAUNCH_CHECK ();
     return 0;
@@ -416,15 +438,15 @@ launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s)
 
 #define LGH_FLAT_INST(T)                                                     \
   template int launch_vc_first<T> (const Csr &, const T *, T *, int,         \
-                                   cudaStream_t);                            \
+                                   cudaStream_t, int);                       \
   template int launch_vc_second<T> (const Csr &, const T *, const T *, T *,  \
-                                    int, double, double, cudaStream_t);      \
+                                    int, double, double, cudaStream_t, int); \
   template int launch_vc_finish<T> (const Csr &, const Csr &, const T *,     \
                                     const T *, const T *, const T *,         \
                                     const T *, T *, int, double, double,     \
-                                    cudaStream_t);                           \
+                                    cudaStream_t, int);                      \
   template int launch_flat_mult<T> (const Csr &, const T *, T *, int,        \
-                                    cudaStream_t);
+                                    cudaStream_t, int);
 LGH_FLAT_INST (double)
 LGH_FLAT_INST (float)
 #undef LGH_FLAT_INST

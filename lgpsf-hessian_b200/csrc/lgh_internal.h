@@ -239,18 +239,21 @@ int launch_scan_counts (int64_t m, const int64_t *counts, int64_t *ptr,
  *   first   R1 = R0 - F1 R0
  *   second  R2 = R1 - a2 (R0 - R1) - s2 F1 R1
  *   finish  Z = D^{-1} (g (R0 + R2) + b2 (R1 + R2 - F1 R2)) + Q Xc
- * and Y = A X for the restriction (rows split over thread groups) */
+ * and Y = A X for the restriction (rows split over thread groups).  wide:
+ * 64-bit entry offsets whatever the entry counts (testing) */
 template <typename T>
-int launch_vc_first (const Csr &F1, const T *R0, T *R1, int ld, cudaStream_t s);
+int launch_vc_first (const Csr &F1, const T *R0, T *R1, int ld, cudaStream_t s,
+                     int wide = 0);
 template <typename T>
 int launch_vc_second (const Csr &F1, const T *R0, const T *R1, T *R2, int ld,
-                      double a2, double s2, cudaStream_t s);
+                      double a2, double s2, cudaStream_t s, int wide = 0);
 template <typename T>
 int launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
                       const T *R1, const T *R2, const T *Xc, T *Z, int ld,
-                      double g, double b2, cudaStream_t s);
+                      double g, double b2, cudaStream_t s, int wide = 0);
 template <typename T>
-int launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s);
+int launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s,
+                      int wide = 0);
 
 /* elementwise / block helpers (k_vec.cu) */
 template <typename T>

@@ -853,12 +853,11 @@ k_row_sum (int64_t n, Sum op, int64_t *counts, const int64_t *ptr,
 constexpr int ROW_SUM_LISTS = 1024;
 
 /* the result as a device Csr of n rows and m columns (rowptr, colidx and
- * vals alone; csr_finish adds the rest); maxlists: the most lists of a row;
- * *fits = 0 (and no result) if they exceed ROW_SUM_LISTS or the entries
- * 2^31 */
+ * vals alone; csr_finish adds the rest); maxlists: the most lists of a row,
+ * at most ROW_SUM_LISTS */
 template <typename Sum>
 static int
-row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
+row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out)
 {
   cudaStream_t s = stream ();
   DBuf<int64_t> counts;
@@ -866,7 +865,6 @@ row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
   out = Csr ();
   out.n = n;
   out.ncols = m;
-  *fits = 1;
   auto pass = [&] (bool fill) -> int {
     auto run = [&] (auto g, auto c) -> int {
       constexpr int G = decltype (g)::value, C = decltype (c)::value;
@@ -889,53 +887,40 @@ row_sum (int64_t n, int64_t m, int maxlists, const Sum &op, Csr &out, int *fits)
       return run (integral_constant<int, 32> (), integral_constant<int, 3> ());
     if (maxlists <= 256)
       return run (integral_constant<int, 32> (), integral_constant<int, 8> ());
-    if (maxlists <= ROW_SUM_LISTS)
-      return run (integral_constant<int, 32> (), integral_constant<int, 32> ());
-    *fits = 0;
-    return 0;
+    LGH_CHECK (maxlists <= ROW_SUM_LISTS, LGH_ERR_SUP, "mg: %d lists a row",
+               maxlists);
+    return run (integral_constant<int, 32> (), integral_constant<int, 32> ());
   };
-  int rc = pass (false);
-  if (rc || !*fits) return rc;
-  rc = dalloc ((void **) &out.rowptr, (size_t) (n + 1) * sizeof (int64_t));
+  LGH_TRY (pass (false));
+  int rc = dalloc ((void **) &out.rowptr, (size_t) (n + 1) * sizeof (int64_t));
   if (!rc) rc = launch_scan_counts (n, counts.p, out.rowptr, s);
   if (!rc && (cudaMemcpyAsync (&out.nnz, out.rowptr + n, sizeof (int64_t),
                                cudaMemcpyDeviceToHost, s) != cudaSuccess
               || cudaStreamSynchronize (s) != cudaSuccess))
     rc = set_error (LGH_ERR_GPU, "mg: sparse product sizes");
-  if (!rc && out.nnz >= FLAT_NNZ_MAX) *fits = 0;
-  if (!rc && *fits) {
-    rc = dalloc ((void **) &out.colidx, (size_t) out.nnz * sizeof (int32_t) + 16);
-    if (!rc) rc = dalloc ((void **) &out.vals, (size_t) out.nnz * sizeof (double) + 16);
-    if (!rc) rc = pass (true);
-  }
-  if (rc || !*fits) csr_free (out);
+  if (!rc) rc = dalloc ((void **) &out.colidx, (size_t) out.nnz * sizeof (int32_t) + 16);
+  if (!rc) rc = dalloc ((void **) &out.vals, (size_t) out.nnz * sizeof (double) + 16);
+  if (!rc) rc = pass (true);
+  if (rc) csr_free (out);
   return rc;
 }
 
 /* lv.Q from the level's device operators (A, F1, P).  Where a row of A
  * holds more than 1022 entries the merge does not fit a group's lists: the
- * level keeps A P instead (hAP, the Galerkin step's).  Both are left empty,
- * and the level on the correction form, where an operator's entries pass
- * 32 bits. */
+ * level keeps A P instead (hAP, the Galerkin step's). */
 static int
 smoothed_correction (MgLevel &lv, const HCsr &hAP)
 {
-  if (lv.A.nnz >= FLAT_NNZ_MAX || lv.P.nnz >= FLAT_NNZ_MAX
-      || lv.R.nnz >= FLAT_NNZ_MAX)
-    return 0;
+  if (lv.A.max_row_nnz + 2 > ROW_SUM_LISTS) return csr_upload (hAP, lv.AP);
   double b1, a2, b2;
   cheb2_coeffs (lv, &b1, &a2, &b2);
   const int64_t m = lv.P.ncols;
-  int fits = 0;
   Csr AP;
-  if (lv.A.max_row_nnz + 2 > ROW_SUM_LISTS)
-    return hAP.rp[hAP.n] < FLAT_NNZ_MAX ? csr_upload (hAP, lv.AP) : 0;
-  LGH_TRY (row_sum (lv.n, m, lv.A.max_row_nnz, SumAP{ lv.A, lv.P }, AP, &fits));
-  if (!fits) return 0;
+  LGH_TRY (row_sum (lv.n, m, lv.A.max_row_nnz, SumAP{ lv.A, lv.P }, AP));
   const SumQ q{ lv.F1, lv.P, AP, lv.A.dinv, b2, b1 * (1. + a2) + b2 };
-  int rc = row_sum (lv.n, m, lv.A.max_row_nnz + 2, q, lv.Q, &fits);
+  int rc = row_sum (lv.n, m, lv.A.max_row_nnz + 2, q, lv.Q);
   csr_free (AP);
-  if (!rc && fits) rc = csr_finish (lv.Q);
+  if (!rc) rc = csr_finish (lv.Q);
   return rc;
 }
 

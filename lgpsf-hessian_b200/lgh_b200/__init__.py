@@ -333,6 +333,8 @@ SIGNATURES = {
     "lgh_test_zsolve": (ctypes.c_int, [P, ctypes.c_int, P, P, ctypes.c_int]),
     "lgh_test_vcycle": (ctypes.c_int, [P, ctypes.c_int, P, P, ctypes.c_int,
                                        P, ctypes.c_int, P]),
+    "lgh_test_vc_level": (ctypes.c_int, [P, ctypes.c_int, P, P, ctypes.c_int,
+                                         ctypes.c_int]),
     "lgh_test_cheb_step": (ctypes.c_int, [P, ctypes.c_int, ctypes.c_double,
                                           ctypes.c_double, ctypes.c_int,
                                           ctypes.c_int, P, P, P, P, P,
@@ -1072,6 +1074,16 @@ def test_vcycle(prior, X, fp32=False):
                                 smax.ctypes.data, 16, ctypes.addressof(nl)),
          "lgh_test_vcycle")
     return Y, smax[:nl.value]
+
+
+def test_vc_level(prior, X, fp32=False, wide=False):
+    """The finest level's V-cycle passes alone (lgh_test_vc_level)."""
+    X = np.ascontiguousarray(X, dtype=np.float64)
+    Y = np.empty_like(X)
+    _chk(load().lgh_test_vc_level(prior.h, X.shape[1], X.ctypes.data,
+                                  Y.ctypes.data, 1 if fp32 else 0,
+                                  1 if wide else 0), "lgh_test_vc_level")
+    return Y
 
 
 CHEB_FIRST, CHEB_ZERO_X, CHEB_STORE_D = 1, 2, 4
