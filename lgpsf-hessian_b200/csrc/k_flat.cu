@@ -267,17 +267,18 @@ fvals (const Csr &A)
 
 /* Column slices: a gathered row is read again by the rows up to the
  * operator's bandwidth away, so the band of 2 bandwidth rows has to stay in
- * L2 (126 MB, shared with the streams); a wider band is swept in slices of
- * whole packs.  f (first pack, packs) runs one slice. */
+ * L2 (126 MB, shared with the streams); a band wider than the smoothers'
+ * budget (smoother_l2_budget) is swept in slices of whole packs.  f (first
+ * pack, packs) runs one slice. */
 template <typename F>
 static int
 flat_slices (int64_t n, int64_t bandwidth, int ld, int nvec, size_t elem, F f)
 {
   const double band = (double) std::min (2 * bandwidth, n) * ld * elem;
-  const double budget = 40. * 1048576.;
+  const double budget = smoother_l2_budget ();
   int ns = (nvec + FLAT_MAXPACKS - 1) / FLAT_MAXPACKS;
-  if (band > budget)
-    ns = std::max (ns, std::min (nvec, (int) (band / budget) + 1));
+  if (budget > 0. && band > budget)
+    ns = std::max (ns, (int) std::min ((double) nvec, band / budget + 1.));
   for (int s = 0; s < ns; s++) {
     const int v0 = (int) ((int64_t) nvec * s / ns);
     const int v1 = (int) ((int64_t) nvec * (s + 1) / ns);

@@ -255,6 +255,11 @@ template <typename T>
 int launch_flat_mult (const Csr &A, const T *X, T *Y, int ld, cudaStream_t s,
                       int wide = 0);
 
+/* L2 bytes that the smoothers' neighbour reuse may span (of 126 MB, shared
+ * with the streaming blocks): 40 MB, or LGH_CHEB_L2MB megabytes (0: never
+ * slice) (zsolve.cu) */
+double smoother_l2_budget ();
+
 /* elementwise / block helpers (k_vec.cu) */
 template <typename T>
 int launch_rowscale (int64_t n, int w, const double *scale, const T *X,

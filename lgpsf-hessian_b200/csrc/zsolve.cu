@@ -956,13 +956,8 @@ template int zsolve_block<float> (const Csr &, const ZsolveCfg &, Hierarchy *,
                                   const double *, float *, int, const double *,
                                   ZsolveStats *, int, cudaStream_t);
 
-/* L2 bytes the smoother's neighbour reuse may span: a row's r and d rows
- * are gathered again by the rows up to the bandwidth away, so the band of
- * 2 bandwidth rows of both blocks must stay in L2 (126 MB, shared with the
- * streaming writes).  A wider band is swept in column slices.
- * LGH_CHEB_L2MB overrides the budget (0: never slice). */
-static double
-cheb_l2_budget ()
+double
+smoother_l2_budget ()
 {
   const char *e = getenv ("LGH_CHEB_L2MB");
   return (e ? atof (e) : 40.0) * 1048576.0;
@@ -981,9 +976,11 @@ launch_cheb_step (const Csr &A, T *X, const T *Ro, T *Rn, const T *Do, T *Dn,
   ZK zk{ A.n, A.rowptr, A.colidx };
   const T *vals = zvals<T> (A);
   const T *dinv = zdinv<T> (A);
-  /* column slices of whole packs so that each slice's reuse band fits */
+  /* a row's r and d rows are gathered again by the rows up to the bandwidth
+   * away, so the band of 2 bandwidth rows of both blocks must stay in L2:
+   * column slices of whole packs so that each slice's band fits */
   const double band = 2. * 2. * (double) A.bandwidth * ld * sizeof (T);
-  const double budget = cheb_l2_budget ();
+  const double budget = smoother_l2_budget ();
   int slices = 1;
   if (budget > 0. && band > budget)
     slices = std::min (nvec_all, (int) std::ceil (band / budget));
