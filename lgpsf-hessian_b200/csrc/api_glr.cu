@@ -725,14 +725,16 @@ batch_op (lgh_glr_t *g, int kind, int nshift, const double *c, int m,
              "batch: a row-sharded object runs the per-shift operations");
   LGH_CHECK (m > 0 && nshift > 0 && ldr >= n && ldx >= n, LGH_ERR_ARG_SIZ, "batch: size");
   std::vector<double> ch (nshift);
-  /* the shifts may lie on either side; a copy from ordinary host memory is
-   * the host's own (cudaMemcpyDefault took 330 us for it) */
+  /* the shifts may lie on either side, and the work queued before this call
+   * may still write them.  Pageable memory is the host's to read once that
+   * work is done (cudaMemcpyDefault took 330 us for it) */
   cudaPointerAttributes pa;
   if (cudaPointerGetAttributes (&pa, c) == cudaSuccess
-      && (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged)) {
+      && pa.type != cudaMemoryTypeUnregistered) {
     LGH_CUDA (cudaMemcpy (ch.data (), c, nshift * sizeof (double), cudaMemcpyDefault));
   } else {
     cudaGetLastError ();
+    LGH_CUDA (cudaStreamSynchronize (s));
     memcpy (ch.data (), c, nshift * sizeof (double));
   }
   for (int i = 0; i < nshift; i++) LGH_TRY (check_shift (g, ch[i], "batch"));
