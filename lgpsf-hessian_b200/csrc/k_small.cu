@@ -308,12 +308,13 @@ jacobi_row (int i, int k, int r, int nblk)
   return b * JB + (i & (JB - 1));
 }
 
-/* 2^-e for the exponent e of x (x normal and below 2^1023) */
+/* a power of two that takes x (normal or infinite) to [1, 2), or to [2, 4)
+ * from the last binade up, whose inverse is no normal number */
 __device__ __forceinline__ double
 exponent_scale (double x)
 {
   const int e = (__double2hiint (x) >> 20) & 0x7ff;
-  return __hiloint2double ((2046 - e) << 20, 0);
+  return __hiloint2double (max (2046 - e, 1) << 20, 0);
 }
 
 /* the rotation that annihilates apq: tan t = s / c with |t| <= 1, from the
