@@ -29,6 +29,7 @@
  */
 
 #include <algorithm>
+#include <type_traits>
 
 #include "lgh_device.cuh"
 #include "lgh_flat.cuh"
@@ -291,19 +292,70 @@ k_strip_f32 (int64_t n, int64_t nstrips, const int64_t *__restrict__ sptr,
   }
 }
 
+/* the product of the k-th entry (see k_strip_flat).  The packs load together
+ * where a thread has 4 of them or 4 rows to multiply each by; two packs of
+ * two rows are faster one after the other (131 columns: FP64 173 us and 187,
+ * FP32 85 and 94) */
+template <int R, int CH, typename T>
+__device__ __forceinline__ void
+strip_step (int k, const int32_t *__restrict__ sc, const T *__restrict__ sv,
+            const T *__restrict__ X, int ldx, int lane, int L, int nvec,
+            T (&acc)[R][CH][Pack<T>::W])
+{
+  constexpr int W = Pack<T>::W;
+  constexpr bool TOGETHER = R == 4 || CH == 4;
+  const T *xr = X + (int64_t) __ldg (sc + k) * ldx;
+  T v[R];
+  Pack<T> x[CH];
+  if constexpr (R >= W) {
+#pragma unroll
+    for (int r = 0; r < R; r += W) {
+      const Pack<T> p = ldp_nc (sv + (size_t) k * R + r);
+#pragma unroll
+      for (int e = 0; e < W; e++) v[r + e] = p.v[e];
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = __ldg (sv + (size_t) k * R + r);
+  }
+  if constexpr (TOGETHER) {
+#pragma unroll
+    for (int h = 0; h < CH; h++) {
+      const int vi = lane + h * L;
+      if (h < CH - 1 || vi < nvec) x[h] = ldp (xr + vi * W);
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < CH; h++) {
+    const int vi = lane + h * L;
+    if (h < CH - 1 || vi < nvec) {
+      if constexpr (!TOGETHER) x[h] = ldp (xr + vi * W);
+#pragma unroll
+      for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int e = 0; e < W; e++)
+          acc[r][h][e] = fma (v[r], x[h].v[e], acc[r][h][e]);
+    }
+  }
+}
+
 /* strips of 2 or 4 rows (operators whose rows share few columns): the flat
- * mapping over strips, a thread holding CH packs of all R rows.  FP64 at 56
- * entries per row, 256^2 x 60 / 131 / 220 columns, R = 4: a warp per 128
- * columns 208 / 228 / 246 us, here 99 / 177 / 269; R = 2: 343 / 373 / 398
- * and 94 / 177 / 277. */
+ * mapping over strips, a thread holding CH packs of all R rows.  256^2 rows
+ * of 56 entries, us at 60 / 131 / 220 / 400 columns, with a warp per strip
+ * and 128 (R = 4) or 256 packs, and here: FP64 R = 2 340 / 369 / 394 / 438
+ * and 94 / 158 / 231 / 409, R = 4 206 / 226 / 246 / 466 and 82 / 157 / 239 /
+ * 402; FP32 R = 2 356 / 365 / 369 / 400 and 47 / 84 / 123 / 207, R = 4 210 /
+ * 216 / 220 / 241 and 45 / 82 / 127 / 204.  A diagonal operator of as many
+ * rows, FP64 at 131 / 400: 48 / 77 and 27 / 81 (64 at the copy rate).  CTAs
+ * per SM: FP64 takes 128 registers at 4 packs of 4 rows, 80 otherwise. */
 template <typename T, int R, int CH>
-__global__ void __launch_bounds__ (FLAT_THREADS, sizeof (T) == 8 ? 3 : 4)
+__global__ void __launch_bounds__ (FLAT_THREADS, sizeof (T) == 4 ? 4 : (R * CH > 8 ? 2 : 3))
 k_strip_flat (int64_t n, int64_t nstrips, const int64_t *__restrict__ sptr,
               const int32_t *__restrict__ scol, const T *__restrict__ sval,
               const T *__restrict__ X, int ldx, T *__restrict__ Y, int ldy,
               int nvec, int L, int rpc)
 {
-  constexpr int W = Pack<T>::W, VW = R < W ? R : W;
+  constexpr int W = Pack<T>::W;
   const int rl = threadIdx.x / L, lane = threadIdx.x - rl * L;
   if (rl >= rpc) return;
   for (int64_t s = (int64_t) blockIdx.x * rpc + rl; s < nstrips;
@@ -315,33 +367,8 @@ k_strip_flat (int64_t n, int64_t nstrips, const int64_t *__restrict__ sptr,
     T acc[R][CH][W];
 #pragma unroll
     for (int r = 0; r < R; r++) flat_zero<T, CH, W> (acc[r]);
-    for (int k = 0; k < cnt; k++) {
-      const T *xr = X + (int64_t) __ldg (sc + k) * ldx;
-      T v[R];
-      if constexpr (VW == W) {
-#pragma unroll
-        for (int r = 0; r < R; r += W) {
-          const Pack<T> p = ldp_nc (sv + (size_t) k * R + r);
-#pragma unroll
-          for (int e = 0; e < W; e++) v[r + e] = p.v[e];
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) v[r] = __ldg (sv + (size_t) k * R + r);
-      }
-#pragma unroll
-      for (int h = 0; h < CH; h++) {
-        const int vi = lane + h * L;
-        if (h < CH - 1 || vi < nvec) {
-          const Pack<T> x = ldp (xr + vi * W);
-#pragma unroll
-          for (int r = 0; r < R; r++)
-#pragma unroll
-            for (int e = 0; e < W; e++)
-              acc[r][h][e] = fma (v[r], x.v[e], acc[r][h][e]);
-        }
-      }
-    }
+    for (int k = 0; k < cnt; k++)
+      strip_step<R, CH, T> (k, sc, sv, X, ldx, lane, L, nvec, acc);
     const int64_t r0 = s * R;
 #pragma unroll
     for (int r = 0; r < R; r++) {
@@ -492,20 +519,34 @@ strip_mma (const StripForm &S, const double *X, int ldx, double *Y, int ldy,
   return 0;
 }
 
-/* strip rows of 2 and 4; two packs per thread where there are that many */
+/* strips of 2 and 4 rows: two packs per thread where there are that many,
+ * in FP64 four above 32 packs (R = 2) or 24 (R = 4); fewer where some SM
+ * would not get two CTAs.  56 entries a row, two packs and four: R = 2 at 60
+ * columns 94 and 99 us, 131 175 and 158; R = 4 at 20 54 and 65, 60 91 and
+ * 80; FP32 keeps two (R = 4 at 60 46 and 51, 400 203 and 239) */
 template <typename T, int R>
 static int
 strip_flat (const StripForm &S, const T *sval, const T *X, int ldx, T *Y,
             int ldy, int nvec, cudaStream_t s)
 {
   constexpr int W = Pack<T>::W;
-  for (int p0 = 0; p0 < nvec; p0 += FLAT_THREADS * 2) {
-    const int nv = std::min (nvec - p0, FLAT_THREADS * 2);
-    const FlatShape f = flat_shape_ch (nv, nv > 2 ? 2 : 1);
-    auto kern = f.ch == 2 ? k_strip_flat<T, R, 2> : k_strip_flat<T, R, 1>;
-    kern<<<flat_grid (f, S.nstrips), FLAT_THREADS, 0, s>>> (
-        S.n, S.nstrips, S.sptr, S.scol, sval, X + p0 * W, ldx, Y + p0 * W,
-        ldy, nv, f.L, f.rpc);
+  for (int p0 = 0; p0 < nvec; p0 += FLAT_THREADS) {
+    const int nv = std::min (nvec - p0, FLAT_THREADS);
+    int ch = nv <= 2 ? 1 : (sizeof (T) == 4 || nv <= (R == 2 ? 32 : 24) ? 2 : 4);
+    FlatShape f = flat_shape_ch (nv, ch);
+    while (ch > 1 && (S.nstrips + f.rpc - 1) / f.rpc < 2 * num_sms ()) {
+      ch /= 2;
+      f = flat_shape_ch (nv, ch);
+    }
+    auto run = [&] (auto chc) {
+      k_strip_flat<T, R, decltype (chc)::value>
+          <<<flat_grid (f, S.nstrips), FLAT_THREADS, 0, s>>> (
+              S.n, S.nstrips, S.sptr, S.scol, sval, X + p0 * W, ldx, Y + p0 * W,
+              ldy, nv, f.L, f.rpc);
+    };
+    if (ch == 1) run (std::integral_constant<int, 1> ());
+    else if (ch == 2) run (std::integral_constant<int, 2> ());
+    else if constexpr (sizeof (T) == 8) run (std::integral_constant<int, 4> ());
     LGH_LAUNCH_CHECK ();
   }
   return 0;
