@@ -252,14 +252,17 @@ spmv_dispatch (const Csr &A, const TV *vals, const T *X, int ldx, T *Y, int ldy,
    * 11 / 16, 7 12 / 16, 9 14 / 25, 19 20 / 31, 27 25 / 37, 40 33 / 76, 57 45
    * / 82, 81 59 / 96, 100 76 / 102, 150 102 / 125, 183 111 / 131 (floor 90),
    * 220 and 256 the same; 300 141 / 160, 400 145 / 145.  Rows of 8 times
-   * what a round covers take the next shape. */
-  auto fits = [&] (int cover) {
-    return A.nnz <= cover * A.n && A.max_row_nnz <= 8 * cover;
+   * what a round covers take the next shape; 8 x 6 goes to 16 rounds, as the
+   * shapes after it cost the short rows more (a row of 400 / 600 entries in
+   * 4096 of 5: 42 / 51 us, 8 x 8 45 / 55, 16 x 6 51 / 55, one entry a lane
+   * and round 65 / 82). */
+  auto fits = [&] (int cover, int rounds = 8) {
+    return A.nnz <= cover * A.n && A.max_row_nnz <= rounds * cover;
   };
   if (fits (5)) LGH_SPV (1, 5);
   if (fits (10)) LGH_SPV (1, 8);
   if (fits (28)) LGH_SPV (4, 7);
-  if (fits (48)) LGH_SPV (8, 6);
+  if (fits (48, 16)) LGH_SPV (8, 6);
   if (fits (64)) LGH_SPV (8, 8);
   if (fits (96)) LGH_SPV (16, 6);
   if (fits (128)) LGH_SPV (16, 8);
