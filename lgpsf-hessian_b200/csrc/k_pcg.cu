@@ -608,10 +608,12 @@ sum_smem (const FlatShape &f, int cols)
   return (f.rpc * cols + FLAT_THREADS) * (int) sizeof (double);
 }
 
+/* two packs per thread at most: the column sums fit the 48 KB of shared
+ * memory that need no opt-in (a Z-solve's tile is 512 columns) */
 int
 pcg_width (int ld, int W)
 {
-  return ld > 0 && ld % W == 0 && ld / W <= FLAT_MAXPACKS
+  return ld > 0 && ld % W == 0 && ld / W <= 2 * FLAT_THREADS
              ? 0
              : set_error (LGH_ERR_SUP, "PCG pass: block width %d unsupported", ld);
 }
@@ -660,9 +662,6 @@ launch_pcg_dots (int64_t n, int w, int ld, const T *R, const TZ *Zb, int first,
           ws.partB.p, ws.counters.p + 1, pc));
     } else {
       auto k = k_pcg_dots<T, TZ, CH_, false>;
-      if (smem > 48 * 1024)   /* FP32 blocks of over 2900 columns */
-        LGH_CUDA (cudaFuncSetAttribute (
-            k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       nb = fit_grid (k, want, FLAT_THREADS, smem);
       LGH_CUDA (launch_pdl (bytes, k, nb, FLAT_THREADS, smem, s, n, ld, nvec, f.L,
           f.rpc, R, Zb, ws.partA.p, ws.partB.p, ws.counters.p + 1, pc));
