@@ -133,8 +133,10 @@ int lgh_prior_create_callbacks (lgh_Vec mass_lumps,
 /* prior.h:76-89.  On this device the Mat path solves Z with blocked,
  * per-column preconditioned CG (blocked_mode 0/1, rtol ksp_rtol, the
  * reference's per-column KSP semantics) or blocked fixed-count Chebyshev
- * (modes 2/3, cheb_rtol, bounds from a CG-Lanczos probe widened 0.9/1.1),
- * preconditioned by a block V-cycle on a smoothed-aggregation hierarchy of
+ * (modes 2/3, cheb_rtol, bounds from a CG-Lanczos probe widened 0.9/1.1;
+ * with the V-cycle and bounds of ratio up to 2.5 the recurrence's direction
+ * term is left out, and the error is 1 to 30 times cheb_rtol on the
+ * isotropic grids that have such bounds), preconditioned by a block V-cycle on a smoothed-aggregation hierarchy of
  * Z (Chebyshev-Jacobi smoothers, nu = nu_force or 2, interval
  * [0.1, smoother_top] lambda_max; dense coarse solve) or by Jacobi
  * (lgh_prior_create_mat_pc).  tile caps the block width of one blocked

@@ -502,11 +502,12 @@ k_pcg_out (int64_t n, int w, int ld, const T *__restrict__ X,
 }
 
 /* One step of the fixed-count iteration around an explicit preconditioner:
- * x += b z, r -= b Z z (first: x = b z).  The step lengths are the
- * Chebyshev recurrence's; its direction term a d is not part of the
- * iteration, so no direction block is kept and r is updated in place, row
- * by row, from the gathered z: 5 block transfers (7 with an x, d and r
- * written beside the old ones: 37 us at 257 x 255 x 48 columns). */
+ * x += b z, r -= b Z z (first: x = b z); r is updated in place, row by row,
+ * from the gathered z: 5 block transfers (7 with an x, d and r written
+ * beside the old ones: 37 us at 257 x 255 x 48 columns).  With z = V(r) and
+ * the Chebyshev recurrence's step lengths b this is the short form of
+ * zsolve_block, without the recurrence's direction term; with the direction
+ * in z's place and b = 1 it is a Chebyshev step. */
 template <typename T, typename I, int CH, bool FIRST>
 __global__ void __launch_bounds__ (FLAT_THREADS, FlatOcc<CH>::v)
 k_pcg_cheb (int64_t n, const int64_t *__restrict__ rowptr,
@@ -548,6 +549,25 @@ k_pcg_cheb (int64_t n, const int64_t *__restrict__ rowptr,
     }
     k0 = k0n;
     k1 = k1n;
+  }
+}
+
+/* the Chebyshev direction, in place: p = a p + b z (first: p = b z) */
+template <typename T>
+__global__ void __launch_bounds__ (256)
+k_pcg_cheb_dir (int64_t n, int ld, const T *__restrict__ Zb, T *__restrict__ P,
+                T a, T b, int first)
+{
+  pdl_wait ();
+  constexpr int W = Pack<T>::W;
+  const int64_t total = n * (ld / W);
+  for (int64_t e = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; e < total;
+       e += (int64_t) gridDim.x * blockDim.x) {
+    const Pack<T> z = ldp (Zb + e * W);
+    Pack<T> p = first ? pzero<T> () : ldp (P + e * W);
+#pragma unroll
+    for (int k = 0; k < W; k++) p.v[k] = fma (b, z.v[k], a * p.v[k]);
+    stp (P + e * W, p);
   }
 }
 
@@ -820,6 +840,18 @@ launch_pcg_cheb (const Csr &Z, const T *Zb, T *R, T *X, int ld, double b,
 
 template <typename T>
 int
+launch_pcg_cheb_dir (int64_t n, int ld, const T *Zb, T *P, double a, double b,
+                     int first, cudaStream_t s)
+{
+  const int64_t bytes = n * ld * (int64_t) sizeof (T);
+  LGH_CUDA (launch_pdl (bytes, k_pcg_cheb_dir<T>, stream_grid (n * (ld / Pack<T>::W)),
+      256, 0, s, n, ld, Zb, P, (T) a, (T) b, first));
+  LGH_LAUNCH_CHECK ();
+  return 0;
+}
+
+template <typename T>
+int
 launch_pcg_cheb_out (int64_t n, int w, int ld, const T *Zb, const T *X, double b,
                      int only, const double *rs, T *Y, int ldy, cudaStream_t s)
 {
@@ -881,6 +913,8 @@ pcg_wait_count (ZWork &ws, cudaStream_t s, int *count)
 #define LGH_PCG_INST_C(T)                                                    \
   template int launch_pcg_cheb<T> (const Csr &, const T *, T *, T *, int,    \
                                    double, int, cudaStream_t);               \
+  template int launch_pcg_cheb_dir<T> (int64_t, int, const T *, T *, double, \
+                                       double, int, cudaStream_t);           \
   template int launch_pcg_cheb_out<T> (int64_t, int, int, const T *,         \
                                        const T *, double, int,               \
                                        const double *, T *, int,             \

@@ -58,10 +58,15 @@ int launch_pcg_out (int64_t n, int w, int ld, const T *X, const T *P,
                     cudaStream_t s);
 
 /* the fixed-count iteration around z = V(r): a step x += b z, r -= b Z z
- * (first: x = b z), and the last step's x with the row scaling */
+ * (first: x = b z), the last step's x with the row scaling, and the
+ * Chebyshev direction p = a p + b z (first: p = b z) that may stand for z,
+ * with b = 1 */
 template <typename T>
 int launch_pcg_cheb (const Csr &Z, const T *Zb, T *R, T *X, int ld, double b,
                      int first, cudaStream_t s);
+template <typename T>
+int launch_pcg_cheb_dir (int64_t n, int ld, const T *Zb, T *P, double a,
+                         double b, int first, cudaStream_t s);
 template <typename T>
 int launch_pcg_cheb_out (int64_t n, int w, int ld, const T *Zb, const T *X,
                          double b, int only, const double *rs, T *Y, int ldy,

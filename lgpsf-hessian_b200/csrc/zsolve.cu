@@ -7,8 +7,10 @@
  *             preconditioned-residual norm, rtol = ksp_rtol, 10000-iteration
  *             cap), run for all columns of a block at once with per-column
  *             alpha/beta and a per-column convergence mask;
- *   mode 2    fixed-count Chebyshev (zsolve_impl.h:94-141), nit from the
- *             margined spectral interval.
+ *   mode 2/3  fixed-count Chebyshev (zsolve_impl.h:94-141), nit from the
+ *             margined spectral interval; around the V-cycle on an interval
+ *             of ratio up to 2.5 its step lengths without the direction
+ *             term (CHEB_SHORT below).
  * The preconditioner is the aggregation V-cycle (mg.cu; the iteration's own
  * passes are those of k_pcg.cu) or Jacobi, whose kernels are here.
  *
@@ -610,6 +612,17 @@ zvd (const Csr &Z)
  * 20 times */
 constexpr double PCG_AHEAD = 32. * 1048576.;
 
+/* lmax / lmin up to which a fixed-count solve around the V-cycle leaves out
+ * the recurrence's direction term, x += b_k V(r).  Without it the count,
+ * which is Chebyshev's, does not reach cheb_rtol, and from 3 + 2 sqrt 2 =
+ * 5.8 on b lmax > 2: the steps grow the error.  Isotropic grids have 1.8 to
+ * 2.1: relative errors of 1 to 30 times cheb_rtol, a transfer of three
+ * blocks a step fewer, and results that callers compare with earlier ones.
+ * Error at cheb_rtol 1e-10 without and with the term, 60^2 with the second
+ * direction's coupling scaled by 0.1 / 0.03 / 0.01 (ratio 3.5, 8.3, 17.7):
+ * 5e-6 / 0.8 / 3e6 and 4e-11 / 6e-11 / 6e-11. */
+constexpr double CHEB_SHORT = 2.5;
+
 template <typename T>
 int
 zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
@@ -789,29 +802,39 @@ zsolve_block (const Csr &Z, const ZsolveCfg &cfg, Hierarchy *mg, ZWork &ws,
       continue;
     } else if (mgcheb) {
       /* fixed count around the V-cycle (modes 2/3: zsolve_impl.h:108-141
-       * with the AMG / harvested-hierarchy preconditioner), at the step
-       * lengths b of the Chebyshev recurrence */
+       * with the AMG / harvested-hierarchy preconditioner): Chebyshev, or
+       * (CHEB_SHORT) its step lengths without the direction term */
+      const bool full = cfg.lmax > CHEB_SHORT * cfg.lmin;
       const double theta = 0.5 * (cfg.lmax + cfg.lmin);
       const double delta = 0.5 * (cfg.lmax - cfg.lmin);
       const double sigma1 = theta / delta;
       double rho_old = 1.0 / sigma1;
       LGH_TRY (launch_pcg_start<T> (n, wt, ldt, Xin + c0, ldx, rs_in, bR, nullptr, s));
       for (int k = 1; k <= cfg.nit; k++) {
-        double b = 1.0 / theta;
+        double a = 0., b = 1.0 / theta;
         if (k > 1) {
           const double rho = 1.0 / (2.0 * sigma1 - rho_old);
+          a = rho * rho_old;
           b = 2.0 * rho / delta;
           rho_old = rho;
         }
         static thread_local KTrace ktc;
         KTrace *tc = (timing && k % 4 == 0) ? &ktc : nullptr;
         LGH_TRY (mg_vcycle<T> (mg, bR, bZ, ldt, wt, s, tc));
+        const T *step = bZ;           /* x += b step */
+        if (full) {
+          if (tc) LGH_TRY (tc->begin (K_PCGX_PFORM, (k == 1 ? 2. : 3.) * n * wt * sizeof (T), s));
+          LGH_TRY (launch_pcg_cheb_dir<T> (n, ldt, bZ, bP0, a, b, k == 1, s));
+          if (tc) LGH_TRY (tc->end (s));
+          step = bP0;
+          b = 1.;
+        }
         if (k == cfg.nit) {
-          LGH_TRY (launch_pcg_cheb_out<T> (n, wt, ldt, bZ, bX, b, k == 1, rs_out,
+          LGH_TRY (launch_pcg_cheb_out<T> (n, wt, ldt, step, bX, b, k == 1, rs_out,
                                            Y + c0, ldy, s));
         } else {
           if (tc) LGH_TRY (tc->begin (K_CHEBX, zbytes + 5. * (double) n * wt * sizeof (T), s));
-          LGH_TRY (launch_pcg_cheb<T> (Z, bZ, bR, bX, ldt, b, k == 1, s));
+          LGH_TRY (launch_pcg_cheb<T> (Z, step, bR, bX, ldt, b, k == 1, s));
           if (tc) LGH_TRY (tc->end (s));
         }
         if (tc) {
