@@ -288,6 +288,94 @@ k_gemm_tn_part (int64_t n, int m1, int m2, const T *__restrict__ A, int lda,
       }
 }
 
+/* acc += one stage of k_gemm_tn_tile (gemm_tile keeps its own copy of this
+ * loop: calling it there cost 13 to 40 % through its registers) */
+template <typename O>
+__device__ __forceinline__ void
+gemm_stage (const double *As, const double *Bs, int wm, int wn, int lane, int ma,
+            int nb, double (&acc)[4][4][2])
+{
+  if (ma == 0 || nb == 0) return;
+#pragma unroll
+  for (int kk = 0; kk < GK; kk += 4) {
+    double a[4], b[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      a[t] = t < ma ? O::frag (As, wm * 32 + t * 8 + (lane >> 2), kk + (lane & 3)) : 0.;
+      b[t] = t < nb ? O::frag (Bs, wn * 32 + t * 8 + (lane >> 2), kk + (lane & 3)) : 0.;
+    }
+#pragma unroll
+    for (int ti = 0; ti < 4; ti++)
+      if (ti < ma)
+#pragma unroll
+        for (int tj = 0; tj < 4; tj++)
+          if (tj < nb)
+            asm volatile ("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
+                          "{%0, %1}, {%2}, {%3}, {%0, %1};"
+                          : "+d"(acc[ti][tj][0]), "+d"(acc[ti][tj][1])
+                          : "d"(a[ti]), "d"(b[tj]));
+  }
+}
+
+/* k_gemm_tn_part for one output tile of FP64 operands, staged through
+ * registers: the next stage is read while the current one is multiplied, in
+ * 8-byte loads at any alignment.  SAME: B is A, loaded once.  The whole
+ * lgh_gram_noalloc with an even / odd ldx, us with the ring of copies (8-byte
+ * ones where ldx is odd) and here: 262144 x 33 130 / 148 and 128 / 129, x 64
+ * 143 / 176 and 143 / 143, 20000 x 48 40 / 46 and 39 / 39.  For A^T B the
+ * ring is kept where its copies are 16 bytes. */
+template <bool SAME>
+__global__ void __launch_bounds__ (128)
+k_gemm_tn_tile (int64_t n, int m1, int m2, const double *__restrict__ A, int lda,
+                const double *__restrict__ B, int ldb, double *__restrict__ work,
+                int64_t kchunk)
+{
+  using O = GOp<double, true, GB>;
+  __shared__ double As[O::ELEMS], Bs[SAME ? 1 : O::ELEMS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = warp >> 1, wn = warp & 1;
+  const int64_t kb0 = (int64_t) blockIdx.x * kchunk;
+  const int64_t kb1 = kb0 + kchunk < n ? kb0 + kchunk : n;
+  const int ma = SAME && wm > wn ? 0 : gemm_frags (wm * 32, m1);
+  const int nb = gemm_frags (wn * 32, m2);
+  double acc[4][4][2];
+  gemm_zero (acc);
+  /* k row tid / 8; columns tid % 8, tid % 8 + 8, ... */
+  const int lk = tid >> 3, lc = tid & 7;
+  double ra[8], rb[SAME ? 1 : 8];
+  auto fetch = [&] (int64_t k0) {
+    const int64_t k = k0 + lk;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const int c = lc + e * 8;
+      ra[e] = k < kb1 && c < m1 ? A[k * lda + c] : 0.;
+      if constexpr (!SAME) rb[e] = k < kb1 && c < m2 ? B[k * ldb + c] : 0.;
+    }
+  };
+  fetch (kb0);
+  for (int64_t k0 = kb0; k0 < kb1; k0 += GK) {
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      As[lk * O::S + lc + e * 8] = ra[e];
+      if constexpr (!SAME) Bs[lk * O::S + lc + e * 8] = rb[e];
+    }
+    __syncthreads ();
+    fetch (k0 + GK);
+    gemm_stage<O> (As, SAME ? As : Bs, wm, wn, lane, ma, nb, acc);
+    __syncthreads ();
+  }
+  double *wz = work + (size_t) blockIdx.x * m1 * m2;
+#pragma unroll
+  for (int ti = 0; ti < 4; ti++)
+#pragma unroll
+    for (int tj = 0; tj < 4; tj++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        const int i = dmma_row (wm, ti, lane), j = dmma_col (wn, tj, c, lane);
+        if (i < m1 && j < m2 && (!SAME || i <= j)) wz[i + (size_t) j * m1] = acc[ti][tj][c];
+      }
+}
+
 /* C = the sum of the slices in slice order; upper: the slices hold the
  * entries on and above the diagonal of a symmetric product */
 __global__ void
@@ -356,6 +444,15 @@ k_gemm_tn_reduce_same (int64_t total, int m1, int nsplit,
   }
 }
 
+/* slices of 256 rows, or of 64 up to 64 of them: few rows are bound by the
+ * stages of a slice (the whole Gram product at 1000 x 130 35 us in 4 slices,
+ * 22 in 16; 5000 x 65 36 in 20, 30 in 64) */
+static int64_t
+tn_max_splits (int64_t n)
+{
+  return std::max ((n + 255) / 256, std::min<int64_t> ((n + 63) / 64, 64));
+}
+
 static int
 tn_splits (int64_t n, int m1, int m2)
 {
@@ -363,7 +460,7 @@ tn_splits (int64_t n, int m1, int m2)
    * (gemm_tn_work_max follows this rule) */
   const int tiles = ((m1 + GB - 1) / GB) * ((m2 + GB - 1) / GB);
   int want = 4 * num_sms () / tiles;
-  int64_t maxs = (n + 255) / 256;
+  const int64_t maxs = tn_max_splits (n);
   if (want > maxs) want = (int) maxs;
   if (want < 1) want = 1;
   if (want > 256) want = 256;
@@ -549,6 +646,14 @@ gemm_tn_run (int64_t n, int m1, int m2, const T *A, int lda, const T *B, int ldb
   using C16 = std::integral_constant<int, 16>;
   using CS = std::integral_constant<int, sizeof (T)>;
   const bool a16 = copy_bytes (A, lda) == 16, b16 = copy_bytes (B, ldb) == 16;
+  if constexpr (sizeof (T) == 8) {
+    if ((upper || !(a16 && b16)) && m1 <= GB && m2 <= GB) {
+      auto k = upper ? k_gemm_tn_tile<true> : k_gemm_tn_tile<false>;
+      k<<<nsplit, 128, 0, s>>> (n, m1, m2, A, lda, B, ldb, work, kchunk);
+      LGH_LAUNCH_CHECK ();
+      return gemm_tn_sum (m1, m2, nsplit, work, C, ldc, sym, upper, s, tiles);
+    }
+  }
   if (a16 && b16) LGH_TRY (run (C16 (), C16 ()));
   else if (a16) LGH_TRY (run (C16 (), CS ()));
   else if (b16) LGH_TRY (run (CS (), C16 ()));
@@ -586,7 +691,7 @@ launch_gemm_tn (int64_t n, int m1, int m2, const T *A, int lda, const T *B,
     const int tm = (m1 + GB - 1) / GB;
     const int64_t want = std::max (1, 4 * num_sms () / (tm * (tm + 1) / 2));
     ns = (int) std::min<int64_t> (std::min<int64_t> (want, 256),
-                                  std::min<int64_t> ((n + 255) / 256,
+                                  std::min<int64_t> (tn_max_splits (n),
                                                      (int64_t) (work_elems / ((size_t) m1 * m2))));
     ns = std::max (ns, 1);
   }
