@@ -120,8 +120,9 @@ k_flat_second (int64_t n, const int64_t *__restrict__ rowptr,
 }
 
 /* z = dinv (g (r0 + r2) + b2 (r1 + r2 - F1 r2)) + Q xc: reads r0, r1, r2
- * (gathered) and the coarse block (gathered), writes z.  487 us, floor 297;
- * the post residual and the two post-smoothing steps took 787 */
+ * (gathered) and the coarse block (gathered), writes z.  487 us in a job
+ * (470 alone), floor 297; the post residual and the two post-smoothing steps
+ * took 787 */
 template <typename T, typename I, int CH>
 __global__ void __launch_bounds__ (FLAT_THREADS, CH == 2 ? 5 : (CH == 3 ? 4 : FlatOcc<CH>::v))
 k_flat_finish (int64_t n, const int64_t *__restrict__ frp,
@@ -275,7 +276,8 @@ static int
 flat_slices (int64_t n, int64_t bandwidth, int ld, int nvec, size_t elem, F f)
 {
   const double band = (double) std::min (2 * bandwidth, n) * ld * elem;
-  const double budget = smoother_l2_budget ();
+  /* a single vector's band is a few KB: no look at the override */
+  const double budget = band > 16384. ? smoother_l2_budget () : 0.;
   int ns = (nvec + FLAT_MAXPACKS - 1) / FLAT_MAXPACKS;
   if (budget > 0. && band > budget)
     ns = std::max (ns, (int) std::min ((double) nvec, band / budget + 1.));
@@ -369,7 +371,7 @@ launch_vc_finish (const Csr &F1, const Csr &Q, const T *dinv, const T *R0,
      * rows are long (3D: 25 entries with Q's; 46 packs FP64 305 us against
      * 375 with four and 340 with two, 110 packs 802, 1036, 824), or divides
      * a 2D block of up to 64 packs (48: 210, 218, 230); 110 packs in 2D
-     * keep four (470, three 522) */
+     * keep four (alone 470, three 522) */
     FlatShape f = flat_shape (nv, F1.n);
     const int L3 = (nv + 2) / 3;
     const bool lng = F1.nnz + Q.nnz > 16 * F1.n;

@@ -34,8 +34,8 @@ namespace lgh
  * by a thread each with theirs in registers; the arithmetic and its order
  * are those of a column at a time.  A column at a time over the whole panel
  * cost three barriers of 1024 threads for each, 0.8 us a column (n = 60: 47
- * us, now 41; 220: 328 and 237; 800: 6.2 and 5.2 ms); what is left is the chain of a square root and a division per
- * column.  The trailing update is m8n8k4 products of the panel, a warp per
+ * us, now 41; 220: 328 and 237; 800: 6.2 and 5.2 ms); what is left is the
+ * chain of a square root and a division per column.  The trailing update is m8n8k4 products of the panel, a warp per
  * 8 x 8 tile.  16 columns: the rows fit the registers of 512 threads. */
 constexpr int NB = 16;
 

@@ -80,7 +80,9 @@ int mg_vcycle (Hierarchy *h, const T *B, T *X, int ld, int w, cudaStream_t s,
  * previous step was a first step with coefficient bp run with
  * CHEB_R_ONLY: Do holds its input residual r_prev, and its d = bp D^{-1}
  * r_prev and its x are formed here with the same roundings, so the pair
- * gives the same bits as two ordinary steps) */
+ * gives the same bits as two ordinary steps).  The last two, and bp below,
+ * are run by lgh_test_cheb_step alone: the V-cycle's two steps are the
+ * passes of k_flat.cu */
 enum { CHEB_FIRST = 1, CHEB_ZERO_X = 2, CHEB_STORE_D = 4, CHEB_R_ONLY = 8,
        CHEB_PREV_R = 16 };
 template <typename T>
