@@ -504,7 +504,9 @@ k_pcg_out (int64_t n, int w, int ld, const T *__restrict__ X,
 /* One step of the fixed-count iteration around an explicit preconditioner:
  * x += b z, r -= b Z z (first: x = b z); r is updated in place, row by row,
  * from the gathered z: 5 block transfers (7 with an x, d and r written
- * beside the old ones: 37 us at 257 x 255 x 48 columns).  With z = V(r) and
+ * beside the old ones: 37 us at 257 x 255 x 48 columns).  The product is of
+ * b z as it is rounded, which r has to follow: with b times the product of
+ * z the error of FP32 solves was 3 to 10 % larger.  With z = V(r) and
  * the Chebyshev recurrence's step lengths b this is the short form of
  * zsolve_block, without the recurrence's direction term; with the direction
  * in z's place and b = 1 it is a Chebyshev step. */
@@ -530,7 +532,7 @@ k_pcg_cheb (int64_t n, const int64_t *__restrict__ rowptr,
     }
     T acc[CH][W];
     flat_zero<T, CH, W> (acc);
-    flat_gather<T, CH> (colidx, vals, k0, k1, 1, Zb, ld, lane, L, nvec, acc);
+    flat_gather<T, CH, true> (colidx, vals, k0, k1, 1, Zb, ld, lane, L, nvec, acc, b);
 #pragma unroll
     for (int h = 0; h < CH; h++) {
       const int vi = lane + h * L;
@@ -541,7 +543,7 @@ k_pcg_cheb (int64_t n, const int64_t *__restrict__ rowptr,
 #pragma unroll
         for (int e = 0; e < W; e++) {
           x.v[e] = fma (b, z.v[e], x.v[e]);
-          r.v[e] = fma (-b, acc[h][e], r.v[e]);
+          r.v[e] -= acc[h][e];
         }
         stp (X + o, x);
         stp (R + o, r);

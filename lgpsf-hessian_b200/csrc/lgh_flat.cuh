@@ -86,12 +86,13 @@ struct FlatOcc
 
 /* one row's product: acc += sum_k v_k X[c_k, :] over its entries k0, k0 +
  * step, ... below k1; I: int for operators of fewer than 2^31 entries (the
- * wider offsets cost the registers that spill) */
-template <typename T, int CH, typename I>
+ * wider offsets cost the registers that spill).  SC: each value of X is
+ * first multiplied by sc, and rounded */
+template <typename T, int CH, bool SC = false, typename I>
 __device__ __forceinline__ void
 flat_gather (const int32_t *__restrict__ ci, const T *__restrict__ va, I k0,
              I k1, int step, const T *__restrict__ X, int ld, int lane,
-             int L, int nvec, T (&acc)[CH][Pack<T>::W])
+             int L, int nvec, T (&acc)[CH][Pack<T>::W], T sc = T (1))
 {
   constexpr int W = Pack<T>::W;
   if constexpr (CH == 1) {
@@ -116,7 +117,7 @@ flat_gather (const int32_t *__restrict__ ci, const T *__restrict__ va, I k0,
         if (k + u * step < k1)
 #pragma unroll
           for (int e = 0; e < W; e++)
-            acc[0][e] = fma (v[u], x[u].v[e], acc[0][e]);
+            acc[0][e] = fma (v[u], SC ? sc * x[u].v[e] : x[u].v[e], acc[0][e]);
     }
     return;
   }
@@ -130,7 +131,8 @@ flat_gather (const int32_t *__restrict__ ci, const T *__restrict__ va, I k0,
       if (h < CH - 1 || vi < nvec) {
         const Pack<T> x = ldp (xr + vi * W);
 #pragma unroll
-        for (int e = 0; e < W; e++) acc[h][e] = fma (v, x.v[e], acc[h][e]);
+        for (int e = 0; e < W; e++)
+          acc[h][e] = fma (v, SC ? sc * x.v[e] : x.v[e], acc[h][e]);
       }
     }
   }
