@@ -280,17 +280,28 @@ launch_trtri_lower (int n, const double *L, double *Linv, int transpose,
 /* ------------------------------------------------------------- jacobi -- */
 
 /* Block Jacobi: the matrix in blocks of JB rows, paired round-robin.  A
- * round diagonalises the 2 JB x 2 JB submatrix of every block pair by one
- * cyclic sweep in shared memory (k_jacobi_pairs, one CTA per pair, the
- * accumulated rotations W kept) and applies the W's to the rest of A and to
- * V as small tensor-core products (k_jacobi_apply, one CTA per tile).  A
- * sweep is nblk - 1 rounds of two launches, 13 at n = 220, where the scalar
- * ordering needs n - 1 rounds, each with a barrier over the whole grid and
- * an update of every entry (5.2 us a round, bound by the barrier and the L2
- * latency behind it: 10.3 ms at n = 220, 2.0 ms at n = 60; now 3.3 and
- * 0.56).  Blocks of 16:
- * the sweep inside a pair is the longest chain of a round, and a 32 x 32
- * submatrix is also one tile of the products. */
+ * round rotates the index pairs of every block pair in shared memory
+ * (k_jacobi_pairs, one CTA per pair, the accumulated rotations W kept) and
+ * applies the W's to the rest of A and to V as small tensor-core products
+ * (k_jacobi_apply, one CTA per tile).  A sweep is nblk - 1 rounds of two
+ * launches, 13 at n = 220, where the scalar ordering needs n - 1 rounds,
+ * each with a barrier over the whole grid and an update of every entry.
+ * Blocks of 16: the steps inside a pair are the longest chain of a round,
+ * and a 32 x 32 submatrix is also one tile of the products.
+ *
+ * Every index pair is rotated once a sweep, as in the scalar ordering: the
+ * pairs across the two blocks in each round, those inside a block in the
+ * sweep's last round.  (All pairs of the submatrix in every round: twice the
+ * rotations and their rounding for the same number of sweeps, 4.1 ms against
+ * 3.0 for a random matrix of n = 220, 0.67 and 0.63 at 60; the scalar
+ * ordering took 11.3 and 2.1.)  The products are of W - I, added to the tile, so that the late
+ * sweeps' small rotations round a tile once, and the eigenvalues are the
+ * Rayleigh quotients of the result.  Residual, loss of orthogonality and
+ * eigenvalue error (Frobenius, over the norm) at n = 220, of the scalar
+ * ordering / all pairs in every round and the diagonal / now: a spectrum
+ * that decays to 1e-12 5.1e-15 9.8e-13 2.0e-15 / 7.2e-15 1.3e-12 4.9e-15 /
+ * 2.7e-15 1.0e-13 1.3e-16; a third of full rank 4.4e-15 8.1e-13 1.4e-15 /
+ * 5.9e-15 9.4e-13 3.6e-15 / 2.5e-15 9.8e-14 1.7e-16. */
 constexpr int JB = 16, JT = 2 * JB, JS = JT + 4;   /* block, tile, row stride */
 
 /* index at position `pos` in round r of the round-robin over np entries */
@@ -319,11 +330,13 @@ exponent_scale (double x)
 
 /* the rotation that annihilates apq: tan t = s / c with |t| <= 1, from the
  * double angle, d = aqq - app, b = 2 apq: cos 2a = |d| / r, c^2 = (1 + cos
- * 2a) / 2, s = b / (2 r c), r^2 = d^2 + b^2.  Two reciprocal square roots
- * long where t, c from the quotient d / b take three divisions and two
- * square roots one after the other (a round of k_jacobi_pairs: 1.3 us); both
- * are scaled by a power of two first, so nothing overflows.  False (no
- * rotation) below the relative threshold 1e-15 sqrt |app aqq|. */
+ * 2a) / 2, t = b / (2 r c^2), r^2 = d^2 + b^2.  Reciprocal square roots
+ * where t from the quotient d / b takes two divisions and a square root one
+ * after the other; d and b are scaled by a power of two first, so nothing
+ * overflows.  c and s are then those of t as it is rounded: from the double
+ * angle itself c^2 + s^2 is off by a few roundings more, which the columns
+ * of V collect (1e-12 at n = 220, now 1e-13).  False (no rotation) below
+ * the relative threshold 1e-15 sqrt |app aqq|. */
 __device__ __forceinline__ bool
 jacobi_rotation (double app, double aqq, double apq, double &c, double &s,
                  double &t)
@@ -340,19 +353,20 @@ jacobi_rotation (double app, double aqq, double apq, double &c, double &s,
   const double ri = rsqrt (fma (d, d, b * b));
   const double c2 = fma (0.5 * fabs (d), ri, 0.5);
   const double ci = rsqrt (c2);
-  c = c2 * ci;
-  s = (d < 0. ? -0.5 : 0.5) * b * ri * ci;
-  t = s * ci;
+  t = (d < 0. ? -0.5 : 0.5) * b * ri * ci * ci;
+  c = rsqrt (fma (t, t, 1.));
+  s = t * c;
   return true;
 }
 
-/* the 2 JB x 2 JB submatrix of each pair: up to `sweeps` cyclic sweeps
- * (stopping at one without a rotation); the diagonalised submatrix goes back
+/* the 2 JB x 2 JB submatrix of each pair: up to `sweeps` passes over its
+ * index pairs, all of them where inner is set, else those across the blocks
+ * (stopping at a pass without a rotation); the rotated submatrix goes back
  * to A, the rotations to W (row-major), whether there were any to rot[pair],
  * and any_rot / done (sweeps run) record the round */
 __global__ void __launch_bounds__ (256)
-k_jacobi_pairs (int n, int nblk, int r, int sweeps, double *A, double *Wg,
-                int *rot, int *any_rot, int *done)
+k_jacobi_pairs (int n, int nblk, int r, int sweeps, int inner, double *A,
+                double *Wg, int *rot, int *any_rot, int *done)
 {
   __shared__ double S[JT][JS], W[JT][JS];
   __shared__ double cs[JB], sn[JB], tt[JB];
@@ -370,9 +384,11 @@ k_jacobi_pairs (int n, int nblk, int r, int sweeps, double *A, double *Wg,
   for (; sw < sweeps; sw++) {
     if (tid == 0) rotated = 0;
     __syncthreads ();
-    for (int q = 0; q < JT - 1; q++) {
+    for (int q = 0; q < (inner ? JT - 1 : JB); q++) {
       if (tid < JB) {
-        const int a = rr_index (tid, q, JT), b = rr_index (JT - 1 - tid, q, JT);
+        const int a = inner ? rr_index (tid, q, JT) : tid;
+        const int b = inner ? rr_index (JT - 1 - tid, q, JT)
+                            : JB + ((tid + q) & (JB - 1));
         const int pi = a < b ? a : b, qi = a < b ? b : a;
         double c, s, t;
         if (jacobi_rotation (S[pi][pi], S[qi][qi], S[pi][qi], c, s, t)) rotated = 1;
@@ -464,7 +480,7 @@ jacobi_mma (const double (*Pm)[JS], const double (*Qm)[JS], double (&acc)[2][2])
 }
 
 /* blockIdx.y < npair: tile (x, y) of A, x < y: W_x^T A W_y, with its mirror;
- * above: 32 rows of V times W_x */
+ * above: 32 rows of V times W_x.  WP and WQ hold W - I. */
 __global__ void __launch_bounds__ (256)
 k_jacobi_apply (int n, int nblk, int r, double *A, double *V,
                 const double *__restrict__ Wg, const int *__restrict__ rot)
@@ -489,12 +505,20 @@ k_jacobi_apply (int n, int nblk, int r, double *A, double *V,
     const double *src = isv ? V : A;
     T[i][j] = (gi < n && gj < n) ? src[gi + (size_t) gj * n] : 0.;
     const int wi = e / JT, wj = e % JT;
-    WQ[wi][wj] = rot[kq] ? Wg[(size_t) kq * JT * JT + e] : (wi == wj ? 1. : 0.);
-    if (!isv)
-      WP[wi][wj] = rot[kp] ? Wg[(size_t) kp * JT * JT + e] : (wi == wj ? 1. : 0.);
+    const double one = wi == wj ? 1. : 0.;
+    WQ[wi][wj] = rot[kq] ? Wg[(size_t) kq * JT * JT + e] - one : 0.;
+    if (!isv) WP[wi][wj] = rot[kp] ? Wg[(size_t) kp * JT * JT + e] - one : 0.;
   }
   __syncthreads ();
+  /* a thread's entries of T are its own to replace */
+  auto add_tile = [&] () {
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) acc[t][c] += T[fi][fj + t * 8 + c];
+  };
   jacobi_mma<false> (T, WQ, acc);
+  add_tile ();
   if (!isv) {
     __syncthreads ();
 #pragma unroll
@@ -503,6 +527,7 @@ k_jacobi_apply (int n, int nblk, int r, double *A, double *V,
       for (int c = 0; c < 2; c++) T[fi][fj + t * 8 + c] = acc[t][c];
     __syncthreads ();
     jacobi_mma<true> (WP, T, acc);
+    add_tile ();
   }
   __syncthreads ();
 #pragma unroll
@@ -534,12 +559,55 @@ k_jacobi_start (int n, double *V, int *flags, int nflags)
     for (int e = threadIdx.x; e < nflags; e += blockDim.x) flags[e] = 0;
 }
 
-__global__ void
-k_jacobi_diag (int n, const double *A, double *w)
+/* w_j = v_j^T A v_j / v_j^T v_j: JR eigenvectors per CTA, a warp per row of
+ * the symmetric A (its contiguous column) */
+constexpr int JR = 2;
+
+__global__ void __launch_bounds__ (256)
+k_jacobi_rayleigh (int n, const double *__restrict__ A,
+                   const double *__restrict__ V, double *w)
 {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gridDim.x * blockDim.x)
-    w[i] = A[i + (size_t) i * n];
+  extern __shared__ double sv[];               /* [JR][n] */
+  __shared__ double red[8][JR][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int j0 = blockIdx.x * JR;
+  for (int e = tid; e < JR * n; e += 256)
+    sv[e] = j0 + e / n < n ? V[(size_t) j0 * n + e] : 0.;
+  __syncthreads ();
+  double num[JR], den[JR];
+#pragma unroll
+  for (int q = 0; q < JR; q++) num[q] = den[q] = 0.;
+  for (int i = warp; i < n; i += 8) {
+    double y[JR];
+#pragma unroll
+    for (int q = 0; q < JR; q++) y[q] = 0.;
+    for (int k = lane; k < n; k += 32) {
+      const double a = A[k + (size_t) i * n];
+#pragma unroll
+      for (int q = 0; q < JR; q++) y[q] = fma (a, sv[q * n + k], y[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < JR; q++) {
+      const double v = sv[q * n + i];
+      num[q] = fma (v, warp_sum (y[q]), num[q]);
+      den[q] = fma (v, v, den[q]);
+    }
+  }
+  if (lane == 0)
+#pragma unroll
+    for (int q = 0; q < JR; q++) {
+      red[warp][q][0] = num[q];
+      red[warp][q][1] = den[q];
+    }
+  __syncthreads ();
+  if (tid < JR && j0 + tid < n) {
+    double a = 0., b = 0.;
+    for (int k = 0; k < 8; k++) {
+      a += red[k][tid][0];
+      b += red[k][tid][1];
+    }
+    w[j0 + tid] = a / b;
+  }
 }
 
 int
@@ -550,9 +618,12 @@ launch_syev_jacobi (int n, double *A, double *V, double *w, int *sweeps,
   LGH_CHECK (n <= 2048, LGH_ERR_SUP, "syev: n=%d > 2048", n);
   constexpr int MAXS = 40;
   const int npair = (n + JT - 1) / JT, nblk = 2 * npair;
-  DBuf<double> Wg;
+  DBuf<double> Wg, A0;
   DBuf<int> flags;     /* rot[npair], any_rot[MAXS], done */
   LGH_TRY (Wg.alloc ((size_t) npair * JT * JT));
+  LGH_TRY (A0.alloc ((size_t) n * n));
+  LGH_CUDA (cudaMemcpyAsync (A0.p, A, (size_t) n * n * sizeof (double),
+                             cudaMemcpyDeviceToDevice, s));
   LGH_TRY (flags.alloc (npair + MAXS + 1));
   int *rot = flags.p, *any = rot + npair, *done = any + MAXS;
   k_jacobi_start<<<std::max (1, std::min (num_sms () * 4, (n * n + 255) / 256)),
@@ -562,7 +633,7 @@ launch_syev_jacobi (int n, double *A, double *V, double *w, int *sweeps,
   const dim3 tiles ((unsigned) npair, (unsigned) (npair + npair));
   if (npair == 1) {
     /* the whole matrix in one CTA, to convergence */
-    k_jacobi_pairs<<<1, 256, 0, s>>> (n, nblk, 0, MAXS, A, Wg.p, rot, any, done);
+    k_jacobi_pairs<<<1, 256, 0, s>>> (n, nblk, 0, MAXS, 1, A, Wg.p, rot, any, done);
     LGH_LAUNCH_CHECK ();
     k_jacobi_apply<<<tiles, 256, 0, s>>> (n, nblk, 0, A, V, Wg.p, rot);
     LGH_LAUNCH_CHECK ();
@@ -571,8 +642,8 @@ launch_syev_jacobi (int n, double *A, double *V, double *w, int *sweeps,
   } else {
     for (; ran < MAXS; ) {
       for (int r = 0; r < nblk - 1; r++) {
-        k_jacobi_pairs<<<npair, 256, 0, s>>> (n, nblk, r, 1, A, Wg.p, rot,
-                                              any + ran, done);
+        k_jacobi_pairs<<<npair, 256, 0, s>>> (n, nblk, r, 1, r == nblk - 2, A, Wg.p,
+                                              rot, any + ran, done);
         k_jacobi_apply<<<tiles, 256, 0, s>>> (n, nblk, r, A, V, Wg.p, rot);
       }
       LGH_LAUNCH_CHECK ();
@@ -586,7 +657,8 @@ launch_syev_jacobi (int n, double *A, double *V, double *w, int *sweeps,
       if (!more) break;
     }
   }
-  k_jacobi_diag<<<std::max (1, (n + 255) / 256), 256, 0, s>>> (n, A, w);
+  k_jacobi_rayleigh<<<(n + JR - 1) / JR, 256, JR * n * (int) sizeof (double), s>>> (
+      n, A0.p, V, w);
   LGH_LAUNCH_CHECK ();
   if (sweeps) *sweeps = std::max (ran, 1);
   return 0;
