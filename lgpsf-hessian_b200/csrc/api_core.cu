@@ -761,6 +761,21 @@ prior_solve_rows (lgh_prior_t *p, int w, const T *X, int ldx,
 }
 
 int
+allow_smem (const void *fn, int bytes)
+{
+  static std::mutex mu;
+  static std::map<const void *, int> limit;
+  if (bytes <= 48 * 1024) return 0;
+  std::lock_guard<std::mutex> lk (mu);
+  int &l = limit[fn];
+  if (l >= bytes) return 0;
+  LGH_CUDA (cudaFuncSetAttribute (fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  bytes));
+  l = bytes;
+  return 0;
+}
+
+int
 resident_ctas (const void *fn, int threads, int smem)
 {
   static std::mutex mu;

@@ -31,8 +31,6 @@
  * build's A^T B and X^T X. */
 
 #include <algorithm>
-#include <mutex>
-#include <set>
 #include <type_traits>
 
 #include "lgh_batch.h"
@@ -225,22 +223,6 @@ copy_bytes (const T *p, int64_t ld)
   if (a % 16 == 0 && l % 16 == 0) return 16;
   if (sizeof (T) == 8 || (a % 8 == 0 && l % 8 == 0)) return 8;
   return 4;
-}
-
-/* opt kernel k into its dynamic shared memory (above 48 KB), once */
-template <typename K>
-static int
-gemm_smem_attr (K k, int bytes)
-{
-  static std::mutex mu;
-  static std::set<const void *> done;
-  std::lock_guard<std::mutex> lk (mu);
-  if (done.count ((const void *) k)) return 0;
-  LGH_CUDA (cudaFuncSetAttribute ((const void *) k,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  bytes));
-  done.insert ((const void *) k);
-  return 0;
 }
 
 /* partial C = A^T B over rows [kb0, kb1) of row-major A (n x m1), B
@@ -638,7 +620,7 @@ gemm_tn_run (int64_t n, int m1, int m2, const T *A, int lda, const T *B, int ldb
   constexpr int smem = gemm_smem<T, true, T, true, GB> ();
   auto run = [&] (auto ca, auto cb) -> int {
     auto k = k_gemm_tn_part<T, decltype (ca)::value, decltype (cb)::value>;
-    LGH_TRY (gemm_smem_attr (k, smem));
+    LGH_TRY (allow_smem ((const void *) k, smem));
     k<<<grid, 128, smem, s>>> (n, m1, m2, A, lda, B, ldb, work, kchunk, upper);
     LGH_LAUNCH_CHECK ();
     return 0;
@@ -855,7 +837,7 @@ launch_shift_combine_variant (int variant, int64_t n, int kept, int m,
     constexpr int smem = gemm_smem<double, false, double, false, BM_> ();
     /* W's rows are padded to 4 values at a 256-byte base */
     auto k = k_shift_combine<BM_, 16, decltype (cb)::value>;
-    LGH_TRY (gemm_smem_attr (k, smem));
+    LGH_TRY (allow_smem ((const void *) k, smem));
     k<<<grid, BM_ * 2, smem, s>>> (n, kept, m, (int) ncol, W, ldw, S, fc, Y0,
                                    ldy0, out, ldo);
     LGH_LAUNCH_CHECK ();
@@ -1004,7 +986,7 @@ launch_gemm_nn (int64_t n, int k, int m2, double alpha, const T *X, int ldx,
   constexpr int smem = gemm_smem<T, false, double, false, GB> ();
   auto run = [&] (auto ca, auto cb) -> int {
     auto f = k_gemm_nn<T, decltype (ca)::value, decltype (cb)::value>;
-    LGH_TRY (gemm_smem_attr (f, smem));
+    LGH_TRY (allow_smem ((const void *) f, smem));
     f<<<(unsigned) tiles, 128, smem, s>>> (n, k, m2, alpha, X, ldx, M, ldm, beta,
                                            Y0, ldy0, Y, ldy, tn);
     LGH_LAUNCH_CHECK ();

@@ -176,9 +176,7 @@ launch_potrf (int n, double *G, double *G0, int jitter_mode, int *info,
   LGH_CHECK (smem <= 220 * 1024, LGH_ERR_SUP, "potrf: n=%d too large", n);
   if (G0) LGH_CUDA (cudaMemcpyAsync (G0, G, (size_t) n * n * sizeof (double),
                                      cudaMemcpyDeviceToDevice, s));
-  LGH_CUDA (cudaFuncSetAttribute (k_potrf,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  smem));
+  LGH_TRY (allow_smem ((const void *) k_potrf, smem));
   k_potrf<<<1, 512, smem, s>>> (n, G, G0, jitter_mode, info);
   LGH_LAUNCH_CHECK ();
   return 0;
@@ -269,9 +267,7 @@ launch_trtri_lower (int n, const double *L, double *Linv, int transpose,
     return 0;
   }
   const int smem = 8 * n * (int) sizeof (double);
-  LGH_CUDA (cudaFuncSetAttribute (k_trtri_lower,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  smem));
+  LGH_TRY (allow_smem ((const void *) k_trtri_lower, smem));
   k_trtri_lower<<<(n + 7) / 8, 256, smem, s>>> (n, L, Linv, transpose);
   LGH_LAUNCH_CHECK ();
   return 0;

@@ -31,7 +31,6 @@
 #include <cmath>
 #include <mutex>
 #include <type_traits>
-#include <unordered_map>
 
 #include "lgh_device.cuh"
 #include "lgh_internal.h"
@@ -510,26 +509,11 @@ k_zresid (ZK z, const double *__restrict__ vals,
 
 /* ---- host side ------------------------------------------------------------ */
 
-/* opt a kernel into > 48 KB of dynamic shared memory, once per kernel */
-static void
-smem_prep (const void *fn, int bytes)
-{
-  static std::mutex mu;
-  static std::unordered_map<const void *, int> done;
-  if (bytes <= 48 * 1024) return;
-  std::lock_guard<std::mutex> lk (mu);
-  auto it = done.find (fn);
-  if (it != done.end () && it->second >= bytes) return;
-  cudaFuncSetAttribute (fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                        bytes);
-  done[fn] = bytes;
-}
-
 template <typename K>
 static void
 set_smem_attr (K kern, int bytes)
 {
-  smem_prep ((const void *) kern, bytes);
+  (void) allow_smem ((const void *) kern, bytes);   /* the launch reports it */
 }
 
 static int
