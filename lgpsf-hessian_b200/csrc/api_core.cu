@@ -764,10 +764,12 @@ int
 allow_smem (const void *fn, int bytes)
 {
   static std::mutex mu;
-  static std::map<const void *, int> limit;
-  if (bytes <= 48 * 1024) return 0;
+  static std::map<std::pair<const void *, int>, int> limit;
+  if (bytes <= 40 * 1024) return 0;
+  int dev = 0;
+  LGH_CUDA (cudaGetDevice (&dev));
   std::lock_guard<std::mutex> lk (mu);
-  int &l = limit[fn];
+  int &l = limit[std::make_pair (fn, dev)];
   if (l >= bytes) return 0;
   LGH_CUDA (cudaFuncSetAttribute (fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   bytes));

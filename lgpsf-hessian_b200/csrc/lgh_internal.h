@@ -221,10 +221,11 @@ fit_grid (K kern, int want, int threads, int smem)
   return (r > 0 && r < want) ? r : want;
 }
 
-/* opt kernel fn into `bytes` of dynamic shared memory (above 48 KB).  The
- * limit belongs to the kernel, not to a launch, and only ever grows here: a
- * thread that set it for a smaller launch of its own between another
- * thread's opt-in and launch would make that launch fail. */
+/* opt kernel fn into `bytes` of dynamic shared memory (from 40 KB: the
+ * default 48 KB hold its static arrays too).  The limit belongs to the kernel
+ * on the current device, not to a launch, and only ever grows here: a thread
+ * that set it for a smaller launch of its own between another thread's opt-in
+ * and launch would make that launch fail. */
 int allow_smem (const void *fn, int bytes);
 
 /* entries up to which 32-bit entry offsets hold, with a batch's step past a
